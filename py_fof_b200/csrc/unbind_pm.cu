@@ -332,6 +332,17 @@ __device__ __forceinline__ uint32_t spread3(uint32_t v) {
   return r;
 }
 
+// C2 cells are numbered brick by brick: a brick is 4^3 cells, its cells in
+// Morton order, so the members of a whole brick, and of each aligned 2^3
+// block of cells, are consecutive in cell order and can be read as one range
+// (sr_gather_kernel picks the node size that fits a target's cutoff).
+__device__ __forceinline__ uint32_t sr_cell(const PmHalo &p, int x, int y, int z) {
+  const int bx = (p.nc[0] + 3) >> 2, by = (p.nc[1] + 3) >> 2;
+  const int64_t brick = (x >> 2) + (int64_t)bx * ((y >> 2) + (int64_t)by * (z >> 2));
+  const uint32_t m = spread3(x & 3) | (spread3(y & 3) << 1) | (spread3(z & 3) << 2);
+  return (uint32_t)(p.cell_off + 64 * brick) + m;
+}
+
 __global__ void pm_cellkey_kernel(const Members m, const PmHalo *__restrict__ H,
                                   const int32_t *__restrict__ mhalo, int64_t M,
                                   uint32_t *__restrict__ key, uint32_t sentinel, int sb,
@@ -360,7 +371,7 @@ __global__ void pm_cellkey_kernel(const Members m, const PmHalo *__restrict__ H,
       fr = fr < 0.0 ? 0.0 : (fr > (double)(sub - 1) ? (double)(sub - 1) : fr);
       f[d] = (uint32_t)fr;
     }
-    const uint32_t cell = (uint32_t)(p.cell_off + c[0] + (int64_t)p.nc[0] * (c[1] + (int64_t)p.nc[1] * c[2]));
+    const uint32_t cell = sr_cell(p, (int)c[0], (int)c[1], (int)c[2]);
     key[k] = cell;
     skey[k] = (cell << sb) | (spread3(f[0]) | (spread3(f[1]) << 1) | (spread3(f[2]) << 2));
   }
@@ -515,17 +526,10 @@ __device__ __forceinline__ T c2_delta(T r, T ht, T hs) {
 // bound_two_level_pp_update :1345-1498): UPDATE sums over those sources only
 // and subtracts.
 //
-// Work is organised by target chunks: a warp takes up to 32 members of one
-// C2 cell, in cell order (within a cell sorted by a Morton sub-key, so a
-// chunk is spatially compact).  Sources are scanned cell by cell in
-// coalesced batches of 32; a source enters the pair loop only if it lies
-// within the chunk's largest cutoff of the chunk's bounding box, so the
-// divergent pair arithmetic runs almost only on pairs that interact.  FP32
-// sums are compensated (Kahan); FP64 sums are plain, which keeps the
-// dependent chain per pair to one add.
-// FP32 product path of the short-range kernel: the spline-softened 1/r of
-// depth_c with its divisions replaced by products with per-h reciprocals and
-// 1/r from rsqrtf (a few ulps; the FP64 path keeps the divisions).
+// FP32 product path: the spline-softened 1/r of depth_c with its divisions
+// replaced by products with per-h reciprocals and 1/r from rsqrtf (a few
+// ulps).  FP32 sums are compensated (Kahan); FP64 sums are plain, which
+// keeps the dependent chain per pair to one add.
 struct DepthConst {
   float h, two_over_h, inv70h, six_h;
 };
@@ -545,198 +549,387 @@ __device__ __forceinline__ float depth_fast(float r, float rinv, const DepthCons
   return (128.0f - prim) * c.inv70h;
 }
 
-// FP64 path of the same kernel without divisions: 1/r from an FP32
-// reciprocal square root seed refined by two Newton-Raphson steps in FP64,
-// y <- y (3/2 - r2 y^2 / 2), which square the relative error each time
-// (2^-22 -> ~1e-13 -> a few FP64 ulps); the per-h constants are FP64
-// reciprocals.  For r2 outside the FP32 normal range the caller keeps the
-// plain sqrt/division form.
+// FP64 path of the same kernel without divisions.  1/r: an FP32 reciprocal
+// square root seed y (relative error about 2^-22) and one step of the
+// binomial series 1/sqrt(r2) = y (1 - g)^(-1/2) = y (1 + g/2 + 3 g^2/8 + ..),
+// g = 1 - r2 y^2 (|g| about 2^-21, so the dropped cubic term is 2^-65).  For r2
+// outside the FP32 normal range the caller keeps the plain sqrt/division
+// form.  The two pieces of the spline are polynomials in e = 2r/h scaled by
+// 1/h, with the 1/70 folded into their coefficients (the 12/e term is 6/(70 r)).
 struct DepthConst64 {
-  double h, two_over_h, inv70h, six_h;
+  double h, two_over_h, inv_h;
 };
-__device__ __forceinline__ DepthConst64 depth_const64(double h) {
-  return DepthConst64{h, 2.0 / h, 1.0 / (70.0 * h), 6.0 * h};
-}
-__device__ __forceinline__ double rsqrt_nr64(double r2) {
-  double y = (double)rsqrtf((float)r2);
-  const double hr2 = 0.5 * r2;
-  y = y * (1.5 - hr2 * y * y);
-  y = y * (1.5 - hr2 * y * y);
-  return y;
+__device__ __forceinline__ DepthConst64 depth_const64(double h) { return DepthConst64{h, 2.0 / h, 1.0 / h}; }
+__device__ __forceinline__ double rsqrt_series64(double r2) {
+  const double y = (double)rsqrtf((float)r2);
+  const double g = fma(-(r2 * y), y, 1.0);
+  return fma(y * g, fma(0.375, g, 0.5), y);
 }
 __device__ __forceinline__ double depth_fast64(double r, double rinv, const DepthConst64 &c) {
   if (r >= c.h) return rinv;
   const double e = r * c.two_over_h;
   if (e <= 1.0) {
-    const double prim = e * e * (112.0 + e * e * (-56.0 + e * (14.0 + e * (8.0 - 3.0 * e))));
-    return (208.0 - prim) * c.inv70h;
+    const double e2 = e * e;
+    double t = fma(e, -3.0 / 70.0, 8.0 / 70.0);
+    t = fma(e, t, 14.0 / 70.0);
+    t = fma(e, t, -56.0 / 70.0);
+    t = fma(e2, t, 112.0 / 70.0);
+    return fma(-e2, t, 208.0 / 70.0) * c.inv_h;
   }
-  const double prim = e * e * (448.0 + e * (-280.0 + e * (56.0 + e * (14.0 + e * (-8.0 + e))))) -
-                      224.0 * e - c.six_h * rinv;
-  return (128.0 - prim) * c.inv70h;
+  double t = fma(e, -1.0 / 70.0, 8.0 / 70.0);
+  t = fma(e, t, -14.0 / 70.0);
+  t = fma(e, t, -56.0 / 70.0);
+  t = fma(e, t, 280.0 / 70.0);
+  t = fma(e, t, -448.0 / 70.0);
+  t = fma(e, t, 224.0 / 70.0);
+  t = fma(e, t, 128.0 / 70.0);
+  return fma(t, c.inv_h, rinv * (6.0 / 70.0));
 }
 
+// A target chunk: up to 32 members of one brick, consecutive in cell order
+// (along the brick's Morton curve, so they are spatially compact), with the
+// range of source nodes its widened bounding box touches.  A node is an
+// aligned block of 2^level cells per axis.
 struct SrChunk {
-  uint32_t cell, e0;
+  uint32_t e0;       // first member (position in cell order)
+  int32_t h;         // halo
+  float lo[3], hi[3];  // bounding box of the targets
+  float amax;        // largest cutoff of the targets, a little widened
+  uint32_t nsrc;     // members of all its nodes
+  int16_t x0[3];     // first node per axis
+  uint16_t nx[3];    // nodes per axis
+  uint8_t cnt, level;
 };
 
+// Chunks whose nodes hold this many members or more are summed by the eight
+// warps of a block together.  The rule looks at the chunk alone, so the order
+// of its sum does not depend on what else is in the call.
+constexpr uint32_t kSrHeavy = 1024;
+constexpr int kSrWarps = 8;
+
+__global__ void sr_chunk_count_kernel(const uint32_t *__restrict__ cstart, int64_t nbrick,
+                                      uint32_t *__restrict__ cnt) {
+  for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nbrick;
+       b += (int64_t)gridDim.x * blockDim.x)
+    cnt[b] = (cstart[64 * (b + 1)] - cstart[64 * b] + 31u) / 32u;
+}
+
+__global__ void sr_chunk_fill_kernel(const uint32_t *__restrict__ cstart, const uint32_t *__restrict__ coff,
+                                     int64_t nbrick, uint2 *__restrict__ span) {
+  for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nbrick;
+       b += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t e0 = cstart[64 * b], e1 = cstart[64 * (b + 1)];
+    const uint32_t n = (e1 - e0 + 31u) / 32u;
+    for (uint32_t i = 0; i < n; ++i) span[coff[b] + i] = make_uint2(e0 + 32u * i, min(32u, e1 - e0 - 32u * i));
+  }
+}
+
+// First member of node (x, y, z) of `level` and the one after its last.
+__device__ __forceinline__ uint2 sr_node_range(const PmHalo &p, const uint32_t *__restrict__ cstart, int x, int y,
+                                               int z, int level) {
+  const uint32_t c = sr_cell(p, x << level, y << level, z << level);
+  return make_uint2(cstart[c], cstart[c + (1u << (3 * level))]);
+}
+
+// Chunk records, a warp per chunk, and their sort keys: most sources first,
+// so that the dynamically fetched chunks end together.
+__global__ void __launch_bounds__(BLK) sr_chunk_setup_kernel(
+    const uint2 *__restrict__ span, int64_t nchunk, const PmHalo *__restrict__ H,
+    const int32_t *__restrict__ mhalo, const uint32_t *__restrict__ cmem, const float4 *__restrict__ src4,
+    const uint8_t *__restrict__ pr, const uint32_t *__restrict__ cstart, SrChunk *__restrict__ out,
+    uint32_t *__restrict__ key, uint32_t *__restrict__ nheavy) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  for (int64_t ch = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5; ch < nchunk;
+       ch += ((int64_t)gridDim.x * BLK) >> 5) {
+    const uint2 sp = span[ch];
+    const bool valid = lane < (int)sp.y;
+    float4 me = make_float4(0.f, 0.f, 0.f, 0.f);
+    int ri = 64;
+    if (valid) {
+      me = src4[sp.x + lane];
+      ri = pr[cmem[sp.x + lane]];
+    }
+    const int h = mhalo[cmem[sp.x]];
+    const PmHalo &p = H[h];
+    SrChunk C;
+    C.e0 = sp.x;
+    C.h = h;
+    C.cnt = (uint8_t)sp.y;
+    const float m3[3] = {me.x, me.y, me.z};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      C.lo[d] = ord_to_flt(__reduce_min_sync(FULL, valid ? flt_to_ord(m3[d]) : 0xffffffffu));
+      C.hi[d] = ord_to_flt(__reduce_max_sync(FULL, valid ? flt_to_ord(m3[d]) : 0u));
+    }
+    const int rmin = __reduce_min_sync(FULL, ri);
+    const double spc = (double)p.spacing;
+    // conservative filter radius (a little above every target's cutoff)
+    C.amax = (float)(3.5 * spc / (double)rmin) * 1.0001f + 1e-30f;
+    // nodes about as wide as the cutoff; wider ones for a chunk that a
+    // sparse brick spreads over many
+    int level = p.two_level ? (p.r_max >= 4 * rmin ? 2 : (p.r_max >= 2 * rmin ? 1 : 0)) : 0;
+    int nodes;
+    for (;; ++level) {
+      nodes = 1;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const double gl = (((double)C.lo[d] - (double)C.amax) / spc - p.u_min[d]) / p.cw_u - 1e-4;
+        const double gh = (((double)C.hi[d] + (double)C.amax) / spc - p.u_min[d]) / p.cw_u + 1e-4;
+        const int top = p.nc[d] - 1;
+        const int a = gl <= 0.0 ? 0 : (gl >= (double)top ? top : (int)gl);
+        const int b = gh <= 0.0 ? 0 : (gh >= (double)top ? top : (int)gh);
+        C.x0[d] = (int16_t)(a >> level);
+        C.nx[d] = (uint16_t)((b >> level) - (a >> level) + 1);
+        nodes *= C.nx[d];
+      }
+      if (level == 2 || nodes <= 128) break;
+    }
+    C.level = (uint8_t)level;
+    uint32_t t = 0;
+    for (int j = lane; j < nodes; j += 32) {
+      const int w0 = C.nx[0], w1 = C.nx[1];
+      const uint2 r = sr_node_range(p, cstart, C.x0[0] + j % w0, C.x0[1] + (j / w0) % w1,
+                                    C.x0[2] + j / (w0 * w1), level);
+      t += r.y - r.x;
+    }
+    C.nsrc = __reduce_add_sync(FULL, t);
+    if (lane == 0) {
+      out[ch] = C;
+      key[ch] = 65535u - min(C.nsrc >> 2, 65535u);
+      if (C.nsrc >= kSrHeavy) atomicAdd(nheavy, 1u);
+    }
+  }
+}
+
+__global__ void sr_chunk_order_kernel(const SrChunk *__restrict__ chunks, const uint32_t *__restrict__ idx,
+                                      int64_t n, SrChunk *__restrict__ out) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    out[i] = chunks[idx[i]];
+}
+
+// What a warp needs of its targets to test and add pairs.
+template <typename R>
+struct SrTarget {
+  float4 me;
+  uint32_t e;     // position in cell order (a target is not its own source)
+  float a2f;      // FP32 bound of the pair test, a little above a2; < 0: no target
+  R a2;
+  bool tl;
+  DepthConst eps, ai;
+  DepthConst64 eps64, ai64;
+  R acc, comp;
+};
+
+// Up to 32 staged sources against the warp's 32 targets.  Every lane first
+// marks the sources inside its own cutoff with an FP32 test (the box filter
+// in front of it keeps a chunk's union, of which a target needs a third or
+// less), then walks its own marks, so the long pair arithmetic runs on
+// interacting pairs only, in ascending source order per target.
 template <typename R, bool UPDATE>
-__global__ void __launch_bounds__(256, 4) sr_gather_kernel(
-    const PmHalo *__restrict__ H, const int32_t *__restrict__ mhalo, const uint8_t *__restrict__ keep,
-    const uint8_t *__restrict__ pr, const SrChunk *__restrict__ chunks, int64_t nchunks,
+__device__ __forceinline__ void sr_pairs(const float4 *__restrict__ buf, const uint32_t *__restrict__ idx, int cnt,
+                                         SrTarget<R> &t) {
+  unsigned mask = 0;
+#pragma unroll 8
+  for (int j = 0; j < cnt; ++j) {
+    const float4 s = buf[j];
+    const float dx = s.x - t.me.x, dy = s.y - t.me.y, dz = s.z - t.me.z;
+    if (dx * dx + dy * dy + dz * dz <= t.a2f) mask |= 1u << j;
+  }
+  while (mask) {
+    const int j = __ffs(mask) - 1;
+    mask &= mask - 1;
+    if (!UPDATE && idx[j] == t.e) continue;
+    const float4 s = buf[j];
+    R dx, dy, dz;
+    if (t.tl) {
+      dx = (R)s.x - (R)t.me.x; dy = (R)s.y - (R)t.me.y; dz = (R)s.z - (R)t.me.z;
+    } else {
+      dx = (R)__fsub_rn(s.x, t.me.x); dy = (R)__fsub_rn(s.y, t.me.y); dz = (R)__fsub_rn(s.z, t.me.z);
+    }
+    const R r2 = dx * dx + dy * dy + dz * dz;
+    if (!(r2 < t.a2)) continue;
+    if constexpr (sizeof(R) == 4) {  // compensated sum of the negated terms
+      const float rinv = rsqrtf(r2), d = r2 * rinv;
+      const float y = -(s.w * (depth_fast(d, rinv, t.eps) - depth_fast(d, rinv, t.ai))) - t.comp;
+      const float v = t.acc + y;
+      t.comp = (v - t.acc) - y;
+      t.acc = v;
+    } else if (r2 > 1e-30 && r2 < 1e30) {
+      const double rinv = rsqrt_series64(r2), d = r2 * rinv;
+      t.acc = fma((double)s.w, depth_fast64(d, rinv, t.ai64) - depth_fast64(d, rinv, t.eps64), t.acc);
+    } else {
+      const R d = sqrt(r2);
+      t.acc += (R)s.w * (depth_c<R>(d, t.ai64.h) - depth_c<R>(d, t.eps64.h));
+    }
+  }
+}
+
+// The sum of one chunk, or every nparts-th batch of its sources.  Nodes are
+// taken 32 at a time: a lane loads one node's member range, the ranges are
+// concatenated by a warp prefix sum and read in batches of 32 (a lane finds
+// its source's node by a binary search over the prefix); sources within the
+// largest cutoff of the targets' bounding box are staged, and every 32
+// staged sources go to sr_pairs.
+template <typename R, bool UPDATE>
+__device__ __forceinline__ void sr_chunk_sum(const SrChunk &C, const PmHalo &p, int part, int nparts,
+                                             const uint32_t *__restrict__ cstart, const float4 *__restrict__ src4,
+                                             const uint32_t *__restrict__ rpos, const uint32_t *__restrict__ rsrc,
+                                             float4 *buf, uint32_t *idx, SrTarget<R> &t) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = lanemask_lt();
+  const float amax2 = C.amax * C.amax;
+  const int w0 = C.nx[0], w1 = C.nx[1], nodes = w0 * w1 * C.nx[2];
+  int fill = 0, turn = 0;
+  for (int n0 = 0; n0 < nodes; n0 += 32) {
+    const int j = n0 + lane;
+    uint32_t s0 = 0, cnt = 0;
+    if (j < nodes) {
+      uint2 r = sr_node_range(p, cstart, C.x0[0] + j % w0, C.x0[1] + (j / w0) % w1, C.x0[2] + j / (w0 * w1),
+                              C.level);
+      if (UPDATE && r.y > r.x) r = make_uint2(rpos[r.x], rpos[r.y]);
+      s0 = r.x;
+      cnt = r.y - r.x;
+    }
+    uint32_t incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += v;
+    }
+    const uint32_t first = s0 - (incl - cnt);  // source of batch index g: first + g
+    const uint32_t T = __shfl_sync(FULL, incl, 31);
+    for (uint32_t g0 = 0; g0 < T; g0 += 32) {
+      if (nparts > 1 && (turn++ & (nparts - 1)) != part) continue;
+      const uint32_t g = g0 + (uint32_t)lane;
+      int owner = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const uint32_t v = __shfl_sync(FULL, incl, owner + step - 1);
+        if (v <= g) owner += step;
+      }
+      owner &= 31;
+      const uint32_t of = __shfl_sync(FULL, first, owner);
+      uint32_t se = 0;
+      float4 sv = make_float4(0.f, 0.f, 0.f, 0.f);
+      bool cand = false;
+      if (g < T) {
+        se = UPDATE ? rsrc[of + g] : of + g;
+        sv = src4[se];
+        const float bx = fmaxf(fmaxf(C.lo[0] - sv.x, sv.x - C.hi[0]), 0.f);
+        const float by = fmaxf(fmaxf(C.lo[1] - sv.y, sv.y - C.hi[1]), 0.f);
+        const float bz = fmaxf(fmaxf(C.lo[2] - sv.z, sv.z - C.hi[2]), 0.f);
+        cand = bx * bx + by * by + bz * bz <= amax2;
+      }
+      const unsigned m = __ballot_sync(FULL, cand);
+      if (cand) {
+        const int q = fill + __popc(m & lt);
+        buf[q] = sv;
+        idx[q] = se;
+      }
+      fill += __popc(m);
+      __syncwarp();
+      if (fill >= 32) {
+        sr_pairs<R, UPDATE>(buf, idx, 32, t);
+        __syncwarp();
+        fill -= 32;
+        if (lane < fill) {
+          buf[lane] = buf[32 + lane];
+          idx[lane] = idx[32 + lane];
+        }
+        __syncwarp();
+      }
+    }
+  }
+  if (fill) sr_pairs<R, UPDATE>(buf, idx, fill, t);
+  __syncwarp();
+}
+
+// Bound by FP64 arithmetic per interacting pair (about 45 operations) once
+// enough warps have work.  Persistent blocks: first the heavy chunks, a
+// block each (eight warps take the source batches in turn and their sums
+// are added in warp order), then the others, a warp each; both most sources
+// first, fetched from a counter.
+template <typename R, bool UPDATE>
+__global__ void __launch_bounds__(32 * kSrWarps, sizeof(R) == 4 ? 4 : 3) sr_gather_kernel(
+    const PmHalo *__restrict__ H, const uint8_t *__restrict__ keep, const uint8_t *__restrict__ pr,
+    const SrChunk *__restrict__ chunks, uint32_t nchunks, const uint32_t *__restrict__ nheavy_p,
     const uint32_t *__restrict__ cstart, const uint32_t *__restrict__ cmem, const float4 *__restrict__ src4,
     const uint32_t *__restrict__ rpos, const uint32_t *__restrict__ rsrc, double a_val, double app,
     R *__restrict__ phi_sr, unsigned *__restrict__ next) {
   constexpr unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  // chunks come heaviest first; each warp takes the next one when it is
-  // free (the sums of a chunk do not depend on which warp runs it)
-  auto fetch = [&]() -> int64_t {
-    unsigned v = 0;
-    if (lane == 0) v = atomicAdd(next, 1u);
-    return (int64_t)__shfl_sync(FULL, v, 0);
+  __shared__ float4 buf[kSrWarps][64];
+  __shared__ uint32_t idx[kSrWarps][64];
+  __shared__ R part[kSrWarps][32];
+  __shared__ unsigned s_ch;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t nheavy = *nheavy_p;
+  const R eps = (R)(double)(float)app;
+  const R fac = (R)(a_val / (6.0 * kPi));
+  SrTarget<R> t;
+  t.eps = depth_const((float)eps);
+  t.eps64 = depth_const64((double)eps);
+  // the chunk's targets; false when it has nothing to do
+  auto begin = [&](const SrChunk &C, const PmHalo &p, int64_t &k) -> bool {
+    if (!p.pending) return false;
+    const bool valid = lane < (int)C.cnt;
+    t.e = C.e0 + lane;
+    k = valid ? (int64_t)cmem[t.e] : -1;
+    const bool active = valid && (!UPDATE || keep[k] != 0);
+    if (!__any_sync(FULL, active)) return false;
+    t.me = valid ? src4[t.e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int ri = active ? (int)pr[k] : 1;
+    const R ai = (R)(3.5 * (double)p.spacing / (double)ri);
+    t.a2 = ai * ai;
+    // the FP32 distance of a pair is within 1e-6 of the exact one
+    t.a2f = active ? (float)t.a2 * 1.00001f + 1e-37f : -1.0f;
+    t.ai = depth_const((float)ai);
+    t.ai64 = depth_const64((double)ai);
+    t.tl = p.two_level != 0;
+    t.acc = t.comp = (R)0;
+    if (!active) k = -1;
+    return true;
   };
-  for (int64_t ch = fetch(); ch < nchunks; ch = fetch()) {
+  auto finish = [&](int64_t k, R acc) {
+    if (k < 0) return;
+    // FP32 accumulates the negated terms, FP64 the terms with the sign taken in
+    const R v = fac * acc;
+    if (UPDATE) phi_sr[k] -= v;
+    else phi_sr[k] = v;
+  };
+  for (;;) {
+    if (threadIdx.x == 0) s_ch = atomicAdd(&next[0], 1u);
+    __syncthreads();
+    const unsigned ch = s_ch;
+    if (ch >= nheavy) break;
     const SrChunk C = chunks[ch];
-    const uint32_t cend = cstart[C.cell + 1];
-    const uint32_t e = C.e0 + lane;
-    const bool valid = e < cend;
-    const int64_t k = valid ? (int64_t)cmem[e] : -1;
-    const int h = mhalo[cmem[C.e0]];
-    const PmHalo &p = H[h];
-    if (!p.pending) continue;
-    const bool active = valid && keep[k] != 0;
-    if (!__any_sync(FULL, active)) continue;
-    float4 me = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (valid) me = src4[e];
-    const double sp = (double)p.spacing;
-    const int ri = active ? (int)pr[k] : 64;
-    const R ai = (R)(3.5 * sp / (double)ri);
-    const R a2 = ai * ai;
-    // chunk bounding box of the active targets and its largest cutoff
-    float lo[3] = {active ? me.x : 3e38f, active ? me.y : 3e38f, active ? me.z : 3e38f};
-    float hi[3] = {active ? me.x : -3e38f, active ? me.y : -3e38f, active ? me.z : -3e38f};
-    int rmin = ri;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        lo[d] = fminf(lo[d], __shfl_xor_sync(FULL, lo[d], o));
-        hi[d] = fmaxf(hi[d], __shfl_xor_sync(FULL, hi[d], o));
-      }
-      rmin = min(rmin, __shfl_xor_sync(FULL, rmin, o));
+    const PmHalo &p = H[C.h];
+    int64_t k;
+    const bool some = begin(C, p, k);  // the same for every warp of the block
+    if (some) {
+      sr_chunk_sum<R, UPDATE>(C, p, warp, kSrWarps, cstart, src4, rpos, rsrc, buf[warp], idx[warp], t);
+      part[warp][lane] = t.acc;
     }
-    // conservative filter radius (a little above every lane's cutoff)
-    const float amax = (float)(3.5 * sp / (double)rmin) * 1.0001f + 1e-30f;
-    const float amax2 = amax * amax;
-    int kk = (int)ceil((3.5 / (double)rmin) / p.cw_u - 1e-9);
-    kk = kk < 1 ? 1 : (kk > 4 ? 4 : kk);
-    const int64_t local = (int64_t)C.cell - p.cell_off;
-    const int64_t n0 = p.nc[0], n1 = p.nc[1], n2 = p.nc[2];
-    const int64_t cx = local % n0, cy = (local / n0) % n1, cz = local / (n0 * n1);
-    const R eps = (R)(double)(float)app;
-    const R fac = (R)(a_val / (6.0 * kPi));
-    const bool tl = p.two_level != 0;
-    const DepthConst k_eps = depth_const((float)eps), k_ai = depth_const((float)ai);
-    const DepthConst64 k64_eps = depth_const64((double)eps), k64_ai = depth_const64((double)ai);
-    R acc = 0, comp = 0;
-    // The (2kk+1)^3 neighbour cells, 32 at a time: a lane loads one cell's
-    // source range, the ranges are concatenated by a warp prefix sum and
-    // streamed in batches of 32 (a lane finds its source's cell by a binary
-    // search over the prefix), so small cells share batches.
-    const int wd = 2 * kk + 1, ncell = wd * wd * wd;
-    for (int cb0 = 0; cb0 < ncell; cb0 += 32) {
-      const int j = cb0 + lane;
-      uint32_t s0 = 0, cnt = 0;
-      if (j < ncell) {
-        const int64_t x = cx + j % wd - kk, y = cy + (j / wd) % wd - kk, z = cz + j / (wd * wd) - kk;
-        if (x >= 0 && x < n0 && y >= 0 && y < n1 && z >= 0 && z < n2) {
-          const int64_t c = p.cell_off + x + n0 * (y + n1 * z);
-          uint32_t a = cstart[c], b = cstart[c + 1];
-          if (UPDATE) {
-            a = rpos[a];
-            b = rpos[b];
-          }
-          s0 = a;
-          cnt = b - a;
-        }
-      }
-      uint32_t incl = cnt;
+    __syncthreads();
+    if (some && warp == 0) {
+      R sum = part[0][lane];
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o) incl += v;
-      }
-      const uint32_t excl = incl - cnt;
-      const uint32_t T = __shfl_sync(FULL, incl, 31);
-      for (uint32_t g0 = 0; g0 < T; g0 += 32) {
-        const uint32_t g = g0 + (uint32_t)lane;
-        int owner = 0;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1) {
-          const uint32_t v = __shfl_sync(FULL, incl, owner + step - 1);
-          if (v <= g) owner += step;
-        }
-        owner &= 31;
-        const uint32_t os0 = __shfl_sync(FULL, s0, owner);
-        const uint32_t oex = __shfl_sync(FULL, excl, owner);
-        uint32_t se = 0;
-        float4 sv = make_float4(0.f, 0.f, 0.f, 0.f);
-        bool cand = false;
-        if (g < T) {
-          const uint32_t t = os0 + (g - oex);
-          se = UPDATE ? rsrc[t] : t;
-          sv = src4[se];
-          cand = UPDATE || keep[cmem[se]] != 0;
-          const float bx = fmaxf(fmaxf(lo[0] - sv.x, sv.x - hi[0]), 0.f);
-          const float by = fmaxf(fmaxf(lo[1] - sv.y, sv.y - hi[1]), 0.f);
-          const float bz = fmaxf(fmaxf(lo[2] - sv.z, sv.z - hi[2]), 0.f);
-          cand = cand && (bx * bx + by * by + bz * bz <= amax2);
-        }
-        unsigned mask = __ballot_sync(FULL, cand);
-        while (mask) {
-          const int bl = __ffs(mask) - 1;
-          mask &= mask - 1;
-          const float jx = __shfl_sync(FULL, sv.x, bl), jy = __shfl_sync(FULL, sv.y, bl);
-          const float jz = __shfl_sync(FULL, sv.z, bl), jw = __shfl_sync(FULL, sv.w, bl);
-          const uint32_t je = __shfl_sync(FULL, se, bl);
-          if (active && je != e) {
-            R dx, dy, dz;
-            if (tl) {
-              dx = (R)jx - (R)me.x; dy = (R)jy - (R)me.y; dz = (R)jz - (R)me.z;
-            } else {
-              dx = (R)__fsub_rn(jx, me.x); dy = (R)__fsub_rn(jy, me.y); dz = (R)__fsub_rn(jz, me.z);
-            }
-            const R r2 = dx * dx + dy * dy + dz * dz;
-            if (r2 < a2) {
-              R dphi;
-              if constexpr (sizeof(R) == 4) {
-                const float rinv = rsqrtf(r2), d = r2 * rinv;
-                dphi = -(fac * (depth_fast(d, rinv, k_eps) - depth_fast(d, rinv, k_ai)));
-              } else if (r2 > 1e-30 && r2 < 1e30) {
-                const double rinv = rsqrt_nr64(r2), d = r2 * rinv;
-                dphi = -(fac * (depth_fast64(d, rinv, k64_eps) - depth_fast64(d, rinv, k64_ai)));
-              } else {
-                const R d = sqrt(r2);
-                dphi = -(fac * (depth_c<R>(d, eps) - depth_c<R>(d, ai)));
-              }
-              if constexpr (sizeof(R) == 4) {  // FP32: compensated sum
-                const R yv = (R)jw * dphi - comp;
-                const R tt = acc + yv;
-                comp = (tt - acc) - yv;
-                acc = tt;
-              } else {  // FP64: a plain sum (one dependent add per pair)
-                acc += (R)jw * dphi;
-              }
-            }
-          }
-        }
-      }
+      for (int w = 1; w < kSrWarps; ++w) sum += part[w][lane];
+      finish(k, sum);
     }
-    if (active) {
-      if (UPDATE) phi_sr[k] -= acc;
-      else phi_sr[k] = acc;
-    }
+  }
+  for (;;) {
+    unsigned ch = 0;
+    if (lane == 0) ch = nheavy + atomicAdd(&next[1], 1u);
+    ch = __shfl_sync(FULL, ch, 0);
+    if (ch >= nchunks) break;
+    const SrChunk C = chunks[ch];
+    const PmHalo &p = H[C.h];
+    int64_t k;
+    if (!begin(C, p, k)) continue;
+    sr_chunk_sum<R, UPDATE>(C, p, 0, 1, cstart, src4, rpos, rsrc, buf[warp], idx[warp], t);
+    finish(k, t.acc);
   }
 }
 
@@ -748,40 +941,6 @@ __global__ void sr_pack_kernel(const Members m, const uint32_t *__restrict__ cme
     const uint32_t k = cmem[e];
     src4[e] = make_float4(m.q[0][k], m.q[1][k], m.q[2][k], m.w[k]);
   }
-}
-
-// Target chunks: ceil(members / 32) per cell.
-__global__ void sr_chunk_count_kernel(const uint32_t *__restrict__ cstart, int64_t ncell,
-                                      uint32_t *__restrict__ cnt) {
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncell;
-       c += (int64_t)gridDim.x * blockDim.x)
-    cnt[c] = (cstart[c + 1] - cstart[c] + 31u) / 32u;
-}
-
-__global__ void sr_chunk_fill_kernel(const uint32_t *__restrict__ cstart, const uint32_t *__restrict__ coff,
-                                     int64_t ncell, SrChunk *__restrict__ chunks) {
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncell;
-       c += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t n = (cstart[c + 1] - cstart[c] + 31u) / 32u;
-    for (uint32_t i = 0; i < n; ++i) chunks[coff[c] + i] = SrChunk{(uint32_t)c, cstart[c] + 32u * i};
-  }
-}
-
-// Work order of the target chunks: heaviest first, the weight being the
-// occupancy of the chunk's cell (the density its targets' cutoff spheres
-// sample), so the dynamically fetched chunks end together.
-__global__ void sr_chunk_key_kernel(const SrChunk *__restrict__ chunks, int64_t n,
-                                    const uint32_t *__restrict__ cstart, uint32_t *__restrict__ key) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t c = chunks[i].cell;
-    key[i] = 65535u - min(cstart[c + 1] - cstart[c], 65535u);
-  }
-}
-
-__global__ void sr_chunk_order_kernel(const SrChunk *__restrict__ chunks, const uint32_t *__restrict__ idx,
-                                      int64_t n, SrChunk *__restrict__ out) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = chunks[idx[i]];
 }
 
 // Members removed since the previous pass, in cell order: flag (and clear
@@ -1787,7 +1946,7 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
       p.u_min[d] = hext[6 * h + d];
       const double span = hext[6 * h + 3 + d] - hext[6 * h + d];
       p.nc[d] = std::max(1, (int)std::floor(span / p.cw_u) + 1);
-      c *= p.nc[d];
+      c *= 4 * (((int64_t)p.nc[d] + 3) / 4);  // whole bricks of 4^3 cells
     }
     ncell += c;
   }
@@ -1814,48 +1973,37 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   // cell-ordered positions and weights, target chunks, removal lists
   uint32_t npm = 0;
   PYFOF_CUDA(cudaMemcpyAsync(&npm, cstart + ncell, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  uint32_t *chcnt = W.carve<uint32_t>(ncell + 1);
+  const int64_t nbrick = ncell / 64;
+  uint32_t *chcnt = W.carve<uint32_t>(nbrick + 1);
   if (!chcnt) { set_error("workspace exhausted (C2 chunks)"); return kAlloc; }
-  PYFOF_CUDA(cudaMemsetAsync(chcnt, 0, sizeof(uint32_t) * (ncell + 1), s));
-  const unsigned gC = (unsigned)std::min<int64_t>(ceil_div(std::max<int64_t>(ncell, 1), BLK), 148 * 16);
-  sr_chunk_count_kernel<<<gC, BLK, 0, s>>>(cstart, ncell, chcnt);
+  PYFOF_CUDA(cudaMemsetAsync(chcnt, 0, sizeof(uint32_t) * (nbrick + 1), s));
+  const unsigned gC = (unsigned)std::min<int64_t>(ceil_div(std::max<int64_t>(nbrick, 1), BLK), 148 * 16);
+  sr_chunk_count_kernel<<<gC, BLK, 0, s>>>(cstart, nbrick, chcnt);
   PYFOF_CHECK_LAUNCH();
-  PYFOF_TRY(exclusive_scan_u32(chcnt, chcnt, ncell + 1, nullptr, W, s));
+  PYFOF_TRY(exclusive_scan_u32(chcnt, chcnt, nbrick + 1, nullptr, W, s));
   uint32_t nchunk = 0;
-  PYFOF_CUDA(cudaMemcpyAsync(&nchunk, chcnt + ncell, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  PYFOF_CUDA(cudaMemcpyAsync(&nchunk, chcnt + nbrick, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   PYFOF_CUDA(cudaStreamSynchronize(s));
   float4 *src4 = W.carve<float4>(std::max<uint32_t>(npm, 1));
   SrChunk *chunks = W.carve<SrChunk>(std::max<uint32_t>(nchunk, 1));
+  uint2 *chspan = W.carve<uint2>(std::max<uint32_t>(nchunk, 1));
   uint32_t *rflag = W.carve<uint32_t>((size_t)npm + 1), *rpos = W.carve<uint32_t>((size_t)npm + 1);
   uint32_t *rsrc = W.carve<uint32_t>(std::max<uint32_t>(npm, 1));
-  if (!src4 || !chunks || !rflag || !rpos || !rsrc) { set_error("workspace exhausted (C2 sources)"); return kAlloc; }
+  // [0..1] the chunk counters of a pass, [2] the heavy chunks
+  unsigned *sr_next = W.carve<unsigned>(3);
+  if (!src4 || !chunks || !chspan || !rflag || !rpos || !rsrc || !sr_next) {
+    set_error("workspace exhausted (C2 sources)");
+    return kAlloc;
+  }
+  PYFOF_CUDA(cudaMemsetAsync(sr_next, 0, 3 * sizeof(unsigned), s));
   PYFOF_CUDA(cudaMemsetAsync(rflag, 0, sizeof(uint32_t) * ((size_t)npm + 1), s));
   const unsigned gP = (unsigned)std::min<int64_t>(ceil_div(std::max<uint32_t>(npm, 1), BLK), 148 * 16);
   sr_pack_kernel<<<gP, BLK, 0, s>>>(m, cmem, npm, src4);
   PYFOF_CHECK_LAUNCH();
-  sr_chunk_fill_kernel<<<gC, BLK, 0, s>>>(cstart, chcnt, ncell, chunks);
+  sr_chunk_fill_kernel<<<gC, BLK, 0, s>>>(cstart, chcnt, nbrick, chspan);
   PYFOF_CHECK_LAUNCH();
-  {
-    // heaviest chunks first (a stable sort on the 16-bit weight key)
-    const int64_t nc = std::max<uint32_t>(nchunk, 1);
-    uint32_t *ck = W.carve<uint32_t>(nc), *c1k = W.carve<uint32_t>(nc), *c1v = W.carve<uint32_t>(nc),
-             *c2k = W.carve<uint32_t>(nc), *c2v = W.carve<uint32_t>(nc);
-    SrChunk *sorted = W.carve<SrChunk>(nc);
-    if (!ck || !c1k || !c1v || !c2k || !c2v || !sorted) { set_error("workspace exhausted (C2 chunks)"); return kAlloc; }
-    const unsigned gK = (unsigned)std::min<int64_t>(ceil_div(nc, BLK), 148 * 16);
-    sr_chunk_key_kernel<<<gK, BLK, 0, s>>>(chunks, nchunk, cstart, ck);
-    PYFOF_CHECK_LAUNCH();
-    uint32_t *sk2, *order;
-    PYFOF_TRY(radix_sort_pairs(ck, nullptr, nchunk, 16, c1k, c1v, c2k, c2v, &sk2, &order, W, s));
-    sr_chunk_order_kernel<<<gK, BLK, 0, s>>>(chunks, order, nchunk, sorted);
-    PYFOF_CHECK_LAUNCH();
-    chunks = sorted;
-  }
-  unsigned *sr_next = W.carve<unsigned>(1);
-  if (!sr_next) { set_error("workspace exhausted (C2 chunks)"); return kAlloc; }
-  // persistent warps: the blocks that fit on the GPU at once (4 per SM)
-  const unsigned gS = (unsigned)std::min<int64_t>(ceil_div((int64_t)std::max<uint32_t>(nchunk, 1) * 32, 256),
-                                                  148 * 4);
+  // persistent blocks: those that fit on the GPU at once, if there is work for them
+  const unsigned gS = (unsigned)std::min<int64_t>(std::max<uint32_t>(nchunk, 1), 148 * (sizeof(R) == 4 ? 4 : 3));
   // per-member refinement ratio, refined-region sources and targets
   const int na = (int)act.size();
   uint8_t *pr = W.carve<uint8_t>(M);
@@ -1877,6 +2025,24 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
     PYFOF_TRY(upload(ctx, dact_of, act_of.data(), sizeof(int32_t) * nh * 512, s));
     tl_particle_kernel<<<gM, BLK, 0, s>>>(m, dH, mhalo, M, dregr, dact_of, pr, preg);
     PYFOF_CHECK_LAUNCH();
+    {
+      // chunk records, then most sources first (a stable sort on a 16-bit key)
+      const int64_t nc = std::max<uint32_t>(nchunk, 1);
+      uint32_t *ck = W.carve<uint32_t>(nc), *c1k = W.carve<uint32_t>(nc), *c1v = W.carve<uint32_t>(nc),
+               *c2k = W.carve<uint32_t>(nc), *c2v = W.carve<uint32_t>(nc);
+      SrChunk *sorted = W.carve<SrChunk>(nc);
+      if (!ck || !c1k || !c1v || !c2k || !c2v || !sorted) { set_error("workspace exhausted (C2 chunks)"); return kAlloc; }
+      const unsigned gW = (unsigned)std::min<int64_t>(ceil_div(nc * 32, BLK), 148 * 16);
+      sr_chunk_setup_kernel<<<gW, BLK, 0, s>>>(chspan, nchunk, dH, mhalo, cmem, src4, pr, cstart, chunks, ck,
+                                               sr_next + 2);
+      PYFOF_CHECK_LAUNCH();
+      const unsigned gK = (unsigned)std::min<int64_t>(ceil_div(nc, BLK), 148 * 16);
+      uint32_t *sk2, *order;
+      PYFOF_TRY(radix_sort_pairs(ck, nullptr, nchunk, 16, c1k, c1v, c2k, c2v, &sk2, &order, W, s));
+      sr_chunk_order_kernel<<<gK, BLK, 0, s>>>(chunks, order, nchunk, sorted);
+      PYFOF_CHECK_LAUNCH();
+      chunks = sorted;
+    }
     if (na > 0) {
       dA = W.carve<TlRegion>(na);
       uint32_t *cnt = W.carve<uint32_t>(na + 1);
@@ -2112,10 +2278,11 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
         PYFOF_CHECK_LAUNCH();
       }
     }
-    PYFOF_CUDA(cudaMemsetAsync(sr_next, 0, sizeof(unsigned), s));
+    PYFOF_CUDA(cudaMemsetAsync(sr_next, 0, 2 * sizeof(unsigned), s));
     if (pass == 1) {
-      sr_gather_kernel<R, false><<<gS, 256, 0, s>>>(dH, mhalo, keep, pr, chunks, nchunk, cstart, cmem, src4,
-                                                    nullptr, nullptr, a.a_val, a.softening, c2, sr_next);
+      sr_gather_kernel<R, false><<<gS, 32 * kSrWarps, 0, s>>>(dH, keep, pr, chunks, nchunk, sr_next + 2, cstart,
+                                                              cmem, src4, nullptr, nullptr, a.a_val, a.softening,
+                                                              c2, sr_next);
       PYFOF_CHECK_LAUNCH();
     } else {
       sr_removed_flag_kernel<<<gP, BLK, 0, s>>>(cmem, npm, jd, rflag);
@@ -2123,8 +2290,9 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
       PYFOF_TRY(exclusive_scan_u32(rflag, rpos, (int64_t)npm + 1, nullptr, W, s));
       sr_removed_fill_kernel<<<gP, BLK, 0, s>>>(rflag, rpos, npm, rsrc);
       PYFOF_CHECK_LAUNCH();
-      sr_gather_kernel<R, true><<<gS, 256, 0, s>>>(dH, mhalo, keep, pr, chunks, nchunk, cstart, cmem, src4,
-                                                   rpos, rsrc, a.a_val, a.softening, c2, sr_next);
+      sr_gather_kernel<R, true><<<gS, 32 * kSrWarps, 0, s>>>(dH, keep, pr, chunks, nchunk, sr_next + 2, cstart,
+                                                             cmem, src4, rpos, rsrc, a.a_val, a.softening, c2,
+                                                             sr_next);
       PYFOF_CHECK_LAUNCH();
     }
     if (!pend_small.empty()) {

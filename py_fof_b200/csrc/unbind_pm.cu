@@ -549,41 +549,30 @@ __device__ __forceinline__ float depth_fast(float r, float rinv, const DepthCons
   return (128.0f - prim) * c.inv70h;
 }
 
-// FP64 path of the same kernel without divisions.  1/r: an FP32 reciprocal
-// square root seed y (relative error about 2^-22) and one step of the
-// binomial series 1/sqrt(r2) = y (1 - g)^(-1/2) = y (1 + g/2 + 3 g^2/8 + ..),
-// g = 1 - r2 y^2 (|g| about 2^-21, so the dropped cubic term is 2^-65).  For r2
-// outside the FP32 normal range the caller keeps the plain sqrt/division
-// form.  The two pieces of the spline are polynomials in e = 2r/h scaled by
-// 1/h, with the 1/70 folded into their coefficients (the 12/e term is 6/(70 r)).
-struct DepthConst64 {
-  double h, two_over_h, inv_h;
-};
-__device__ __forceinline__ DepthConst64 depth_const64(double h) { return DepthConst64{h, 2.0 / h, 1.0 / h}; }
+// FP64 path of the same kernel without divisions or branches on the spline
+// piece.  With e = 2r/h the two pieces and the 1/r beyond them are one
+// expression in truncated powers (expand it to get depth_c's polynomials):
+//     r D(r, h) = 1 - S(e) / 140,
+//     S(e) = (2-e)_+^6 (e^2 + 4e + 2) + 4 (1-e)_+^7 (3 + e),
+// so a pair's term D(r, a) - D(r, eps) is (S(2r/eps) - S(2r/a)) / (140 r).
+// Its rounding error is that of 1/r, above the softened kernel's own
+// once r is far below eps: pairs closer than eps/20 keep depth_c.  1/r: an
+// FP32 reciprocal square root seed y (relative error about 2^-22) and one step
+// of the binomial series 1/sqrt(r2) = y (1 - g)^(-1/2) = y (1 + g/2 + 3 g^2/8
+// + ..), g = 1 - r2 y^2 (|g| about 2^-21, so the dropped cubic term is 2^-65).
 __device__ __forceinline__ double rsqrt_series64(double r2) {
   const double y = (double)rsqrtf((float)r2);
   const double g = fma(-(r2 * y), y, 1.0);
   return fma(y * g, fma(0.375, g, 0.5), y);
 }
-__device__ __forceinline__ double depth_fast64(double r, double rinv, const DepthConst64 &c) {
-  if (r >= c.h) return rinv;
-  const double e = r * c.two_over_h;
-  if (e <= 1.0) {
-    const double e2 = e * e;
-    double t = fma(e, -3.0 / 70.0, 8.0 / 70.0);
-    t = fma(e, t, 14.0 / 70.0);
-    t = fma(e, t, -56.0 / 70.0);
-    t = fma(e2, t, 112.0 / 70.0);
-    return fma(-e2, t, 208.0 / 70.0) * c.inv_h;
-  }
-  double t = fma(e, -1.0 / 70.0, 8.0 / 70.0);
-  t = fma(e, t, -14.0 / 70.0);
-  t = fma(e, t, -56.0 / 70.0);
-  t = fma(e, t, 280.0 / 70.0);
-  t = fma(e, t, -448.0 / 70.0);
-  t = fma(e, t, 224.0 / 70.0);
-  t = fma(e, t, 128.0 / 70.0);
-  return fma(t, c.inv_h, rinv * (6.0 / 70.0));
+// S(e) for 0 <= e <= 2
+__device__ __forceinline__ double spline_s64(double e) {
+  const double u = 2.0 - e, v = 1.0 - e;
+  const int neg = __double2hiint(v) >> 31;  // all ones when e > 1
+  const double vp = __hiloint2double(__double2hiint(v) & ~neg, __double2loint(v) & ~neg);
+  const double u2 = u * u, v2 = vp * vp;
+  const double u6 = u2 * u2 * u2, v7 = v2 * v2 * v2 * (4.0 * vp);
+  return fma(v7, 3.0 + e, u6 * fma(e, e + 4.0, 2.0));
 }
 
 // A target chunk: up to 32 members of one brick, consecutive in cell order
@@ -604,7 +593,8 @@ struct SrChunk {
 // Chunks whose nodes hold this many members or more are summed by the eight
 // warps of a block together.  The rule looks at the chunk alone, so the order
 // of its sum does not depend on what else is in the call.
-constexpr uint32_t kSrHeavy = 1024;
+// Update passes sum over the removed members only, a few per cent of them.
+constexpr uint32_t kSrHeavy = 1024, kSrHeavyUpdate = 16384;
 constexpr int kSrWarps = 8;
 
 __global__ void sr_chunk_count_kernel(const uint32_t *__restrict__ cstart, int64_t nbrick,
@@ -697,7 +687,8 @@ __global__ void __launch_bounds__(BLK) sr_chunk_setup_kernel(
     if (lane == 0) {
       out[ch] = C;
       key[ch] = 65535u - min(C.nsrc >> 2, 65535u);
-      if (C.nsrc >= kSrHeavy) atomicAdd(nheavy, 1u);
+      if (C.nsrc >= kSrHeavy) atomicAdd(&nheavy[0], 1u);
+      if (C.nsrc >= kSrHeavyUpdate) atomicAdd(&nheavy[1], 1u);
     }
   }
 }
@@ -712,12 +703,12 @@ __global__ void sr_chunk_order_kernel(const SrChunk *__restrict__ chunks, const 
 template <typename R>
 struct SrTarget {
   float4 me;
-  uint32_t e;     // position in cell order (a target is not its own source)
+  uint32_t e0;    // the chunk's first target (position in cell order)
   float a2f;      // FP32 bound of the pair test, a little above a2; < 0: no target
   R a2;
   bool tl;
-  DepthConst eps, ai;
-  DepthConst64 eps64, ai64;
+  DepthConst eps, ai;  // FP32 path
+  double two_over_eps, two_over_ai, eps64, r2_min;  // FP64 path
   R acc, comp;
 };
 
@@ -736,10 +727,19 @@ __device__ __forceinline__ void sr_pairs(const float4 *__restrict__ buf, const u
     const float dx = s.x - t.me.x, dy = s.y - t.me.y, dz = s.z - t.me.z;
     if (dx * dx + dy * dy + dz * dz <= t.a2f) mask |= 1u << j;
   }
+  if constexpr (!UPDATE) {  // a target is not its own source
+    const int lane = threadIdx.x & 31;
+    const uint32_t own = lane < cnt ? idx[lane] - t.e0 : 32u;
+    unsigned self = __ballot_sync(0xffffffffu, own < 32u);
+    while (self) {
+      const int j = __ffs(self) - 1;
+      self &= self - 1;
+      if (__shfl_sync(0xffffffffu, own, j) == (uint32_t)lane) mask &= ~(1u << j);
+    }
+  }
   while (mask) {
     const int j = __ffs(mask) - 1;
     mask &= mask - 1;
-    if (!UPDATE && idx[j] == t.e) continue;
     const float4 s = buf[j];
     R dx, dy, dz;
     if (t.tl) {
@@ -755,12 +755,15 @@ __device__ __forceinline__ void sr_pairs(const float4 *__restrict__ buf, const u
       const float v = t.acc + y;
       t.comp = (v - t.acc) - y;
       t.acc = v;
-    } else if (r2 > 1e-30 && r2 < 1e30) {
+    } else if (r2 > t.r2_min) {
       const double rinv = rsqrt_series64(r2), d = r2 * rinv;
-      t.acc = fma((double)s.w, depth_fast64(d, rinv, t.ai64) - depth_fast64(d, rinv, t.eps64), t.acc);
+      double sd = -spline_s64(d * t.two_over_ai);
+      const double ee = d * t.two_over_eps;
+      if (ee < 2.0) sd += spline_s64(ee);
+      t.acc = fma((double)s.w * rinv, sd, t.acc);
     } else {
       const R d = sqrt(r2);
-      t.acc += (R)s.w * (depth_c<R>(d, t.ai64.h) - depth_c<R>(d, t.eps64.h));
+      t.acc += (R)140 * (R)s.w * (depth_c<R>(d, sqrt(t.a2)) - depth_c<R>(d, t.eps64));
     }
   }
 }
@@ -781,28 +784,38 @@ __device__ __forceinline__ void sr_chunk_sum(const SrChunk &C, const PmHalo &p, 
   const unsigned lt = lanemask_lt();
   const float amax2 = C.amax * C.amax;
   const int w0 = C.nx[0], w1 = C.nx[1], nodes = w0 * w1 * C.nx[2];
-  int fill = 0, turn = 0;
-  for (int n0 = 0; n0 < nodes; n0 += 32) {
-    const int j = n0 + lane;
-    uint32_t s0 = 0, cnt = 0;
-    if (j < nodes) {
-      uint2 r = sr_node_range(p, cstart, C.x0[0] + j % w0, C.x0[1] + (j / w0) % w1, C.x0[2] + j / (w0 * w1),
-                              C.level);
-      if (UPDATE && r.y > r.x) r = make_uint2(rpos[r.x], rpos[r.y]);
-      s0 = r.x;
-      cnt = r.y - r.x;
-    }
-    uint32_t incl = cnt;
+  int fill = 0, n0 = -32;
+  uint32_t T = 0, g0 = 0, incl = 0, first = 0, turn = 0;  // the 32 nodes in hand; batches so far
+  for (;;) {
+    bool more = true;
+    while (fill < 32) {
+      if (g0 >= T) {
+        n0 += 32;
+        more = n0 < nodes;
+        if (!more) break;
+        const int j = n0 + lane;
+        uint32_t s0 = 0, cnt = 0;
+        if (j < nodes) {
+          uint2 r = sr_node_range(p, cstart, C.x0[0] + j % w0, C.x0[1] + (j / w0) % w1, C.x0[2] + j / (w0 * w1),
+                                  C.level);
+          if (UPDATE && r.y > r.x) r = make_uint2(rpos[r.x], rpos[r.y]);
+          s0 = r.x;
+          cnt = r.y - r.x;
+        }
+        incl = cnt;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(FULL, incl, o);
-      if (lane >= o) incl += v;
-    }
-    const uint32_t first = s0 - (incl - cnt);  // source of batch index g: first + g
-    const uint32_t T = __shfl_sync(FULL, incl, 31);
-    for (uint32_t g0 = 0; g0 < T; g0 += 32) {
-      if (nparts > 1 && (turn++ & (nparts - 1)) != part) continue;
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t v = __shfl_up_sync(FULL, incl, o);
+          if (lane >= o) incl += v;
+        }
+        first = s0 - (incl - cnt);  // source of batch index g: first + g
+        T = __shfl_sync(FULL, incl, 31);
+        g0 = 0;
+        continue;
+      }
       const uint32_t g = g0 + (uint32_t)lane;
+      g0 += 32;
+      if (nparts > 1 && (turn++ & (uint32_t)(nparts - 1)) != (uint32_t)part) continue;
       int owner = 0;
 #pragma unroll
       for (int step = 16; step > 0; step >>= 1) {
@@ -830,20 +843,17 @@ __device__ __forceinline__ void sr_chunk_sum(const SrChunk &C, const PmHalo &p, 
       }
       fill += __popc(m);
       __syncwarp();
-      if (fill >= 32) {
-        sr_pairs<R, UPDATE>(buf, idx, 32, t);
-        __syncwarp();
-        fill -= 32;
-        if (lane < fill) {
-          buf[lane] = buf[32 + lane];
-          idx[lane] = idx[32 + lane];
-        }
-        __syncwarp();
-      }
     }
+    if (fill) sr_pairs<R, UPDATE>(buf, idx, min(fill, 32), t);
+    __syncwarp();
+    if (!more) break;
+    fill -= 32;
+    if (lane < fill) {
+      buf[lane] = buf[32 + lane];
+      idx[lane] = idx[32 + lane];
+    }
+    __syncwarp();
   }
-  if (fill) sr_pairs<R, UPDATE>(buf, idx, fill, t);
-  __syncwarp();
 }
 
 // Bound by FP64 arithmetic per interacting pair (about 45 operations) once
@@ -864,102 +874,96 @@ __global__ void __launch_bounds__(32 * kSrWarps, sizeof(R) == 4 ? 4 : 3) sr_gath
   __shared__ R part[kSrWarps][32];
   __shared__ unsigned s_ch;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t nheavy = *nheavy_p;
+  const uint32_t nheavy = nheavy_p[UPDATE ? 1 : 0];
   const R eps = (R)(double)(float)app;
-  const R fac = (R)(a_val / (6.0 * kPi));
+  // FP64 sums carry the 140 of S(e)
+  const R fac = (R)(a_val / (6.0 * kPi) / (sizeof(R) == 8 ? 140.0 : 1.0));
   SrTarget<R> t;
   t.eps = depth_const((float)eps);
-  t.eps64 = depth_const64((double)eps);
+  t.eps64 = (double)eps;
+  t.two_over_eps = 2.0 / (double)eps;
+  t.r2_min = fmax(2.5e-3 * (double)eps * (double)eps, 1e-30);
   // the chunk's targets; false when it has nothing to do
   auto begin = [&](const SrChunk &C, const PmHalo &p, int64_t &k) -> bool {
     if (!p.pending) return false;
     const bool valid = lane < (int)C.cnt;
-    t.e = C.e0 + lane;
-    k = valid ? (int64_t)cmem[t.e] : -1;
+    t.e0 = C.e0;
+    k = valid ? (int64_t)cmem[C.e0 + lane] : -1;
     const bool active = valid && (!UPDATE || keep[k] != 0);
     if (!__any_sync(FULL, active)) return false;
-    t.me = valid ? src4[t.e] : make_float4(0.f, 0.f, 0.f, 0.f);
+    t.me = valid ? src4[C.e0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int ri = active ? (int)pr[k] : 1;
     const R ai = (R)(3.5 * (double)p.spacing / (double)ri);
     t.a2 = ai * ai;
     // the FP32 distance of a pair is within 1e-6 of the exact one
     t.a2f = active ? (float)t.a2 * 1.00001f + 1e-37f : -1.0f;
     t.ai = depth_const((float)ai);
-    t.ai64 = depth_const64((double)ai);
+    t.two_over_ai = 2.0 / (double)ai;
     t.tl = p.two_level != 0;
     t.acc = t.comp = (R)0;
     if (!active) k = -1;
     return true;
   };
-  auto finish = [&](int64_t k, R acc) {
-    if (k < 0) return;
-    // FP32 accumulates the negated terms, FP64 the terms with the sign taken in
-    const R v = fac * acc;
-    if (UPDATE) phi_sr[k] -= v;
-    else phi_sr[k] = v;
-  };
-  for (;;) {
-    if (threadIdx.x == 0) s_ch = atomicAdd(&next[0], 1u);
-    __syncthreads();
-    const unsigned ch = s_ch;
-    if (ch >= nheavy) break;
-    const SrChunk C = chunks[ch];
-    const PmHalo &p = H[C.h];
-    int64_t k;
-    const bool some = begin(C, p, k);  // the same for every warp of the block
-    if (some) {
-      sr_chunk_sum<R, UPDATE>(C, p, warp, kSrWarps, cstart, src4, rpos, rsrc, buf[warp], idx[warp], t);
-      part[warp][lane] = t.acc;
-    }
-    __syncthreads();
-    if (some && warp == 0) {
-      R sum = part[0][lane];
-#pragma unroll
-      for (int w = 1; w < kSrWarps; ++w) sum += part[w][lane];
-      finish(k, sum);
-    }
-  }
+  bool heavy = true;  // the same for every warp of the block at its barriers
   for (;;) {
     unsigned ch = 0;
-    if (lane == 0) ch = nheavy + atomicAdd(&next[1], 1u);
-    ch = __shfl_sync(FULL, ch, 0);
-    if (ch >= nchunks) break;
-    const SrChunk C = chunks[ch];
+    if (heavy) {
+      if (threadIdx.x == 0) s_ch = atomicAdd(&next[0], 1u);
+      __syncthreads();
+      ch = s_ch;
+      if (ch >= nheavy) {
+        heavy = false;
+        continue;
+      }
+    } else {
+      if (lane == 0) ch = nheavy + atomicAdd(&next[1], 1u);
+      ch = __shfl_sync(FULL, ch, 0);
+      if (ch >= nchunks) break;
+    }
+    const SrChunk &C = chunks[ch];  // read where needed (L1), not held in registers
     const PmHalo &p = H[C.h];
     int64_t k;
-    if (!begin(C, p, k)) continue;
-    sr_chunk_sum<R, UPDATE>(C, p, 0, 1, cstart, src4, rpos, rsrc, buf[warp], idx[warp], t);
-    finish(k, t.acc);
+    const bool some = begin(C, p, k);
+    if (some)
+      sr_chunk_sum<R, UPDATE>(C, p, heavy ? warp : 0, heavy ? kSrWarps : 1, cstart, src4, rpos, rsrc, buf[warp],
+                              idx[warp], t);
+    if (heavy) {
+      if (some) part[warp][lane] = t.acc;
+      __syncthreads();
+      if (warp != 0 || !some) continue;
+#pragma unroll
+      for (int w = 1; w < kSrWarps; ++w) t.acc += part[w][lane];
+    }
+    if (some && k >= 0) {
+      const R v = fac * t.acc;
+      if (UPDATE) phi_sr[k] -= v;
+      else phi_sr[k] = v;
+    }
   }
 }
 
-// Cell-ordered copy of the members' positions and weights.
+// Cell-ordered copy of the members' positions and weights, and every
+// member's position in cell order.
 __global__ void sr_pack_kernel(const Members m, const uint32_t *__restrict__ cmem, int64_t n,
-                               float4 *__restrict__ src4) {
+                               float4 *__restrict__ src4, uint32_t *__restrict__ epos) {
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t k = cmem[e];
     src4[e] = make_float4(m.q[0][k], m.q[1][k], m.q[2][k], m.w[k]);
+    epos[k] = (uint32_t)e;
   }
 }
 
-// Members removed since the previous pass, in cell order: flag (and clear
-// the removal mark) per cell-ordered position.
-__global__ void sr_removed_flag_kernel(const uint32_t *__restrict__ cmem, int64_t n, uint8_t *__restrict__ jd,
-                                       uint32_t *__restrict__ flag) {
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t k = cmem[e];
-    flag[e] = jd[k];
-    jd[k] = 0;
-  }
-}
-
-__global__ void sr_removed_fill_kernel(const uint32_t *__restrict__ flag, const uint32_t *__restrict__ rpos,
+// The members removed since the previous pass (flagged per cell-ordered
+// position by the removal kernels), compacted in cell order; clears the flags.
+__global__ void sr_removed_fill_kernel(uint32_t *__restrict__ flag, const uint32_t *__restrict__ rpos,
                                        int64_t n, uint32_t *__restrict__ rsrc) {
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x)
-    if (flag[e]) rsrc[rpos[e]] = (uint32_t)e;
+    if (flag[e]) {
+      rsrc[rpos[e]] = (uint32_t)e;
+      flag[e] = 0;
+    }
 }
 
 // ---------------------------------------------------------------- two-level
@@ -1237,7 +1241,8 @@ template <typename R>
 __global__ void __launch_bounds__(IBLK) pm_inner_kernel(const Members m, PmHalo *__restrict__ H,
                                                         const int32_t *__restrict__ list, int nlist,
                                                         uint8_t *__restrict__ keep,
-                                                        uint8_t *__restrict__ jd,
+                                                        const uint32_t *__restrict__ epos,
+                                                        uint32_t *__restrict__ rflag,
                                                         const R *__restrict__ phi_c1,
                                                         const R *__restrict__ phi_in,
                                                         const R *__restrict__ phi_c2,
@@ -1358,7 +1363,7 @@ __global__ void __launch_bounds__(IBLK) pm_inner_kernel(const Members m, PmHalo 
         const float e = en[k];
         if (e >= 0.0f && __float_as_uint(e + 0.0f) >= thr) {
           keep[k] = 0;
-          jd[k] = 1;
+          rflag[epos[k]] = 1;
         }
       }
       __syncthreads();
@@ -1389,7 +1394,7 @@ __global__ void __launch_bounds__(IBLK) pm_inner_kernel(const Members m, PmHalo 
       for (int w = 0; w < IBLK / 32; ++w) chunk_eq += red_i[w];
       if (i < np && (del_gt || (is_eq && before < need))) {
         keep[k] = 0;
-        jd[k] = 1;
+        rflag[epos[k]] = 1;
       }
       taken_eq += chunk_eq;
       __syncthreads();
@@ -1535,7 +1540,9 @@ __global__ void __launch_bounds__(IBLK) big_select_kernel(BigHalo *__restrict__ 
                                                           const uint32_t *__restrict__ ulist,
                                                           uint32_t *__restrict__ eqbuf,
                                                           const float *__restrict__ en,
-                                                          uint8_t *__restrict__ keep, uint8_t *__restrict__ jd,
+                                                          uint8_t *__restrict__ keep,
+                                                          const uint32_t *__restrict__ epos,
+                                                          uint32_t *__restrict__ rflag,
                                                           int nmin, int32_t *__restrict__ nactive,
                                                           const int32_t *flags) {
   BigHalo &bh = B[blockIdx.x];
@@ -1605,7 +1612,7 @@ __global__ void __launch_bounds__(IBLK) big_select_kernel(BigHalo *__restrict__ 
     const unsigned key = __float_as_uint(E[li] + 0.0f);
     if (key > thr) {
       keep[bh.off + li] = 0;
-      jd[bh.off + li] = 1;
+      rflag[epos[bh.off + li]] = 1;
     } else if (key == thr) {
       EQ[atomicAdd(&s_neq, 1)] = li;
     }
@@ -1618,7 +1625,7 @@ __global__ void __launch_bounds__(IBLK) big_select_kernel(BigHalo *__restrict__ 
     for (int j = 0; j < neq; ++j) rank += EQ[j] < li;
     if (rank < need) {
       keep[bh.off + li] = 0;
-      jd[bh.off + li] = 1;
+      rflag[epos[bh.off + li]] = 1;
     }
   }
   __syncthreads();
@@ -1760,7 +1767,7 @@ int bits_for(uint64_t v) {
 // One pass of the removal loop of the large halos (see BigHalo).
 template <typename R>
 int32_t big_removal(Context &ctx, const Members &m, BigHalo *dB, int nbig, const BigChunk *dCh, int nchb,
-                    PmHalo *dH, uint8_t *keep, uint8_t *jd, const R *c1, const R *phi_in, const R *c2,
+                    PmHalo *dH, uint8_t *keep, const uint32_t *epos, uint32_t *rflag, const R *c1, const R *phi_in, const R *c2,
                     float *phi, float *en, double *part, int32_t *ucount, uint32_t *ulist, uint32_t *eqbuf,
                     int32_t *nactive, float b_val, int nmin, int phi_only) {
   cudaStream_t s = ctx.stream;
@@ -1786,7 +1793,7 @@ int32_t big_removal(Context &ctx, const Members &m, BigHalo *dB, int nbig, const
         PYFOF_CHECK_LAUNCH();
         big_energy_kernel<<<nchb, 256, 0, s>>>(m, dCh, dB, keep, phi, en, b_val, ucount, ulist, ctx.d_flags);
         PYFOF_CHECK_LAUNCH();
-        big_select_kernel<<<nbig, IBLK, 0, s>>>(dB, ucount, ulist, eqbuf, en, keep, jd, nmin, nactive,
+        big_select_kernel<<<nbig, IBLK, 0, s>>>(dB, ucount, ulist, eqbuf, en, keep, epos, rflag, nmin, nactive,
                                                 ctx.d_flags);
         PYFOF_CHECK_LAUNCH();
       }
@@ -1838,9 +1845,8 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   R *selfv = W.carve<R>(M), *c1 = W.carve<R>(M), *c2 = W.carve<R>(M);
   float *phi = W.carve<float>(M), *en = W.carve<float>(M);
   R *tl_self_in = nullptr;
-  uint8_t *jd = W.carve<uint8_t>(M);  // removed since the previous pass
-  if (!jd) { set_error("workspace exhausted (removal marks)"); return kAlloc; }
-  PYFOF_CUDA(cudaMemsetAsync(jd, 0, M, s));
+  uint32_t *epos = W.carve<uint32_t>(M);  // positions in cell order (PM members)
+  if (!epos) { set_error("workspace exhausted (cell positions)"); return kAlloc; }
   double *ext = W.carve<double>(6 * (size_t)nh);
   if (!dH || !dlist || !dselfs || !mhalo || !first || !wt || !selfv || !c1 || !c2 || !phi || !en || !ext) {
     set_error("workspace exhausted (PM members)");
@@ -1989,16 +1995,16 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   uint2 *chspan = W.carve<uint2>(std::max<uint32_t>(nchunk, 1));
   uint32_t *rflag = W.carve<uint32_t>((size_t)npm + 1), *rpos = W.carve<uint32_t>((size_t)npm + 1);
   uint32_t *rsrc = W.carve<uint32_t>(std::max<uint32_t>(npm, 1));
-  // [0..1] the chunk counters of a pass, [2] the heavy chunks
-  unsigned *sr_next = W.carve<unsigned>(3);
+  // [0..1] the chunk counters of a pass, [2..3] the heavy chunks (first pass, updates)
+  unsigned *sr_next = W.carve<unsigned>(4);
   if (!src4 || !chunks || !chspan || !rflag || !rpos || !rsrc || !sr_next) {
     set_error("workspace exhausted (C2 sources)");
     return kAlloc;
   }
-  PYFOF_CUDA(cudaMemsetAsync(sr_next, 0, 3 * sizeof(unsigned), s));
+  PYFOF_CUDA(cudaMemsetAsync(sr_next, 0, 4 * sizeof(unsigned), s));
   PYFOF_CUDA(cudaMemsetAsync(rflag, 0, sizeof(uint32_t) * ((size_t)npm + 1), s));
   const unsigned gP = (unsigned)std::min<int64_t>(ceil_div(std::max<uint32_t>(npm, 1), BLK), 148 * 16);
-  sr_pack_kernel<<<gP, BLK, 0, s>>>(m, cmem, npm, src4);
+  sr_pack_kernel<<<gP, BLK, 0, s>>>(m, cmem, npm, src4, epos);
   PYFOF_CHECK_LAUNCH();
   sr_chunk_fill_kernel<<<gC, BLK, 0, s>>>(cstart, chcnt, nbrick, chspan);
   PYFOF_CHECK_LAUNCH();
@@ -2285,8 +2291,6 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
                                                               c2, sr_next);
       PYFOF_CHECK_LAUNCH();
     } else {
-      sr_removed_flag_kernel<<<gP, BLK, 0, s>>>(cmem, npm, jd, rflag);
-      PYFOF_CHECK_LAUNCH();
       PYFOF_TRY(exclusive_scan_u32(rflag, rpos, (int64_t)npm + 1, nullptr, W, s));
       sr_removed_fill_kernel<<<gP, BLK, 0, s>>>(rflag, rpos, npm, rsrc);
       PYFOF_CHECK_LAUNCH();
@@ -2298,12 +2302,13 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
     if (!pend_small.empty()) {
       PYFOF_CUDA(wait_velocities(ctx, s));
       pm_inner_kernel<R><<<(unsigned)pend_small.size(), IBLK, 0, s>>>(m, dH, dpend, (int)pend_small.size(), keep,
-                                                                     jd, c1, phi_in, c2, phi, en,
+                                                                     epos, rflag, c1, phi_in, c2, phi, en,
                                                                      (float)a.b_val, a.np_halo_min, phi_only,
                                                                      ctx.d_flags);
       PYFOF_CHECK_LAUNCH();
     }
-    if (nbig) PYFOF_TRY(big_removal<R>(ctx, m, dB, nbig, dCh, nchb, dH, keep, jd, c1, phi_in, c2, phi, en, bpart,
+    if (nbig) PYFOF_TRY(big_removal<R>(ctx, m, dB, nbig, dCh, nchb, dH, keep, epos, rflag, c1, phi_in, c2, phi, en,
+                                       bpart,
                                        bucount, bulist, beq, nactive, (float)a.b_val, a.np_halo_min,
                                        phi_only));
     if (ctx.timing) ctx.gap_timer.begin(s);

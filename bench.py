@@ -27,8 +27,9 @@ background sigma 1; link 0.2, np_halo_min 10, s_15 = 15 * 0.67 * 256 / 300.
 * e2e: the same metric through the public API ``py_fof_b200.fof`` with
   pinned host inputs, host<->device copies inside the timed region.
 * roofline: the dominant kernel group.  With unbinding: the particle-mesh
-  convolutions (the FFT kernels), algorithmic bytes 4 s (n+2) n^2 per solve
-  on an n^3 grid of s-byte reals over their event-timed device time.  Plain
+  convolutions (the FFT kernels), algorithmic bytes what their five passes
+  read and write on the halos' support boxes, each line once, over their
+  event-timed device time.  Plain
   FoF: the linking kernels, 20 B per particle + 4 B per cell.
   roofline_fof_link: the linking kernels on every workload.
 * cpu_baseline: the CPU restatement of the reference (oracle/, OpenMP, the
@@ -631,8 +632,8 @@ def run_b200(args):
     if bound:
         roof_main = roof("pm_convolve_fp64", st["pm_fft"], st["pm_fft_bytes"],
                          {"kernels": "k_x_r2c, k_lines (3 launches), k_x_c2r per batch (FP64 grids)",
-                          "algorithmic_bytes": "32 (n+2) n^2 per solve on FP64 grids (a read and a "
-                                               "write of the padded grid per transform, two transforms)",
+                          "algorithmic_bytes": "what the five passes read and write on the halos' support "
+                                               "boxes, each line once",
                           "solves_per_call": counts["pm_solves"]})
     else:
         roof_main = roof_link

@@ -107,9 +107,8 @@ int32_t pyfof_host_free(void *ptr);
  * particle mesh), "valid_halos" (halos written to the output),
  * "refined_regions" (two-level inner regions), "pm_passes" (passes of the
  * particle-mesh removal loop), "pm_solves" (halo-grid
- * convolutions over all passes), "pm_fft_bytes" (their algorithmic bytes:
- * 4 s (n+2) n^2 per solve on an n^3 grid of s-byte reals: a read and a
- * write of the padded grid per transform, two transforms). */
+ * convolutions over all passes), "pm_fft_bytes" (the bytes their five
+ * passes read and write on the halos' support boxes, each line once). */
 int32_t pyfof_get_stat(const char *key, int64_t *value);
 
 /* Device time of the linking kernel of the last call, when timing is on. */

@@ -84,9 +84,7 @@ struct Context {
   GroupTimer gap_timer;
   int64_t last_pm_passes = 0;
   bool side_timed = false;  // ev[9..11] hold this call's fork timing
-  // statistics of the last call: PM solves and their algorithmic FFT bytes
-  // (one read and one write of the padded (n+2) n^2 grid per transform, two
-  // transforms per solve)
+  // statistics of the last call: PM solves and their FFT bytes (conv_bytes)
   int64_t last_pm_solves = 0;
   double last_pm_fft_bytes = 0.0;
   // statistics of the last call

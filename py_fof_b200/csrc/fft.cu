@@ -221,14 +221,21 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int K>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(K) : "memory"); }
 
-// tw[j] = exp(-2 pi i j / N), from double-precision sincospi
-template <typename R, int N, int T>
-__device__ __forceinline__ void load_twiddles(cplx_t<R> *tw) {
-  for (int j = threadIdx.x; j < N; j += T) {
+// tw[j] = exp(-2 pi i j / N), from double-precision sincospi, computed once
+// per grid size: a block's own N calls would be a tenth of its FP64 work.
+template <typename R>
+__global__ void k_twiddles(cplx_t<R> *tw, int n) {
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
     double s, c;
-    sincospi(2.0 * (double)j / (double)N, &s, &c);
+    sincospi(2.0 * (double)j / (double)n, &s, &c);
     tw[j] = mk<cplx_t<R>>((R)c, (R)-s);
   }
+}
+
+template <typename R, int N, int T>
+__device__ __forceinline__ void load_twiddles(cplx_t<R> *tw, const cplx_t<R> *__restrict__ table) {
+#pragma unroll
+  for (int j = threadIdx.x; j < N; j += T) tw[j] = table[j];
 }
 
 // Stage A in place on `buf`: every thread first reads all the elements of
@@ -289,47 +296,57 @@ __device__ __forceinline__ void stage_b_smem(const cplx_t<R> *src, cplx_t<R> *ds
 
 // ------------------------------------------------------------------ kernels
 
-// x pass, forward r2c.  Real lines L = (b*SUP + z)*SUP + y, x < SUP
-// (SUP = N/2 + 1), are taken in pairs as one complex line (a + i b); the two
-// half spectra are separated with the Hermitian symmetry of real
-// transforms.  All loops have compile-time trip counts, so every thread
-// issues its loads before the first one returns.
-// FIX: the input is the fixed-point deposit grid (64-bit integers, grid b
-// scaled by inv_scale[b]) instead of R values.
-template <typename R, int N, bool FIX>
-__global__ void __launch_bounds__(Cfg<R, N>::T) k_x_r2c(const R *__restrict__ rho, cplx_t<R> *__restrict__ spec,
-                                                        int nhp, int nlines,
-                                                        const unsigned long long *__restrict__ acc,
-                                                        const double *__restrict__ inv_scale) {
+// Grid of every pass but the fused z pass: blockIdx.y = grid of the batch,
+// blockIdx.x = tile within it; a grid with fewer tiles than the largest
+// leaves the rest of its blocks at once (the host batches grids of similar
+// size).
+
+// Spectrum offset of line (y, z), z-major over ny lines per plane.
+template <int N>
+__device__ __forceinline__ int64_t line_off(int line, int ny, int y0, int z0, int nhp) {
+  const int z = line / ny, y = line - z * ny;
+  return ((int64_t)(z0 + z) * N + (y0 + y)) * nhp;
+}
+
+// x pass, forward r2c.  The in[1] x in[2] real lines of a grid (in[0]
+// fixed-point values each, scaled by the grid's inv_scale) are taken in
+// pairs as one complex line (a + i b); the two half spectra are separated
+// with the Hermitian symmetry of real transforms.  All loops have
+// compile-time trip counts, so every thread issues its loads before the
+// first one returns.
+template <typename R, int N>
+__global__ void __launch_bounds__(Cfg<R, N>::T) k_x_r2c(const unsigned long long *__restrict__ acc,
+                                                        const double *__restrict__ inv_scale,
+                                                        cplx_t<R> *__restrict__ spec,
+                                                        const cplx_t<R> *__restrict__ twt,
+                                                        const ConvBox *__restrict__ boxes, int nhp) {
   using C = cplx_t<R>;
   constexpr int T = Cfg<R, N>::T, W = kW<R>, WP = W + 1, NH = N / 2 + 1, SUP = N / 2 + 1;
+  const ConvBox &bx = boxes[blockIdx.y];
+  const int sx = bx.in[0], sy = bx.in[1];
+  const int L0 = blockIdx.x * (2 * W);
+  const int nl = min(2 * W, sy * bx.in[2] - L0);
+  if (nl <= 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int64_t loff[2 * W];
   C *tw = reinterpret_cast<C *>(smem_raw);
   C *t0 = tw + N;
-  load_twiddles<R, N, T>(tw);
-  const int L0 = blockIdx.x * (2 * W);
-  const int nl = min(2 * W, nlines - L0);
-  const R *src = rho + (int64_t)L0 * SUP;
+  load_twiddles<R, N, T>(tw, twt);
+  if (threadIdx.x < 2 * W) loff[threadIdx.x] = bx.spec_off + line_off<N>(L0 + threadIdx.x, sy, 0, 0, nhp);
+  const double inv = inv_scale[blockIdx.y];
+  const unsigned long long *src = acc + bx.in_off + (int64_t)L0 * sx;
 #pragma unroll
   for (int it = 0; it < (W * SUP + T - 1) / T; ++it) {
     const int idx = threadIdx.x + it * T;
-    if (idx < W * SUP) {
-      const int p = idx / SUP, x = idx - p * SUP;
-      R va, vb;
-      if constexpr (FIX) {
-        const int la = L0 + 2 * p;
-        va = 2 * p < nl ? (R)((double)acc[(int64_t)la * SUP + x] * inv_scale[la / (SUP * SUP)]) : (R)0;
-        vb = 2 * p + 1 < nl ? (R)((double)acc[(int64_t)(la + 1) * SUP + x] * inv_scale[(la + 1) / (SUP * SUP)])
-                            : (R)0;
-      } else {
-        va = 2 * p < nl ? src[(2 * p) * SUP + x] : (R)0;
-        vb = 2 * p + 1 < nl ? src[(2 * p + 1) * SUP + x] : (R)0;
-      }
+    const int p = idx / SUP, x = idx - p * SUP;
+    if (idx < W * SUP && x < sx) {
+      const R va = 2 * p < nl ? (R)((double)src[(2 * p) * sx + x] * inv) : (R)0;
+      const R vb = 2 * p + 1 < nl ? (R)((double)src[(2 * p + 1) * sx + x] * inv) : (R)0;
       t0[p + WP * x] = mk<C>(va, vb);
     }
   }
   __syncthreads();
-  stage_a_inplace<R, N, -1>(t0, tw, SUP);
+  stage_a_inplace<R, N, -1>(t0, tw, sx);
   __syncthreads();
   stage_b_smem<R, N, -1>(t0, t0);
   __syncthreads();
@@ -338,52 +355,49 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_x_r2c(const R *__restrict__ rh
     const int idx = threadIdx.x + it * T;
     const int lr = idx / NH, kx = idx - lr * NH;
     if (lr < nl) {
-      const int L = L0 + lr, p = lr >> 1;
-      const int b = L / (SUP * SUP), rem = L - b * (SUP * SUP);
-      const int z = rem / SUP, y = rem - z * SUP;
+      const int p = lr >> 1;
       const C zk = t0[p + WP * kx];
       const C zm = t0[p + WP * ((N - kx) % N)];
       C out;
       if ((lr & 1) == 0) out = mk<C>((R)0.5 * (zk.x + zm.x), (R)0.5 * (zk.y - zm.y));
       else out = mk<C>((R)0.5 * (zk.y + zm.y), (R)0.5 * (zm.x - zk.x));
-      spec[(((int64_t)b * N + z) * N + y) * nhp + kx] = out;
+      spec[loff[lr] + kx] = out;
     }
   }
 }
 
-// x pass, c2r into compact cubes of side OLIM: lines L = (b*OLIM + z)*OLIM
-// + y, out[L*OLIM + x] = x-th real value / scale.  Two Hermitian half
-// spectra become one complex line (a + i b); only the real parts of the DC
-// and Nyquist bins are used.
-template <typename R, int N, int OLIM>
-__global__ void __launch_bounds__(Cfg<R, N>::T) k_x_c2r(const cplx_t<R> *__restrict__ spec, R *__restrict__ out,
-                                                        int nhp, int nlines, R scale) {
+// x pass, c2r of the lines (y, z) of a grid's output window; the values
+// [out0[0], out0[0] + out[0]) of each, divided by `scale`, go to the compact
+// output.  Two Hermitian half spectra become one complex line (a + i b); only
+// the real parts of the DC and Nyquist bins are used.  SUP: the largest
+// out[0] of the launch.
+template <typename R, int N, int SUP>
+__global__ void __launch_bounds__(Cfg<R, N>::T) k_x_c2r(const cplx_t<R> *__restrict__ spec, R *__restrict__ phi,
+                                                        const cplx_t<R> *__restrict__ twt,
+                                                        const ConvBox *__restrict__ boxes, int nhp, R scale) {
   using C = cplx_t<R>;
   constexpr int T = Cfg<R, N>::T, W = kW<R>, WP = W + 1, NH = N / 2 + 1;
+  const ConvBox &bx = boxes[blockIdx.y];
+  const int ox = bx.out[0], x0 = bx.out0[0], oy = bx.out[1];
+  const int L0 = blockIdx.x * (2 * W);
+  const int nl = min(2 * W, oy * bx.out[2] - L0);
+  if (nl <= 0) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int64_t loff[2 * W];
   C *tw = reinterpret_cast<C *>(smem_raw);
   C *t0 = tw + N;
-  load_twiddles<R, N, T>(tw);
-  const int L0 = blockIdx.x * (2 * W);
-  const int nl = min(2 * W, nlines - L0);
+  load_twiddles<R, N, T>(tw, twt);
+  if (threadIdx.x < 2 * W)
+    loff[threadIdx.x] = bx.spec_off + line_off<N>(L0 + threadIdx.x, oy, bx.out0[1], bx.out0[2], nhp);
+  __syncthreads();
 #pragma unroll
   for (int it = 0; it < (W * NH + T - 1) / T; ++it) {
     const int idx = threadIdx.x + it * T;
     if (idx < W * NH) {
       const int p = idx / NH, kx = idx - p * NH;
       C a = mk<C>(0, 0), b = mk<C>(0, 0);
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        const int lr = 2 * p + hh;
-        if (lr < nl) {
-          const int L = L0 + lr;
-          const int bb = L / (OLIM * OLIM), rem = L - bb * (OLIM * OLIM);
-          const int z = rem / OLIM, y = rem - z * OLIM;
-          const C v = spec[(((int64_t)bb * N + z) * N + y) * nhp + kx];
-          if (hh == 0) a = v;
-          else b = v;
-        }
-      }
+      if (2 * p < nl) a = spec[loff[2 * p] + kx];
+      if (2 * p + 1 < nl) b = spec[loff[2 * p + 1] + kx];
       if (kx == 0 || kx == N / 2) {
         a.y = 0;
         b.y = 0;
@@ -397,46 +411,57 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_x_c2r(const cplx_t<R> *__restr
   __syncthreads();
   stage_b_smem<R, N, +1>(t0, t0);
   __syncthreads();
-  R *dst = out + (int64_t)L0 * OLIM;
+  R *dst = phi + bx.out_off + (int64_t)L0 * ox;
+  // a power of two divides exactly as its reciprocal multiplies
+  constexpr bool pow2 = (N & (N - 1)) == 0;
+  const R inv = (R)1 / scale;
 #pragma unroll
-  for (int it = 0; it < (W * OLIM + T - 1) / T; ++it) {
+  for (int it = 0; it < (W * SUP + T - 1) / T; ++it) {
     const int idx = threadIdx.x + it * T;
-    if (idx < W * OLIM) {
-      const int p = idx / OLIM, x = idx - p * OLIM;
-      const C v = t0[p + WP * x];
-      if (2 * p < nl) dst[(2 * p) * OLIM + x] = v.x / scale;
-      if (2 * p + 1 < nl) dst[(2 * p + 1) * OLIM + x] = v.y / scale;
+    const int p = idx / SUP, x = idx - p * SUP;
+    if (idx < W * SUP && x < ox) {
+      const C v = t0[p + WP * (x0 + x)];
+      if (2 * p < nl) dst[(2 * p) * ox + x] = pow2 ? v.x * inv : v.x / scale;
+      if (2 * p + 1 < nl) dst[(2 * p + 1) * ox + x] = pow2 ? v.y * inv : v.y / scale;
     }
   }
 }
 
-// Strided pass over tiles of W consecutive kx.  Line (b, other, kx) starts at
-// spec + b*bstride + other*ostride + kx, element e at + e*estride.  Elements
-// e >= in_lim are zero; elements e < out_lim are written.  CONV: forward
-// transform, multiplication by the real Green table (index ((e*N + other)*NH
-// + kx)) and inverse transform; otherwise one transform of sign SIGN.  A
-// block handles halos [b0, b0 + nbb) of the batch.
-template <typename R, int N, int SIGN, bool CONV>
+// Strided passes over tiles of W consecutive kx.
+enum { kYForward = 0, kZConv = 1, kYInverse = 2, kZInverse = 3 };
+
+// kYForward: lines (kx, z < in[2]), values y < in[1] in, all N out.
+// kZConv: lines (kx, ky), values z < in[2] in, forward transform,
+//   multiplication by the real Green table (index ((kz*N + ky)*NH + kx)),
+//   inverse transform, the output window's z out; a block handles the grids
+//   [b0, b0 + nbb) of the batch with its Green values in registers.
+// kYInverse: lines (kx, z of the output window), all N in, its y out.
+// kZInverse: lines (kx, ky), all N in and out (the self kernel).
+template <typename R, int N, int PASS>
 __global__ void __launch_bounds__(Cfg<R, N>::T) k_lines(cplx_t<R> *__restrict__ spec, const R *__restrict__ green,
-                                                        int64_t bstride, int64_t ostride, int64_t estride,
-                                                        int nother, int ntiles, int nbb, int batch, int in_lim,
-                                                        int out_lim) {
+                                                        const cplx_t<R> *__restrict__ twt,
+                                                        const ConvBox *__restrict__ boxes, int nhp, int ntiles,
+                                                        int nbb, int batch) {
   using C = cplx_t<R>;
+  constexpr bool CONV = PASS == kZConv, FWD = PASS == kYForward || CONV, ZLINE = CONV || PASS == kZInverse;
   constexpr int N1 = Cfg<R, N>::N1, N2 = Cfg<R, N>::N2, T = Cfg<R, N>::T;
   constexpr int W = kW<R>, WP = W + 1, NH = N / 2 + 1;
   constexpr int UA = W * N2, UB = W * N1;
   constexpr int IA = (UA + T - 1) / T, IB = (UB + T - 1) / T;
+  const int tile = (int)(blockIdx.x % (unsigned)ntiles);
+  const int other = (int)(blockIdx.x / (unsigned)ntiles);
+  const int kx0 = tile * W;
+  const int b0 = (int)blockIdx.y * nbb;
+  const int b1 = CONV ? min(batch, b0 + nbb) : b0 + 1;
+  if constexpr (PASS == kYForward) {
+    if (other >= boxes[b0].in[2]) return;
+  } else if constexpr (PASS == kYInverse) {
+    if (other >= boxes[b0].out[2]) return;
+  }
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *tw = reinterpret_cast<C *>(smem_raw);
   C *const buf0 = tw + N;
-  load_twiddles<R, N, T>(tw);
-  int64_t bid = blockIdx.x;
-  const int tile = (int)(bid % ntiles);
-  bid /= ntiles;
-  const int other = (int)(bid % nother);
-  const int b0 = (int)(bid / nother) * nbb;
-  const int b1 = min(batch, b0 + nbb);
-  const int kx0 = tile * W;
+  load_twiddles<R, N, T>(tw, twt);
   R g[CONV ? IB : 1][CONV ? N2 : 1];
   if constexpr (CONV) {
 #pragma unroll
@@ -451,15 +476,22 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_lines(cplx_t<R> *__restrict__ 
     }
   }
   __syncthreads();
-  // CONV: the input rows of the next halo are copied into a staging buffer
+  const int64_t estride = ZLINE ? (int64_t)N * nhp : nhp;
+  // first element of the line tile of grid b
+  auto tile_base = [&](int b) -> C * {
+    const int64_t o = ZLINE ? other : (int64_t)N * (other + (PASS == kYInverse ? boxes[b].out0[2] : 0));
+    return spec + boxes[b].spec_off + o * nhp + kx0;
+  };
+  // CONV: the input rows of the next grid are copied into a staging buffer
   // while the current one is transformed (two buffers of N/2+1 rows of W
-  // complex; in_lim <= N/2+1 there)
+  // complex)
   constexpr int SROWS = N / 2 + 1, CPR = (int)(W * sizeof(C) / 16);
   C *const stage0 = buf0 + WP * N;
-  auto prefetch = [&](int bb, int slot) {
-    const C *src = spec + (int64_t)bb * bstride + (int64_t)other * ostride + kx0;
+  auto prefetch = [&](int b, int slot) {
+    const C *src = tile_base(b);
+    const int rows = boxes[b].in[2];
     C *dst = stage0 + slot * (SROWS * W);
-    for (int c = threadIdx.x; c < in_lim * CPR; c += T) {
+    for (int c = threadIdx.x; c < rows * CPR; c += T) {
       const int e = c / CPR, part = c - e * CPR;
       cp_async16(reinterpret_cast<char *>(dst + e * W) + 16 * part,
                  reinterpret_cast<const char *>(src + (int64_t)e * estride) + 16 * part);
@@ -470,7 +502,12 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_lines(cplx_t<R> *__restrict__ 
     if (b0 < b1) prefetch(b0, 0);
   }
   for (int b = b0, i = 0; b < b1; ++b, ++i) {
-    C *base = spec + (int64_t)b * bstride + (int64_t)other * ostride + kx0;
+    C *const base = tile_base(b);
+    const ConvBox &bx = boxes[b];
+    const int in_lim = CONV ? bx.in[2] : (PASS == kYForward ? bx.in[1] : N);
+    // values [lo, lo + cnt) are written
+    const int lo = CONV ? bx.out0[2] : (PASS == kYInverse ? bx.out0[1] : 0);
+    const unsigned cnt = CONV ? bx.out[2] : (PASS == kYInverse ? bx.out[1] : N);
     C *bA = buf0;
     const C *stg = stage0 + (i & 1) * (SROWS * W);
     if constexpr (CONV) {
@@ -496,11 +533,11 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_lines(cplx_t<R> *__restrict__ 
           if constexpr (CONV) v[q] = (col && e < in_lim) ? stg[e * W + li] : mk<C>(0, 0);
           else v[q] = (col && e < in_lim) ? base[(int64_t)e * estride + li] : mk<C>(0, 0);
         }
-        dft<N1, CONV ? -1 : SIGN>(v);
+        dft<N1, FWD ? -1 : +1>(v);
 #pragma unroll
         for (int k1 = 0; k1 < N1; ++k1) {
           const C w = tw[s * k1];
-          bA[li + WP * (k1 + N1 * s)] = (CONV || SIGN < 0) ? cmul(v[k1], w) : cmulc(v[k1], w);
+          bA[li + WP * (k1 + N1 * s)] = FWD ? cmul(v[k1], w) : cmulc(v[k1], w);
         }
       }
     }
@@ -517,7 +554,7 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_lines(cplx_t<R> *__restrict__ 
         C v[N2];
 #pragma unroll
         for (int s = 0; s < N2; ++s) v[s] = bA[li + WP * (k1 + N1 * s)];
-        dft<N2, CONV ? -1 : SIGN>(v);
+        dft<N2, FWD ? -1 : +1>(v);
         if constexpr (CONV) {
 #pragma unroll
           for (int k2 = 0; k2 < N2; ++k2) {
@@ -532,7 +569,7 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_lines(cplx_t<R> *__restrict__ 
 #pragma unroll
             for (int k2 = 0; k2 < N2; ++k2) {
               const int e = k1 + N1 * k2;
-              if (e < out_lim) base[(int64_t)e * estride + li] = v[k2];
+              if ((unsigned)(e - lo) < cnt) base[(int64_t)e * estride + li] = v[k2];
             }
           }
         }
@@ -554,15 +591,14 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_lines(cplx_t<R> *__restrict__ 
 #pragma unroll
             for (int q = 0; q < N1; ++q) {
               const int e = s + N2 * q;
-              if (e < out_lim) base[(int64_t)e * estride + li] = v[q];
+              if ((unsigned)(e - lo) < cnt) base[(int64_t)e * estride + li] = v[q];
             }
           }
         }
       }
     }
-    // the next halo's stage A rewrites the tile: every thread must have
-    // finished reading it (CONV: the barrier at the top of the loop)
-    if constexpr (!CONV) __syncthreads();
+    // the next grid's stage A rewrites the tile: every thread has finished
+    // reading it at the barrier at the top of the loop
   }
 }
 
@@ -592,47 +628,41 @@ int32_t prepare() {
   std::call_once(once, [] {
     const size_t sm = smem_lines_bytes<R, N>();
     int32_t r = kOk;
-    if (r == kOk) r = allow_smem(k_x_r2c<R, N, false>, sm);
-    if (r == kOk) r = allow_smem(k_x_r2c<R, N, true>, sm);
+    if (r == kOk) r = allow_smem(k_x_r2c<R, N>, sm);
     if (r == kOk) r = allow_smem(k_x_c2r<R, N, N / 2 + 1>, sm);
     if (r == kOk) r = allow_smem(k_x_c2r<R, N, N>, sm);
-    if (r == kOk) r = allow_smem(k_lines<R, N, -1, false>, smem_lines_bytes<R, N>());
-    if (r == kOk) r = allow_smem(k_lines<R, N, +1, false>, smem_lines_bytes<R, N>());
-    if (r == kOk) r = allow_smem(k_lines<R, N, -1, true>, smem_conv_bytes<R, N>());
+    if (r == kOk) r = allow_smem(k_lines<R, N, kYForward>, sm);
+    if (r == kOk) r = allow_smem(k_lines<R, N, kYInverse>, sm);
+    if (r == kOk) r = allow_smem(k_lines<R, N, kZInverse>, sm);
+    if (r == kOk) r = allow_smem(k_lines<R, N, kZConv>, smem_conv_bytes<R, N>());
     status = r;
   });
   return status;
 }
 
 template <typename R, int N>
-int32_t convolve_n(R *rho, cplx_t<R> *spec, const R *green, int sup, int batch, cudaStream_t s,
-                   const unsigned long long *acc, const double *inv_scale, int waves) {
+int32_t convolve_n(const unsigned long long *acc, const double *inv_scale, R *phi, cplx_t<R> *spec, const R *green,
+                   const cplx_t<R> *tw, const ConvBox *boxes, const ConvExtent &ext, int batch, cudaStream_t s,
+                   int waves) {
   PYFOF_TRY((prepare<R, N>()));
   constexpr int W = kW<R>, T = Cfg<R, N>::T;
   const int nhp = (int)spec_row<R>(N);
   const int ntiles = nhp / W;
   const size_t sm = smem_lines_bytes<R, N>();
-  const int64_t bstride = (int64_t)N * N * nhp;
-  const int64_t nlines = (int64_t)batch * sup * sup;
-  if (acc)
-    k_x_r2c<R, N, true><<<(unsigned)ceil_div(nlines, 2 * W), T, sm, s>>>(rho, spec, nhp, (int)nlines, acc,
-                                                                         inv_scale);
-  else
-    k_x_r2c<R, N, false><<<(unsigned)ceil_div(nlines, 2 * W), T, sm, s>>>(rho, spec, nhp, (int)nlines, nullptr,
-                                                                          nullptr);
+  const dim3 gx_in((unsigned)ceil_div(ext.in_lines, 2 * W), (unsigned)batch);
+  const dim3 gx_out((unsigned)ceil_div(ext.out_lines, 2 * W), (unsigned)batch);
+  k_x_r2c<R, N><<<gx_in, T, sm, s>>>(acc, inv_scale, spec, tw, boxes, nhp);
   PYFOF_CHECK_LAUNCH();
-  // y forward: lines (kx, z < sup), input y < sup, output all y
-  k_lines<R, N, -1, false><<<(unsigned)((int64_t)ntiles * sup * batch), T, smem_lines_bytes<R, N>(), s>>>(
-      spec, nullptr, bstride, (int64_t)N * nhp, nhp, sup, ntiles, 1, batch, sup, N);
+  k_lines<R, N, kYForward><<<dim3((unsigned)(ntiles * ext.in_z), (unsigned)batch), T, sm, s>>>(
+      spec, nullptr, tw, boxes, nhp, ntiles, 1, batch);
   PYFOF_CHECK_LAUNCH();
-  // z: forward, Green, inverse; lines (kx, ky), input and output z < sup;
-  // halos split into chunks so that the grid is at least `waves` full waves
+  // z: grids split into chunks so that the launch is at least `waves` full waves
   const int64_t per = (int64_t)ntiles * N;
   static int conv_blocks_per_sm = 0;
   if (!conv_blocks_per_sm) {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_lines<R, N, -1, true>, T,
-                                                      smem_conv_bytes<R, N>()) != cudaSuccess || b < 1)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_lines<R, N, kZConv>, T, smem_conv_bytes<R, N>()) !=
+            cudaSuccess || b < 1)
       b = 1;
     conv_blocks_per_sm = b;
   }
@@ -640,21 +670,20 @@ int32_t convolve_n(R *rho, cplx_t<R> *spec, const R *green, int sup, int batch, 
   const int nchunk = (int)std::max<int64_t>(1, std::min<int64_t>(batch, ceil_div((int64_t)waves * slots, per)));
   const int nbb = (int)ceil_div(batch, nchunk);
   const int nchunk_used = (int)ceil_div(batch, nbb);
-  k_lines<R, N, -1, true><<<(unsigned)(per * nchunk_used), T, smem_conv_bytes<R, N>(), s>>>(
-      spec, green, bstride, nhp, (int64_t)N * nhp, N, ntiles, nbb, batch, sup, sup);
+  k_lines<R, N, kZConv><<<dim3((unsigned)per, (unsigned)nchunk_used), T, smem_conv_bytes<R, N>(), s>>>(
+      spec, green, tw, boxes, nhp, ntiles, nbb, batch);
   PYFOF_CHECK_LAUNCH();
-  // y inverse: lines (kx, z < sup), input all y, output y < sup
-  k_lines<R, N, +1, false><<<(unsigned)((int64_t)ntiles * sup * batch), T, smem_lines_bytes<R, N>(), s>>>(
-      spec, nullptr, bstride, (int64_t)N * nhp, nhp, sup, ntiles, 1, batch, N, sup);
+  k_lines<R, N, kYInverse><<<dim3((unsigned)(ntiles * ext.out_z), (unsigned)batch), T, sm, s>>>(
+      spec, nullptr, tw, boxes, nhp, ntiles, 1, batch);
   PYFOF_CHECK_LAUNCH();
   const R n3 = (R)((double)N * N * N);
-  k_x_c2r<R, N, N / 2 + 1><<<(unsigned)ceil_div(nlines, 2 * W), T, sm, s>>>(spec, rho, nhp, (int)nlines, n3);
+  k_x_c2r<R, N, N / 2 + 1><<<gx_out, T, sm, s>>>(spec, phi, tw, boxes, nhp, n3);
   PYFOF_CHECK_LAUNCH();
   return kOk;
 }
 
 template <typename R, int N>
-int32_t c2r_full_n(const R *green, cplx_t<R> *spec, R *out, cudaStream_t s) {
+int32_t c2r_full_n(const R *green, cplx_t<R> *spec, R *out, const cplx_t<R> *tw, const ConvBox *box, cudaStream_t s) {
   PYFOF_TRY((prepare<R, N>()));
   constexpr int W = kW<R>, T = Cfg<R, N>::T;
   const int nhp = (int)spec_row<R>(N);
@@ -663,16 +692,12 @@ int32_t c2r_full_n(const R *green, cplx_t<R> *spec, R *out, cudaStream_t s) {
   const int64_t cnt = (int64_t)(N / 2 + 1) * N * N;
   k_real_to_cplx<R><<<(unsigned)std::min<int64_t>(ceil_div(cnt, 256), 4096), 256, 0, s>>>(green, spec, N, nhp);
   PYFOF_CHECK_LAUNCH();
-  const int64_t bstride = (int64_t)N * N * nhp;
   // z inverse over all ky, then y inverse over all z
-  k_lines<R, N, +1, false><<<(unsigned)((int64_t)ntiles * N), T, smem_lines_bytes<R, N>(), s>>>(
-      spec, nullptr, bstride, nhp, (int64_t)N * nhp, N, ntiles, 1, 1, N, N);
+  k_lines<R, N, kZInverse><<<(unsigned)(ntiles * N), T, sm, s>>>(spec, nullptr, tw, box, nhp, ntiles, 1, 1);
   PYFOF_CHECK_LAUNCH();
-  k_lines<R, N, +1, false><<<(unsigned)((int64_t)ntiles * N), T, smem_lines_bytes<R, N>(), s>>>(
-      spec, nullptr, bstride, (int64_t)N * nhp, nhp, N, ntiles, 1, 1, N, N);
+  k_lines<R, N, kYInverse><<<(unsigned)(ntiles * N), T, sm, s>>>(spec, nullptr, tw, box, nhp, ntiles, 1, 1);
   PYFOF_CHECK_LAUNCH();
-  const int64_t nlines = (int64_t)N * N;
-  k_x_c2r<R, N, N><<<(unsigned)ceil_div(nlines, 2 * W), T, sm, s>>>(spec, out, nhp, (int)nlines, (R)1);
+  k_x_c2r<R, N, N><<<(unsigned)ceil_div((int64_t)N * N, 2 * W), T, sm, s>>>(spec, out, tw, box, nhp, (R)1);
   PYFOF_CHECK_LAUNCH();
   return kOk;
 }
@@ -680,39 +705,57 @@ int32_t c2r_full_n(const R *green, cplx_t<R> *spec, R *out, cudaStream_t s) {
 }  // namespace
 
 template <typename R>
-int32_t pm_convolve_batch(R *rho, cplx_t<R> *spec, const R *green, int n, int sup, int batch,
-                          cudaStream_t s, const unsigned long long *acc, const double *inv_scale, int waves) {
-  if (sup != n / 2 + 1 || batch < 1 || (int64_t)batch * sup * sup >= (int64_t)1 << 30) {
-    set_error("invalid convolution batch (n %d, support %d, batch %d)", n, sup, batch);
-    return kInvalid;
-  }
-  switch (n) {
-    case 48: return convolve_n<R, 48>(rho, spec, green, sup, batch, s, acc, inv_scale, waves);
-    case 64: return convolve_n<R, 64>(rho, spec, green, sup, batch, s, acc, inv_scale, waves);
-    case 128: return convolve_n<R, 128>(rho, spec, green, sup, batch, s, acc, inv_scale, waves);
-    case 216: return convolve_n<R, 216>(rho, spec, green, sup, batch, s, acc, inv_scale, waves);
-    case 256: return convolve_n<R, 256>(rho, spec, green, sup, batch, s, acc, inv_scale, waves);
-    default: set_error("unsupported FFT size %d", n); return kInvalid;
-  }
+int32_t fill_twiddles(cplx_t<R> *tw, int n, cudaStream_t s) {
+  k_twiddles<R><<<1, 256, 0, s>>>(tw, n);
+  PYFOF_CHECK_LAUNCH();
+  return kOk;
 }
 
 template <typename R>
-int32_t c2r_full(const R *green, cplx_t<R> *spec, R *out, int n, cudaStream_t s) {
+int32_t pm_convolve_batch(const unsigned long long *acc, const double *inv_scale, R *phi, cplx_t<R> *spec,
+                          const R *green, const cplx_t<R> *tw, int n, const ConvBox *boxes, const ConvExtent &ext,
+                          int batch, cudaStream_t s, int waves) {
+  const int sup = n / 2 + 1;
+  if (batch < 1 || batch > 65535 || ext.in_lines < 1 || ext.out_lines < 1 || ext.in_y > sup || ext.in_z > sup ||
+      ext.out_y > sup || ext.out_z > sup) {
+    set_error("invalid convolution batch (n %d, batch %d)", n, batch);
+    return kInvalid;
+  }
+#define PYFOF_CONV(N) return convolve_n<R, N>(acc, inv_scale, phi, spec, green, tw, boxes, ext, batch, s, waves)
   switch (n) {
-    case 48: return c2r_full_n<R, 48>(green, spec, out, s);
-    case 64: return c2r_full_n<R, 64>(green, spec, out, s);
-    case 128: return c2r_full_n<R, 128>(green, spec, out, s);
-    case 216: return c2r_full_n<R, 216>(green, spec, out, s);
-    case 256: return c2r_full_n<R, 256>(green, spec, out, s);
+    case 48: PYFOF_CONV(48);
+    case 64: PYFOF_CONV(64);
+    case 128: PYFOF_CONV(128);
+    case 216: PYFOF_CONV(216);
+    case 256: PYFOF_CONV(256);
+    default: set_error("unsupported FFT size %d", n); return kInvalid;
+  }
+#undef PYFOF_CONV
+}
+
+template <typename R>
+int32_t c2r_full(const R *green, cplx_t<R> *spec, R *out, const cplx_t<R> *tw, const ConvBox *box, int n,
+                 cudaStream_t s) {
+  switch (n) {
+    case 48: return c2r_full_n<R, 48>(green, spec, out, tw, box, s);
+    case 64: return c2r_full_n<R, 64>(green, spec, out, tw, box, s);
+    case 128: return c2r_full_n<R, 128>(green, spec, out, tw, box, s);
+    case 216: return c2r_full_n<R, 216>(green, spec, out, tw, box, s);
+    case 256: return c2r_full_n<R, 256>(green, spec, out, tw, box, s);
     default: set_error("unsupported FFT size %d", n); return kInvalid;
   }
 }
 
-template int32_t pm_convolve_batch<float>(float *, float2 *, const float *, int, int, int, cudaStream_t,
-                                          const unsigned long long *, const double *, int);
-template int32_t pm_convolve_batch<double>(double *, double2 *, const double *, int, int, int, cudaStream_t,
-                                           const unsigned long long *, const double *, int);
-template int32_t c2r_full<float>(const float *, float2 *, float *, int, cudaStream_t);
-template int32_t c2r_full<double>(const double *, double2 *, double *, int, cudaStream_t);
+template int32_t fill_twiddles<float>(float2 *, int, cudaStream_t);
+template int32_t fill_twiddles<double>(double2 *, int, cudaStream_t);
+template int32_t pm_convolve_batch<float>(const unsigned long long *, const double *, float *, float2 *, const float *,
+                                          const float2 *, int, const ConvBox *, const ConvExtent &, int, cudaStream_t,
+                                          int);
+template int32_t pm_convolve_batch<double>(const unsigned long long *, const double *, double *, double2 *,
+                                           const double *, const double2 *, int, const ConvBox *, const ConvExtent &,
+                                           int, cudaStream_t, int);
+template int32_t c2r_full<float>(const float *, float2 *, float *, const float2 *, const ConvBox *, int, cudaStream_t);
+template int32_t c2r_full<double>(const double *, double2 *, double *, const double2 *, const ConvBox *, int,
+                                  cudaStream_t);
 
 }  // namespace pyfof

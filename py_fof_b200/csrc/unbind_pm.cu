@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <memory>
 
 #include "context.cuh"
@@ -128,10 +129,12 @@ struct GreenTable {
   int n = 0;
   void *g = nullptr;     // half-spectrum table (R)
   void *self = nullptr;  // 125 self-kernel values (R), device
+  void *tw = nullptr;    // the transforms' twiddles (complex R), device
   bool fp64 = false;
   ~GreenTable() {
     if (g) cudaFree(g);
     if (self) cudaFree(self);
+    if (tw) cudaFree(tw);
   }
 };
 
@@ -154,21 +157,29 @@ int32_t get_green(Context &ctx, int n, double soft, double range, int truncated,
   cudaStream_t s = ctx.stream;
   PYFOF_CUDA(cudaMalloc(&t->g, sizeof(R) * cnt));
   PYFOF_CUDA(cudaMalloc(&t->self, sizeof(R) * 125));
+  PYFOF_CUDA(cudaMalloc(&t->tw, sizeof(cplx_t<R>) * n));
+  PYFOF_TRY(fill_twiddles<R>((cplx_t<R> *)t->tw, n, s));
   PYFOF_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(int32_t), s));
   green_kernel<R><<<(unsigned)std::min<int64_t>(ceil_div(cnt, 128), 148 * 64), 128, 0, s>>>(
       (R *)t->g, n, soft, range, truncated, ctx.d_flags);
   PYFOF_CHECK_LAUNCH();
   R *grid = nullptr;
   cplx_t<R> *spec = nullptr;
+  ConvBox *dbox = nullptr;
+  ConvBox box{};
+  for (int d = 0; d < 3; ++d) box.in[d] = box.out[d] = n;
   PYFOF_CUDA(cudaMallocAsync(&grid, sizeof(R) * (size_t)n * n * n, s));
-  PYFOF_CUDA(cudaMallocAsync(&spec, sizeof(cplx_t<R>) * spec_elems<R>(n), s));
-  int32_t r = c2r_full<R>((const R *)t->g, spec, grid, n, s);
+  PYFOF_CUDA(cudaMallocAsync(&spec, sizeof(cplx_t<R>) * spec_elems<R>(n, n), s));
+  PYFOF_CUDA(cudaMallocAsync(&dbox, sizeof(ConvBox), s));
+  PYFOF_CUDA(cudaMemcpyAsync(dbox, &box, sizeof(ConvBox), cudaMemcpyHostToDevice, s));
+  int32_t r = c2r_full<R>((const R *)t->g, spec, grid, (const cplx_t<R> *)t->tw, dbox, n, s);
   if (r == kOk) {
     self_extract_kernel<R><<<1, 128, 0, s>>>(grid, n, (R *)t->self);
     PYFOF_CHECK_LAUNCH();
   }
   cudaFreeAsync(grid, s);
   cudaFreeAsync(spec, s);
+  cudaFreeAsync(dbox, s);
   PYFOF_CUDA(cudaMemcpyAsync(ctx.h_flags, ctx.d_flags, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   PYFOF_CUDA(cudaStreamSynchronize(s));
   if (r != kOk) return r;
@@ -186,7 +197,8 @@ int32_t get_green(Context &ctx, int n, double soft, double range, int truncated,
 struct PmHalo {      // device copy of one PM halo's parameters
   int64_t off;       // first member
   int32_t np;
-  int32_t n, sup;    // grid size and support side (n/2+1)
+  int32_t n;         // grid size
+  int32_t sup[3];    // nodes [0, sup) per axis the members' TSC clouds touch
   float spacing;
   float origin[3];
   int64_t cell_off;  // first C2 cell
@@ -308,7 +320,8 @@ __global__ void __launch_bounds__(BLK) pm_extent_kernel(const Members m, const P
 }
 
 __global__ void pm_extent_final_kernel(const PmHalo *__restrict__ H, int nh, const uint32_t *__restrict__ omin,
-                                       const uint32_t *__restrict__ omax, double *__restrict__ ext) {
+                                       const uint32_t *__restrict__ omax, double *__restrict__ ext,
+                                       int32_t *__restrict__ sup) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 3 * nh) return;
   const int h = i / 3, d = i % 3;
@@ -316,8 +329,13 @@ __global__ void pm_extent_final_kernel(const PmHalo *__restrict__ H, int nh, con
   if (p.np <= 0) {
     ext[6 * h + d] = 1e30;
     ext[6 * h + 3 + d] = -1e30;
+    sup[i] = 3;
     return;
   }
+  // the highest node of any member's TSC cloud (pm_setup_kernel's rounding
+  // is monotone in q; members outside the domain are refused there)
+  const float t = __fdiv_rn(__fsub_rn(ord_to_flt(omax[i]), p.origin[d]), p.spacing);
+  sup[i] = t >= 0.0f && t < (float)(p.n / 2 - 1) ? max(3, min((int)lroundf(t) + 2, p.n / 2 + 1)) : p.n / 2 + 1;
   const double sp = (double)p.spacing;
   ext[6 * h + d] = (double)ord_to_flt(omin[i]) / sp;
   ext[6 * h + 3 + d] = (double)ord_to_flt(omax[i]) / sp;
@@ -401,16 +419,6 @@ __device__ __forceinline__ unsigned long long fx_quantum(float v, double scale) 
   return __double2ull_rn((double)v * scale);
 }
 
-// Inverse scale of every grid of a batch: inv[j] = 2^(e - 61) of the halo
-// that owns grid j (its region's halo for refined regions, A != nullptr).
-__global__ void pm_batch_scale_kernel(const PmHalo *__restrict__ H, const int32_t *__restrict__ batch, int nb,
-                                      const TlRegion *__restrict__ A, double *__restrict__ inv) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nb; j += gridDim.x * blockDim.x) {
-    const int h = A ? A[batch[j]].h : batch[j];
-    inv[j] = scalbn(1.0, fx_exp(H[h].mkeep) - 61);
-  }
-}
-
 // Last entry e0 of the ascending array off[0..n] with off[e0] <= idx.
 __device__ __forceinline__ int seg_of(const uint32_t *__restrict__ off, int n, uint32_t idx) {
   int lo = 0, hi = n;  // off[lo] <= idx < off[hi]
@@ -423,18 +431,22 @@ __device__ __forceinline__ int seg_of(const uint32_t *__restrict__ off, int n, u
 }
 
 // Deposit of the kept members of a batch of halos (batch[j] = halo of
-// grid j, bpre = prefix of their member counts), flat over the batch's
-// members in their stored order (coalesced member reads).  Each of a
-// member's 27 contributions is one 64-bit integer atomic add.
+// grid j, boxes[j] its support box, bpre = prefix of their member counts),
+// flat over the batch's members in their stored order (coalesced member
+// reads).  Each of a member's 27 contributions is one 64-bit integer atomic
+// add.  Block 0 also writes the grids' inverse scales inv[j] = 2^(e - 61).
 __global__ void __launch_bounds__(BLK) pm_deposit_kernel(const Members m, const PmHalo *__restrict__ H,
+                                                         const ConvBox *__restrict__ boxes,
                                                          const int32_t *__restrict__ batch,
                                                          const uint32_t *__restrict__ bpre, int nb,
                                                          const uint8_t *__restrict__ keep,
                                                          const int3 *__restrict__ first,
-                                                         const float *__restrict__ wt, int sup,
-                                                         unsigned long long *__restrict__ acc) {
+                                                         const float *__restrict__ wt,
+                                                         unsigned long long *__restrict__ acc,
+                                                         double *__restrict__ inv) {
+  if (blockIdx.x == 0)
+    for (int j = threadIdx.x; j < nb; j += blockDim.x) inv[j] = scalbn(1.0, fx_exp(H[batch[j]].mkeep) - 61);
   const uint32_t total = bpre[nb];
-  const int64_t sup3 = (int64_t)sup * sup * sup;
   for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
     const int j = seg_of(bpre, nb, idx);
     const PmHalo &p = H[batch[j]];
@@ -444,13 +456,13 @@ __global__ void __launch_bounds__(BLK) pm_deposit_kernel(const Members m, const 
     const int3 f = first[k];
     const float *w9 = wt + 9 * k;
     const float wk = m.w[k];
-    unsigned long long *g = acc + (int64_t)j * sup3;
+    const int nx = boxes[j].in[0], ny = boxes[j].in[1];
+    unsigned long long *g = acc + boxes[j].in_off + (((int64_t)(f.z - 1) * ny + (f.y - 1)) * nx + (f.x - 1));
     for (int sz = 0; sz < 3; ++sz)
       for (int sy = 0; sy < 3; ++sy)
         for (int sx = 0; sx < 3; ++sx) {
           const float v = __fmul_rn(__fmul_rn(__fmul_rn(wk, w9[sx]), w9[3 + sy]), w9[6 + sz]);
-          atomicAdd(&g[((int64_t)(f.z + sz - 1) * sup + (f.y + sy - 1)) * sup + (f.x + sx - 1)],
-                    fx_quantum(v, sc));
+          atomicAdd(&g[((int64_t)sz * ny + sy) * nx + sx], fx_quantum(v, sc));
         }
   }
 }
@@ -458,10 +470,10 @@ __global__ void __launch_bounds__(BLK) pm_deposit_kernel(const Members m, const 
 // TSC gather and the C1 potential (bound_fortran.f90:2681-2703) at the kept
 // members of a batch; grid j holds the potential of halo batch[j].
 template <typename R>
-__global__ void pm_gather_kernel(const Members m, const PmHalo *__restrict__ H,
+__global__ void pm_gather_kernel(const Members m, const PmHalo *__restrict__ H, const ConvBox *__restrict__ boxes,
                                  const int32_t *__restrict__ batch, const uint32_t *__restrict__ bpre, int nb,
                                  const uint8_t *__restrict__ keep, const int3 *__restrict__ first,
-                                 const float *__restrict__ wt, const R *__restrict__ selfv, int sup,
+                                 const float *__restrict__ wt, const R *__restrict__ selfv,
                                  const R *__restrict__ rho, double a_val, R *__restrict__ phi_c1) {
   const uint32_t total = bpre[nb];
   for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
@@ -469,20 +481,15 @@ __global__ void pm_gather_kernel(const Members m, const PmHalo *__restrict__ H,
     const PmHalo &p = H[batch[j]];
     const int64_t k = p.off + (idx - bpre[j]);
     if (!keep[k]) continue;
-    const R *g = rho + (int64_t)j * sup * sup * sup;
     const int3 f = first[k];
+    const int nx = boxes[j].out[0], ny = boxes[j].out[1];  // the window starts at node 0
+    const R *g = rho + boxes[j].out_off + (((int64_t)(f.z - 1) * ny + (f.y - 1)) * nx + (f.x - 1));
     const float *w9 = wt + 9 * k;
     R raw = 0;
-    for (int sz = 0; sz < 3; ++sz) {
-      const int z = f.z + sz - 1;
-      for (int sy = 0; sy < 3; ++sy) {
-        const int y = f.y + sy - 1;
-        for (int sx = 0; sx < 3; ++sx) {
-          const int x = f.x + sx - 1;
-          raw += g[((int64_t)z * sup + y) * sup + x] * (R)w9[sx] * (R)w9[3 + sy] * (R)w9[6 + sz];
-        }
-      }
-    }
+    for (int sz = 0; sz < 3; ++sz)
+      for (int sy = 0; sy < 3; ++sy)
+        for (int sx = 0; sx < 3; ++sx)
+          raw += g[((int64_t)sz * ny + sy) * nx + sx] * (R)w9[sx] * (R)w9[3 + sy] * (R)w9[6 + sz];
     const R wk = (R)m.w[k];
     const double rest = p.mkeep - (double)m.w[k];
     const R radius = (R)p.n / (R)2;
@@ -1125,11 +1132,13 @@ __global__ void tl_self_kernel(const Members m, const PmHalo *__restrict__ H,
 // Inner PM of a batch of refined regions of one inner grid size
 // (bound_two_level_run_pm, :825-942): deposit of the kept sources ...
 __global__ void tl_deposit_kernel(const Members m, const PmHalo *__restrict__ H,
-                                  const TlRegion *__restrict__ A, const int32_t *__restrict__ batch,
-                                  const uint32_t *__restrict__ bpre, int nb,
+                                  const TlRegion *__restrict__ A, const ConvBox *__restrict__ boxes,
+                                  const int32_t *__restrict__ batch, const uint32_t *__restrict__ bpre, int nb,
                                   const uint32_t *__restrict__ src_start, const uint32_t *__restrict__ src,
-                                  const uint8_t *__restrict__ keep, int sup,
-                                  unsigned long long *__restrict__ acc) {
+                                  const uint8_t *__restrict__ keep, unsigned long long *__restrict__ acc,
+                                  double *__restrict__ inv) {
+  if (blockIdx.x == 0)
+    for (int j = threadIdx.x; j < nb; j += blockDim.x) inv[j] = scalbn(1.0, fx_exp(H[A[batch[j]].h].mkeep) - 61);
   // flat over the sources of the batch: bpre[j] = first index of region j;
   // fixed-point integer adds as pm_deposit_kernel (order-independent)
   const uint32_t total = bpre[nb];
@@ -1140,19 +1149,19 @@ __global__ void tl_deposit_kernel(const Members m, const PmHalo *__restrict__ H,
     const PmHalo &p = H[Rg.h];
     const int64_t k = src[src_start[a] + (idx - bpre[j])];
     if (!keep[k]) continue;
-    unsigned long long *g = acc + (int64_t)j * sup * sup * sup;
     const double sc = scalbn(1.0, 61 - fx_exp(p.mkeep));
     float t[3], w9[9];
     int f[3];
     tl_t(m, p, k, t);
     tl_tsc(Rg, t, f, w9);
     const float wk = m.w[k];
+    const int nx = boxes[j].in[0], ny = boxes[j].in[1];
+    unsigned long long *g = acc + boxes[j].in_off + (((int64_t)(f[2] - 1) * ny + (f[1] - 1)) * nx + (f[0] - 1));
     for (int sz = 0; sz < 3; ++sz)
       for (int sy = 0; sy < 3; ++sy)
         for (int sx = 0; sx < 3; ++sx) {
           const float v = __fmul_rn(__fmul_rn(__fmul_rn(wk, w9[sx]), w9[3 + sy]), w9[6 + sz]);
-          atomicAdd(&g[((int64_t)(f[2] + sz - 1) * sup + (f[1] + sy - 1)) * sup + (f[0] + sx - 1)],
-                    fx_quantum(v, sc));
+          atomicAdd(&g[((int64_t)sz * ny + sy) * nx + sx], fx_quantum(v, sc));
         }
   }
 }
@@ -1160,10 +1169,10 @@ __global__ void tl_deposit_kernel(const Members m, const PmHalo *__restrict__ H,
 // ... and gather at the kept targets: phi_in = a r/(6 pi sp) (raw - w self_in)
 template <typename R>
 __global__ void tl_gather_kernel(const Members m, const PmHalo *__restrict__ H,
-                                 const TlRegion *__restrict__ A, const int32_t *__restrict__ batch,
-                                 const uint32_t *__restrict__ bpre, int nb,
+                                 const TlRegion *__restrict__ A, const ConvBox *__restrict__ boxes,
+                                 const int32_t *__restrict__ batch, const uint32_t *__restrict__ bpre, int nb,
                                  const uint32_t *__restrict__ tgt_start, const uint32_t *__restrict__ tgt,
-                                 const uint8_t *__restrict__ keep, const R *__restrict__ self_in, int sup,
+                                 const uint8_t *__restrict__ keep, const R *__restrict__ self_in,
                                  const R *__restrict__ rho, double a_val, R *__restrict__ phi_in) {
   const uint32_t total = bpre[nb];
   for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
@@ -1173,18 +1182,20 @@ __global__ void tl_gather_kernel(const Members m, const PmHalo *__restrict__ H,
     const PmHalo &p = H[Rg.h];
     const int64_t k = tgt[tgt_start[a] + (idx - bpre[j])];
     if (!keep[k]) continue;
-    const R *g = rho + (int64_t)j * sup * sup * sup;
     const R pref = (R)(a_val * (double)Rg.r / (6.0 * kPi * (double)p.spacing));
     float t[3], w9[9];
     int f[3];
     tl_t(m, p, k, t);
     tl_tsc(Rg, t, f, w9);
+    const ConvBox &bx = boxes[j];
+    const int nx = bx.out[0], ny = bx.out[1];
+    const R *g = rho + bx.out_off +
+                 (((int64_t)(f[2] - 1 - bx.out0[2]) * ny + (f[1] - 1 - bx.out0[1])) * nx + (f[0] - 1 - bx.out0[0]));
     R raw = 0;
     for (int sz = 0; sz < 3; ++sz)
       for (int sy = 0; sy < 3; ++sy)
         for (int sx = 0; sx < 3; ++sx)
-          raw += g[((int64_t)(f[2] + sz - 1) * sup + (f[1] + sy - 1)) * sup + (f[0] + sx - 1)] *
-                 (R)w9[sx] * (R)w9[3 + sy] * (R)w9[6 + sz];
+          raw += g[((int64_t)sz * ny + sy) * nx + sx] * (R)w9[sx] * (R)w9[3 + sy] * (R)w9[6 + sz];
     phi_in[k] = pref * (raw - (R)m.w[k] * self_in[k]);
   }
 }
@@ -1720,10 +1731,24 @@ __global__ void pm_mkeep_kernel(const Members m, PmHalo *__restrict__ H, const i
   if (threadIdx.x == 0) p.mkeep = s;
 }
 
-__global__ void pm_mark_halo_kernel(const PmHalo *__restrict__ H, int nh, int32_t *__restrict__ mhalo) {
+// Members of every PM halo: their halo, and kept.
+__global__ void pm_mark_halo_kernel(const PmHalo *__restrict__ H, int nh, int32_t *__restrict__ mhalo,
+                                    uint8_t *__restrict__ keep) {
   const int h = blockIdx.x;
   if (h >= nh) return;
-  for (int64_t i = threadIdx.x; i < H[h].np; i += blockDim.x) mhalo[H[h].off + i] = h;
+  for (int64_t i = threadIdx.x; i < H[h].np; i += blockDim.x) {
+    mhalo[H[h].off + i] = h;
+    keep[H[h].off + i] = 1;
+  }
+}
+
+// Results of the PM halos into the candidates' table.
+__global__ void pm_result_kernel(const PmHalo *__restrict__ H, const int32_t *__restrict__ cand, int nh,
+                                 HaloResult *__restrict__ res) {
+  const int h = blockIdx.x * blockDim.x + threadIdx.x;
+  if (h >= nh) return;
+  res[cand[h]].status = H[h].pending ? 5 : H[h].status;
+  res[cand[h]].np_bound = H[h].np_bound;
 }
 
 __global__ void pm_fill_i32(int32_t *a, int64_t n, int32_t v) {
@@ -1827,7 +1852,6 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
     p.off = t.off;
     p.np = t.np;
     p.n = t.n;
-    p.sup = t.n / 2 + 1;
     p.spacing = t.spacing;
     for (int d = 0; d < 3; ++d) p.origin[d] = t.origin[d];
     p.np_bound = t.np;
@@ -1848,26 +1872,21 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   uint32_t *epos = W.carve<uint32_t>(M);  // positions in cell order (PM members)
   if (!epos) { set_error("workspace exhausted (cell positions)"); return kAlloc; }
   double *ext = W.carve<double>(6 * (size_t)nh);
-  if (!dH || !dlist || !dselfs || !mhalo || !first || !wt || !selfv || !c1 || !c2 || !phi || !en || !ext) {
+  int32_t *dsup = W.carve<int32_t>(3 * (size_t)nh);
+  if (!dH || !dlist || !dselfs || !mhalo || !first || !wt || !selfv || !c1 || !c2 || !phi || !en || !ext || !dsup) {
     set_error("workspace exhausted (PM members)");
     return kAlloc;
   }
-  std::vector<int32_t> hl(nh);
-  for (int h = 0; h < nh; ++h) hl[h] = h;
   PYFOF_TRY(upload(ctx, dH, H.data(), sizeof(PmHalo) * nh, s));
-  PYFOF_TRY(upload(ctx, dlist, hl.data(), sizeof(int32_t) * nh, s));
+  PYFOF_TRY(upload(ctx, dlist, list.data(), sizeof(int32_t) * nh, s));
   PYFOF_TRY(upload(ctx, dselfs, selfs.data(), sizeof(R *) * nh, s));
   const unsigned gM = (unsigned)std::min<int64_t>(ceil_div(M, BLK), (int64_t)kNumSMs * 16);
   pm_fill_i32<<<gM, BLK, 0, s>>>(mhalo, M, -1);
   PYFOF_CHECK_LAUNCH();
-  pm_mark_halo_kernel<<<nh, BLK, 0, s>>>(dH, nh, mhalo);
+  pm_mark_halo_kernel<<<nh, BLK, 0, s>>>(dH, nh, mhalo, keep);
   PYFOF_CHECK_LAUNCH();
   pm_setup_kernel<R><<<gM, BLK, 0, s>>>(m, dH, mhalo, M, dselfs, first, wt, selfv, ctx.d_flags);
   PYFOF_CHECK_LAUNCH();
-  // mark PM members kept
-  for (int h = 0; h < nh; ++h) {
-    PYFOF_CUDA(cudaMemsetAsync(keep + H[h].off, 1, (size_t)H[h].np, s));
-  }
   // two-level refinement of dense 16-cell regions of 256-grid halos
   // (bound_two_level_setup_ratios / build_halo, bound_fortran.f90:551-823)
   std::vector<TlRegion> act;
@@ -1936,11 +1955,14 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
       pm_extent_kernel<<<(unsigned)work.size(), BLK, 0, s>>>(m, dH, dwork, omin, omax);
       PYFOF_CHECK_LAUNCH();
     }
-    pm_extent_final_kernel<<<(unsigned)ceil_div(3 * (int64_t)nh, 128), 128, 0, s>>>(dH, nh, omin, omax, ext);
+    pm_extent_final_kernel<<<(unsigned)ceil_div(3 * (int64_t)nh, 128), 128, 0, s>>>(dH, nh, omin, omax, ext,
+                                                                                       dsup);
     PYFOF_CHECK_LAUNCH();
   }
   std::vector<double> hext(6 * (size_t)nh);
+  std::vector<int32_t> hsup(3 * (size_t)nh);
   PYFOF_CUDA(cudaMemcpyAsync(hext.data(), ext, sizeof(double) * 6 * nh, cudaMemcpyDeviceToHost, s));
+  PYFOF_CUDA(cudaMemcpyAsync(hsup.data(), dsup, sizeof(int32_t) * 3 * nh, cudaMemcpyDeviceToHost, s));
   PYFOF_CUDA(cudaStreamSynchronize(s));
   int64_t ncell = 0;
   for (int h = 0; h < nh; ++h) {
@@ -1950,6 +1972,7 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
     int64_t c = 1;
     for (int d = 0; d < 3; ++d) {
       p.u_min[d] = hext[6 * h + d];
+      p.sup[d] = hsup[3 * h + d];
       const double span = hext[6 * h + 3 + d] - hext[6 * h + d];
       p.nc[d] = std::max(1, (int)std::floor(span / p.cw_u) + 1);
       c *= 4 * (((int64_t)p.nc[d] + 3) / 4);  // whole bricks of 4^3 cells
@@ -2111,41 +2134,130 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   // sized for the largest batch, serves every batch of every pass
   const size_t budget = ctx.pm_budget;
   auto round256 = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  // per grid: the fixed-point deposit grid (8 B a node; the convolved
-  // potential, R, is written back over it) and the half spectrum
-  auto batch_bytes = [&](int n, int nb) {
-    const size_t sup = n / 2 + 1;
-    return round256(sizeof(unsigned long long) * nb * sup * sup * sup) +
-           sizeof(cplx_t<R>) * (size_t)nb * spec_elems<R>(n);
-  };
-  auto max_batch = [&](int n) {
-    const int by_budget = (int)std::max<size_t>(1, budget / batch_bytes(n, 1));
-    const int cap = a.tiles.pm_batch[kGridIndex(n)];
-    return cap > 0 ? std::min(cap, by_budget) : by_budget;
-  };
   auto waves = [&](int n) { return a.tiles.conv_waves[kGridIndex(n)]; };
+  // the box of a halo's own grid, and of a region's inner grid: its sources
+  // lie within 3.5 + 3/r grid cells of the region, its targets inside it
+  // (tl_source_kernel, tl_particle_kernel), one node of slack each side
+  auto halo_box = [&](int h) {
+    ConvBox b{};
+    for (int d = 0; d < 3; ++d) b.in[d] = b.out[d] = H[h].sup[d];
+    return b;
+  };
+  auto region_box = [&](int ia) {
+    const TlRegion &Rg = act[ia];
+    ConvBox b{};
+    for (int d = 0; d < 3; ++d) {
+      b.in[d] = std::min(Rg.n_in / 2 + 1, (int)((16.0f + 2.0f * Rg.bo) * Rg.r + 1.0f) + 3);
+      b.out0[d] = (int)(Rg.bo * Rg.r + 1.0f) - 2;
+      b.out[d] = 16 * Rg.r + 5;
+    }
+    return b;
+  };
+  // bytes of a grid: the fixed-point deposit nodes (8 B each; the convolved
+  // potential, R, is written back over them) and the half spectrum
+  auto acc_bytes = [&](const ConvBox &b) {
+    return round256(sizeof(unsigned long long) * b.in[0] * (size_t)b.in[1] * b.in[2]);
+  };
+  auto spec_bytes = [&](int n, const ConvBox &b) { return sizeof(cplx_t<R>) * (size_t)spec_elems<R>(n, b.in[2]); };
   size_t scratch_bytes = 256;
-  for (int n : {48, 64, 128, 256}) {
-    int cnt = 0;
-    for (int h = 0; h < nh; ++h) cnt += H[h].n == n;
-    if (cnt) scratch_bytes = std::max(scratch_bytes, batch_bytes(n, std::min(cnt, max_batch(n))));
-  }
-  for (int r : {2, 4}) {
-    int cnt = 0;
-    for (int ia = 0; ia < na; ++ia) cnt += act[ia].r == r;
-    const int nin = r == 2 ? 128 : 216;
-    if (cnt) scratch_bytes = std::max(scratch_bytes, batch_bytes(nin, std::min(cnt, max_batch(nin))));
+  int64_t nbat = 1;
+  {
+    std::vector<size_t> sizes;
+    auto room = [&](int n) {
+      if (sizes.empty()) return;
+      std::sort(sizes.begin(), sizes.end(), std::greater<size_t>());
+      const int cap = a.tiles.pm_batch[kGridIndex(n)];
+      size_t need = 0;
+      for (size_t i = 0; i < sizes.size() && (cap <= 0 || i < (size_t)cap); ++i) need += sizes[i];
+      scratch_bytes = std::max(scratch_bytes, std::min(need, std::max(budget, sizes[0])));
+      nbat = std::max<int64_t>(nbat, (int64_t)sizes.size());
+    };
+    for (int n : {48, 64, 128, 256}) {
+      sizes.clear();
+      for (int h = 0; h < nh; ++h)
+        if (H[h].n == n) {
+          const ConvBox b = halo_box(h);
+          sizes.push_back(acc_bytes(b) + spec_bytes(n, b));
+        }
+      room(n);
+    }
+    for (int n : {128, 216}) {
+      sizes.clear();
+      for (int ia = 0; ia < na; ++ia)
+        if (act[ia].n_in == n) {
+          const ConvBox b = region_box(ia);
+          sizes.push_back(acc_bytes(b) + spec_bytes(n, b));
+        }
+      room(n);
+    }
   }
   unsigned char *scratch = W.carve<unsigned char>(scratch_bytes);
   int32_t *dpend = W.carve<int32_t>(nh);
-  const int nbat = std::max(std::max(na, nh), 1);
-  int32_t *dbatch = W.carve<int32_t>(nbat);
-  uint32_t *dbpre = W.carve<uint32_t>(2 * (size_t)(nbat + 1));
+  // a batch's tables, uploaded together: boxes, ids, member prefixes
+  unsigned char *dmeta = W.carve<unsigned char>((size_t)nbat * (sizeof(ConvBox) + 12) + 64);
   double *dinv = W.carve<double>(nbat);
-  if (!scratch || !dpend || !dbatch || !dbpre || !dinv) {
+  if (!scratch || !dpend || !dmeta || !dinv) {
     set_error("workspace exhausted (PM grids)");
     return kAlloc;
   }
+  struct Batch {
+    std::vector<int32_t> ids;
+    std::vector<ConvBox> boxes;
+    ConvExtent ext;
+    size_t acc = 0, spec = 0;  // bytes
+    const ConvBox *dbox;
+    const int32_t *did;
+    const uint32_t *dpre0, *dpre1;
+    uint32_t n0, n1;  // members: sources and targets (the same for a halo's own grid)
+  };
+  // takes grids from items[at..] while they fit, and uploads the tables
+  std::vector<unsigned char> meta;
+  auto next_batch = [&](const std::vector<int32_t> &items, size_t &at, int n, bool region, Batch &B) -> int32_t {
+    B = Batch();
+    const int cap = a.tiles.pm_batch[kGridIndex(n)];
+    std::vector<uint32_t> p0(1, 0), p1(1, 0);
+    for (; at < items.size() && (cap <= 0 || (int)B.ids.size() < cap) && B.ids.size() < 65535; ++at) {
+      ConvBox b = region ? region_box(items[at]) : halo_box(items[at]);
+      const size_t ab = acc_bytes(b), sb = spec_bytes(n, b);
+      if (!B.ids.empty() && B.acc + B.spec + ab + sb > scratch_bytes) break;
+      b.in_off = (int64_t)(B.acc / sizeof(unsigned long long));
+      b.out_off = (int64_t)(B.acc / sizeof(R));
+      b.spec_off = (int64_t)(B.spec / sizeof(cplx_t<R>));
+      B.acc += ab;
+      B.spec += sb;
+      B.ext.add(b);
+      ctx.last_pm_fft_bytes += conv_bytes<R>(n, b);
+      B.ids.push_back(items[at]);
+      B.boxes.push_back(b);
+      if (region) {
+        p0.push_back(p0.back() + (hsrc[items[at] + 1] - hsrc[items[at]]));
+        p1.push_back(p1.back() + (htgt[items[at] + 1] - htgt[items[at]]));
+      } else {
+        p0.push_back(p0.back() + (uint32_t)H[items[at]].np);
+      }
+    }
+    const size_t nb = B.ids.size(), ob = sizeof(ConvBox) * nb, oi = ob + 4 * nb, op = oi + 4 * (nb + 1);
+    meta.resize(op + (region ? 4 * (nb + 1) : 0));
+    std::memcpy(meta.data(), B.boxes.data(), ob);
+    std::memcpy(meta.data() + ob, B.ids.data(), 4 * nb);
+    std::memcpy(meta.data() + oi, p0.data(), 4 * (nb + 1));
+    if (region) std::memcpy(meta.data() + op, p1.data(), 4 * (nb + 1));
+    PYFOF_TRY(upload(ctx, dmeta, meta.data(), meta.size(), s));
+    B.dbox = reinterpret_cast<const ConvBox *>(dmeta);
+    B.did = reinterpret_cast<const int32_t *>(dmeta + ob);
+    B.dpre0 = reinterpret_cast<const uint32_t *>(dmeta + oi);
+    B.dpre1 = region ? reinterpret_cast<const uint32_t *>(dmeta + op) : B.dpre0;
+    B.n0 = p0.back();
+    B.n1 = region ? p1.back() : p0.back();
+    ctx.last_pm_solves += (int64_t)nb;
+    PYFOF_CUDA(cudaMemsetAsync(scratch, 0, B.acc, s));
+    return kOk;
+  };
+  auto flat_grid = [&](uint32_t n) {
+    return (unsigned)std::min<int64_t>(ceil_div(std::max<uint32_t>(n, 1), BLK), 148 * 16);
+  };
+  unsigned long long *const acc = reinterpret_cast<unsigned long long *>(scratch);
+  R *const rho = reinterpret_cast<R *>(scratch);  // the convolved grids overwrite acc
   // halos above kBigNp members: chunked removal loop
   std::vector<BigHalo> hbig;
   std::vector<BigChunk> hch;
@@ -2206,36 +2318,26 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
       big_mass_sum_kernel<<<(unsigned)ceil_div(nbig, 128), 128, 0, s>>>(dB, nbig, bpart, dH);
       PYFOF_CHECK_LAUNCH();
     }
+    Batch B;
     for (int n : {48, 64, 128, 256}) {
       std::vector<int32_t> grp;
       for (int h : pend) if (H[h].n == n) grp.push_back(h);
-      if (grp.empty()) continue;
-      const int sup = n / 2 + 1;
-      const int maxb = max_batch(n);
-      for (size_t g0 = 0; g0 < grp.size(); g0 += maxb) {
-        const int nb = (int)std::min<size_t>(maxb, grp.size() - g0);
-        // the batch's halos, their member prefix and their first cmem position
-        std::vector<uint32_t> bp((size_t)nb + 1, 0);
-        for (int j = 0; j < nb; ++j) bp[j + 1] = bp[j] + (uint32_t)H[grp[g0 + j]].np;
-        PYFOF_TRY(upload(ctx, dbatch, grp.data() + g0, sizeof(int32_t) * nb, s));
-        PYFOF_TRY(upload(ctx, dbpre, bp.data(), sizeof(uint32_t) * (nb + 1), s));
-        unsigned long long *acc = reinterpret_cast<unsigned long long *>(scratch);
-        R *rho = reinterpret_cast<R *>(scratch);  // the convolved grids overwrite acc
-        cplx_t<R> *spec = reinterpret_cast<cplx_t<R> *>(
-            scratch + round256(sizeof(unsigned long long) * (size_t)nb * sup * sup * sup));
-        const int64_t ng = (int64_t)nb * sup * sup * sup;
-        PYFOF_CUDA(cudaMemsetAsync(acc, 0, sizeof(unsigned long long) * ng, s));
-        pm_batch_scale_kernel<<<(unsigned)ceil_div(nb, 128), 128, 0, s>>>(dH, dbatch, nb, nullptr, dinv);
-        PYFOF_CHECK_LAUNCH();
-        const unsigned gb = (unsigned)std::min<int64_t>(ceil_div(std::max<uint32_t>(bp[nb], 1), BLK), 148 * 16);
-        pm_deposit_kernel<<<gb, BLK, 0, s>>>(m, dH, dbatch, dbpre, nb, keep, first, wt, sup, acc);
+      // boxes of similar size together: a launch is shaped by the largest
+      std::stable_sort(grp.begin(), grp.end(), [&](int x, int y) {
+        return (int64_t)H[x].sup[1] * H[x].sup[2] > (int64_t)H[y].sup[1] * H[y].sup[2];
+      });
+      for (size_t at = 0; at < grp.size();) {
+        PYFOF_TRY(next_batch(grp, at, n, false, B));
+        const int nb = (int)B.ids.size();
+        const unsigned gb = flat_grid(B.n0);
+        pm_deposit_kernel<<<gb, BLK, 0, s>>>(m, dH, B.dbox, B.did, B.dpre0, nb, keep, first, wt, acc, dinv);
         PYFOF_CHECK_LAUNCH();
         if (ctx.timing) ctx.conv_timer.begin(s);
-        PYFOF_TRY(pm_convolve_batch<R>(rho, spec, (const R *)green_of[n]->g, n, sup, nb, s, acc, dinv, waves(n)));
+        PYFOF_TRY(pm_convolve_batch<R>(acc, dinv, rho, reinterpret_cast<cplx_t<R> *>(scratch + B.acc),
+                                       (const R *)green_of[n]->g, (const cplx_t<R> *)green_of[n]->tw, n, B.dbox,
+                                       B.ext, nb, s, waves(n)));
         if (ctx.timing) ctx.conv_timer.end(s);
-        ctx.last_pm_solves += nb;
-        ctx.last_pm_fft_bytes += 4.0 * sizeof(R) * nb * (n + 2.0) * n * n;
-        pm_gather_kernel<R><<<gb, BLK, 0, s>>>(m, dH, dbatch, dbpre, nb, keep, first, wt, selfv, sup, rho,
+        pm_gather_kernel<R><<<gb, BLK, 0, s>>>(m, dH, B.dbox, B.did, B.dpre0, nb, keep, first, wt, selfv, rho,
                                                a.a_val, c1);
         PYFOF_CHECK_LAUNCH();
       }
@@ -2245,42 +2347,21 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
       std::vector<int32_t> regs;
       for (int ia = 0; ia < na; ++ia)
         if (act[ia].r == r && H[act[ia].h].pending) regs.push_back(ia);
-      if (regs.empty()) continue;
       const int nin = r == 2 ? 128 : 216;
-      const int sup = nin / 2 + 1;
-      const int maxb = max_batch(nin);
-      const R *gin = (const R *)(r == 2 ? g_r2 : g_r4)->g;
-      for (size_t g0 = 0; g0 < regs.size(); g0 += maxb) {
-        const int nb = (int)std::min<size_t>(maxb, regs.size() - g0);
-        unsigned long long *acc = reinterpret_cast<unsigned long long *>(scratch);
-        R *rho = reinterpret_cast<R *>(scratch);  // the convolved grids overwrite acc
-        cplx_t<R> *spec = reinterpret_cast<cplx_t<R> *>(
-            scratch + round256(sizeof(unsigned long long) * (size_t)nb * sup * sup * sup));
-        // prefix counts of the batch's sources and targets (flat launches)
-        std::vector<uint32_t> bp(2 * (size_t)(nb + 1), 0);
-        for (int j = 0; j < nb; ++j) {
-          const int ia = regs[g0 + j];
-          bp[j + 1] = bp[j] + (hsrc[ia + 1] - hsrc[ia]);
-          bp[nb + 1 + j + 1] = bp[nb + 1 + j] + (htgt[ia + 1] - htgt[ia]);
-        }
-        PYFOF_TRY(upload(ctx, dbatch, regs.data() + g0, sizeof(int32_t) * nb, s));
-        PYFOF_TRY(upload(ctx, dbpre, bp.data(), sizeof(uint32_t) * bp.size(), s));
-        const int64_t ng = (int64_t)nb * sup * sup * sup;
-        PYFOF_CUDA(cudaMemsetAsync(acc, 0, sizeof(unsigned long long) * ng, s));
-        pm_batch_scale_kernel<<<(unsigned)ceil_div(nb, 128), 128, 0, s>>>(dH, dbatch, nb, dA, dinv);
-        PYFOF_CHECK_LAUNCH();
-        const unsigned gd = (unsigned)std::min<int64_t>(ceil_div(std::max<uint32_t>(bp[nb], 1), BLK), 148 * 16);
-        tl_deposit_kernel<<<gd, BLK, 0, s>>>(m, dH, dA, dbatch, dbpre, nb, src_start, src, keep, sup, acc);
+      const GreenTable *gin = (r == 2 ? g_r2 : g_r4).get();
+      for (size_t at = 0; at < regs.size();) {
+        PYFOF_TRY(next_batch(regs, at, nin, true, B));
+        const int nb = (int)B.ids.size();
+        tl_deposit_kernel<<<flat_grid(B.n0), BLK, 0, s>>>(m, dH, dA, B.dbox, B.did, B.dpre0, nb, src_start, src,
+                                                          keep, acc, dinv);
         PYFOF_CHECK_LAUNCH();
         if (ctx.timing) ctx.conv_timer.begin(s);
-        PYFOF_TRY(pm_convolve_batch<R>(rho, spec, gin, nin, sup, nb, s, acc, dinv, waves(nin)));
+        PYFOF_TRY(pm_convolve_batch<R>(acc, dinv, rho, reinterpret_cast<cplx_t<R> *>(scratch + B.acc),
+                                       (const R *)gin->g, (const cplx_t<R> *)gin->tw, nin, B.dbox, B.ext, nb, s,
+                                       waves(nin)));
         if (ctx.timing) ctx.conv_timer.end(s);
-        ctx.last_pm_solves += nb;
-        ctx.last_pm_fft_bytes += 4.0 * sizeof(R) * nb * (nin + 2.0) * nin * nin;
-        const unsigned gg = (unsigned)std::min<int64_t>(
-            ceil_div(std::max<uint32_t>(bp[2 * nb + 1], 1), BLK), 148 * 16);
-        tl_gather_kernel<R><<<gg, BLK, 0, s>>>(m, dH, dA, dbatch, dbpre + nb + 1, nb, tgt_start, tgt, keep,
-                                               tl_self_in, sup, rho, a.a_val, phi_in);
+        tl_gather_kernel<R><<<flat_grid(B.n1), BLK, 0, s>>>(m, dH, dA, B.dbox, B.did, B.dpre1, nb, tgt_start, tgt,
+                                                            keep, tl_self_in, rho, a.a_val, phi_in);
         PYFOF_CHECK_LAUNCH();
       }
     }
@@ -2321,13 +2402,8 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
       return ctx.h_flags[FLAG_ERR];
     }
   }
-  std::vector<HaloResult> hr(nh);
-  for (int h = 0; h < nh; ++h) {
-    hr[h].status = H[h].pending ? 5 : H[h].status;
-    hr[h].np_bound = H[h].np_bound;
-  }
-  for (int h = 0; h < nh; ++h)
-    PYFOF_TRY(upload(ctx, res + list[h], &hr[h], sizeof(HaloResult), s));
+  pm_result_kernel<<<(unsigned)ceil_div(nh, 128), 128, 0, s>>>(dH, dlist, nh, res);
+  PYFOF_CHECK_LAUNCH();
   if (phi_out) PYFOF_CUDA(cudaMemcpyAsync(phi_out, phi, sizeof(float) * M, cudaMemcpyDeviceToDevice, s));
   PYFOF_CUDA(cudaStreamSynchronize(s));
   return kOk;

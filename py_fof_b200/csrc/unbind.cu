@@ -435,6 +435,28 @@ static int32_t launch_direct_loop(bool fp64, int threads, unsigned nb, int cap, 
 #undef PYFOF_DIRECT_NT
 }
 
+// First-pass potentials of the direct-summation halos `list` (`dl` on the
+// device), flat over (halo, target tile).
+static int32_t direct_first_pass(Context &ctx, bool fp64, const Members &m, const int64_t *off, const int32_t *dl,
+                                 const std::vector<int32_t> &list, const std::vector<HaloTask> &tasks,
+                                 const direct::DirectParams &P, double *phi1, cudaStream_t s) {
+  const int pt = fp64 ? direct::kPhi1Targets<true> : direct::kPhi1Targets<false>;
+  std::vector<int2> tl;
+  for (size_t e = 0; e < list.size(); ++e)
+    for (int t0 = 0; t0 < tasks[list[e]].np; t0 += pt) tl.push_back(make_int2((int)e, t0));
+  int2 *dtl = ctx.work.carve<int2>(tl.size());
+  if (!dtl) { set_error("workspace exhausted (direct potentials)"); return kAlloc; }
+  PYFOF_TRY(upload(ctx, dtl, tl.data(), sizeof(int2) * tl.size(), s));
+  if (fp64)
+    direct::ub_direct_phi1_kernel<true><<<(unsigned)tl.size(), direct::kPhi1Threads<true>, 0, s>>>(m, off, dl, dtl, P,
+                                                                                                  phi1);
+  else
+    direct::ub_direct_phi1_kernel<false><<<(unsigned)tl.size(), direct::kPhi1Threads<false>, 0, s>>>(m, off, dl, dtl,
+                                                                                                    P, phi1);
+  PYFOF_CHECK_LAUNCH();
+  return kOk;
+}
+
 int32_t unbind_stage(Context &ctx, const FofArgs &a, FofState &st) {
   cudaStream_t s = ctx.stream;
   Arena &W = ctx.work;
@@ -602,19 +624,10 @@ int32_t unbind_stage(Context &ctx, const FofArgs &a, FofState &st) {
       // removal loops, one block per halo, launched per halo-size bucket
       // with the tile table's block size and shared memory for the bucket's
       // largest halo
-      std::vector<int2> tl;
-      for (size_t e = 0; e < direct.size(); ++e)
-        for (int t0 = 0; t0 < tasks[direct[e]].np; t0 += direct::PT) tl.push_back(make_int2((int)e, t0));
-      int2 *dtl = W.carve<int2>(tl.size());
       double *phi1 = W.carve<double>((size_t)std::max<int64_t>(M, 1));
       int32_t *dbl = W.carve<int32_t>(direct.size());
-      if (!dtl || !phi1 || !dbl) { set_error("workspace exhausted (direct potentials)"); return kAlloc; }
-      PYFOF_TRY(upload(ctx, dtl, tl.data(), sizeof(int2) * tl.size(), s));
-      if (a.bound_fp64)
-        direct::ub_direct_phi1_kernel<true><<<(unsigned)tl.size(), direct::PT, 0, s>>>(m, off, dl, dtl, P, phi1);
-      else
-        direct::ub_direct_phi1_kernel<false><<<(unsigned)tl.size(), direct::PT, 0, s>>>(m, off, dl, dtl, P, phi1);
-      PYFOF_CHECK_LAUNCH();
+      if (!phi1 || !dbl) { set_error("workspace exhausted (direct potentials)"); return kAlloc; }
+      PYFOF_TRY(direct_first_pass(ctx, a.bound_fp64 != 0, m, off, dl, direct, tasks, P, phi1, s));
       // per bucket, largest halos first (they run longest)
       std::vector<int32_t> bl;
       std::vector<size_t> bstart(7, 0);
@@ -799,16 +812,11 @@ int32_t unbind_potential(Context &ctx, const float *q_soa, const float *w, int32
     P.b = 0.0f;
     P.nmin = 1;
     P.phi_only = 1;
-    if (fp64) {
-      PYFOF_CUDA(cudaFuncSetAttribute(direct::ub_direct_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kDirectSmem));
-      direct::ub_direct_kernel<true><<<1, BLK, kDirectSmem, s>>>(m, off, dl, P, res, keep, phid, ctx.d_flags);
-    } else {
-      PYFOF_CUDA(cudaFuncSetAttribute(direct::ub_direct_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)kDirectSmem));
-      direct::ub_direct_kernel<false><<<1, BLK, kDirectSmem, s>>>(m, off, dl, P, res, keep, phid, ctx.d_flags);
-    }
-    PYFOF_CHECK_LAUNCH();
+    double *phi1 = W.carve<double>(np);
+    if (!phi1) { set_error("workspace exhausted"); return kAlloc; }
+    PYFOF_TRY(direct_first_pass(ctx, fp64 != 0, m, off, dl, std::vector<int32_t>(1, 0), tasks, P, phi1, s));
+    PYFOF_TRY(launch_direct_loop(fp64 != 0, 256, 1, (np + 31) / 32 * 32, m, off, dl, P, res, keep, phid, ctx.d_flags,
+                                 phi1, s));
   } else {
     const float spf = (float)sp;
     tasks[0].spacing = spf;

@@ -84,79 +84,95 @@ struct DirectParams {
   int phi_only;   // stop after the first potential
 };
 
-// Sources j0 .. j0+cnt-1 (staged at sx[0..cnt)) of a target's first-pass
-// potential, in ascending index, skipping the target itself: the
-// reference's accumulation order (bound_fortran.f90:2619-2640; its i<j loop
-// adds each pair term to both ends, so every target sums its sources in
-// ascending order) and the same operations as the in-kernel first pass of
-// ub_direct_kernel.
-template <bool FP64>
-__device__ __forceinline__ void phi1_sources(const float *sx, const float *sy, const float *sz,
-                                             const float *sw, int j0, int cnt, int i, float xi, float yi,
-                                             float zi, const DirectParams &P, double &acc64, Kahan &acc32,
-                                             float h32, float inv_h, float inv70h) {
-  for (int k = 0; k < cnt; ++k) {
-    if (j0 + k == i) continue;
-    if (FP64) {
-      const double dx = (double)__fsub_rn(sx[k], xi);
-      const double dy = (double)__fsub_rn(sy[k], yi);
-      const double dz = (double)__fsub_rn(sz[k], zi);
-      const double r = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
-                                            __dmul_rn(dz, dz)));
-      const double dd = __dmul_rn(P.fac, depth_continuous<double>(r, P.app));
-      acc64 = __dadd_rn(acc64, -__dmul_rn((double)sw[k], dd));
-    } else {
-      const float dx = sx[k] - xi, dy = sy[k] - yi, dz = sz[k] - zi;
-      const float r2 = dx * dx + dy * dy + dz * dz;
-      acc32.add(-sw[k] * depth_f32(r2, h32, inv_h, inv70h));
-    }
+// One FP64 pair term of the first pass, -(w_j * fac D(r)), with the
+// reference's operations (bound_fortran.f90:2619-2640).
+__device__ __forceinline__ double pair_depth64(float xj, float yj, float zj, float xi, float yi, float zi, double app) {
+  const double dx = (double)__fsub_rn(xj, xi);
+  const double dy = (double)__fsub_rn(yj, yi);
+  const double dz = (double)__fsub_rn(zj, zi);
+  const double r = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
+  return depth_continuous<double>(r, app);
+}
+
+// Adds the terms t of a group of G lanes to acc in lane order, the same on
+// every lane of the group: a serial sum whose terms were computed in parallel.
+template <int G>
+__device__ __forceinline__ void add_in_order(double &acc, double t, int n, unsigned group) {
+#pragma unroll
+  for (int u = 0; u < G; ++u) {
+    const double v = __shfl_sync(group, t, u, G);
+    if (u < n) acc = __dadd_rn(acc, v);
   }
 }
 
-// The first-pass potentials of many direct-summation halos, spread over
-// the whole GPU: block b takes the PT targets tiles[b] = (entry of list,
-// first target) of one halo and streams the halo's members through shared
-// memory in ascending order.  Each target's sum has exactly the order and
-// operations of the in-kernel first pass of ub_direct_kernel, so the
-// results are the same bits; the removal loop then starts from phi1.
-constexpr int PT = 64;
+// The first-pass potentials of many direct-summation halos, spread over the
+// whole GPU: block b takes the kPhi1Targets targets tiles[b] = (entry of list, first
+// target) of one halo and streams the halo's members through shared memory
+// in ascending order.  Each target adds its sources in ascending index,
+// skipping itself: the reference's accumulation order (bound_fortran.f90:
+// 2619-2640; its i<j loop adds each pair term to both ends) with the
+// operations of the in-kernel first pass of ub_direct_kernel, so the results
+// are the same bits; the removal loop then starts from phi1.
+// FP64: latency-bound (a square root and a division per term in one
+// dependent chain per target), so G = 8 lanes share a target: they compute
+// eight terms at once and add them in order (add_in_order).  A halo of 450
+// members took 184 us with a lane per target.  FP32: a lane per target (its
+// terms are as short as the ordered adds would be).
+constexpr int kPhi1Lanes64 = 8;
 template <bool FP64>
-__global__ void __launch_bounds__(PT) ub_direct_phi1_kernel(Members m, const int64_t *__restrict__ off,
-                                                            const int32_t *__restrict__ list,
-                                                            const int2 *__restrict__ tiles, DirectParams P,
-                                                            double *__restrict__ phi1) {
-  __shared__ float sx[PT], sy[PT], sz[PT], sw[PT];
+constexpr int kPhi1Targets = FP64 ? 32 : 64;
+template <bool FP64>
+constexpr int kPhi1Threads = FP64 ? 32 * kPhi1Lanes64 : 64;
+template <bool FP64>
+__global__ void __launch_bounds__(kPhi1Threads<FP64>) ub_direct_phi1_kernel(
+    Members m, const int64_t *__restrict__ off, const int32_t *__restrict__ list, const int2 *__restrict__ tiles,
+    DirectParams P, double *__restrict__ phi1) {
+  constexpr int G = FP64 ? kPhi1Lanes64 : 1, NT = kPhi1Threads<FP64>;
+  __shared__ float4 src[NT];
   const int2 t = tiles[blockIdx.x];
   const int c = list[t.x];
   const int64_t b0 = off[c];
   const int np = (int)(off[c + 1] - b0);
-  const int i = t.y + threadIdx.x;
+  const int i = t.y + threadIdx.x / G, gl = threadIdx.x % G;
   const bool act = i < np;
+  const unsigned group = G == 1 ? 0u : ((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
   const float xi = act ? m.q[0][b0 + i] : 0.f, yi = act ? m.q[1][b0 + i] : 0.f,
               zi = act ? m.q[2][b0 + i] : 0.f;
   const float h32 = (float)P.app, inv_h = (float)(1.0 / P.app), inv70h = (float)(1.0 / (70.0 * P.app));
   double acc64 = 0.0;
   Kahan acc32;
-  for (int j0 = 0; j0 < np; j0 += PT) {
+  for (int j0 = 0; j0 < np; j0 += NT) {
     const int j = j0 + threadIdx.x;
-    if (j < np) {
-      sx[threadIdx.x] = m.q[0][b0 + j];
-      sy[threadIdx.x] = m.q[1][b0 + j];
-      sz[threadIdx.x] = m.q[2][b0 + j];
-      sw[threadIdx.x] = m.w[b0 + j];
+    __syncthreads();
+    if (j < np) src[threadIdx.x] = make_float4(m.q[0][b0 + j], m.q[1][b0 + j], m.q[2][b0 + j], m.w[b0 + j]);
+    __syncthreads();
+    const int cnt = min(NT, np - j0);
+    if (FP64) {
+      if (act)
+        for (int k0 = 0; k0 < cnt; k0 += G) {
+          const int k = k0 + gl;
+          double v = 0.0;  // adding +0 leaves the sum as it is: the target itself
+          if (k < cnt && j0 + k != i) {
+            const float4 s = src[k];
+            v = -__dmul_rn((double)s.w, __dmul_rn(P.fac, pair_depth64(s.x, s.y, s.z, xi, yi, zi, P.app)));
+          }
+          add_in_order<G>(acc64, v, cnt - k0, group);
+        }
+    } else if (act) {
+      for (int k = 0; k < cnt; ++k) {
+        if (j0 + k == i) continue;
+        const float4 s = src[k];
+        const float dx = s.x - xi, dy = s.y - yi, dz = s.z - zi;
+        acc32.add(-s.w * depth_f32(dx * dx + dy * dy + dz * dz, h32, inv_h, inv70h));
+      }
     }
-    __syncthreads();
-    if (act)
-      phi1_sources<FP64>(sx, sy, sz, sw, j0, min(PT, np - j0), i, xi, yi, zi, P, acc64, acc32, h32, inv_h,
-                         inv70h);
-    __syncthreads();
   }
-  if (act) phi1[b0 + i] = FP64 ? acc64 : (double)((float)P.fac * acc32.s);
+  if (act && gl == 0) phi1[b0 + i] = FP64 ? acc64 : (double)((float)P.fac * acc32.s);
 }
 
 // Dynamic shared memory of ub_direct_kernel for halos of up to cap members
-// (cap a multiple of 32): nine float and two int arrays, one double array
-// and the keep flags.
+// (cap a multiple of 32): eight float arrays and one int array, two 64-bit
+// arrays and the keep flags.
 __host__ __device__ constexpr size_t direct_smem(int cap) { return (size_t)cap * (11 * 4 + 8 + 1); }
 
 // One block of NT threads per halo: bound_check_grid for gid 0
@@ -164,9 +180,18 @@ __host__ __device__ constexpr size_t direct_smem(int cap) { return (size_t)cap *
 // reference arithmetic; FP64=false the FP32 product path with compensated
 // sums.  phi1 (optional): the first-pass potentials from
 // ub_direct_phi1_kernel; null computes them here.  Every halo of the launch
-// has at most cap members.  No result depends on NT: every sum runs in an
-// order fixed by the member indices alone (per-target serial sums, the
-// FP64 centre sums in thread 0, the FP32 ones in warp 0 by index mod 32).
+// has at most cap members.  No result depends on NT: every sum is the one of
+// an order fixed by the member indices alone (per-target serial sums; for the
+// centre sums see s_amax below).
+//
+// One block per halo is a chain of short steps, so what counts is their
+// latency.  The centre sums in their fixed order cost one dependent add per
+// member and iteration (8 ms of a 128^3 box for its largest halos); here the
+// block sums them in parallel, bounds the distance to the ordered sums, and
+// runs the ordered sums only if that bound leaves the FP32 centre open.  The
+// refresh of the potential shares a target among eight lanes as
+// ub_direct_phi1_kernel does, and the removal order is a count over 64-bit
+// keys (energy, then index).
 template <bool FP64, int NT = BLK>
 __global__ void __launch_bounds__(NT) ub_direct_kernel(Members m, const int64_t *__restrict__ off,
                                                        const int32_t *__restrict__ list,
@@ -183,15 +208,24 @@ __global__ void __launch_bounds__(NT) ub_direct_kernel(Members m, const int64_t 
   float *qx = reinterpret_cast<float *>(smem);
   float *qy = qx + cap, *qz = qy + cap;
   float *vx = qz + cap, *vy = vx + cap, *vz = vy + cap;
-  float *w = vz + cap, *phi = w + cap, *en = phi + cap;
-  int *jdel = reinterpret_cast<int *>(en + cap);
-  int *unb = jdel + cap;
-  double *phid = reinterpret_cast<double *>(unb + cap);
+  float *w = vz + cap, *phi = w + cap;
+  int *jdel = reinterpret_cast<int *>(phi + cap);
+  // unbound members: bits of E (E >= 0, so they order like E) over ~index, so
+  // that a larger key is removed first (equal energies: lower index first)
+  unsigned long long *ukey = reinterpret_cast<unsigned long long *>(jdel + cap);
+  double *phid = reinterpret_cast<double *>(ukey + cap);
   unsigned char *keep = reinterpret_cast<unsigned char *>(phid + cap);
+  constexpr int G = FP64 ? kPhi1Lanes64 : 1;
   __shared__ int red_i[NT / 32];
-  __shared__ double s_qc[3], s_vc[3], s_sum[7];
-  __shared__ int s_nu, s_err;
+  __shared__ double red_d[7][NT / 32];
+  __shared__ double s_sum[7];
+  __shared__ float s_c[6];          // centre and mean velocity
+  __shared__ unsigned s_amax[6];    // largest |component| of q and v over the members
+  __shared__ int s_nu, s_err, s_open;
 
+  if (threadIdx.x < 6) s_amax[threadIdx.x] = 0;
+  __syncthreads();
+  float am[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (int i = threadIdx.x; i < np; i += NT) {
     const int64_t k = b0 + i;
     qx[i] = m.q[0][k]; qy[i] = m.q[1][k]; qz[i] = m.q[2][k];
@@ -199,6 +233,14 @@ __global__ void __launch_bounds__(NT) ub_direct_kernel(Members m, const int64_t 
     w[i] = m.w[k];
     keep[i] = 1;
     phid[i] = 0.0;
+    const float v6[6] = {qx[i], qy[i], qz[i], vx[i], vy[i], vz[i]};
+#pragma unroll
+    for (int d = 0; d < 6; ++d) am[d] = fmaxf(am[d], fabsf(v6[d]));
+  }
+#pragma unroll
+  for (int d = 0; d < 6; ++d) {
+    const unsigned o = __reduce_max_sync(0xffffffffu, __float_as_uint(am[d]));
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_amax[d], o);
   }
   if (threadIdx.x == 0) s_err = 0;
   __syncthreads();
@@ -211,63 +253,47 @@ __global__ void __launch_bounds__(NT) ub_direct_kernel(Members m, const int64_t 
     for (int i = threadIdx.x; i < np; i += NT) ks += keep[i];
     const int n_source = block_sum_i(ks, red_i);
     // potential: full sum on the first pass, later passes add back the
-    // sources removed since the previous refresh
-    for (int i = threadIdx.x; i < np; i += NT) {
+    // sources removed since the previous refresh, in removal order; G lanes
+    // per target (the same targets for every lane of a group)
+    const int gl = threadIdx.x % G;
+    const unsigned group = G == 1 ? 0u : ((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
+    for (int i = threadIdx.x / G; i < np; i += NT / G) {
       if (pass == 1 && phi1) {
-        phid[i] = phi1[b0 + i];
-      } else if (pass == 1) {
-        if (FP64) {
-          double acc = 0.0;
-          for (int j = 0; j < np; ++j) {
-            if (j == i) continue;
-            const double dx = (double)__fsub_rn(qx[j], qx[i]);
-            const double dy = (double)__fsub_rn(qy[j], qy[i]);
-            const double dz = (double)__fsub_rn(qz[j], qz[i]);
-            const double r = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
-                                                  __dmul_rn(dz, dz)));
-            const double dd = __dmul_rn(P.fac, depth_continuous<double>(r, P.app));
-            acc = __dadd_rn(acc, -__dmul_rn((double)w[j], dd));
-          }
-          phid[i] = acc;
-        } else {
-          Kahan acc;
-          const float xi = qx[i], yi = qy[i], zi = qz[i];
-          for (int j = 0; j < np; ++j) {
-            if (j == i) continue;
-            const float dx = qx[j] - xi, dy = qy[j] - yi, dz = qz[j] - zi;
-            const float r2 = dx * dx + dy * dy + dz * dz;
-            acc.add(-w[j] * depth_f32(r2, h32, inv_h, inv70h));
-          }
-          phid[i] = (double)(fac32 * acc.s);
-        }
-      } else if (keep[i]) {
-        if (FP64) {
-          double acc = phid[i];
-          for (int k = 0; k < njd; ++k) {
+        if (gl == 0) phid[i] = phi1[b0 + i];
+      } else if (FP64 && (pass == 1 || keep[i])) {
+        const float xi = qx[i], yi = qy[i], zi = qz[i];
+        const int nk = pass == 1 ? np : njd;
+        double acc = pass == 1 ? 0.0 : phid[i];
+        for (int k0 = 0; k0 < nk; k0 += G) {
+          const int k = k0 + gl;
+          double v = 0.0;
+          if (pass == 1) {
+            if (k < nk && k != i)
+              v = -__dmul_rn((double)w[k], __dmul_rn(P.fac, pair_depth64(qx[k], qy[k], qz[k], xi, yi, zi, P.app)));
+          } else if (k < nk) {
             const int j = jdel[k];
-            const double dx = (double)__fsub_rn(qx[j], qx[i]);
-            const double dy = (double)__fsub_rn(qy[j], qy[i]);
-            const double dz = (double)__fsub_rn(qz[j], qz[i]);
-            const double r = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
-                                                  __dmul_rn(dz, dz)));
-            acc = __dadd_rn(acc, __dmul_rn(__dmul_rn((double)w[j], P.fac),
-                                           depth_continuous<double>(r, P.app)));
+            v = __dmul_rn(__dmul_rn((double)w[j], P.fac), pair_depth64(qx[j], qy[j], qz[j], xi, yi, zi, P.app));
           }
-          phid[i] = acc;
-        } else {
-          Kahan acc;
-          const float xi = qx[i], yi = qy[i], zi = qz[i];
-          for (int k = 0; k < njd; ++k) {
-            const int j = jdel[k];
-            const float dx = qx[j] - xi, dy = qy[j] - yi, dz = qz[j] - zi;
-            acc.add(w[j] * depth_f32(dx * dx + dy * dy + dz * dz, h32, inv_h, inv70h));
-          }
-          phid[i] += (double)(fac32 * acc.s);
+          add_in_order<G>(acc, v, nk - k0, group);
         }
+        __syncwarp(group);  // every lane has read phid[i]
+        if (gl == 0) phid[i] = acc;
+      } else if (!FP64 && (pass == 1 || keep[i])) {
+        Kahan acc;
+        const float xi = qx[i], yi = qy[i], zi = qz[i];
+        const int nk = pass == 1 ? np : njd;
+        for (int k = 0; k < nk; ++k) {
+          const int j = pass == 1 ? k : jdel[k];
+          if (pass == 1 && j == i) continue;
+          const float dx = qx[j] - xi, dy = qy[j] - yi, dz = qz[j] - zi;
+          const float t = w[j] * depth_f32(dx * dx + dy * dy + dz * dz, h32, inv_h, inv70h);
+          acc.add(pass == 1 ? -t : t);
+        }
+        phid[i] = (pass == 1 ? 0.0 : phid[i]) + (double)(fac32 * acc.s);
       }
     }
-    njd = 0;
     __syncthreads();
+    njd = 0;
     for (int i = threadIdx.x; i < np; i += NT) {
       if (!keep[i]) continue;
       float v = FP64 ? __double2float_rn(phid[i]) : (float)phid[i];
@@ -280,53 +306,87 @@ __global__ void __launch_bounds__(NT) ub_direct_kernel(Members m, const int64_t 
     if (P.phi_only) { status = 0; break; }
     int deleted = 0;
     for (;;) {
-      // centre of mass and mean velocity of the kept set, FP64
-      if (FP64) {
-        // seven sequential sums in ascending index (the reference's order),
-        // one per lane of warp 0: the kept mass and the mass-weighted
-        // positions and velocities
-        if (threadIdx.x < 7) {
-          const int qi = threadIdx.x;
-          const float *src = qi == 1 ? qx : qi == 2 ? qy : qi == 3 ? qz : qi == 4 ? vx : qi == 5 ? vy : vz;
-          double acc = 0.0;
-#pragma unroll 4
-          for (int i = 0; i < np; ++i) {
-            if (!keep[i]) continue;
-            const double wi = (double)w[i];
-            acc = __dadd_rn(acc, qi == 0 ? wi : __dmul_rn(wi, (double)src[i]));
-          }
-          s_sum[qi] = acc;
-        }
-        __syncwarp();
-        if (threadIdx.x == 0) {
-          const double ws = s_sum[0];
-          for (int d = 0; d < 3; ++d) {
-            s_qc[d] = __ddiv_rn(s_sum[1 + d], ws);
-            s_vc[d] = __ddiv_rn(s_sum[4 + d], ws);
-          }
-        }
-      } else if (threadIdx.x < 32) {
-        // warp 0: lane l sums the members l, l+32, ...; then a butterfly
+      // centre of mass and mean velocity of the kept set.  The FP64 sums of
+      // w, w q and w v over n members in two orders, here this block's and
+      // the fixed one, differ by at most 2 (n-1) u sum |terms| (u = 2^-53), and
+      // sum |w x| <= max |x| sum w; so the two quotients differ by less than
+      // err = 5 (n + 4) u max |x|.  If q - err and q + err round to the same
+      // FP32 value, that is the fixed order's; if not (about one iteration in
+      // a hundred), the sums are run in the fixed order.
+      {
         double a[7] = {0, 0, 0, 0, 0, 0, 0};
-        for (int i = threadIdx.x; i < np; i += 32) {
+        for (int i = threadIdx.x; i < np; i += NT) {
           if (!keep[i]) continue;
           const double wi = (double)w[i];
           a[0] += wi;
-          a[1] += wi * qx[i]; a[2] += wi * qy[i]; a[3] += wi * qz[i];
-          a[4] += wi * vx[i]; a[5] += wi * vy[i]; a[6] += wi * vz[i];
+          a[1] += wi * (double)qx[i]; a[2] += wi * (double)qy[i]; a[3] += wi * (double)qz[i];
+          a[4] += wi * (double)vx[i]; a[5] += wi * (double)vy[i]; a[6] += wi * (double)vz[i];
         }
+#pragma unroll
         for (int k = 0; k < 7; ++k)
+#pragma unroll
           for (int o = 16; o > 0; o >>= 1) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
-        if (threadIdx.x == 0) {
-          for (int d = 0; d < 3; ++d) { s_qc[d] = a[1 + d] / a[0]; s_vc[d] = a[4 + d] / a[0]; }
+        if ((threadIdx.x & 31) == 0)
+#pragma unroll
+          for (int k = 0; k < 7; ++k) red_d[k][threadIdx.x >> 5] = a[k];
+        if (threadIdx.x == 0) s_nu = 0;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+          double v = 0.0;
+          if (threadIdx.x < 7)
+#pragma unroll
+            for (int u = 0; u < NT / 32; ++u) v += red_d[threadIdx.x][u];
+          const double ws = __shfl_sync(0xffffffffu, v, 0);
+          bool open = false;
+          if (threadIdx.x >= 1 && threadIdx.x < 7) {
+            const double q = v / ws;
+            const double err = 5.0 * (double)(np + 4) * 1.1102230246251566e-16 *
+                               (double)__uint_as_float(s_amax[threadIdx.x - 1]);
+            const float lo = __double2float_rn(q - err), hi = __double2float_rn(q + err);
+            open = !(lo == hi);
+            s_c[threadIdx.x - 1] = hi;
+          }
+          open = __any_sync(0xffffffffu, open);
+          if (threadIdx.x == 0) s_open = open;
         }
+        __syncthreads();
       }
-      if (threadIdx.x == 0) s_nu = 0;
-      __syncthreads();
-      const float qc0 = __double2float_rn(s_qc[0]), qc1 = __double2float_rn(s_qc[1]),
-                  qc2 = __double2float_rn(s_qc[2]);
-      const float vc0 = __double2float_rn(s_vc[0]), vc1 = __double2float_rn(s_vc[1]),
-                  vc2 = __double2float_rn(s_vc[2]);
+      if (s_open) {
+        if (FP64) {
+          // seven sequential sums in ascending index (the reference's order),
+          // one per lane of warp 0
+          if (threadIdx.x < 7) {
+            const int qi = threadIdx.x;
+            const float *src = qi == 1 ? qx : qi == 2 ? qy : qi == 3 ? qz : qi == 4 ? vx : qi == 5 ? vy : vz;
+            double acc = 0.0;
+#pragma unroll 4
+            for (int i = 0; i < np; ++i) {
+              if (!keep[i]) continue;
+              const double wi = (double)w[i];
+              acc = __dadd_rn(acc, qi == 0 ? wi : __dmul_rn(wi, (double)src[i]));
+            }
+            s_sum[qi] = acc;
+          }
+        } else if (threadIdx.x < 32) {
+          // warp 0: lane l sums the members l, l+32, ...; then a butterfly
+          double a[7] = {0, 0, 0, 0, 0, 0, 0};
+          for (int i = threadIdx.x; i < np; i += 32) {
+            if (!keep[i]) continue;
+            const double wi = (double)w[i];
+            a[0] += wi;
+            a[1] += wi * qx[i]; a[2] += wi * qy[i]; a[3] += wi * qz[i];
+            a[4] += wi * vx[i]; a[5] += wi * vy[i]; a[6] += wi * vz[i];
+          }
+          for (int k = 0; k < 7; ++k)
+            for (int o = 16; o > 0; o >>= 1) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
+          if (threadIdx.x == 0)
+            for (int k = 0; k < 7; ++k) s_sum[k] = a[k];
+        }
+        __syncthreads();
+        if (threadIdx.x < 6) s_c[threadIdx.x] = __double2float_rn(__ddiv_rn(s_sum[1 + threadIdx.x], s_sum[0]));
+        __syncthreads();
+      }
+      const float qc0 = s_c[0], qc1 = s_c[1], qc2 = s_c[2], vc0 = s_c[3], vc1 = s_c[4], vc2 = s_c[5];
       // specific energies (bound_fortran.f90:2773-2786), FP32
       for (int i = threadIdx.x; i < np; i += NT) {
         if (!keep[i]) continue;
@@ -338,8 +398,9 @@ __global__ void __launch_bounds__(NT) ub_direct_kernel(Members m, const int64_t 
         s = __fadd_rn(s, __fmul_rn(d2, d2));
         const float e = __fadd_rn(__fdiv_rn(s, 2.0f), phi[i]);
         if (!isfinite(e)) s_err = kInvalid;
-        en[i] = e;
-        if (e >= 0.0f) unb[atomicAdd(&s_nu, 1)] = i;
+        if (e >= 0.0f)
+          ukey[atomicAdd(&s_nu, 1)] =
+              ((unsigned long long)__float_as_uint(e + 0.0f) << 32) | (0xffffffffu - (unsigned)i);
       }
       __syncthreads();
       if (s_err) break;
@@ -354,15 +415,12 @@ __global__ void __launch_bounds__(NT) ub_direct_kernel(Members m, const int64_t 
       nb = max(1, nb);
       nb = min(nu, nb);
       for (int t = threadIdx.x; t < nu; t += NT) {
-        const int i = unb[t];
-        const float ei = en[i];
+        const unsigned long long key = ukey[t];
         int rank = 0;
-        for (int u = 0; u < nu; ++u) {
-          const int j = unb[u];
-          const float ej = en[j];
-          rank += (ej > ei) || (ej == ei && j < i);
-        }
+#pragma unroll 8
+        for (int u = 0; u < nu; ++u) rank += ukey[u] > key;
         if (rank < nb) {
+          const int i = (int)(0xffffffffu - (unsigned)key);
           keep[i] = 0;
           jdel[njd + rank] = i;
         }

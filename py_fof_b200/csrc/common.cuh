@@ -112,9 +112,17 @@ __device__ __forceinline__ double fmodulo(double a, double p) {
 }
 
 // Unwrap a coordinate about an anchor: MODULO(x - anchor + half, L) - half,
-// evaluated left to right in FP64 (fof_fortran.f90:525).
+// evaluated left to right in FP64 (fof_fortran.f90:525).  Within one period
+// either side of [0, L) the remainder is known without a division and exact:
+// fmod(a, L) is a for |a| < L and a - L for L <= a < 2L.
 __device__ __forceinline__ double unwrap(double x, double anchor, double half, double L) {
-  return __dadd_rn(fmodulo(__dadd_rn(__dadd_rn(x, -anchor), half), L), -half);
+  const double a = __dadd_rn(__dadd_rn(x, -anchor), half);
+  double r;
+  if (a >= 0.0 && a < L) r = a;
+  else if (a < 0.0 && a > -L) r = __dadd_rn(a, L);
+  else if (a >= L && a < 2.0 * L) r = __dadd_rn(a, -L);
+  else r = fmodulo(a, L);
+  return __dadd_rn(r, -half);
 }
 
 // Order-preserving maps between doubles and unsigned 64-bit integers, for

@@ -6,18 +6,23 @@
 //   1. fof_bbox_kernel    per-region unwrap about the first particle + bbox
 //   2. host               reference cell geometry per region (same formulas,
 //                         same libm pow) -> region table
-//   3. fof_key_kernel     global cell key per particle + cell histogram
-//   4. stable cell order  (cell key, particle index): the reference CRS order,
-//                         by a scatter to per-cell slots and a sort of each
-//                         cell (a stable radix sort when a cell is large)
-//   5. fof_gather_kernel  FP32 sorted coordinates (real(x_rel,4))
+//   3. fof_key_kernel     global cell key per particle, cell histogram and the
+//                         particle's slot in its cell
+//   4. fof_scatter_kernel FP32 coordinates (real(x_rel,4)) in cell order.  The
+//                         order inside a cell is arbitrary; where the
+//                         reference's CRS order (cell, then ascending index)
+//                         decides something, the numbering of the candidates
+//                         and their first member, step 8 restores it.  (Option
+//                         cell_order: the CRS order itself.)
+//   5. fof_cells_kernel   dense cells and their warp chunks
 //   6. link kernels       pair tests over the reference's neighbour cells
 //                         (fof_link_dense_kernel for cells with more than
 //                         DENSE_T particles and their pairs with sparse
 //                         cells, fof_link_kernel for sparse-cell pairs),
 //                         lock-free atomicCAS union (lower index wins)
 //   7. fof_root_kernel    full compression + warp-aggregated group sizes
-//   8. scan of root flags -> candidate ranks (region order, then root CRS
+//   8. ordered compaction of the roots of large groups, then by index inside
+//                         a cell -> candidate ids (region order, then root CRS
 //                         position: the reference halo numbering)
 //   9. outputs, FP64 centre-of-mass / angular momentum per candidate
 #include <algorithm>
@@ -70,6 +75,7 @@ __global__ void __launch_bounds__(BLK) fof_bbox_kernel(Coords xp, const RegionDe
     mx[d] = -INFINITY;
   }
   bool bad = false;
+#pragma unroll 4
   for (int64_t i = t.begin + threadIdx.x; i < t.end; i += BLK) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -99,55 +105,91 @@ __global__ void __launch_bounds__(BLK) fof_bbox_kernel(Coords xp, const RegionDe
   }
 }
 
-__device__ __forceinline__ int64_t cell_coord(double x, double origin, double size, int32_t n) {
-  double f = floor(__ddiv_rn(__dadd_rn(x, -origin), size)) + 1.0;
-  if (!(f >= 1.0)) f = 1.0;
-  if (f > (double)n) f = (double)n;
-  return (int64_t)f - 1;
+// Zero-based cell of a coordinate, floor((x - origin) / size) clamped to the
+// grid (fof_fortran.f90:598).  The product with the reciprocal is within a
+// few ulps of the quotient, so its floor is the quotient's unless it lies
+// that close to a cell boundary; only then is the division done.
+__device__ __forceinline__ int32_t cell_coord(double x, double origin, double size, double inv, int32_t n) {
+  const double y = __dadd_rn(x, -origin);
+  const double q = y * inv;
+  double f = floor(q);
+  const double tol = 1e-15 * fabs(q) + 1e-300;
+  if (!(q - f > tol && f + 1.0 - q > tol)) f = floor(__ddiv_rn(y, size));
+  if (!(f >= 0.0)) f = 0.0;
+  const double top = (double)(n - 1);
+  if (f > top) f = top;
+  return __double2int_rz(f);
 }
 
+// sentinel != 0: particles of inactive regions get that key and a slot too
+// (the sorts of option cell_order take all particles).
 __global__ void __launch_bounds__(BLK) fof_key_kernel(Coords xp, const RegionDev *__restrict__ R,
                                                       const Tile *__restrict__ T, double L,
-                                                      double half, uint32_t sentinel,
+                                                      double half, uint32_t sentinel, int all,
                                                       uint32_t *__restrict__ keys,
                                                       uint32_t *__restrict__ counts,
                                                       uint32_t *__restrict__ rank) {
   const Tile t = T[blockIdx.x];
   const RegionDev &r = R[t.region];
   if (!r.active) {
-    for (int64_t i = t.begin + threadIdx.x; i < t.end; i += BLK) {
-      keys[i] = sentinel;
-      rank[i] = atomicAdd(&counts[sentinel], 1u);
-    }
+    if (all)
+      for (int64_t i = t.begin + threadIdx.x; i < t.end; i += BLK) {
+        keys[i] = sentinel;
+        rank[i] = atomicAdd(&counts[sentinel], 1u);
+      }
     return;
   }
   double anc[3];
   for (int d = 0; d < 3; ++d) anc[d] = xp.get(r.start, d);
+#pragma unroll 4
   for (int64_t i = t.begin + threadIdx.x; i < t.end; i += BLK) {
-    int64_t c[3];
+    uint32_t c[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d)
-      c[d] = cell_coord(unwrap(xp.get(i, d), anc[d], half, L), r.origin[d], r.size[d], r.N[d]);
-    uint64_t key = r.cell_off + (uint64_t)(c[0] + (int64_t)r.N[0] * (c[1] + (int64_t)r.N[1] * c[2]));
-    keys[i] = (uint32_t)key;
+      c[d] = (uint32_t)cell_coord(unwrap(xp.get(i, d), anc[d], half, L), r.origin[d], r.size[d], r.inv_size[d],
+                                  r.N[d]);
+    const uint32_t key =
+        (uint32_t)r.cell_off + c[0] + (uint32_t)r.N[0] * (c[1] + (uint32_t)r.N[1] * c[2]);
+    keys[i] = key;
     rank[i] = atomicAdd(&counts[key], 1u);  // a slot in the cell, in no particular order
   }
 }
 
-// ---- cell order without a radix sort ---------------------------------------
+// FP32 coordinates to cell start + slot.  Reads the coordinates again, in
+// input order (24 B a particle, coalesced), and writes 20 B at the sorted
+// position: bound by those writes when the input order is not spatial.  (A
+// gather by sorted index reads three sectors per particle instead, after a
+// sort of the indices: 1.75 ms against 0.6 ms for a shuffled 256^3 box.)
+__global__ void __launch_bounds__(BLK) fof_scatter_kernel(Coords xp, const RegionDev *__restrict__ R,
+                                                          const Tile *__restrict__ T, double L, double half,
+                                                          const uint32_t *__restrict__ keys,
+                                                          const uint32_t *__restrict__ rank,
+                                                          const uint32_t *__restrict__ cstart,
+                                                          float4 *__restrict__ pos, uint32_t *__restrict__ skey,
+                                                          uint32_t *__restrict__ prid) {
+  const Tile t = T[blockIdx.x];
+  const RegionDev &r = R[t.region];
+  if (!r.active) return;
+  double anc[3];
+  for (int d = 0; d < 3; ++d) anc[d] = xp.get(r.start, d);
+#pragma unroll 4
+  for (int64_t i = t.begin + threadIdx.x; i < t.end; i += BLK) {
+    const uint32_t k = keys[i];
+    const uint32_t p = cstart[k] + rank[i];
+    float v[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) v[d] = __double2float_rn(unwrap(xp.get(i, d), anc[d], half, L));
+    pos[p] = make_float4(v[0], v[1], v[2], __int_as_float((int)i));
+    skey[p] = k;
+    if (prid) prid[p] = (uint32_t)t.region;
+  }
+}
+
+// ---- the CRS order itself (option cell_order) ------------------------------
 // The key kernel's counters give every particle a distinct slot in its
 // cell; scattering to cell start + slot groups the particles by cell, and
 // sorting each cell's original indices restores the stable order of the
 // reference's counting sort (ascending original index within a cell).
-
-__global__ void fof_max_count_kernel(const uint32_t *__restrict__ counts, int64_t ncell,
-                                     uint32_t *__restrict__ out) {
-  uint32_t m = 0;
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncell; c += (int64_t)gridDim.x * blockDim.x)
-    m = max(m, counts[c]);
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(out, m);
-}
 
 __global__ void fof_cell_scatter_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ rank,
                                         const uint32_t *__restrict__ cstart, int64_t n,
@@ -233,7 +275,7 @@ __global__ void __launch_bounds__(BLK) fof_gather_kernel(
     for (int d = 0; d < 3; ++d)
       v[d] = __double2float_rn(unwrap(xp.get(i, d), xp.get(r.start, d), half, L));
     pos[p] = make_float4(v[0], v[1], v[2], __int_as_float((int)i));
-    prid[p] = (uint32_t)rid;
+    if (prid) prid[p] = (uint32_t)rid;
   }
 }
 
@@ -318,10 +360,9 @@ constexpr int DENSE_T = 24;
 constexpr int SUB_MAX = 216;
 
 struct DenseIndex {
-  const uint32_t *rank;  // exclusive scan of dense-cell flags, per cell
+  const uint32_t *rank;  // number of each dense cell (set for dense cells only)
   const uint32_t *tab;   // per dense cell: S+1 offsets (relative to cell start)
   const float4 *dpos;    // dense cells' particles listed by sub-cell; .w = sorted position
-  const uint32_t *order; // work order: dense-cell particles first, then the rest
   int stride;            // entries per dense cell in tab
   float reach;           // linking length plus FP32 rounding slack
 };
@@ -402,104 +443,152 @@ __device__ __forceinline__ void link_pair(int *parent, int p, int q, int &rp, in
 // Ordered-integer image of a float (monotone: a < b  <=>  key(a) < key(b)
 // for non-NaN values), so warp min/max reductions of coordinates can use the
 // integer reduction instructions.  The map is its own inverse.
-// Sparse-cell particles, a warp per 32 consecutive entries of the sparse
-// work order.  Each lane lists the source ranges of its particle: the
-// sparse cells among the neighbour cells that the cube of half-width
-// `reach` around it touches, from its own cell on (higher keys; in the own
-// cell, the higher sorted positions).  That is at most 8 cells where cells
-// are wider than two linking lengths; narrower cells, and the key order of
-// wrapped periodic neighbours, allow up to all 27, and a lane tests the
-// ranges beyond the first MAX_RANGES itself, right away.  The warp then
-// runs all pairs of all lanes in rounds of 32, one pair per lane (a lane
-// finds its pair's particle by a binary search over the lanes' pair
-// offsets and its source by walking that particle's ranges), so the lanes
-// stay busy however unevenly the pairs are spread over the particles.
-// Pairs with dense-cell particles are the dense kernel's.
+// Sparse-cell particles, a warp per 32 consecutive sorted positions.  Each
+// lane lists the source ranges of its particle: the sparse cells among the
+// neighbour cells that the cube of half-width `reach` around it touches,
+// from its own cell on (higher keys; in the own cell, the higher positions).
+// Cells that are neighbours along x are consecutive in cell order, so a row
+// of them is one range: at most four rows and two wrapped cells where cells
+// are wider than two linking lengths.  Narrower cells, and rows broken up by
+// dense cells, can give more; a lane tests the ranges beyond the first
+// MAX_RANGES itself, right away.  The warp then runs all pairs of all lanes
+// in rounds of 32, one pair per lane (a lane finds its pair's particle by a
+// binary search over the lanes' pair offsets and its source by walking that
+// particle's ranges), so the lanes stay busy however unevenly the pairs are
+// spread over the particles.  Pairs with dense-cell particles are the dense
+// kernel's.
+// Bound by instruction issue: what a particle costs before its first pair
+// test.  So the cell is decoded by multiplication, the cells its reach
+// touches follow from its FP32 place in the cell (RegionDev::near) and the
+// rows need two loads each.
 constexpr int MAX_RANGES = 8;
+
+// Pairs of particle ip with the sorted positions [b, e), tested at once.
+__device__ __noinline__ void link_range(const float4 *__restrict__ pos, float4 me, int ip, uint32_t b, uint32_t e,
+                                        int periodic, const LinkParams &P, int *parent, int32_t *flags) {
+  for (uint32_t q = b; q < e; ++q) {
+    const float4 o = pos[q];
+    const bool lk = periodic ? linked_pbc(me, o, P) : linked_open(me, o, P.rp2_open);
+    if (lk) {
+      int rp = -1;
+      link_pair(parent, ip, (int)q, rp, flags);
+    }
+  }
+}
 
 __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
     const float4 *__restrict__ pos, const uint32_t *__restrict__ skey,
     const uint32_t *__restrict__ prid, const RegionDev *__restrict__ R,
-    const uint32_t *__restrict__ cell_start, int *parent, int64_t w0, int64_t w1, LinkParams P,
-    DenseIndex D, int32_t *flags) {
+    const uint32_t *__restrict__ cs, int *parent, int64_t n, LinkParams P, int32_t *flags) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ uint2 ranges[BLK][MAX_RANGES];  // (first source, count)
+  __shared__ float4 target[BLK];
   const int lane = threadIdx.x & 31;
   const int wbase_t = threadIdx.x & ~31;
   const int64_t nw = ((int64_t)gridDim.x * BLK) >> 5;
-  for (int64_t wb = w0 + (((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5) * 32; wb < w1; wb += nw * 32) {
+  for (int64_t wb = (((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5) * 32; wb < n; wb += nw * 32) {
     const int64_t w = wb + lane;
-    const bool valid = w < w1;
-    const int ip = valid ? (int)D.order[w] : 0;
-    const float4 me = valid ? pos[ip] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const RegionDev &r = R[valid ? prid[ip] : 0];
+    const int ip = (int)w;
     uint32_t total = 0;
     int nr = 0;
-    if (valid) {
-      const uint32_t local = skey[ip] - (uint32_t)r.cell_off;
-      const int64_t N0 = r.N[0], N1 = r.N[1], N2 = r.N[2];
-      int64_t ixyz[3];
-      {
-        const uint32_t n0 = (uint32_t)N0, n1 = (uint32_t)N1;
-        const uint32_t q0 = local / n0;
-        ixyz[0] = local - q0 * n0;
-        ixyz[1] = q0 % n1;
-        ixyz[2] = q0 / n1;
-      }
-      const int64_t Nd[3] = {N0, N1, N2};
-      const float mexyz[3] = {me.x, me.y, me.z};
-      int lo[3], hi[3];
+    bool per = false;
+    if (w < n) {
+      const uint32_t cell = skey[w];
+      const uint32_t own_end = cs[cell + 1];
+      if (own_end - cs[cell] <= (uint32_t)DENSE_T) {
+        const float4 me = pos[w];
+        const RegionDev &r = R[prid ? prid[w] : 0];
+        per = r.periodic != 0;
+        target[threadIdx.x] = me;
+        const uint32_t coff = (uint32_t)r.cell_off, local = cell - coff;
+        const int N0 = r.N[0], N1 = r.N[1], N2 = r.N[2];
+        const uint32_t q0 = div_by(local, r.div[0]);
+        const int ix = (int)(local - q0 * (uint32_t)N0);
+        const int iz = (int)div_by(q0, r.div[1]);
+        const int iy = (int)(q0 - (uint32_t)iz * (uint32_t)N1);
+        // which neighbour cells the reach touches, per axis; both sides where
+        // FP32 cannot tell the cell
+        const float xyz[3] = {me.x, me.y, me.z};
+        bool below[3], above[3];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const bool pd = (r.pdim >> d) & 1;
-        if (Nd[d] == 1) { lo[d] = 0; hi[d] = 0; continue; }
-        const float clo = cell_lower(r, d, ixyz[d]);
-        const float chi = cell_lower(r, d, ixyz[d] + 1);
-        const bool below = __fsub_rn(mexyz[d], D.reach) < clo;
-        const bool above = __fadd_rn(mexyz[d], D.reach) >= chi;
-        if (pd && Nd[d] == 2) { lo[d] = 0; hi[d] = (below || above) ? 1 : 0; }
-        else { lo[d] = below ? -1 : 0; hi[d] = above ? 1 : 0; }
-      }
-      // (the distance test takes the minimum image itself: a wrapped cell
-      // needs no coordinate shift)
-      for (int dz = lo[2]; dz <= hi[2]; ++dz) {
-        int64_t jz = ixyz[2] + dz;
-        if ((r.pdim >> 2) & 1) {
-          if (jz < 0) jz += N2; else if (jz >= N2) jz -= N2;
-        } else if (jz < 0 || jz >= N2) continue;
-        for (int dy = lo[1]; dy <= hi[1]; ++dy) {
-          int64_t jy = ixyz[1] + dy;
-          if ((r.pdim >> 1) & 1) {
-            if (jy < 0) jy += N1; else if (jy >= N1) jy -= N1;
-          } else if (jy < 0 || jy >= N1) continue;
-          for (int dx = lo[0]; dx <= hi[0]; ++dx) {
-            int64_t jx = ixyz[0] + dx;
-            if (r.pdim & 1) {
-              if (jx < 0) jx += N0; else if (jx >= N0) jx -= N0;
-            } else if (jx < 0 || jx >= N0) continue;
-            const int64_t jl = jx + N0 * (jy + N1 * jz);
-            if (jl < (int64_t)local) continue;
-            const uint64_t jc = r.cell_off + (uint64_t)jl;
-            uint32_t b = cell_start[jc];
-            const uint32_t e = cell_start[jc + 1];
-            if (e - b > (uint32_t)DENSE_T) continue;  // pairs with a dense cell: the dense kernel
-            if (jl == (int64_t)local) b = (uint32_t)ip + 1;
-            if (e <= b) continue;
-            if (nr < MAX_RANGES) {
-              ranges[threadIdx.x][nr++] = make_uint2(b, e - b);
-              total += e - b;
-            } else {
-              const bool per = r.periodic != 0;
-              for (uint32_t q = b; q < e; ++q) {
-                const float4 o = pos[q];
-                const bool lk = per ? linked_pbc(me, o, P) : linked_open(me, o, P.rp2_open);
-                if (lk) {
-                  int rp = -1;
-                  link_pair(parent, ip, (int)q, rp, flags);
-                }
-              }
-            }
+        for (int d = 0; d < 3; ++d) {
+          const float f = (xyz[d] - r.org[d]) * r.cinv[d];
+          const float fr = f - floorf(f);
+          below[d] = fr < r.near[d] || fr > 1.0f - r.slack[d];
+          above[d] = fr > 1.0f - r.near[d] || fr < r.slack[d];
+        }
+        auto add = [&](uint32_t b, uint32_t e) {
+          if (e <= b) return;
+          if (nr < MAX_RANGES) {
+            ranges[threadIdx.x][nr++] = make_uint2(b, e - b);
+            total += e - b;
+          } else {
+            link_range(pos, me, ip, b, e, r.periodic, P, parent, flags);
           }
+        };
+        // the sparse cells c0..c1 (consecutive along x), positions from `from` on
+        auto add_row = [&](uint32_t c0, uint32_t c1, uint32_t from) {
+          const uint32_t b = cs[c0], e = cs[c1 + 1];
+          if (e == b) return;
+          if (e - b <= (uint32_t)DENSE_T) {
+            add(max(b, from), e);
+            return;
+          }
+          for (uint32_t c = c0; c <= c1; ++c) {
+            const uint32_t cb = cs[c], ce = cs[c + 1];
+            if (ce - cb <= (uint32_t)DENSE_T) add(max(cb, from), ce);
+          }
+        };
+        const bool px = r.pdim & 1;
+        if (N0 >= 3 && iy > 0 && iy < N1 - 1 && iz > 0 && iz < N2 - 1) {
+          // x neighbours: a run of cells, and the cell around the box's edge
+          const int x0 = below[0] && ix > 0 ? -1 : 0, x1 = above[0] && ix < N0 - 1 ? 1 : 0;
+          const bool lo_wrap = px && below[0] && ix == 0, hi_wrap = px && above[0] && ix == N0 - 1;
+          add_row(cell, cell + x1, (uint32_t)ip + 1);
+          if (lo_wrap) add_row(cell + (N0 - 1), cell + (N0 - 1), 0);
+          auto forward = [&](int dy, int dz) {
+            const uint32_t c = cell + (uint32_t)(N0 * (dy + N1 * dz));
+            add_row(c + x0, c + x1, 0);
+            if (lo_wrap) add_row(c + (N0 - 1), c + (N0 - 1), 0);
+            if (hi_wrap) add_row(c - (N0 - 1), c - (N0 - 1), 0);
+          };
+          if (above[1]) forward(1, 0);
+          if (above[2]) {
+            if (below[1]) forward(-1, 1);
+            forward(0, 1);
+            if (above[1]) forward(1, 1);
+          }
+        } else {
+          const int ic[3] = {ix, iy, iz}, Nd[3] = {N0, N1, N2};
+          int lo[3], hi[3];
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            if (Nd[d] == 1) { lo[d] = 0; hi[d] = 0; }
+            else if (((r.pdim >> d) & 1) && Nd[d] == 2) { lo[d] = 0; hi[d] = (below[d] || above[d]) ? 1 : 0; }
+            else { lo[d] = below[d] ? -1 : 0; hi[d] = above[d] ? 1 : 0; }
+          }
+          // (the distance test takes the minimum image itself: a wrapped cell
+          // needs no coordinate shift)
+          for (int dz = lo[2]; dz <= hi[2]; ++dz)
+            for (int dy = lo[1]; dy <= hi[1]; ++dy)
+              for (int dx = lo[0]; dx <= hi[0]; ++dx) {
+                const int dd[3] = {dx, dy, dz};
+                int j[3];
+                bool in = true;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                  j[d] = ic[d] + dd[d];
+                  if ((r.pdim >> d) & 1) {
+                    if (j[d] < 0) j[d] += Nd[d]; else if (j[d] >= Nd[d]) j[d] -= Nd[d];
+                  } else if (j[d] < 0 || j[d] >= Nd[d]) {
+                    in = false;
+                  }
+                }
+                if (!in) continue;
+                const uint32_t jl = (uint32_t)j[0] + (uint32_t)N0 * ((uint32_t)j[1] + (uint32_t)N1 * (uint32_t)j[2]);
+                if (jl < local) continue;
+                add_row(coff + jl, coff + jl, jl == local ? (uint32_t)ip + 1 : 0);
+              }
         }
       }
     }
@@ -512,6 +601,7 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
     }
     const uint32_t excl = incl - total;
     const uint32_t T = __shfl_sync(FULL, incl, 31);
+    const unsigned per_mask = __ballot_sync(FULL, per);
     __syncwarp();
     for (uint32_t g0 = 0; g0 < T; g0 += 32) {
       const uint32_t g = g0 + (uint32_t)lane;
@@ -523,16 +613,8 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
         if (v <= g) owner += step;
       }
       owner &= 31;
-      const uint32_t oexcl = __shfl_sync(FULL, excl, owner);
-      const int po = __shfl_sync(FULL, ip, owner);
-      float4 pm;
-      pm.x = __shfl_sync(FULL, me.x, owner);
-      pm.y = __shfl_sync(FULL, me.y, owner);
-      pm.z = __shfl_sync(FULL, me.z, owner);
-      pm.w = 0.f;
-      const bool per = __shfl_sync(FULL, r.periodic, owner) != 0;
+      uint32_t j = g - __shfl_sync(FULL, excl, owner);
       if (g < T) {
-        uint32_t j = g - oexcl;
         const uint2 *rg = ranges[wbase_t + owner];
         int k = 0;
         while (j >= rg[k].y) {
@@ -541,10 +623,11 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
         }
         const int q = (int)(rg[k].x + j);
         const float4 o = pos[q];
-        const bool lk = per ? linked_pbc(pm, o, P) : linked_open(pm, o, P.rp2_open);
+        const float4 pm = target[wbase_t + owner];
+        const bool lk = (per_mask >> owner) & 1 ? linked_pbc(pm, o, P) : linked_open(pm, o, P.rp2_open);
         if (lk) {
           int rp = -1;
-          link_pair(parent, po, q, rp, flags);
+          link_pair(parent, (int)(wb + owner), q, rp, flags);
         }
       }
     }
@@ -591,7 +674,7 @@ __global__ void __launch_bounds__(BLK, 3) fof_link_dense_kernel(
     float4 me = make_float4(0.f, 0.f, 0.f, 0.f);
     if (valid) me = D.dpos[cb + k];
     const int ip = valid ? __float_as_int(me.w) : -1;
-    const RegionDev &r = R[prid[cb]];
+    const RegionDev &r = R[prid ? prid[cb] : 0];
     const bool my_vd = is_vd(r, cn);
     const int64_t local = (int64_t)C.cell - (int64_t)r.cell_off;
     const int64_t N0 = r.N[0], N1 = r.N[1], N2 = r.N[2];
@@ -799,63 +882,44 @@ __global__ void __launch_bounds__(BLK, 3) fof_link_dense_kernel(
   }
 }
 
-// Chunks of up to 32 particles per dense cell.
-__global__ void fof_dense_chunk_count_kernel(const uint32_t *__restrict__ list, const uint32_t *__restrict__ cs,
-                                             int64_t ndense, uint32_t *__restrict__ cnt) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ndense;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t c = list[i];
-    cnt[i] = (cs[c + 1] - cs[c] + 31u) / 32u;
+// Dense cells, their numbers and their chunks of up to 32 particles, in no
+// particular order, and the fullest cell.  out: [0] dense cells, [1] chunks,
+// [2] largest count (zeroed before).
+__global__ void __launch_bounds__(BLK) fof_cells_kernel(const uint32_t *__restrict__ cs, int64_t ncell,
+                                                        uint32_t *__restrict__ out, uint32_t *__restrict__ list,
+                                                        uint32_t *__restrict__ rank, DenseChunk *__restrict__ chunks) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  uint32_t most = 0;
+  for (int64_t base = (int64_t)blockIdx.x * BLK; base < ncell; base += (int64_t)gridDim.x * BLK) {
+    const int64_t c = base + threadIdx.x;
+    const uint32_t n = c < ncell ? cs[c + 1] - cs[c] : 0u;
+    most = max(most, n);
+    const unsigned m = __ballot_sync(FULL, n > (uint32_t)DENSE_T);
+    if (!m) continue;
+    const uint32_t nch = n > (uint32_t)DENSE_T ? (n + 31u) / 32u : 0u;
+    uint32_t incl = nch;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += v;
+    }
+    uint32_t r0 = 0, k0 = 0;
+    if (lane == 31) {
+      r0 = atomicAdd(&out[0], (uint32_t)__popc(m));
+      k0 = atomicAdd(&out[1], incl);
+    }
+    r0 = __shfl_sync(FULL, r0, 31);
+    k0 = __shfl_sync(FULL, k0, 31) + incl - nch;
+    if (nch) {
+      const uint32_t r = r0 + __popc(m & lanemask_lt());
+      list[r] = (uint32_t)c;
+      rank[c] = r;
+      for (uint32_t j = 0; j < nch; ++j) chunks[k0 + j] = DenseChunk{(uint32_t)c, 32u * j};
+    }
   }
-}
-
-__global__ void fof_dense_chunk_fill_kernel(const uint32_t *__restrict__ list, const uint32_t *__restrict__ cs,
-                                            const uint32_t *__restrict__ off, int64_t ndense,
-                                            DenseChunk *__restrict__ chunks) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ndense;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t c = list[i];
-    const uint32_t n = (cs[c + 1] - cs[c] + 31u) / 32u;
-    for (uint32_t j = 0; j < n; ++j) chunks[off[i] + j] = DenseChunk{c, 32u * j};
-  }
-}
-
-__global__ void fof_dense_flag_kernel(const uint32_t *__restrict__ cs,
-                                      const uint64_t *__restrict__ cell_off,
-                                      const RegionDev *__restrict__ R, int nreg, int64_t ncell,
-                                      uint32_t *__restrict__ flag) {
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncell;
-       c += (int64_t)gridDim.x * blockDim.x) {
-    flag[c] = cs[c + 1] - cs[c] > (uint32_t)DENSE_T ? 1u : 0u;
-  }
-}
-
-__global__ void fof_dense_pos_flag_kernel(const uint32_t *__restrict__ skey,
-                                          const uint32_t *__restrict__ cflag, int64_t n,
-                                          uint32_t *__restrict__ pflag) {
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n;
-       p += (int64_t)gridDim.x * blockDim.x)
-    pflag[p] = cflag[skey[p]];
-}
-
-// Dense-cell particles first (they carry most of the pair tests, so they
-// start early), the rest after them; both parts keep the sorted order.
-__global__ void fof_order_kernel(const uint32_t *__restrict__ pflag,
-                                 const uint32_t *__restrict__ prank, int64_t n, int64_t ndense_p,
-                                 uint32_t *__restrict__ order) {
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n;
-       p += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k = pflag[p] ? (int64_t)prank[p] : ndense_p + (p - (int64_t)prank[p]);
-    order[k] = (uint32_t)p;
-  }
-}
-
-__global__ void fof_dense_list_kernel(const uint32_t *__restrict__ flag,
-                                      const uint32_t *__restrict__ rank, int64_t ncell,
-                                      uint32_t *__restrict__ list) {
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncell;
-       c += (int64_t)gridDim.x * blockDim.x)
-    if (flag[c]) list[rank[c]] = (uint32_t)c;
+  most = __reduce_max_sync(FULL, most);
+  if (lane == 0 && most > 0) atomicMax(&out[2], most);
 }
 
 // One block per dense cell: counting sort of its particles by sub-cell.
@@ -1050,10 +1114,12 @@ __global__ void __launch_bounds__(BLK) fof_vd_inter_kernel(
   }
 }
 
-__global__ void fof_init_parent(int *parent, int64_t n) {
+__global__ void fof_init_kernel(int *__restrict__ parent, uint32_t *__restrict__ gsize, int64_t n) {
   for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n;
-       p += (int64_t)gridDim.x * blockDim.x)
+       p += (int64_t)gridDim.x * blockDim.x) {
     parent[p] = (int)p;
+    gsize[p] = 0;
+  }
 }
 
 // Final labels.  The forest is static after linking; find() may still
@@ -1076,11 +1142,98 @@ __global__ void __launch_bounds__(BLK) fof_root_kernel(int *parent, int *lab, ui
   }
 }
 
-__global__ void fof_cand_flag_kernel(const int *lab, const uint32_t *gsize, int64_t n,
-                                     uint32_t np_min, uint32_t *flag) {
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n;
-       p += (int64_t)gridDim.x * blockDim.x)
-    flag[p] = (lab[p] == (int)p && gsize[p] >= np_min) ? 1u : 0u;
+// Candidates: roots whose group has at least nmin members (gsize is 0 at
+// every other position).  Compacted in position order, tile by tile: counts
+// per tile, a scan of the tiles, then the fill.
+constexpr int CTILE = 4096;
+
+__global__ void __launch_bounds__(BLK) fof_cand_count_kernel(const uint32_t *__restrict__ gsize, int64_t n,
+                                                             uint32_t nmin, uint32_t *__restrict__ cnt) {
+  __shared__ uint32_t red[BLK / 32];
+  uint32_t c = 0;
+  const int64_t b = (int64_t)blockIdx.x * CTILE, e = min(n, b + CTILE);
+#pragma unroll
+  for (int k = 0; k < CTILE / BLK; ++k) {
+    const int64_t p = b + k * BLK + threadIdx.x;
+    c += p < e && gsize[p] >= nmin;
+  }
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t t = 0;
+    for (int w = 0; w < BLK / 32; ++w) t += red[w];
+    cnt[blockIdx.x] = t;
+  }
+}
+
+__global__ void __launch_bounds__(BLK) fof_cand_fill_kernel(const uint32_t *__restrict__ gsize, int64_t n,
+                                                            uint32_t nmin, const uint32_t *__restrict__ off,
+                                                            int32_t *__restrict__ root) {
+  if (off[blockIdx.x + 1] == off[blockIdx.x]) return;  // no candidate in the tile
+  __shared__ uint32_t wsum[BLK / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t at = off[blockIdx.x];
+  const int64_t b = (int64_t)blockIdx.x * CTILE, e = min(n, b + CTILE);
+  for (int k = 0; k < CTILE / BLK; ++k) {
+    const int64_t p = b + k * BLK + threadIdx.x;
+    const bool f = p < e && gsize[p] >= nmin;
+    const unsigned m = __ballot_sync(0xffffffffu, f);
+    __syncthreads();
+    if (lane == 0) wsum[warp] = __popc(m);
+    __syncthreads();
+    uint32_t before = at;
+    for (int w = 0; w < BLK / 32; ++w) {
+      if (w < warp) before += wsum[w];
+      at += wsum[w];
+    }
+    if (f) root[before + __popc(m & lanemask_lt())] = (int32_t)p;
+  }
+}
+
+// First member of every candidate in the reference's order (cell, then
+// ascending original index): the root is the lowest position, so it lies in
+// the group's first cell, and the first member is the lowest index among the
+// group's members there (they follow the root).  A warp per candidate.
+__global__ void __launch_bounds__(BLK) fof_cand_anchor_kernel(const int32_t *__restrict__ root, int64_t ncand,
+                                                              const int *__restrict__ lab,
+                                                              const uint32_t *__restrict__ skey,
+                                                              const uint32_t *__restrict__ cs,
+                                                              const float4 *__restrict__ pos,
+                                                              uint32_t *__restrict__ first) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t c = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5; c < ncand; c += ((int64_t)gridDim.x * BLK) >> 5) {
+    const int r = root[c];
+    const int64_t e = cs[skey[r] + 1];
+    uint32_t m = 0xffffffffu;
+    for (int64_t q = (int64_t)r + lane; q < e; q += 32)
+      if (lab[q] == r) m = min(m, (uint32_t)__float_as_int(pos[q].w));
+    m = __reduce_min_sync(0xffffffffu, m);
+    if (lane == 0) first[c] = m;
+  }
+}
+
+// Candidate ids: position order, and by first member among candidates whose
+// roots share a cell.
+__global__ void fof_cand_info_kernel(const int32_t *__restrict__ root, int64_t ncand,
+                                     const uint32_t *__restrict__ first, const uint32_t *__restrict__ skey,
+                                     const uint32_t *__restrict__ prid, const uint32_t *__restrict__ gsize,
+                                     uint32_t *__restrict__ crank, int64_t *__restrict__ cand_anchor,
+                                     int32_t *__restrict__ cand_region, int32_t *__restrict__ cand_np,
+                                     int32_t *__restrict__ cand_root) {
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncand;
+       c += (int64_t)gridDim.x * blockDim.x) {
+    const int r = root[c];
+    const uint32_t cell = skey[r], f = first[c];
+    int64_t id = c;
+    for (int64_t k = c - 1; k >= 0 && skey[root[k]] == cell; --k) id -= first[k] > f;
+    for (int64_t k = c + 1; k < ncand && skey[root[k]] == cell; ++k) id += first[k] < f;
+    crank[r] = (uint32_t)id;
+    cand_anchor[id] = f;
+    cand_region[id] = prid ? (int32_t)prid[r] : 0;
+    cand_np[id] = (int32_t)gsize[r];
+    cand_root[id] = r;
+  }
 }
 
 // Candidate of every sorted particle (-1 if its group is too small), plus
@@ -1172,22 +1325,6 @@ __global__ void __launch_bounds__(BLK) fof_angmom_kernel(Coords xp, Coords vp, c
   }
 }
 
-// anchor (first member in CRS order = the root) and region of each candidate
-__global__ void fof_cand_info_kernel(const uint32_t *flag, const uint32_t *crank,
-                                     const float4 *pos, const uint32_t *prid,
-                                     const uint32_t *gsize, int64_t n, int64_t *cand_anchor,
-                                     int32_t *cand_region, int32_t *cand_np, int32_t *cand_root) {
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n;
-       p += (int64_t)gridDim.x * blockDim.x)
-    if (flag[p]) {
-      const uint32_t c = crank[p];
-      cand_anchor[c] = __float_as_int(pos[p].w);
-      cand_region[c] = (int32_t)prid[p];
-      cand_np[c] = (int32_t)gsize[p];
-      cand_root[c] = (int32_t)p;
-    }
-}
-
 int bits_for(uint64_t v) {
   int b = 0;
   while (b < 64 && (v >> b) != 0) ++b;
@@ -1197,6 +1334,13 @@ int bits_for(uint64_t v) {
 }  // namespace
 
 // ------------------------------------------------------- host geometry
+
+// Half-width of the cube that holds every partner the distance test can
+// accept: slack relative 1e-4 for the FP32 distance arithmetic, 8 FP32 ulps
+// of the box size for the rounding of positions and query endpoints.
+static double link_reach(double L, double link) {
+  return link * (1.0 + 1e-4) + 8.0 * 1.1920928955078125e-07 * (std::fabs(L) + 1.0);
+}
 
 // Reference cell geometry of one region (fof_fortran.f90:528-570) from its
 // unwrapped bounding box.  64-bit integers are used where the reference's
@@ -1251,6 +1395,18 @@ void region_geometry(double L, double link, int32_t np, const double *xmin, cons
   }
   r.sub_ok = prod > 1 ? 1 : 0;
   for (int d = 0; d < 3; ++d) r.inv_sub[d] = (float)((double)r.sub[d] / r.size[d]);
+  const double reach = link_reach(L, link);
+  for (int d = 0; d < 3; ++d) {
+    r.inv_size[d] = 1.0 / r.size[d];
+    r.org[d] = (float)r.origin[d];
+    r.cinv[d] = (float)r.inv_size[d];
+    // FP32 error of (x - org) * cinv: a few ulps of the coordinates, in
+    // cells, and of the product (at most N)
+    const double sl = 1e-4 + 4e-7 * (double)N[d] + 4e-7 * (std::fabs(L) + std::fabs(r.origin[d])) / r.size[d];
+    r.slack[d] = (float)std::min(sl, 2.0);
+    r.near[d] = (float)std::min(reach / r.size[d] + sl, 2.0);
+    if (d < 2) r.div[d] = N[d] > 1 ? ~(uint64_t)0 / (uint64_t)N[d] + 1 : 0;
+  }
   // merge sub-cells: width at most link/sqrt(3) * 0.999 less 8 FP32 ulps of
   // the box size (the rounding of positions and sub-cell boundaries), so the
   // largest distance inside one, as the FP32/FP64 test computes it, stays
@@ -1361,79 +1517,94 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
   uint64_t *dcoff = W.carve<uint64_t>(nreg + 1);
   uint32_t *keys = W.carve<uint32_t>(std::max<int64_t>(n, 1));
   uint32_t *cstart = W.carve<uint32_t>(total_cells + 2);
-  uint32_t *ka = W.carve<uint32_t>(std::max<int64_t>(n, 1));
-  uint32_t *va = W.carve<uint32_t>(std::max<int64_t>(n, 1));
-  uint32_t *kb = W.carve<uint32_t>(std::max<int64_t>(n, 1));
-  uint32_t *vb = W.carve<uint32_t>(std::max<int64_t>(n, 1));
-  if (!dcoff || !keys || !cstart || !ka || !va || !kb || !vb) {
+  if (!dcoff || !keys || !cstart) {
     set_error("workspace exhausted (keys)");
     return kAlloc;
   }
   PYFOF_TRY(upload(ctx, dcoff, cell_off.data(), sizeof(uint64_t) * (nreg + 1), s));
   PYFOF_CUDA(cudaMemsetAsync(cstart, 0, sizeof(uint32_t) * (total_cells + 2), s));
+  // the particles' slots within their cells (sort scratch in the sorted modes)
+  uint32_t *slot = W.carve<uint32_t>(std::max<int64_t>(n, 1));
+  uint32_t *skey = W.carve<uint32_t>(std::max<int64_t>(n, 1));
+  float4 *pos = W.carve<float4>(std::max<int64_t>(n_active, 1));
+  uint32_t *prid = nreg > 1 ? W.carve<uint32_t>(std::max<int64_t>(n_active, 1)) : nullptr;
+  if (!slot || !skey || !pos || (nreg > 1 && !prid)) { set_error("workspace exhausted (keys)"); return kAlloc; }
   const uint32_t sentinel = (uint32_t)total_cells;
-  // slots within the cells go to va (radix scratch when the sort is needed)
   if (ntiles) {
-    fof_key_kernel<<<(unsigned)ntiles, BLK, 0, s>>>(xp, dR, dT, L, half, sentinel, keys, cstart, va);
+    fof_key_kernel<<<(unsigned)ntiles, BLK, 0, s>>>(xp, dR, dT, L, half, sentinel, a.cell_order != 0, keys, cstart,
+                                                    slot);
     PYFOF_CHECK_LAUNCH();
   }
-  // Per-cell sorts pay off where the radix sort needs a fourth pass (keys of
-  // more than 24 bits) and every cell fits one block's sort; otherwise, and
-  // always with cell_order 2, a stable radix sort of all keys.
-  const uint64_t max_key = (n_active < n) ? total_cells : (total_cells ? total_cells - 1 : 0);
-  const bool try_cells = a.cell_order == 1 || (a.cell_order == 0 && bits_for(max_key) > 24);
-  uint32_t *dmax = reinterpret_cast<uint32_t *>(ctx.d_flags + FLAG_COUNT_A);
-  PYFOF_CUDA(cudaMemsetAsync(dmax, 0, sizeof(uint32_t), s));
-  const unsigned cgrid0 = (unsigned)std::max<int64_t>(
-      1, std::min<int64_t>(ceil_div((int64_t)std::max<uint64_t>(total_cells, 1), (int64_t)BLK),
-                           (int64_t)kNumSMs * 16));
-  if (total_cells > 0) {
-    fof_max_count_kernel<<<cgrid0, BLK, 0, s>>>(cstart, (int64_t)total_cells, dmax);
-    PYFOF_CHECK_LAUNCH();
-  }
-  PYFOF_CUDA(cudaMemcpyAsync(ctx.h_flags + FLAG_COUNT_A, dmax, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   PYFOF_TRY(exclusive_scan_u32(cstart, cstart, (int64_t)total_cells + 1, nullptr, W, s));
-  PYFOF_CUDA(cudaStreamSynchronize(s));
-  const uint32_t max_occ = (uint32_t)ctx.h_flags[FLAG_COUNT_A];
-  ctx.last_max_cell = max_occ;
-  ctx.last_cell_sorts = 0;
-  uint32_t *skey, *sidx;
-  if (try_cells && max_occ <= (uint32_t)CELL_SORT_MAX) {
-    ctx.last_cell_sorts = 1;
-    // cells of more than CELL_SORT_SMALL particles: at most n / (CELL_SORT_SMALL + 1)
-    uint32_t *big = W.carve<uint32_t>(
-        (size_t)std::min<int64_t>(n_active / (CELL_SORT_SMALL + 1) + 1, (int64_t)total_cells + 1));
-    uint32_t *nbig = W.carve<uint32_t>(1);
-    if (!big || !nbig) { set_error("workspace exhausted (cell sort)"); return kAlloc; }
-    PYFOF_CUDA(cudaMemsetAsync(nbig, 0, sizeof(uint32_t), s));
-    const unsigned sgrid = (unsigned)std::max<int64_t>(
-        1, std::min<int64_t>(ceil_div(std::max<int64_t>(n, 1), (int64_t)BLK), (int64_t)kNumSMs * 16));
-    fof_cell_scatter_kernel<<<sgrid, BLK, 0, s>>>(keys, va, cstart, n, ka, vb);
+  // dense cells: at most n / (DENSE_T + 1); their chunks: one per 32
+  // particles and one more per cell
+  const size_t dense_cap = (size_t)n_active / (DENSE_T + 1) + 1;
+  uint32_t *list = W.carve<uint32_t>(dense_cap);
+  uint32_t *drank = W.carve<uint32_t>(total_cells + 1);
+  DenseChunk *dchunks = W.carve<DenseChunk>((size_t)n_active / 32 + dense_cap);
+  if (!list || !drank || !dchunks) { set_error("workspace exhausted (dense cells)"); return kAlloc; }
+  uint32_t *dcells = reinterpret_cast<uint32_t *>(ctx.d_flags + FLAG_COUNT_A);  // A, B, C
+  PYFOF_CUDA(cudaMemsetAsync(dcells, 0, 3 * sizeof(uint32_t), s));
+  if (total_cells > 0) {
+    const unsigned cgrid = (unsigned)std::min<int64_t>(ceil_div((int64_t)total_cells, (int64_t)BLK), (int64_t)kNumSMs * 16);
+    fof_cells_kernel<<<cgrid, BLK, 0, s>>>(cstart, (int64_t)total_cells, dcells, list, drank, dchunks);
     PYFOF_CHECK_LAUNCH();
-    if (total_cells > 0) {
-      fof_cell_sort_small_kernel<<<cgrid0, BLK, 0, s>>>(cstart, (int64_t)total_cells, vb, big, nbig);
+  }
+  PYFOF_CUDA(cudaMemcpyAsync(ctx.h_flags, ctx.d_flags, sizeof(int32_t) * FLAG_COUNT, cudaMemcpyDeviceToHost, s));
+  ctx.last_cell_sorts = 0;
+  if (a.cell_order == 0 && n_active > 0) {
+    fof_scatter_kernel<<<(unsigned)ntiles, BLK, 0, s>>>(xp, dR, dT, L, half, keys, slot, cstart, pos, skey, prid);
+    PYFOF_CHECK_LAUNCH();
+  }
+  PYFOF_CUDA(cudaStreamSynchronize(s));
+  const int64_t ndense = (uint32_t)ctx.h_flags[FLAG_COUNT_A], ndense_chunks = (uint32_t)ctx.h_flags[FLAG_COUNT_B];
+  const uint32_t max_occ = (uint32_t)ctx.h_flags[FLAG_COUNT_C];
+  ctx.last_max_cell = max_occ;
+  ctx.last_dense = ndense;
+  if (a.cell_order != 0) {
+    // the reference's CRS order itself
+    uint32_t *sidx = nullptr;
+    uint32_t *ka = skey, *va = slot, *kb = W.carve<uint32_t>(std::max<int64_t>(n, 1)),
+             *vb = W.carve<uint32_t>(std::max<int64_t>(n, 1));
+    if (!kb || !vb) { set_error("workspace exhausted (cell order)"); return kAlloc; }
+    if (a.cell_order == 1 && max_occ <= (uint32_t)CELL_SORT_MAX) {
+      ctx.last_cell_sorts = 1;
+      // cells of more than CELL_SORT_SMALL particles: at most n / (CELL_SORT_SMALL + 1)
+      uint32_t *big = W.carve<uint32_t>(
+          (size_t)std::min<int64_t>(n_active / (CELL_SORT_SMALL + 1) + 1, (int64_t)total_cells + 1));
+      uint32_t *nbig = W.carve<uint32_t>(1);
+      if (!big || !nbig) { set_error("workspace exhausted (cell sort)"); return kAlloc; }
+      PYFOF_CUDA(cudaMemsetAsync(nbig, 0, sizeof(uint32_t), s));
+      const unsigned sgrid = (unsigned)std::max<int64_t>(
+          1, std::min<int64_t>(ceil_div(std::max<int64_t>(n, 1), (int64_t)BLK), (int64_t)kNumSMs * 16));
+      fof_cell_scatter_kernel<<<sgrid, BLK, 0, s>>>(keys, slot, cstart, n, ka, vb);
       PYFOF_CHECK_LAUNCH();
-      fof_cell_sort_big_kernel<<<kNumSMs * 2, 1024, 0, s>>>(cstart, big, nbig, vb);
+      if (total_cells > 0) {
+        const unsigned cgrid = (unsigned)std::min<int64_t>(ceil_div((int64_t)total_cells, (int64_t)BLK),
+                                                           (int64_t)kNumSMs * 16);
+        fof_cell_sort_small_kernel<<<cgrid, BLK, 0, s>>>(cstart, (int64_t)total_cells, vb, big, nbig);
+        PYFOF_CHECK_LAUNCH();
+        fof_cell_sort_big_kernel<<<kNumSMs * 2, 1024, 0, s>>>(cstart, big, nbig, vb);
+        PYFOF_CHECK_LAUNCH();
+      }
+      sidx = vb;
+    } else {
+      const uint64_t max_key = (n_active < n) ? total_cells : (total_cells ? total_cells - 1 : 0);
+      PYFOF_TRY(radix_sort_pairs(keys, nullptr, n, bits_for(max_key), ka, va, kb, vb, &skey, &sidx, W, s));
+    }
+    if (n_active > 0) {
+      const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(n_active, BLK), (int64_t)kNumSMs * 16);
+      fof_gather_kernel<<<grid, BLK, 0, s>>>(xp, dR, dcoff, nreg, skey, sidx, n_active, L, half, pos, prid);
       PYFOF_CHECK_LAUNCH();
     }
-    skey = ka;
-    sidx = vb;
-  } else {
-    PYFOF_TRY(radix_sort_pairs(keys, nullptr, n, bits_for(max_key), ka, va, kb, vb, &skey, &sidx,
-                               W, s));
   }
-  // --- sorted FP32 coordinates, DSU
-  float4 *pos = W.carve<float4>(std::max<int64_t>(n_active, 1));
-  uint32_t *prid = W.carve<uint32_t>(std::max<int64_t>(n_active, 1));
   int *parent = W.carve<int>(std::max<int64_t>(n_active, 1));
-  if (!pos || !prid || !parent) { set_error("workspace exhausted (link)"); return kAlloc; }
+  uint32_t *gsize = W.carve<uint32_t>(std::max<int64_t>(n_active, 1));
+  if (!parent || !gsize) { set_error("workspace exhausted (link)"); return kAlloc; }
   const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(std::max<int64_t>(n_active, 1), BLK),
                                                     (int64_t)kNumSMs * 16);
   if (n_active > 0) {
-    fof_gather_kernel<<<grid, BLK, 0, s>>>(xp, dR, dcoff, nreg, skey, sidx, n_active, L, half, pos,
-                                           prid);
-    PYFOF_CHECK_LAUNCH();
-    fof_init_parent<<<grid, BLK, 0, s>>>(parent, n_active);
+    fof_init_kernel<<<grid, BLK, 0, s>>>(parent, gsize, n_active);
     PYFOF_CHECK_LAUNCH();
     LinkParams P;
     P.L = L;
@@ -1448,16 +1619,10 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
     P.rp2_lo = (float)(P.rp2 * (1.0 - 4e-6));
     P.rp2_hi = (float)(P.rp2 * (1.0 + 4e-6));
     DenseIndex D{};
-    const uint32_t *D_list = nullptr;  // dense cells in rank order
     bool any_vd = false;               // a region where very dense cells can occur
     for (int r = 0; r < nreg; ++r) any_vd = any_vd || (reg[r].active && reg[r].vd_k[0] > 0);
-    int64_t ndense_p = 0;  // particles in dense cells (the head of D.order)
-    int64_t ndense_chunks = 0;
-    DenseChunk *dchunks = nullptr;
-    // slack: relative 1e-4 for the FP32 distance arithmetic, 8 FP32 ulps of
-    // the box size for the rounding of positions and query endpoints
-    D.reach = (float)(a.link * (1.0 + 1e-4) + 8.0 * 1.1920928955078125e-07 * (std::fabs(L) + 1.0));
-    {
+    D.reach = (float)link_reach(L, a.link);
+    if (ndense > 0) {
       int smax = 1;
       for (int r = 0; r < nreg; ++r)
         if (reg[r].active) {
@@ -1465,73 +1630,25 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
           smax = std::max(smax, reg[r].vd_k[0] * reg[r].vd_k[1] * reg[r].vd_k[2]);
         }
       D.stride = smax + 1;
-      const int64_t nc = (int64_t)total_cells;
-      uint32_t *dflag = W.carve<uint32_t>(nc + 1);
-      uint32_t *drank = W.carve<uint32_t>(nc + 1);
       float4 *dpos = W.carve<float4>(n_active);
-      uint32_t *order = W.carve<uint32_t>(n_active);
-      uint32_t *pflag = W.carve<uint32_t>(n_active + 1);
-      uint32_t *prank = W.carve<uint32_t>(n_active + 1);
-      if (!dflag || !drank || !dpos || !order || !pflag || !prank) {
-        set_error("workspace exhausted (dense index)");
-        return kAlloc;
-      }
-      const unsigned cgrid = (unsigned)std::min<int64_t>(ceil_div(nc, BLK), (int64_t)kNumSMs * 16);
-      fof_dense_flag_kernel<<<cgrid, BLK, 0, s>>>(cstart, dcoff, dR, nreg, nc, dflag);
+      uint32_t *tab = W.carve<uint32_t>(ndense * D.stride);
+      if (!dpos || !tab) { set_error("workspace exhausted (dense tables)"); return kAlloc; }
+      fof_dense_build_kernel<<<(unsigned)ndense, BLK, 0, s>>>(list, cstart, pos, dR, dcoff, nreg, D.stride, tab,
+                                                              dpos);
       PYFOF_CHECK_LAUNCH();
-      PYFOF_TRY(exclusive_scan_u32(dflag, drank, nc, reinterpret_cast<uint32_t *>(ctx.d_flags + FLAG_COUNT_B), W, s));
-      fof_dense_pos_flag_kernel<<<grid, BLK, 0, s>>>(skey, dflag, n_active, pflag);
-      PYFOF_CHECK_LAUNCH();
-      PYFOF_TRY(exclusive_scan_u32(pflag, prank, n_active, reinterpret_cast<uint32_t *>(ctx.d_flags + FLAG_COUNT_C), W, s));
-      PYFOF_CUDA(cudaMemcpyAsync(ctx.h_flags, ctx.d_flags, sizeof(int32_t) * FLAG_COUNT,
-                                 cudaMemcpyDeviceToHost, s));
-      PYFOF_CUDA(cudaStreamSynchronize(s));
-      const int64_t ndense = (uint32_t)ctx.h_flags[FLAG_COUNT_B];
-      ndense_p = (uint32_t)ctx.h_flags[FLAG_COUNT_C];
-      fof_order_kernel<<<grid, BLK, 0, s>>>(pflag, prank, n_active, ndense_p, order);
-      PYFOF_CHECK_LAUNCH();
-      uint32_t *tab = W.carve<uint32_t>(std::max<int64_t>(ndense, 1) * D.stride);
-      uint32_t *list = W.carve<uint32_t>(std::max<int64_t>(ndense, 1));
-      if (!tab || !list) { set_error("workspace exhausted (dense tables)"); return kAlloc; }
-      if (ndense > 0) {
-        fof_dense_list_kernel<<<cgrid, BLK, 0, s>>>(dflag, drank, nc, list);
-        PYFOF_CHECK_LAUNCH();
-        fof_dense_build_kernel<<<(unsigned)ndense, BLK, 0, s>>>(list, cstart, pos, dR, dcoff, nreg,
-                                                                D.stride, tab, dpos);
-        PYFOF_CHECK_LAUNCH();
-        // warp chunks of the dense cells
-        uint32_t *coff = W.carve<uint32_t>(ndense + 1);
-        if (!coff) { set_error("workspace exhausted (dense chunks)"); return kAlloc; }
-        PYFOF_CUDA(cudaMemsetAsync(coff, 0, sizeof(uint32_t) * (ndense + 1), s));
-        const unsigned lgrid = (unsigned)std::min<int64_t>(ceil_div(ndense, BLK), (int64_t)kNumSMs * 16);
-        fof_dense_chunk_count_kernel<<<lgrid, BLK, 0, s>>>(list, cstart, ndense, coff);
-        PYFOF_CHECK_LAUNCH();
-        PYFOF_TRY(exclusive_scan_u32(coff, coff, ndense + 1, nullptr, W, s));
-        uint32_t nch = 0;
-        PYFOF_CUDA(cudaMemcpyAsync(&nch, coff + ndense, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-        PYFOF_CUDA(cudaStreamSynchronize(s));
-        ndense_chunks = nch;
-        dchunks = W.carve<DenseChunk>(std::max<uint32_t>(nch, 1));
-        if (!dchunks) { set_error("workspace exhausted (dense chunks)"); return kAlloc; }
-        fof_dense_chunk_fill_kernel<<<lgrid, BLK, 0, s>>>(list, cstart, coff, ndense, dchunks);
-        PYFOF_CHECK_LAUNCH();
-      }
       D.rank = drank;
-      D_list = list;
       D.tab = tab;
       D.dpos = dpos;
-      D.order = order;
-      ctx.last_dense = ndense;
     }
     // dense-cell particles and the rest as two launches: the long pair loops
     // of the dense part do not hold back blocks of the short sparse work
     if (ctx.timing) cudaEventRecord(ctx.ev[0], s);
     PYFOF_CUDA(cudaMemsetAsync(ctx.d_flags + FLAG_VD, 0, sizeof(int32_t), s));
     if (ctx.last_dense > 0 && any_vd) {
-      fof_vd_intra_kernel<<<(unsigned)ctx.last_dense, BLK, 0, s>>>(D_list, cstart, dR, dcoff, nreg, D.stride,
+      fof_vd_intra_kernel<<<(unsigned)ctx.last_dense, BLK, 0, s>>>(list, cstart, dR, dcoff, nreg, D.stride,
                                                                    D.tab, D.dpos, parent, ctx.d_flags);
       PYFOF_CHECK_LAUNCH();
-      fof_vd_inter_kernel<<<(unsigned)ctx.last_dense, BLK, 0, s>>>(D_list, cstart, dR, dcoff, nreg, D.stride,
+      fof_vd_inter_kernel<<<(unsigned)ctx.last_dense, BLK, 0, s>>>(list, cstart, dR, dcoff, nreg, D.stride,
                                                                    D.tab, D.rank, D.dpos, parent, P, D.reach,
                                                                    ctx.d_flags);
       PYFOF_CHECK_LAUNCH();
@@ -1544,11 +1661,8 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
                                                   ctx.d_flags);
       PYFOF_CHECK_LAUNCH();
     }
-    if (n_active > ndense_p) {
-      fof_link_kernel<<<grid, BLK, 0, s>>>(pos, skey, prid, dR, cstart, parent, ndense_p, n_active, P,
-                                           D, ctx.d_flags);
-      PYFOF_CHECK_LAUNCH();
-    }
+    fof_link_kernel<<<grid, BLK, 0, s>>>(pos, skey, prid, dR, cstart, parent, n_active, P, ctx.d_flags);
+    PYFOF_CHECK_LAUNCH();
     if (ctx.timing) cudaEventRecord(ctx.ev[1], s);
   }
   st.dR = dR;
@@ -1556,7 +1670,7 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
   st.prid = prid;
   st.parent = parent;
   st.skey = skey;
-  st.sidx = sidx;
+  st.gsize = gsize;
   st.cell_start = cstart;
   st.keys_free = keys;
   st.reg = reg;
@@ -1567,25 +1681,25 @@ int32_t fof_candidates_stage(Context &ctx, const FofArgs &a, FofState &st, bool 
   cudaStream_t s = ctx.stream;
   Arena &W = ctx.work;
   const int64_t na = st.n_active;
-  uint32_t *gsize = W.carve<uint32_t>(std::max<int64_t>(na, 1));
-  uint32_t *flag = W.carve<uint32_t>(std::max<int64_t>(na, 1) + 1);
-  uint32_t *crank = W.carve<uint32_t>(std::max<int64_t>(na, 1) + 1);
+  uint32_t *crank = W.carve<uint32_t>(std::max<int64_t>(na, 1));
   int32_t *pcand = W.carve<int32_t>(std::max<int64_t>(na, 1));
-  if (!gsize || !flag || !crank || !pcand) { set_error("workspace exhausted (labels)"); return kAlloc; }
+  const int64_t ntile = std::max<int64_t>(ceil_div(na, (int64_t)CTILE), 1);
+  uint32_t *toff = W.carve<uint32_t>(ntile + 1);
+  if (!crank || !pcand || !toff) { set_error("workspace exhausted (labels)"); return kAlloc; }
+  // (every root has at least itself: a minimum of 0 takes all of them too)
+  const uint32_t nmin = a.np_halo_min == 0 ? 1u : (uint32_t)a.np_halo_min;
+  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(std::max<int64_t>(na, 1), BLK), (int64_t)kNumSMs * 16);
   st.ncand = 0;
   if (na > 0) {
-    const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(na, BLK), (int64_t)kNumSMs * 16);
-    PYFOF_CUDA(cudaMemsetAsync(gsize, 0, sizeof(uint32_t) * na, s));
-    st.lab = reinterpret_cast<int *>(st.keys_free);  // keys are dead after the sort
-    fof_root_kernel<<<grid, BLK, 0, s>>>(st.parent, st.lab, gsize, na);
+    st.lab = reinterpret_cast<int *>(st.keys_free);  // keys are dead after the scatter
+    fof_root_kernel<<<grid, BLK, 0, s>>>(st.parent, st.lab, st.gsize, na);
     PYFOF_CHECK_LAUNCH();
-    fof_cand_flag_kernel<<<grid, BLK, 0, s>>>(st.lab, gsize, na, (uint32_t)a.np_halo_min, flag);
+    PYFOF_CUDA(cudaMemsetAsync(toff + ntile, 0, sizeof(uint32_t), s));
+    fof_cand_count_kernel<<<(unsigned)ntile, BLK, 0, s>>>(st.gsize, na, nmin, toff);
     PYFOF_CHECK_LAUNCH();
-    PYFOF_TRY(exclusive_scan_u32(flag, crank, na, reinterpret_cast<uint32_t *>(ctx.d_flags + FLAG_COUNT_A), W, s));
-    fof_member_kernel<<<grid, BLK, 0, s>>>(st.lab, gsize, crank, st.pos, na,
-                                           (uint32_t)a.np_halo_min, write_plain ? 1 : 0, pcand,
-                                           a.in_halo, a.halo_id);
-    PYFOF_CHECK_LAUNCH();
+    PYFOF_TRY(exclusive_scan_u32(toff, toff, ntile + 1, nullptr, W, s));
+    PYFOF_CUDA(cudaMemcpyAsync(ctx.d_flags + FLAG_COUNT_A, toff + ntile, sizeof(uint32_t), cudaMemcpyDeviceToDevice,
+                               s));
     PYFOF_CUDA(cudaMemcpyAsync(ctx.h_flags, ctx.d_flags, sizeof(int32_t) * FLAG_COUNT,
                                cudaMemcpyDeviceToHost, s));
     PYFOF_CUDA(cudaStreamSynchronize(s));
@@ -1596,8 +1710,6 @@ int32_t fof_candidates_stage(Context &ctx, const FofArgs &a, FofState &st, bool 
     st.ncand = (uint32_t)ctx.h_flags[FLAG_COUNT_A];
   }
   ctx.last_candidates = st.ncand;
-  st.gsize = gsize;
-  st.flag = flag;
   st.crank = crank;
   st.pcand = pcand;
   const int64_t nc = std::max<int64_t>(st.ncand, 1);
@@ -1605,15 +1717,24 @@ int32_t fof_candidates_stage(Context &ctx, const FofArgs &a, FofState &st, bool 
   st.cand_region = W.carve<int32_t>(nc);
   st.cand_np = W.carve<int32_t>(nc);
   st.cand_root = W.carve<int32_t>(nc);
-  if (!st.cand_anchor || !st.cand_region || !st.cand_np || !st.cand_root) {
+  int32_t *root = W.carve<int32_t>(nc);
+  uint32_t *first = W.carve<uint32_t>(nc);
+  if (!st.cand_anchor || !st.cand_region || !st.cand_np || !st.cand_root || !root || !first) {
     set_error("workspace exhausted (candidates)");
     return kAlloc;
   }
   if (st.ncand > 0) {
-    const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(na, BLK), (int64_t)kNumSMs * 16);
-    fof_cand_info_kernel<<<grid, BLK, 0, s>>>(flag, crank, st.pos, st.prid, gsize, na,
-                                              st.cand_anchor, st.cand_region, st.cand_np,
-                                              st.cand_root);
+    fof_cand_fill_kernel<<<(unsigned)ntile, BLK, 0, s>>>(st.gsize, na, nmin, toff, root);
+    PYFOF_CHECK_LAUNCH();
+    const unsigned gw = (unsigned)std::min<int64_t>(ceil_div(nc * 32, (int64_t)BLK), (int64_t)kNumSMs * 16);
+    fof_cand_anchor_kernel<<<gw, BLK, 0, s>>>(root, nc, st.lab, st.skey, st.cell_start, st.pos, first);
+    PYFOF_CHECK_LAUNCH();
+    const unsigned gc = (unsigned)std::min<int64_t>(ceil_div(nc, (int64_t)BLK), (int64_t)kNumSMs * 16);
+    fof_cand_info_kernel<<<gc, BLK, 0, s>>>(root, nc, first, st.skey, st.prid, st.gsize, crank, st.cand_anchor,
+                                            st.cand_region, st.cand_np, st.cand_root);
+    PYFOF_CHECK_LAUNCH();
+    fof_member_kernel<<<grid, BLK, 0, s>>>(st.lab, st.gsize, crank, st.pos, na, nmin, write_plain ? 1 : 0, pcand,
+                                           a.in_halo, a.halo_id);
     PYFOF_CHECK_LAUNCH();
   }
   return kOk;

@@ -32,7 +32,17 @@ struct RegionDev {
   // particles of one are linked by the exact distance test
   int32_t vd_k[3];
   float vd_inv[3];
+  double inv_size[3];  // 1 / size
+  uint64_t div[2];     // floor(2^64 / N) + 1 of the x and y axes (div_by)
+  // FP32 place of a particle in its cell (link kernel): (x - org) * cinv,
+  // within `slack` cells of the exact one; `near` = reach in cells + slack
+  float org[3], cinv[3], slack[3], near[3];
 };
+
+// n / N for 32-bit n, with div = floor(2^64 / N) + 1 (N > 1; N = 1: div = 0)
+__device__ __forceinline__ uint32_t div_by(uint32_t n, uint64_t div) {
+  return div ? (uint32_t)__umul64hi((uint64_t)n, div) : n;
+}
 
 struct Tile {
   int32_t region;
@@ -47,14 +57,15 @@ struct FofState {
   std::vector<RegionDev> reg;
   RegionDev *dR = nullptr;
   float4 *pos = nullptr;      // sorted FP32 coordinates, .w = original index bits
-  uint32_t *prid = nullptr;   // region of each sorted particle
+  uint32_t *prid = nullptr;   // region of each sorted particle (null: one region)
   int *parent = nullptr;      // DSU forest over sorted positions
   int *lab = nullptr;         // root (minimum sorted position) of every particle
-  uint32_t *skey = nullptr, *sidx = nullptr, *cell_start = nullptr, *keys_free = nullptr;
-  uint32_t *gsize = nullptr, *flag = nullptr, *crank = nullptr;
+  uint32_t *skey = nullptr, *cell_start = nullptr, *keys_free = nullptr;
+  uint32_t *gsize = nullptr;  // group size at each root, 0 elsewhere
+  uint32_t *crank = nullptr;  // candidate id at each candidate's root
   int32_t *pcand = nullptr;   // candidate of each sorted particle or -1
   uint32_t ncand = 0;
-  int64_t *cand_anchor = nullptr;  // original index of each candidate's first CRS member
+  int64_t *cand_anchor = nullptr;  // original index of each candidate's first member in the reference's order
   int32_t *cand_region = nullptr, *cand_np = nullptr, *cand_root = nullptr;
   float *phi_out = nullptr;   // optional: final potential of every packed member
 };

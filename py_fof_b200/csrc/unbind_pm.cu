@@ -1757,12 +1757,6 @@ __global__ void pm_fill_i32(int32_t *a, int64_t n, int32_t v) {
     a[i] = v;
 }
 
-__global__ void pm_fill_u8(uint8_t *a, int64_t n, uint8_t v) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    a[i] = v;
-}
-
 // Members per 16-cell region of every 256-grid halo
 // (bound_two_level_setup_ratios, bound_fortran.f90:551-568).
 __global__ void pm_region_count_kernel(const Members m, const PmHalo *__restrict__ H,

@@ -307,6 +307,19 @@ __device__ __forceinline__ void dsu_union(int *parent, int a, int b, int32_t *fl
   atomicExch(&flags[FLAG_ERR], kInvalid);  // unreachable: retry cap as a safety net
 }
 
+// Joins the sets of a and b; returns a root of the joined set.
+__device__ __forceinline__ int dsu_join(int *parent, int a, int b, int32_t *flags) {
+  for (int it = 0; it < (1 << 22); ++it) {
+    a = dsu_find(parent, a);
+    b = dsu_find(parent, b);
+    if (a == b) return a;
+    if (a > b) { int t = a; a = b; b = t; }
+    if (atomicCAS(parent + b, b, a) == b) return a;
+  }
+  atomicExch(&flags[FLAG_ERR], kInvalid);  // unreachable: retry cap as a safety net
+  return a;
+}
+
 struct LinkParams {
   double L, half, rp2;
   float rp2_open;   // largest float f with (double)f <= link^2
@@ -433,16 +446,6 @@ __device__ __forceinline__ void link_pair(int *parent, int p, int q, int &rp, in
   }
 }
 
-// Root hints: a root of q's set found earlier in the call.  Sets only
-// merge, so a hint equal to p's cached root rp means p and q already share a
-// set and the pair needs neither its distance test nor a union; any other
-// hint decides nothing (either may have been hung under a lower root since).
-// The dense kernel finds the hints of a batch of 32 sources in parallel, one
-// find per lane, instead of one dependent parent read per source and pair.
-
-// Ordered-integer image of a float (monotone: a < b  <=>  key(a) < key(b)
-// for non-NaN values), so warp min/max reductions of coordinates can use the
-// integer reduction instructions.  The map is its own inverse.
 // Sparse-cell particles, a warp per 32 consecutive sorted positions.  Each
 // lane lists the source ranges of its particle: the sparse cells among the
 // neighbour cells that the cube of half-width `reach` around it touches,
@@ -654,16 +657,70 @@ struct DenseChunk {
   uint32_t cell, e0;  // dense cell (global cell index), first index in its dpos list
 };
 
+// The warp's 32 particles against up to 32 sources, one per lane (o, q; hq a
+// root of q's set found earlier in the call, or -2 for no source).  Sets only
+// merge, so a source whose root is a particle's needs no test with it; and
+// once all particles of the chunk share a root, sources of that set are
+// dropped together.  A linked pair joins two whole sets: one lane joins them
+// and the others take the new root over, so a set is joined once and not by
+// every lane that links to it (in a dense core the kernel used to spend its
+// time on those repeated finds and compare-and-swaps).
+// rp: root of this lane's particle (-1: no particle).  own: the sources that
+// are to be tested from the lower sorted position only, as a lane mask.
+struct ChunkPair {
+  float4 me;
+  int ip, rp;
+};
+
+__device__ __forceinline__ void link_batch(ChunkPair &c, float4 o, int q, int hq, unsigned own, bool per,
+                                           const LinkParams &P, int *parent, int32_t *flags) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  // the root the whole chunk shares, or -1 (invalid lanes agree with any)
+  auto shared_root = [&]() -> int {
+    const unsigned valid = __ballot_sync(FULL, c.rp >= 0);
+    const int r0 = __shfl_sync(FULL, c.rp, __ffs(valid) - 1);
+    return __all_sync(FULL, c.rp < 0 || c.rp == r0) ? r0 : -1;
+  };
+  int all = shared_root();
+  unsigned mask = __ballot_sync(FULL, hq >= 0 && hq != all);
+  while (mask) {
+    const int src = __ffs(mask) - 1;
+    mask &= mask - 1;
+    int hs = __shfl_sync(FULL, hq, src);
+    const int qs = __shfl_sync(FULL, q, src);
+    bool lk = c.rp >= 0 && c.rp != hs && !(((own >> src) & 1) && qs <= c.ip);
+    if (!__any_sync(FULL, lk)) continue;
+    float4 so;
+    so.x = __shfl_sync(FULL, o.x, src);
+    so.y = __shfl_sync(FULL, o.y, src);
+    so.z = __shfl_sync(FULL, o.z, src);
+    so.w = 0.f;
+    if (lk) lk = per ? linked_pbc(c.me, so, P) : linked_open(c.me, so, P.rp2_open);
+    unsigned m = __ballot_sync(FULL, lk);
+    if (!m) continue;
+    do {
+      const int leader = __ffs(m) - 1;
+      const int old = __shfl_sync(FULL, c.rp, leader);
+      int r = 0;
+      if (lane == leader) r = dsu_join(parent, old, hs, flags);
+      r = __shfl_sync(FULL, r, leader);
+      if (c.rp == old || c.rp == hs) c.rp = r;
+      if (hq == old || hq == hs) hq = r;
+      hs = r;
+      m = __ballot_sync(FULL, lk && c.rp != r);
+    } while (m);
+    all = shared_root();
+    mask &= __ballot_sync(FULL, hq >= 0 && hq != all);
+  }
+}
+
 __global__ void __launch_bounds__(BLK, 3) fof_link_dense_kernel(
     const float4 *__restrict__ pos, const uint32_t *__restrict__ prid, const RegionDev *__restrict__ R,
     const uint32_t *__restrict__ cell_start, int *parent, const DenseChunk *__restrict__ chunks,
     int64_t nchunks, LinkParams P, DenseIndex D, int32_t *flags) {
   constexpr unsigned FULL = 0xffffffffu;
-  __shared__ float4 sbuf[BLK];
-  __shared__ int shint[BLK];
   const int lane = threadIdx.x & 31;
-  float4 *wbuf = sbuf + (threadIdx.x & ~31);
-  int *whint = shint + (threadIdx.x & ~31);
   const int64_t nw = ((int64_t)gridDim.x * BLK) >> 5;
   for (int64_t ch = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5; ch < nchunks; ch += nw) {
     const DenseChunk C = chunks[ch];
@@ -740,7 +797,10 @@ __global__ void __launch_bounds__(BLK, 3) fof_link_dense_kernel(
         }
       }
     }
-    int rp = valid ? dsu_find(parent, ip) : -1;  // cached root of this lane's particle
+    ChunkPair c{me, ip, valid ? dsu_find(parent, ip) : -1};
+    // the chunk with itself first: in a dense cell that already joins most of
+    // it, and the sources of its set are then skipped
+    if (!my_vd) link_batch(c, me, ip, c.rp, FULL, per, P, parent, flags);
     // --- cells that are one source range (sparse cells, dense cells of one
     // sub-cell): their sources packed into shared batches of 32
     {
@@ -768,11 +828,10 @@ __global__ void __launch_bounds__(BLK, 3) fof_link_dense_kernel(
         const bool oown = __shfl_sync(FULL, (int)own, owner) != 0;
         const float osh0 = __shfl_sync(FULL, sh[0], owner), osh1 = __shfl_sync(FULL, sh[1], owner),
                     osh2 = __shfl_sync(FULL, sh[2], owner);
-        bool cand = false;
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+        int q = -1, hq = -2;
         if (g < T) {
           const uint32_t t = ob + (g - oex);
-          float4 o;
-          int q;
           if (od) {
             o = D.dpos[t];
             q = __float_as_int(o.w);
@@ -782,7 +841,7 @@ __global__ void __launch_bounds__(BLK, 3) fof_link_dense_kernel(
           }
           const float osh[3] = {osh0, osh1, osh2};
           const float oc[3] = {o.x, o.y, o.z};
-          cand = true;
+          bool cand = true;
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
             if (open_ax[d]) continue;
@@ -790,25 +849,10 @@ __global__ void __launch_bounds__(BLK, 3) fof_link_dense_kernel(
             const float wh = __fadd_rn(__fadd_rn(bh[d], osh[d]), D.reach);
             cand = cand && oc[d] >= wl && oc[d] <= wh;
           }
-          o.w = __int_as_float(oown ? ~q : q);  // own-cell sources carry their flag
-          wbuf[lane] = o;
-          whint[lane] = cand ? dsu_find(parent, q) : -2;
+          if (cand) hq = dsu_find(parent, q);
         }
-        __syncwarp();
-        unsigned mask = __ballot_sync(FULL, cand);
-        while (mask) {
-          const int src = __ffs(mask) - 1;
-          mask &= mask - 1;
-          const float4 so = wbuf[src];
-          const int qw = __float_as_int(so.w);
-          const bool sown = qw < 0;
-          const int qs = sown ? ~qw : qw;
-          if (valid && whint[src] != rp && !(sown && qs <= ip)) {
-            const bool lk = per ? linked_pbc(me, so, P) : linked_open(me, so, P.rp2_open);
-            if (lk) link_pair(parent, ip, qs, rp, flags);
-          }
-        }
-        __syncwarp();
+        if (c.rp >= 0) c.rp = dsu_find(parent, c.rp);
+        link_batch(c, o, q, hq, __ballot_sync(FULL, oown), per, P, parent, flags);
       }
     }
     // --- dense cells of several sub-cells: one after the other, a source
@@ -852,30 +896,14 @@ __global__ void __launch_bounds__(BLK, 3) fof_link_dense_kernel(
             const int64_t t = base + lane;
             float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
             int q = -1, hq = -2;
-            bool cand = false;
             if (t < k1) {
               o = D.dpos[b + t];
               q = __float_as_int(o.w);
-              cand = o.x >= wl[0] && o.x <= wh[0] && o.y >= wl[1] && o.y <= wh[1] && o.z >= wl[2] &&
-                     o.z <= wh[2];
-              if (cand) hq = dsu_find(parent, q);
+              if (o.x >= wl[0] && o.x <= wh[0] && o.y >= wl[1] && o.y <= wh[1] && o.z >= wl[2] && o.z <= wh[2])
+                hq = dsu_find(parent, q);
             }
-            unsigned mask = __ballot_sync(FULL, cand);
-            while (mask) {
-              const int src = __ffs(mask) - 1;
-              mask &= mask - 1;
-              float4 so;
-              so.x = __shfl_sync(FULL, o.x, src);
-              so.y = __shfl_sync(FULL, o.y, src);
-              so.z = __shfl_sync(FULL, o.z, src);
-              so.w = 0.f;
-              const int qs = __shfl_sync(FULL, q, src);
-              const int hs = __shfl_sync(FULL, hq, src);
-              if (valid && hs != rp && !(own_n && qs <= ip)) {
-                const bool lk = per ? linked_pbc(me, so, P) : linked_open(me, so, P.rp2_open);
-                if (lk) link_pair(parent, ip, qs, rp, flags);
-              }
-            }
+            if (c.rp >= 0) c.rp = dsu_find(parent, c.rp);
+            link_batch(c, o, q, hq, own_n ? FULL : 0u, per, P, parent, flags);
           }
         }
     }

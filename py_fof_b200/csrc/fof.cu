@@ -640,11 +640,12 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
 
 // Dense cells, warp-cooperative: a warp takes a chunk of up to 32 particles
 // of one dense cell (consecutive in sub-cell order, so the chunk is
-// compact) and walks the neighbour cells and sub-cells that the chunk's
-// bounding box widened by `reach` can touch.  Sources come in coalesced
-// batches of 32; a source enters the pair loop only if it lies inside the
-// widened box, and then every lane tests it against its own particle with
-// the exact reference test.
+// compact) and walks the neighbour cells and sub-cell rows that the chunk's
+// bounding box widened by `reach` can touch: a lane per neighbour cell, then
+// a lane per row, whose source ranges are concatenated and read in full
+// batches of 32 (row by row, most batches held a few sources and each cost a
+// chain of dependent loads).  A source inside the widened box is tested by
+// every lane against its own particle with the exact reference test.
 //
 // Which side tests a pair: two dense cells, this kernel from the lower cell
 // (in one cell, from the lower sorted position); a dense and a sparse cell,
@@ -655,6 +656,17 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
 // reference's.
 struct DenseChunk {
   uint32_t cell, e0;  // dense cell (global cell index), first index in its dpos list
+};
+
+// A neighbour cell of a chunk: its particles, or the sub-cell rows of them
+// that the chunk's widened box [wl, wh] overlaps (ny x nz rows of nx
+// sub-cells, the first at s00; ny = 0: one range, all n particles).
+struct NbCell {
+  const uint32_t *tab;
+  uint32_t b, n;
+  float wl[3], wh[3];
+  int s00, sy, sz, nx, ny;
+  int dense, own;
 };
 
 // The warp's 32 particles against up to 32 sources, one per lane (o, q; hq a
@@ -715,12 +727,14 @@ __device__ __forceinline__ void link_batch(ChunkPair &c, float4 o, int q, int hq
   }
 }
 
-__global__ void __launch_bounds__(BLK, 3) fof_link_dense_kernel(
+__global__ void __launch_bounds__(BLK, 4) fof_link_dense_kernel(
     const float4 *__restrict__ pos, const uint32_t *__restrict__ prid, const RegionDev *__restrict__ R,
     const uint32_t *__restrict__ cell_start, int *parent, const DenseChunk *__restrict__ chunks,
     int64_t nchunks, LinkParams P, DenseIndex D, int32_t *flags) {
   constexpr unsigned FULL = 0xffffffffu;
+  __shared__ NbCell nb_cells[BLK / 32][27];
   const int lane = threadIdx.x & 31;
+  NbCell *cells = nb_cells[threadIdx.x >> 5];
   const int64_t nw = ((int64_t)gridDim.x * BLK) >> 5;
   for (int64_t ch = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5; ch < nchunks; ch += nw) {
     const DenseChunk C = chunks[ch];
@@ -763,57 +777,107 @@ __global__ void __launch_bounds__(BLK, 3) fof_link_dense_kernel(
       else { lo[d] = below ? -1 : 0; hi[d] = above ? 1 : 0; }
     }
     // --- neighbour cells, one per lane (lane = 9 (dz+1) + 3 (dy+1) + dx+1)
-    bool use = false, dense = false, own = false, single = false;
-    int64_t nb_b = 0, nb_e = 0, jcoord[3] = {0, 0, 0};
-    uint64_t jc = 0;
-    float sh[3] = {0.f, 0.f, 0.f};
+    uint32_t nrow = 0;  // source ranges of this lane's cell
     if (lane < 27) {
       const int off[3] = {lane % 3 - 1, (lane / 3) % 3 - 1, lane / 9 - 1};
-      use = true;
+      bool use = true;
+      int64_t jcoord[3];
+      NbCell &nc = cells[lane];
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
         if (off[d] < lo[d] || off[d] > hi[d]) use = false;
         int64_t j = ixyz[d] + off[d];
+        float sh = 0.f;
         if ((r.pdim >> d) & 1) {
-          if (j < 0) { j += Nd[d]; sh[d] = (float)P.L; } else if (j >= Nd[d]) { j -= Nd[d]; sh[d] = -(float)P.L; }
+          if (j < 0) { j += Nd[d]; sh = (float)P.L; } else if (j >= Nd[d]) { j -= Nd[d]; sh = -(float)P.L; }
         } else if (j < 0 || j >= Nd[d]) use = false;
         jcoord[d] = j;
+        // the widened box, in the neighbour's frame; none along periodic axes
+        // of one or two cells
+        nc.wl[d] = open_ax[d] ? -3e38f : __fsub_rn(__fadd_rn(bl[d], sh), D.reach);
+        nc.wh[d] = open_ax[d] ? 3e38f : __fadd_rn(__fadd_rn(bh[d], sh), D.reach);
       }
       if (use) {
         const int64_t jl = jcoord[0] + N0 * (jcoord[1] + N1 * jcoord[2]);
-        jc = r.cell_off + (uint64_t)jl;
-        nb_b = cell_start[jc];
-        nb_e = cell_start[jc + 1];
-        dense = nb_e - nb_b > DENSE_T;
+        const uint64_t jc = r.cell_off + (uint64_t)jl;
+        const uint32_t nb_b = cell_start[jc], n = cell_start[jc + 1] - nb_b;
+        const bool dense = n > (uint32_t)DENSE_T;
         // pairs with a lower dense cell are that cell's; pairs with sparse
         // cells are all tested here; pairs of two very dense cells are the
         // merge kernels'
-        if ((dense && jl < local) || nb_e == nb_b) use = false;
-        if (use && dense && my_vd && is_vd(r, nb_e - nb_b)) use = false;
-        own = jl == local;
-        if (use) {
-          const SubGrid g = dense ? dense_sub(r, nb_e - nb_b) : SubGrid{{1, 1, 1}, {0.f, 0.f, 0.f}};
-          single = g.s[0] * g.s[1] * g.s[2] == 1;
+        if (n > 0 && !(dense && jl < local) && !(dense && my_vd && is_vd(r, n))) {
+          nc.b = nb_b;
+          nc.n = n;
+          nc.dense = dense;
+          nc.own = jl == local;
+          nc.ny = 0;  // one range
+          nrow = 1;
+          if (dense) {
+            const SubGrid g = dense_sub(r, n);
+            if (g.s[0] * g.s[1] * g.s[2] > 1) {
+              int slo[3], shi[3];
+#pragma unroll
+              for (int d = 0; d < 3; ++d) {
+                const float clo = cell_lower(r, d, jcoord[d]);
+                slo[d] = sub_of(nc.wl[d], clo, g.inv[d], g.s[d]);
+                shi[d] = sub_of(nc.wh[d], clo, g.inv[d], g.s[d]);
+              }
+              nc.tab = D.tab + (int64_t)D.rank[jc] * D.stride;
+              nc.s00 = slo[0] + g.s[0] * (slo[1] + g.s[1] * slo[2]);
+              nc.sy = g.s[0];
+              nc.sz = g.s[0] * g.s[1];
+              nc.nx = shi[0] - slo[0] + 1;
+              nc.ny = shi[1] - slo[1] + 1;
+              nrow = (uint32_t)(nc.ny * (shi[2] - slo[2] + 1));
+            }
+          }
         }
       }
     }
+    uint32_t row_end = nrow;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(FULL, row_end, o);
+      if (lane >= o) row_end += v;
+    }
+    const uint32_t rows = __shfl_sync(FULL, row_end, 31);
+    __syncwarp();
     ChunkPair c{me, ip, valid ? dsu_find(parent, ip) : -1};
-    // the chunk with itself first: in a dense cell that already joins most of
-    // it, and the sources of its set are then skipped
-    if (!my_vd) link_batch(c, me, ip, c.rp, FULL, per, P, parent, flags);
-    // --- cells that are one source range (sparse cells, dense cells of one
-    // sub-cell): their sources packed into shared batches of 32
-    {
-      const uint32_t cnt = (use && single) ? (uint32_t)(nb_e - nb_b) : 0u;
+    for (uint32_t r0 = 0; r0 < rows; r0 += 32) {
+      // --- a row per lane
+      const uint32_t row = r0 + (uint32_t)lane;
+      int cell = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const uint32_t v = __shfl_sync(FULL, row_end, cell + step - 1);
+        if (v <= row) cell += step;
+      }
+      cell &= 31;
+      const uint32_t cell_row0 = __shfl_sync(FULL, row_end - nrow, cell);
+      uint32_t first = 0, cnt = 0;
+      if (row < rows) {
+        const NbCell &nc = cells[cell];
+        if (nc.ny == 0) {
+          first = nc.b;
+          cnt = nc.n;
+        } else {
+          const int k = (int)(row - cell_row0), z = k / nc.ny, y = k - z * nc.ny;
+          const uint32_t *t = nc.tab + nc.s00 + y * nc.sy + z * nc.sz;
+          const uint32_t k0 = t[0];
+          first = nc.b + k0;
+          cnt = t[nc.nx] - k0;
+        }
+      }
       uint32_t incl = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const uint32_t v = __shfl_up_sync(FULL, incl, o);
         if (lane >= o) incl += v;
       }
-      const uint32_t excl = incl - cnt;
       const uint32_t T = __shfl_sync(FULL, incl, 31);
+      const uint32_t at = first - (incl - cnt);  // source of batch index g: at + g
       for (uint32_t g0 = 0; g0 < T; g0 += 32) {
+        // --- a source per lane
         const uint32_t g = g0 + (uint32_t)lane;
         int owner = 0;
 #pragma unroll
@@ -822,91 +886,29 @@ __global__ void __launch_bounds__(BLK, 3) fof_link_dense_kernel(
           if (v <= g) owner += step;
         }
         owner &= 31;
-        const uint32_t ob = (uint32_t)__shfl_sync(FULL, (unsigned)nb_b, owner);
-        const uint32_t oex = __shfl_sync(FULL, excl, owner);
-        const bool od = __shfl_sync(FULL, (int)dense, owner) != 0;
-        const bool oown = __shfl_sync(FULL, (int)own, owner) != 0;
-        const float osh0 = __shfl_sync(FULL, sh[0], owner), osh1 = __shfl_sync(FULL, sh[1], owner),
-                    osh2 = __shfl_sync(FULL, sh[2], owner);
+        const uint32_t t = __shfl_sync(FULL, at, owner) + g;
+        const NbCell &nc = cells[__shfl_sync(FULL, cell, owner)];
         float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
         int q = -1, hq = -2;
+        bool own = false;
         if (g < T) {
-          const uint32_t t = ob + (g - oex);
-          if (od) {
+          if (nc.dense) {
             o = D.dpos[t];
             q = __float_as_int(o.w);
           } else {
             o = pos[t];
             q = (int)t;
           }
-          const float osh[3] = {osh0, osh1, osh2};
-          const float oc[3] = {o.x, o.y, o.z};
-          bool cand = true;
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            if (open_ax[d]) continue;
-            const float wl = __fsub_rn(__fadd_rn(bl[d], osh[d]), D.reach);
-            const float wh = __fadd_rn(__fadd_rn(bh[d], osh[d]), D.reach);
-            cand = cand && oc[d] >= wl && oc[d] <= wh;
-          }
-          if (cand) hq = dsu_find(parent, q);
+          own = nc.own != 0;
+          if (o.x >= nc.wl[0] && o.x <= nc.wh[0] && o.y >= nc.wl[1] && o.y <= nc.wh[1] && o.z >= nc.wl[2] &&
+              o.z <= nc.wh[2])
+            hq = dsu_find(parent, q);
         }
         if (c.rp >= 0) c.rp = dsu_find(parent, c.rp);
-        link_batch(c, o, q, hq, __ballot_sync(FULL, oown), per, P, parent, flags);
+        link_batch(c, o, q, hq, __ballot_sync(FULL, own), per, P, parent, flags);
       }
     }
-    // --- dense cells of several sub-cells: one after the other, a source
-    // range per sub-cell row the widened box overlaps
-    unsigned multi = __ballot_sync(FULL, use && !single);
-    while (multi) {
-      const int nl = __ffs(multi) - 1;
-      multi &= multi - 1;
-      const int64_t b = (int64_t)__shfl_sync(FULL, (unsigned long long)nb_b, nl);
-      const int64_t e = (int64_t)__shfl_sync(FULL, (unsigned long long)nb_e, nl);
-      const uint64_t jcn = __shfl_sync(FULL, (unsigned long long)jc, nl);
-      const bool own_n = __shfl_sync(FULL, (int)own, nl) != 0;
-      int64_t jcn3[3];
-      float wl[3], wh[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        jcn3[d] = (int64_t)__shfl_sync(FULL, (unsigned long long)jcoord[d], nl);
-        const float s = __shfl_sync(FULL, sh[d], nl);
-        if (open_ax[d]) {
-          wl[d] = -3e38f;
-          wh[d] = 3e38f;
-        } else {
-          wl[d] = __fsub_rn(__fadd_rn(bl[d], s), D.reach);
-          wh[d] = __fadd_rn(__fadd_rn(bh[d], s), D.reach);
-        }
-      }
-      const uint32_t *tab = D.tab + (int64_t)D.rank[jcn] * D.stride;
-      const SubGrid g = dense_sub(r, e - b);
-      int slo[3], shi[3];
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const float clo = cell_lower(r, d, jcn3[d]);
-        slo[d] = sub_of(wl[d], clo, g.inv[d], g.s[d]);
-        shi[d] = sub_of(wh[d], clo, g.inv[d], g.s[d]);
-      }
-      for (int sz = slo[2]; sz <= shi[2]; ++sz)
-        for (int sy = slo[1]; sy <= shi[1]; ++sy) {
-          const int s0 = slo[0] + g.s[0] * (sy + g.s[1] * sz);
-          const int64_t k0 = tab[s0], k1 = tab[s0 + (shi[0] - slo[0]) + 1];
-          for (int64_t base = k0; base < k1; base += 32) {
-            const int64_t t = base + lane;
-            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-            int q = -1, hq = -2;
-            if (t < k1) {
-              o = D.dpos[b + t];
-              q = __float_as_int(o.w);
-              if (o.x >= wl[0] && o.x <= wh[0] && o.y >= wl[1] && o.y <= wh[1] && o.z >= wl[2] && o.z <= wh[2])
-                hq = dsu_find(parent, q);
-            }
-            if (c.rp >= 0) c.rp = dsu_find(parent, c.rp);
-            link_batch(c, o, q, hq, own_n ? FULL : 0u, per, P, parent, flags);
-          }
-        }
-    }
+    __syncwarp();
   }
 }
 
@@ -950,12 +952,43 @@ __global__ void __launch_bounds__(BLK) fof_cells_kernel(const uint32_t *__restri
   if (lane == 0 && most > 0) atomicMax(&out[2], most);
 }
 
-// One block per dense cell: counting sort of its particles by sub-cell.
+// The pairs inside one chunk: the warp's adjacency as a 32-bit mask per lane,
+// its transitive closure (Warshall's algorithm, one lane per row), and every
+// particle hung under its component's lowest sorted position.  No other
+// thread touches these parents yet, so plain stores do.  Left to the linking
+// kernel, these are up to 31 dependent joins by compare-and-swap per chunk,
+// and every chunk nearby sees the members as separate sets meanwhile.
+__device__ __forceinline__ void link_chunk(float4 me, int ip, bool per, const LinkParams &P, int *parent) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  unsigned comp = 0;
+#pragma unroll 4
+  for (int j = 0; j < 32; ++j) {
+    float4 o;
+    o.x = __shfl_sync(FULL, me.x, j);
+    o.y = __shfl_sync(FULL, me.y, j);
+    o.z = __shfl_sync(FULL, me.z, j);
+    o.w = 0.f;
+    const int oip = __shfl_sync(FULL, ip, j);
+    const bool lk = ip >= 0 && oip >= 0 && (per ? linked_pbc(me, o, P) : linked_open(me, o, P.rp2_open));
+    if (lk || j == lane) comp |= 1u << j;
+  }
+  // (masks, not predicates: 32 of those do not fit)
+#pragma unroll 8
+  for (int j = 0; j < 32; ++j) comp |= __shfl_sync(FULL, comp, j) & (0u - ((comp >> j) & 1u));
+  unsigned root = (unsigned)ip;
+#pragma unroll 8
+  for (int j = 0; j < 32; ++j) root = min(root, (unsigned)__shfl_sync(FULL, ip, j) | (((comp >> j) & 1u) - 1u));
+  if ((int)root != ip) parent[ip] = (int)root;
+}
+
+// One block per dense cell: counting sort of its particles by sub-cell, then
+// the pairs inside its chunks.
 __global__ void __launch_bounds__(BLK) fof_dense_build_kernel(
     const uint32_t *__restrict__ list, const uint32_t *__restrict__ cs,
     const float4 *__restrict__ pos, const RegionDev *__restrict__ R,
     const uint64_t *__restrict__ cell_off, int nreg, int stride, uint32_t *__restrict__ tab,
-    float4 *__restrict__ dpos) {
+    float4 *dpos, LinkParams P, int *parent) {
   __shared__ uint32_t hist[SUB_MAX + 1];
   __shared__ uint32_t cur[SUB_MAX + 1];
   const uint32_t c = list[blockIdx.x];
@@ -1000,6 +1033,15 @@ __global__ void __launch_bounds__(BLK) fof_dense_build_kernel(
     const int sz = sub_of(v.z, clo[2], g.inv[2], g.s[2]);
     const uint32_t slot = atomicAdd(&cur[sx + g.s[0] * (sy + g.s[1] * sz)], 1u);
     dpos[base + slot] = make_float4(v.x, v.y, v.z, __int_as_float((int)(base + k)));
+  }
+  __syncthreads();
+  if (!is_vd(r, n)) {  // (very dense cells are joined sub-cell by sub-cell)
+    const int lane = threadIdx.x & 31, m = (int)n;
+    for (int e0 = 32 * (threadIdx.x >> 5); e0 < m; e0 += BLK) {
+      const bool valid = e0 + lane < m;
+      const float4 me = valid ? dpos[base + e0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+      link_chunk(me, valid ? __float_as_int(me.w) : -1, r.periodic != 0, P, parent);
+    }
   }
 }
 
@@ -1662,7 +1704,7 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
       uint32_t *tab = W.carve<uint32_t>(ndense * D.stride);
       if (!dpos || !tab) { set_error("workspace exhausted (dense tables)"); return kAlloc; }
       fof_dense_build_kernel<<<(unsigned)ndense, BLK, 0, s>>>(list, cstart, pos, dR, dcoff, nreg, D.stride, tab,
-                                                              dpos);
+                                                              dpos, P, parent);
       PYFOF_CHECK_LAUNCH();
       D.rank = drank;
       D.tab = tab;

@@ -40,7 +40,8 @@ namespace pyfof {
 
 namespace {
 
-constexpr int TILE = 4096;  // particles per block of the bbox and key kernels (16 per thread)
+constexpr int TILE = 4096;  // particles per block of the bbox, key and scatter kernels (16 per thread)
+constexpr int LU = 4;       // particles whose loads a thread has in flight there
 constexpr int BLK = 256;
 
 __device__ __forceinline__ int region_of_key(const uint64_t *cell_off, int nreg, uint64_t key) {
@@ -60,6 +61,19 @@ __device__ __forceinline__ void warp_minmax(double &mn, double &mx) {
   }
 }
 
+// Coordinates of particles i0, i0 + BLK, ..: all loads issued before any is
+// used (left in the loop, the branches of unwrap keep them apart, and the
+// kernels ran at a third of the memory rate).  Past `end`: `fill`.
+__device__ __forceinline__ void load_tile(const Coords &xp, int64_t i0, int64_t end, const double (&fill)[3],
+                                          double (&x)[LU][3]) {
+#pragma unroll
+  for (int u = 0; u < LU; ++u) {
+    const int64_t i = i0 + u * BLK;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) x[u][d] = i < end ? xp.get(i, d) : fill[d];
+  }
+}
+
 __global__ void __launch_bounds__(BLK) fof_bbox_kernel(Coords xp, const RegionDev *__restrict__ R,
                                                        const Tile *__restrict__ T, double L,
                                                        double half,
@@ -75,16 +89,18 @@ __global__ void __launch_bounds__(BLK) fof_bbox_kernel(Coords xp, const RegionDe
     mx[d] = -INFINITY;
   }
   bool bad = false;
-#pragma unroll 4
-  for (int64_t i = t.begin + threadIdx.x; i < t.end; i += BLK) {
+  for (int64_t i0 = t.begin + threadIdx.x; i0 < t.end; i0 += LU * BLK) {
+    double x[LU][3];
+    load_tile(xp, i0, t.end, anc, x);
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      double x = xp.get(i, d);
-      bad |= !isfinite(x);
-      double v = unwrap(x, anc[d], half, L);
-      mn[d] = fmin(mn[d], v);
-      mx[d] = fmax(mx[d], v);
-    }
+    for (int u = 0; u < LU; ++u)  // (past the end: the anchor, a particle of the region)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        bad |= !isfinite(x[u][d]);
+        const double v = unwrap(x[u][d], anc[d], half, L);
+        mn[d] = fmin(mn[d], v);
+        mx[d] = fmax(mx[d], v);
+      }
   }
   if (bad) atomicExch(&flags[FLAG_ERR], kNonFinite);
   __shared__ double smn[3][BLK / 32], smx[3][BLK / 32];
@@ -141,17 +157,27 @@ __global__ void __launch_bounds__(BLK) fof_key_kernel(Coords xp, const RegionDev
   }
   double anc[3];
   for (int d = 0; d < 3; ++d) anc[d] = xp.get(r.start, d);
-#pragma unroll 4
-  for (int64_t i = t.begin + threadIdx.x; i < t.end; i += BLK) {
-    uint32_t c[3];
+  for (int64_t i0 = t.begin + threadIdx.x; i0 < t.end; i0 += LU * BLK) {
+    double x[LU][3];
+    load_tile(xp, i0, t.end, anc, x);
+    uint32_t key[LU];
 #pragma unroll
-    for (int d = 0; d < 3; ++d)
-      c[d] = (uint32_t)cell_coord(unwrap(xp.get(i, d), anc[d], half, L), r.origin[d], r.size[d], r.inv_size[d],
-                                  r.N[d]);
-    const uint32_t key =
-        (uint32_t)r.cell_off + c[0] + (uint32_t)r.N[0] * (c[1] + (uint32_t)r.N[1] * c[2]);
-    keys[i] = key;
-    rank[i] = atomicAdd(&counts[key], 1u);  // a slot in the cell, in no particular order
+    for (int u = 0; u < LU; ++u) {
+      uint32_t c[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        c[d] = (uint32_t)cell_coord(unwrap(x[u][d], anc[d], half, L), r.origin[d], r.size[d], r.inv_size[d],
+                                    r.N[d]);
+      key[u] = (uint32_t)r.cell_off + c[0] + (uint32_t)r.N[0] * (c[1] + (uint32_t)r.N[1] * c[2]);
+    }
+#pragma unroll
+    for (int u = 0; u < LU; ++u) {
+      const int64_t i = i0 + u * BLK;
+      if (i < t.end) {
+        keys[i] = key[u];
+        rank[i] = atomicAdd(&counts[key[u]], 1u);  // a slot in the cell, in no particular order
+      }
+    }
   }
 }
 
@@ -172,16 +198,29 @@ __global__ void __launch_bounds__(BLK) fof_scatter_kernel(Coords xp, const Regio
   if (!r.active) return;
   double anc[3];
   for (int d = 0; d < 3; ++d) anc[d] = xp.get(r.start, d);
-#pragma unroll 4
-  for (int64_t i = t.begin + threadIdx.x; i < t.end; i += BLK) {
-    const uint32_t k = keys[i];
-    const uint32_t p = cstart[k] + rank[i];
-    float v[3];
+  for (int64_t i0 = t.begin + threadIdx.x; i0 < t.end; i0 += LU * BLK) {
+    double x[LU][3];
+    uint32_t k[LU], p[LU];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) v[d] = __double2float_rn(unwrap(xp.get(i, d), anc[d], half, L));
-    pos[p] = make_float4(v[0], v[1], v[2], __int_as_float((int)i));
-    skey[p] = k;
-    if (prid) prid[p] = (uint32_t)t.region;
+    for (int u = 0; u < LU; ++u) {
+      const int64_t i = i0 + u * BLK;
+      k[u] = i < t.end ? keys[i] : 0u;
+      p[u] = i < t.end ? rank[i] : 0u;
+    }
+    load_tile(xp, i0, t.end, anc, x);
+#pragma unroll
+    for (int u = 0; u < LU; ++u) p[u] += cstart[k[u]];
+#pragma unroll
+    for (int u = 0; u < LU; ++u) {
+      const int64_t i = i0 + u * BLK;
+      if (i >= t.end) break;
+      float v[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) v[d] = __double2float_rn(unwrap(x[u][d], anc[d], half, L));
+      pos[p[u]] = make_float4(v[0], v[1], v[2], __int_as_float((int)i));
+      skey[p[u]] = k[u];
+      if (prid) prid[p[u]] = (uint32_t)t.region;
+    }
   }
 }
 
@@ -465,6 +504,7 @@ __device__ __forceinline__ void link_pair(int *parent, int p, int q, int &rp, in
 // touches follow from its FP32 place in the cell (RegionDev::near) and the
 // rows need two loads each.
 constexpr int MAX_RANGES = 8;
+constexpr int kRounds = 2;
 
 // Pairs of particle ip with the sorted positions [b, e), tested at once.
 __device__ __noinline__ void link_range(const float4 *__restrict__ pos, float4 me, int ip, uint32_t b, uint32_t e,
@@ -486,7 +526,20 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ uint2 ranges[BLK][MAX_RANGES];  // (first source, count)
   __shared__ float4 target[BLK];
+  // linked pairs of the warp, joined 32 at a time: a join is a chain of
+  // dependent loads and a compare-and-swap, and only a few pairs of a round link
+  __shared__ int2 joins[BLK / 32][32 + 32 * kRounds];
+  int njoin = 0;
   const int lane = threadIdx.x & 31;
+  int2 *wjoin = joins[threadIdx.x >> 5];
+  auto join_queue = [&](int m) {  // the first m pairs of the queue, a lane each
+    if (lane < m) {
+      const int2 e = wjoin[lane];
+      int rp = -1;
+      link_pair(parent, e.x, e.y, rp, flags);
+    }
+    __syncwarp();
+  };
   const int wbase_t = threadIdx.x & ~31;
   const int64_t nw = ((int64_t)gridDim.x * BLK) >> 5;
   for (int64_t wb = (((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5) * 32; wb < n; wb += nw * 32) {
@@ -606,36 +659,63 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
     const uint32_t T = __shfl_sync(FULL, incl, 31);
     const unsigned per_mask = __ballot_sync(FULL, per);
     __syncwarp();
-    for (uint32_t g0 = 0; g0 < T; g0 += 32) {
-      const uint32_t g = g0 + (uint32_t)lane;
-      // owner lane of pair g: the number of lanes whose pairs end at or before g
-      int owner = 0;
+    // kRounds rounds at a time, so that their position loads overlap
+    for (uint32_t g0 = 0; g0 < T; g0 += 32 * kRounds) {
+      int own[kRounds], q[kRounds];
+      float4 o[kRounds];
 #pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const uint32_t v = __shfl_sync(FULL, incl, owner + step - 1);
-        if (v <= g) owner += step;
+      for (int u = 0; u < kRounds; ++u) {
+        const uint32_t g = g0 + 32 * u + (uint32_t)lane;
+        // owner lane of pair g: the number of lanes whose pairs end at or before g
+        int owner = 0;
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1) {
+          const uint32_t v = __shfl_sync(FULL, incl, owner + step - 1);
+          if (v <= g) owner += step;
+        }
+        owner &= 31;
+        uint32_t j = g - __shfl_sync(FULL, excl, owner);
+        own[u] = owner;
+        q[u] = -1;
+        if (g < T) {
+          const uint2 *rg = ranges[wbase_t + owner];
+          int k = 0;
+          while (j >= rg[k].y) {
+            j -= rg[k].y;
+            ++k;
+          }
+          q[u] = (int)(rg[k].x + j);
+          o[u] = pos[q[u]];
+        }
       }
-      owner &= 31;
-      uint32_t j = g - __shfl_sync(FULL, excl, owner);
-      if (g < T) {
-        const uint2 *rg = ranges[wbase_t + owner];
-        int k = 0;
-        while (j >= rg[k].y) {
-          j -= rg[k].y;
-          ++k;
+#pragma unroll
+      for (int u = 0; u < kRounds; ++u) {
+        bool lk = false;
+        if (q[u] >= 0) {
+          const float4 pm = target[wbase_t + own[u]];
+          lk = (per_mask >> own[u]) & 1 ? linked_pbc(pm, o[u], P) : linked_open(pm, o[u], P.rp2_open);
         }
-        const int q = (int)(rg[k].x + j);
-        const float4 o = pos[q];
-        const float4 pm = target[wbase_t + owner];
-        const bool lk = (per_mask >> owner) & 1 ? linked_pbc(pm, o, P) : linked_open(pm, o, P.rp2_open);
-        if (lk) {
-          int rp = -1;
-          link_pair(parent, (int)(wb + owner), q, rp, flags);
-        }
+        const unsigned m = __ballot_sync(FULL, lk);
+        if (lk) wjoin[njoin + __popc(m & lanemask_lt())] = make_int2((int)(wb + own[u]), q[u]);
+        njoin += __popc(m);
+      }
+      __syncwarp();
+      while (njoin >= 32) {
+        join_queue(32);
+        njoin -= 32;
+        // (at most 32 kRounds pairs are left)
+        int2 e[kRounds];
+#pragma unroll
+        for (int u = 0; u < kRounds; ++u) e[u] = wjoin[32 + 32 * u + lane];
+        __syncwarp();
+#pragma unroll
+        for (int u = 0; u < kRounds; ++u) wjoin[32 * u + lane] = e[u];
+        __syncwarp();
       }
     }
     __syncwarp();
   }
+  join_queue(njoin);
 }
 
 // Dense cells, warp-cooperative: a warp takes a chunk of up to 32 particles
@@ -1206,9 +1286,13 @@ __global__ void __launch_bounds__(BLK) fof_root_kernel(int *parent, int *lab, ui
       root = dsu_find(parent, (int)p);
       lab[p] = root;
     }
-    const unsigned peers = __match_any_sync(0xffffffffu, root);
-    const int leader = __ffs(peers) - 1;
-    if (root >= 0 && (int)(threadIdx.x & 31) == leader) atomicAdd(&gsize[root], (uint32_t)__popc(peers));
+    // one add per run of lanes with the same root (a match over the warp
+    // costs more than the adds it saves)
+    const int lane = threadIdx.x & 31;
+    const int prev = __shfl_up_sync(0xffffffffu, root, 1);
+    const bool head = lane == 0 || prev != root;
+    const unsigned later = __ballot_sync(0xffffffffu, head) & ~(0xffffffffu >> (31 - lane));
+    if (root >= 0 && head) atomicAdd(&gsize[root], (uint32_t)((later ? __ffs(later) - 1 : 32) - lane));
   }
 }
 

@@ -137,14 +137,16 @@ __device__ __forceinline__ int32_t cell_coord(double x, double origin, double si
   return __double2int_rz(f);
 }
 
-// sentinel != 0: particles of inactive regions get that key and a slot too
-// (the sorts of option cell_order take all particles).
+// all != 0: particles of inactive regions get the sentinel key and a slot too
+// (the sorts of option cell_order take all particles).  flags[FLAG_SPREAD]:
+// warps, one sample of 32 consecutive particles each, whose keys span more
+// than `far`.
 __global__ void __launch_bounds__(BLK) fof_key_kernel(Coords xp, const RegionDev *__restrict__ R,
                                                       const Tile *__restrict__ T, double L,
                                                       double half, uint32_t sentinel, int all,
-                                                      uint32_t *__restrict__ keys,
+                                                      uint32_t far, uint32_t *__restrict__ keys,
                                                       uint32_t *__restrict__ counts,
-                                                      uint32_t *__restrict__ rank) {
+                                                      uint32_t *__restrict__ rank, int32_t *flags) {
   const Tile t = T[blockIdx.x];
   const RegionDev &r = R[t.region];
   if (!r.active) {
@@ -170,6 +172,11 @@ __global__ void __launch_bounds__(BLK) fof_key_kernel(Coords xp, const RegionDev
                                     r.N[d]);
       key[u] = (uint32_t)r.cell_off + c[0] + (uint32_t)r.N[0] * (c[1] + (uint32_t)r.N[1] * c[2]);
     }
+    if (i0 < t.begin + BLK) {  // the tile's first round (past the end: the anchor's key)
+      const unsigned act = __activemask();
+      const uint32_t lo = __reduce_min_sync(act, key[0]), hi = __reduce_max_sync(act, key[0]);
+      if (hi - lo > far && (threadIdx.x & 31) == 0) atomicAdd(&flags[FLAG_SPREAD], 1);
+    }
 #pragma unroll
     for (int u = 0; u < LU; ++u) {
       const int64_t i = i0 + u * BLK;
@@ -182,17 +189,16 @@ __global__ void __launch_bounds__(BLK) fof_key_kernel(Coords xp, const RegionDev
 }
 
 // FP32 coordinates to cell start + slot.  Reads the coordinates again, in
-// input order (24 B a particle, coalesced), and writes 20 B at the sorted
-// position: bound by those writes when the input order is not spatial.  (A
-// gather by sorted index reads three sectors per particle instead, after a
-// sort of the indices: 1.75 ms against 0.6 ms for a shuffled 256^3 box.)
+// input order (24 B a particle, coalesced), and writes 16 B at the sorted
+// position (its cell there, skey, comes from fof_cells_kernel, in order).
+// (A gather by sorted index reads three sectors per particle
+// instead, after a sort of the indices.)
 __global__ void __launch_bounds__(BLK) fof_scatter_kernel(Coords xp, const RegionDev *__restrict__ R,
                                                           const Tile *__restrict__ T, double L, double half,
                                                           const uint32_t *__restrict__ keys,
                                                           const uint32_t *__restrict__ rank,
                                                           const uint32_t *__restrict__ cstart,
-                                                          float4 *__restrict__ pos, uint32_t *__restrict__ skey,
-                                                          uint32_t *__restrict__ prid) {
+                                                          float4 *__restrict__ pos, uint32_t *__restrict__ prid) {
   const Tile t = T[blockIdx.x];
   const RegionDev &r = R[t.region];
   if (!r.active) return;
@@ -218,10 +224,103 @@ __global__ void __launch_bounds__(BLK) fof_scatter_kernel(Coords xp, const Regio
 #pragma unroll
       for (int d = 0; d < 3; ++d) v[d] = __double2float_rn(unwrap(x[u][d], anc[d], half, L));
       pos[p[u]] = make_float4(v[0], v[1], v[2], __int_as_float((int)i));
-      skey[p[u]] = k[u];
       if (prid) prid[p[u]] = (uint32_t)t.region;
     }
   }
+}
+
+// The same in two steps for one region whose consecutive particles lie far
+// apart (use_partition).  The direct scatter then writes single 16-byte pieces
+// all over an output larger than L2, each a sector read and written in HBM:
+// 1.26 ms (with the cells) for a shuffled box of 15.8 M particles; five passes
+// over windows of the output that fit L2 took 0.94 ms.  Here a tile first deals its particles
+// to kBuckets ranges of cells, whose places in the output are known (cell
+// starts): a run of the output per tile and bucket, reserved by one atomic;
+// then the particles move on to their slots, a bucket's megabyte at a time.
+constexpr int kBuckets = 256;
+
+__device__ __forceinline__ uint32_t bucket_of(uint32_t key, uint32_t ncell) {
+  return (uint32_t)(((uint64_t)key * kBuckets) / ncell);
+}
+
+// cursor[b] = first position of bucket b (its first cell: the lowest key
+// with bucket_of(key) = b)
+__global__ void fof_bucket_start_kernel(const uint32_t *__restrict__ cstart, uint32_t ncell,
+                                        uint32_t *__restrict__ cursor) {
+  const uint32_t b = threadIdx.x;
+  if (b < (uint32_t)kBuckets) cursor[b] = cstart[((uint64_t)b * ncell + kBuckets - 1) / kBuckets];
+}
+
+constexpr int PTILE = 4096;
+
+__global__ void __launch_bounds__(BLK) fof_partition_kernel(Coords xp, int64_t n, double L, double half,
+                                                            const uint32_t *__restrict__ keys,
+                                                            const uint32_t *__restrict__ rank, uint32_t ncell,
+                                                            uint32_t *__restrict__ cursor, float4 *__restrict__ tpos,
+                                                            uint2 *__restrict__ tkey) {
+  __shared__ uint32_t cnt[kBuckets], base[kBuckets];
+  static_assert(kBuckets == BLK, "a bucket per thread");
+  cnt[threadIdx.x] = 0;
+  __syncthreads();
+  const int64_t b0 = (int64_t)blockIdx.x * PTILE, end = min(n, b0 + PTILE);
+  uint32_t key[PTILE / BLK], at[PTILE / BLK];
+#pragma unroll
+  for (int j = 0; j < PTILE / BLK; ++j) {
+    const int64_t i = b0 + j * BLK + threadIdx.x;
+    key[j] = i < end ? keys[i] : 0u;
+  }
+#pragma unroll
+  for (int j = 0; j < PTILE / BLK; ++j)
+    if (b0 + j * BLK + threadIdx.x < end) at[j] = atomicAdd(&cnt[bucket_of(key[j], ncell)], 1u);
+  __syncthreads();
+  const uint32_t c = cnt[threadIdx.x];
+  base[threadIdx.x] = c ? atomicAdd(&cursor[threadIdx.x], c) : 0u;
+  __syncthreads();
+  double anc[3];
+  for (int d = 0; d < 3; ++d) anc[d] = xp.get(0, d);
+#pragma unroll
+  for (int j0 = 0; j0 < PTILE / BLK; j0 += LU) {
+    const int64_t i0 = b0 + j0 * BLK + threadIdx.x;
+    double x[LU][3];
+    load_tile(xp, i0, end, anc, x);
+    uint32_t s[LU];
+#pragma unroll
+    for (int u = 0; u < LU; ++u) s[u] = i0 + u * BLK < end ? rank[i0 + u * BLK] : 0u;
+#pragma unroll
+    for (int u = 0; u < LU; ++u) {
+      if (i0 + u * BLK >= end) break;
+      float v[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) v[d] = __double2float_rn(unwrap(x[u][d], anc[d], half, L));
+      const uint32_t q = base[bucket_of(key[j0 + u], ncell)] + at[j0 + u];
+      tpos[q] = make_float4(v[0], v[1], v[2], __int_as_float((int)(i0 + u * BLK)));
+      tkey[q] = make_uint2(key[j0 + u], s[u]);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(BLK) fof_place_kernel(const float4 *__restrict__ tpos,
+                                                        const uint2 *__restrict__ tkey, int64_t n,
+                                                        const uint32_t *__restrict__ cstart,
+                                                        float4 *__restrict__ pos) {
+  const int64_t i0 = (int64_t)blockIdx.x * (LU * BLK) + threadIdx.x;
+  uint2 k[LU];
+  float4 v[LU];
+#pragma unroll
+  for (int u = 0; u < LU; ++u)
+    if (i0 + u * BLK < n) {
+      k[u] = tkey[i0 + u * BLK];
+      v[u] = tpos[i0 + u * BLK];
+    }
+#pragma unroll
+  for (int u = 0; u < LU; ++u)
+    if (i0 + u * BLK < n) pos[cstart[k[u].x] + k[u].y] = v[u];
+}
+
+// Whether the two-step scatter pays: one region, most sampled warps hold
+// particles far apart, and the output (20 B a particle) does not fit half of L2.
+static bool use_partition(int nreg, int64_t n_active, int64_t ntiles, int32_t spread) {
+  return nreg == 1 && 16.0 * (double)n_active > 64e6 && (int64_t)spread * 2 >= ntiles * (BLK / 32);
 }
 
 // ---- the CRS order itself (option cell_order) ------------------------------
@@ -490,10 +589,9 @@ __device__ __forceinline__ void link_pair(int *parent, int p, int q, int &rp, in
 // neighbour cells that the cube of half-width `reach` around it touches,
 // from its own cell on (higher keys; in the own cell, the higher positions).
 // Cells that are neighbours along x are consecutive in cell order, so a row
-// of them is one range: at most four rows and two wrapped cells where cells
-// are wider than two linking lengths.  Narrower cells, and rows broken up by
-// dense cells, can give more; a lane tests the ranges beyond the first
-// MAX_RANGES itself, right away.  The warp then runs all pairs of all lanes
+// of them is one range: at most five rows and as many wrapped cells.  Rows
+// broken up by dense cells, and axes of one or two cells, can give more; a
+// lane tests the ranges beyond the first MAX_RANGES itself, right away.  The warp then runs all pairs of all lanes
 // in rounds of 32, one pair per lane (a lane finds its pair's particle by a
 // binary search over the lanes' pair offsets and its source by walking that
 // particle's ranges), so the lanes stay busy however unevenly the pairs are
@@ -503,7 +601,7 @@ __device__ __forceinline__ void link_pair(int *parent, int p, int q, int &rp, in
 // test.  So the cell is decoded by multiplication, the cells its reach
 // touches follow from its FP32 place in the cell (RegionDev::near) and the
 // rows need two loads each.
-constexpr int MAX_RANGES = 8;
+constexpr int MAX_RANGES = 10;
 constexpr int kRounds = 2;
 
 // Pairs of particle ip with the sorted positions [b, e), tested at once.
@@ -541,18 +639,26 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
     __syncwarp();
   };
   const int wbase_t = threadIdx.x & ~31;
-  const int64_t nw = ((int64_t)gridDim.x * BLK) >> 5;
-  for (int64_t wb = (((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5) * 32; wb < n; wb += nw * 32) {
+  const int64_t step_w = (int64_t)gridDim.x * BLK;
+  int64_t wb = (((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5) * 32;
+  // the next particle's cell and position are loaded an iteration ahead
+  uint32_t next_cell = wb + lane < n ? skey[wb + lane] : 0u;
+  float4 next_me = wb + lane < n ? pos[wb + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (; wb < n; wb += step_w) {
     const int64_t w = wb + lane;
     const int ip = (int)w;
     uint32_t total = 0;
     int nr = 0;
     bool per = false;
+    const uint32_t cell = next_cell;
+    const float4 me = next_me;
+    const uint32_t own_begin = cs[cell], own_end = cs[cell + 1];
+    if (w + step_w < n) {
+      next_cell = skey[w + step_w];
+      next_me = pos[w + step_w];
+    }
     if (w < n) {
-      const uint32_t cell = skey[w];
-      const uint32_t own_end = cs[cell + 1];
-      if (own_end - cs[cell] <= (uint32_t)DENSE_T) {
-        const float4 me = pos[w];
+      if (own_end - own_begin <= (uint32_t)DENSE_T) {
         const RegionDev &r = R[prid ? prid[w] : 0];
         per = r.periodic != 0;
         target[threadIdx.x] = me;
@@ -582,14 +688,9 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
             link_range(pos, me, ip, b, e, r.periodic, P, parent, flags);
           }
         };
-        // the sparse cells c0..c1 (consecutive along x), positions from `from` on
-        auto add_row = [&](uint32_t c0, uint32_t c1, uint32_t from) {
-          const uint32_t b = cs[c0], e = cs[c1 + 1];
-          if (e == b) return;
-          if (e - b <= (uint32_t)DENSE_T) {
-            add(max(b, from), e);
-            return;
-          }
+        // the sparse cells among c0..c1, positions from `from` on
+        auto add_cells = [&](uint32_t c0, uint32_t c1, uint32_t from) {
+#pragma unroll 1
           for (uint32_t c = c0; c <= c1; ++c) {
             const uint32_t cb = cs[c], ce = cs[c + 1];
             if (ce - cb <= (uint32_t)DENSE_T) add(max(cb, from), ce);
@@ -600,19 +701,35 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
           // x neighbours: a run of cells, and the cell around the box's edge
           const int x0 = below[0] && ix > 0 ? -1 : 0, x1 = above[0] && ix < N0 - 1 ? 1 : 0;
           const bool lo_wrap = px && below[0] && ix == 0, hi_wrap = px && above[0] && ix == N0 - 1;
-          add_row(cell, cell + x1, (uint32_t)ip + 1);
-          if (lo_wrap) add_row(cell + (N0 - 1), cell + (N0 - 1), 0);
-          auto forward = [&](int dy, int dz) {
-            const uint32_t c = cell + (uint32_t)(N0 * (dy + N1 * dz));
-            add_row(c + x0, c + x1, 0);
-            if (lo_wrap) add_row(c + (N0 - 1), c + (N0 - 1), 0);
-            if (hi_wrap) add_row(c - (N0 - 1), c - (N0 - 1), 0);
-          };
-          if (above[1]) forward(1, 0);
-          if (above[2]) {
-            if (below[1]) forward(-1, 1);
-            forward(0, 1);
-            if (above[1]) forward(1, 1);
+          // the rows to visit: own, then (y, z) = (+1, 0), (-1, +1), (0, +1),
+          // (+1, +1); all their bounds are loaded before the first is used
+          const bool need[5] = {true, above[1], above[2] && below[1], above[2], above[2] && above[1]};
+          const int step[5] = {0, N0, N0 * (N1 - 1), N0 * N1, N0 * (N1 + 1)};
+          uint32_t rb[5], re[5];
+#pragma unroll
+          for (int i = 0; i < 5; ++i) {
+            const uint32_t c = cell + (uint32_t)step[i];
+            rb[i] = i ? (need[i] ? cs[c + x0] : 0u) : own_begin;
+            re[i] = need[i] ? cs[c + x1 + 1] : 0u;
+          }
+#pragma unroll
+          for (int i = 0; i < 5; ++i) {
+            if (re[i] == rb[i]) continue;
+            if (re[i] - rb[i] <= (uint32_t)DENSE_T) {
+              add(i ? rb[i] : (uint32_t)ip + 1, re[i]);
+            } else {
+              const uint32_t c = cell + (uint32_t)step[i];
+              add_cells(i ? c + x0 : c, c + x1, i ? 0u : (uint32_t)ip + 1);
+            }
+          }
+          if (lo_wrap || hi_wrap) {
+#pragma unroll 1
+            for (int i = lo_wrap ? 0 : 1; i < 5; ++i) {
+              const int dz = i > 1 ? 1 : 0, dy = i > 1 ? i - 3 : i;
+              if ((dz && !above[2]) || (dy > 0 && !above[1]) || (dy < 0 && !below[1])) continue;
+              const uint32_t c = cell + (uint32_t)(N0 * (dy + N1 * dz)) + (lo_wrap ? N0 - 1 : 1 - N0);
+              add_cells(c, c, 0);
+            }
           }
         } else {
           const int ic[3] = {ix, iy, iz}, Nd[3] = {N0, N1, N2};
@@ -643,7 +760,7 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
                 if (!in) continue;
                 const uint32_t jl = (uint32_t)j[0] + (uint32_t)N0 * ((uint32_t)j[1] + (uint32_t)N1 * (uint32_t)j[2]);
                 if (jl < local) continue;
-                add_row(coff + jl, coff + jl, jl == local ? (uint32_t)ip + 1 : 0);
+                add_cells(coff + jl, coff + jl, jl == local ? (uint32_t)ip + 1 : 0);
               }
         }
       }
@@ -992,20 +1109,30 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_dense_kernel(
   }
 }
 
-// Dense cells, their numbers and their chunks of up to 32 particles, in no
-// particular order, and the fullest cell.  out: [0] dense cells, [1] chunks,
+// The cell of every sorted position (skey), the dense cells, their numbers and
+// their chunks of up to 32 particles, in no particular order, and the
+// fullest cell.  out: [0] dense cells, [1] chunks,
 // [2] largest count (zeroed before).
 __global__ void __launch_bounds__(BLK) fof_cells_kernel(const uint32_t *__restrict__ cs, int64_t ncell,
                                                         uint32_t *__restrict__ out, uint32_t *__restrict__ list,
-                                                        uint32_t *__restrict__ rank, DenseChunk *__restrict__ chunks) {
+                                                        uint32_t *__restrict__ rank, DenseChunk *__restrict__ chunks,
+                                                        uint32_t *__restrict__ skey) {
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   uint32_t most = 0;
   for (int64_t base = (int64_t)blockIdx.x * BLK; base < ncell; base += (int64_t)gridDim.x * BLK) {
     const int64_t c = base + threadIdx.x;
-    const uint32_t n = c < ncell ? cs[c + 1] - cs[c] : 0u;
+    const uint32_t b = c < ncell ? cs[c] : 0u, n = c < ncell ? cs[c + 1] - b : 0u;
     most = max(most, n);
+    // the cell of every sorted position: small cells by their lane, in step
+    // with the neighbour lanes' stores, the others by the warp
     const unsigned m = __ballot_sync(FULL, n > (uint32_t)DENSE_T);
+    for (uint32_t j = 0; j < n && n <= (uint32_t)DENSE_T; ++j) skey[b + j] = (uint32_t)c;
+    for (unsigned k = m; k; k &= k - 1) {
+      const int src = __ffs(k) - 1;
+      const uint32_t sb = __shfl_sync(FULL, b, src), sn = __shfl_sync(FULL, n, src);
+      for (uint32_t j = lane; j < sn; j += 32) skey[sb + j] = (uint32_t)(c - lane + src);
+    }
     if (!m) continue;
     const uint32_t nch = n > (uint32_t)DENSE_T ? (n + 31u) / 32u : 0u;
     uint32_t incl = nch;
@@ -1685,8 +1812,8 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
   if (!slot || !skey || !pos || (nreg > 1 && !prid)) { set_error("workspace exhausted (keys)"); return kAlloc; }
   const uint32_t sentinel = (uint32_t)total_cells;
   if (ntiles) {
-    fof_key_kernel<<<(unsigned)ntiles, BLK, 0, s>>>(xp, dR, dT, L, half, sentinel, a.cell_order != 0, keys, cstart,
-                                                    slot);
+    fof_key_kernel<<<(unsigned)ntiles, BLK, 0, s>>>(xp, dR, dT, L, half, sentinel, a.cell_order != 0,
+                                                    (uint32_t)(total_cells / 64), keys, cstart, slot, ctx.d_flags);
     PYFOF_CHECK_LAUNCH();
   }
   PYFOF_TRY(exclusive_scan_u32(cstart, cstart, (int64_t)total_cells + 1, nullptr, W, s));
@@ -1701,16 +1828,32 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
   PYFOF_CUDA(cudaMemsetAsync(dcells, 0, 3 * sizeof(uint32_t), s));
   if (total_cells > 0) {
     const unsigned cgrid = (unsigned)std::min<int64_t>(ceil_div((int64_t)total_cells, (int64_t)BLK), (int64_t)kNumSMs * 16);
-    fof_cells_kernel<<<cgrid, BLK, 0, s>>>(cstart, (int64_t)total_cells, dcells, list, drank, dchunks);
+    fof_cells_kernel<<<cgrid, BLK, 0, s>>>(cstart, (int64_t)total_cells, dcells, list, drank, dchunks, skey);
     PYFOF_CHECK_LAUNCH();
   }
   PYFOF_CUDA(cudaMemcpyAsync(ctx.h_flags, ctx.d_flags, sizeof(int32_t) * FLAG_COUNT, cudaMemcpyDeviceToHost, s));
   ctx.last_cell_sorts = 0;
-  if (a.cell_order == 0 && n_active > 0) {
-    fof_scatter_kernel<<<(unsigned)ntiles, BLK, 0, s>>>(xp, dR, dT, L, half, keys, slot, cstart, pos, skey, prid);
-    PYFOF_CHECK_LAUNCH();
-  }
   PYFOF_CUDA(cudaStreamSynchronize(s));
+  float4 *spare = nullptr;  // a float4 per particle, free after the scatter
+  if (a.cell_order == 0 && n_active > 0) {
+    if (use_partition(nreg, n_active, ntiles, ctx.h_flags[FLAG_SPREAD])) {
+      spare = W.carve<float4>(n_active);
+      uint2 *tkey = W.carve<uint2>(n_active);
+      uint32_t *cursor = W.carve<uint32_t>(kBuckets);
+      if (!spare || !tkey || !cursor) { set_error("workspace exhausted (scatter)"); return kAlloc; }
+      fof_bucket_start_kernel<<<1, kBuckets, 0, s>>>(cstart, (uint32_t)total_cells, cursor);
+      PYFOF_CHECK_LAUNCH();
+      fof_partition_kernel<<<(unsigned)ceil_div(n, (int64_t)PTILE), BLK, 0, s>>>(xp, n, L, half, keys, slot,
+                                                                                 (uint32_t)total_cells, cursor, spare,
+                                                                                 tkey);
+      PYFOF_CHECK_LAUNCH();
+      fof_place_kernel<<<(unsigned)ceil_div(n, (int64_t)LU * BLK), BLK, 0, s>>>(spare, tkey, n, cstart, pos);
+      PYFOF_CHECK_LAUNCH();
+    } else {
+      fof_scatter_kernel<<<(unsigned)ntiles, BLK, 0, s>>>(xp, dR, dT, L, half, keys, slot, cstart, pos, prid);
+      PYFOF_CHECK_LAUNCH();
+    }
+  }
   const int64_t ndense = (uint32_t)ctx.h_flags[FLAG_COUNT_A], ndense_chunks = (uint32_t)ctx.h_flags[FLAG_COUNT_B];
   const uint32_t max_occ = (uint32_t)ctx.h_flags[FLAG_COUNT_C];
   ctx.last_max_cell = max_occ;
@@ -1784,7 +1927,7 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
           smax = std::max(smax, reg[r].vd_k[0] * reg[r].vd_k[1] * reg[r].vd_k[2]);
         }
       D.stride = smax + 1;
-      float4 *dpos = W.carve<float4>(n_active);
+      float4 *dpos = spare ? spare : W.carve<float4>(n_active);
       uint32_t *tab = W.carve<uint32_t>(ndense * D.stride);
       if (!dpos || !tab) { set_error("workspace exhausted (dense tables)"); return kAlloc; }
       fof_dense_build_kernel<<<(unsigned)ndense, BLK, 0, s>>>(list, cstart, pos, dR, dcoff, nreg, D.stride, tab,

@@ -1213,17 +1213,6 @@ __device__ __forceinline__ double bsum_d(double v, double *red) {
   return t;
 }
 
-__device__ __forceinline__ int bsum_i(int v, int *red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  int t = 0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-  __syncthreads();
-  return t;
-}
-
 // Seven block sums at once: each value is reduced in the same order as by
 // bsum_d (warp butterfly, then the warp partials in warp order), so the
 // results are bit-identical, with 2 barriers instead of 21.
@@ -1245,9 +1234,55 @@ __device__ __forceinline__ void bsum7_d(double *v, double *red) {
   }
 }
 
+// The digit of the need-th largest key, from a 256-bin histogram of one digit
+// of the keys: bins are summed from the top.  Every warp does it alone (eight
+// bins per lane, a suffix scan over the lanes).  Returns the digit; above =
+// keys in higher bins, count = keys in it.
+__device__ __forceinline__ int digit_of(const unsigned *hist, int need, int &above, int &count) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  int c[8], sum = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    c[j] = (int)hist[8 * lane + j];
+    sum += c[j];
+  }
+  int suffix = sum;  // this lane's bins and all higher ones
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_down_sync(FULL, suffix, o);
+    if (lane + o < 32) suffix += v;
+  }
+  // the highest lane whose suffix reaches `need` holds the digit
+  const int src = 31 - __clz(__ballot_sync(FULL, suffix >= need));
+  int ab = suffix - sum, digit = 0, cnt = 0;
+  bool found = false;
+#pragma unroll
+  for (int j = 7; j >= 0; --j) {
+    if (!found && ab + c[j] >= need) {
+      digit = 8 * lane + j;
+      cnt = c[j];
+      found = true;
+    }
+    if (!found) ab += c[j];
+  }
+  above = __shfl_sync(FULL, ab, src);
+  count = __shfl_sync(FULL, cnt, src);
+  return __shfl_sync(FULL, digit, src);
+}
+
 // One block per pending halo: combine the potential, then the inner
 // removal loop of bound_check_grid (:2739-2855).  Leaves status -1 when the
 // potential must be refreshed (next pass).
+//
+// A chain of sweeps over the members with a barrier between them, bound by
+// latency.  An iteration sweeps all members twice (centre, energies); the
+// unbound ones go as 64-bit keys (energy, then ~index, so the order is total)
+// to shared memory, and the nb-th largest key is found by a radix select over
+// that list.  Only when more than KCAP are unbound are the energies selected
+// from memory, by sweeps over all members.
+constexpr int KCAP = 4096;
+
 template <typename R>
 __global__ void __launch_bounds__(IBLK) pm_inner_kernel(const Members m, PmHalo *__restrict__ H,
                                                         const int32_t *__restrict__ list, int nlist,
@@ -1266,12 +1301,15 @@ __global__ void __launch_bounds__(IBLK) pm_inner_kernel(const Members m, PmHalo 
   __shared__ double red7[7 * (IBLK / 32)];
   __shared__ int red_i[IBLK / 32];
   __shared__ unsigned hist[256];
-  __shared__ int s_err;
-  const int64_t b0 = p.off, np = p.np;
+  __shared__ unsigned long long ukey[KCAP];
+  __shared__ int s_err, s_nu;
+  const int64_t b0 = p.off;
+  const int np = p.np;
+  const int lane = threadIdx.x & 31;
   if (threadIdx.x == 0) s_err = 0;
   int np_bound = p.np_bound;
   const int n_source = np_bound;
-  for (int64_t i = threadIdx.x; i < np; i += IBLK) {
+  for (int i = threadIdx.x; i < np; i += IBLK) {
     const int64_t k = b0 + i;
     if (!keep[k]) continue;
     float v = (float)((phi_c1[k] + phi_in[k]) + phi_c2[k]);
@@ -1288,12 +1326,17 @@ __global__ void __launch_bounds__(IBLK) pm_inner_kernel(const Members m, PmHalo 
     if (threadIdx.x == 0) { p.status = 0; p.pending = 0; }
     return;
   }
+  auto remove = [&](int i) {
+    const int64_t k = b0 + i;
+    keep[k] = 0;
+    rflag[epos[k]] = 1;
+  };
   int deleted = 0, status = -1;
   for (;;) {
     double a7[7] = {0, 0, 0, 0, 0, 0, 0};
-    // top-digit histogram of the energies, filled by the energy sweep below
-    for (int t = threadIdx.x; t < 256; t += IBLK) hist[t] = 0;
-    for (int64_t i = threadIdx.x; i < np; i += IBLK) {
+    if (threadIdx.x == 0) s_nu = 0;
+#pragma unroll 2
+    for (int i = threadIdx.x; i < np; i += IBLK) {
       const int64_t k = b0 + i;
       if (!keep[k]) continue;
       const double wi = (double)m.w[k];
@@ -1306,110 +1349,118 @@ __global__ void __launch_bounds__(IBLK) pm_inner_kernel(const Members m, PmHalo 
       qc[d] = __double2float_rn(a7[1 + d] / a7[0]);
       vc[d] = __double2float_rn(a7[4 + d] / a7[0]);
     }
-    int nu = 0;
-    for (int64_t i = threadIdx.x; i < np; i += IBLK) {
+#pragma unroll 2
+    for (int i0 = threadIdx.x - lane; i0 < np; i0 += IBLK) {
+      const int i = i0 + lane;
       const int64_t k = b0 + i;
-      if (!keep[k]) continue;
-      float s = 0.f;
-      for (int d = 0; d < 3; ++d) {
-        const float dv = __fadd_rn(__fsub_rn(m.v[d][k], vc[d]), __fmul_rn(b_val, __fsub_rn(m.q[d][k], qc[d])));
-        s = d == 0 ? __fmul_rn(dv, dv) : __fadd_rn(s, __fmul_rn(dv, dv));
+      float e = -1.0f;
+      if (i < np && keep[k]) {
+        float s = 0.f;
+        for (int d = 0; d < 3; ++d) {
+          const float dv = __fadd_rn(__fsub_rn(m.v[d][k], vc[d]), __fmul_rn(b_val, __fsub_rn(m.q[d][k], qc[d])));
+          s = d == 0 ? __fmul_rn(dv, dv) : __fadd_rn(s, __fmul_rn(dv, dv));
+        }
+        e = __fadd_rn(__fdiv_rn(s, 2.0f), phi[k]);
+        if (!isfinite(e)) s_err = kInvalid;
+        en[k] = e;
       }
-      const float e = __fadd_rn(__fdiv_rn(s, 2.0f), phi[k]);
-      if (!isfinite(e)) s_err = kInvalid;
-      en[k] = e;
-      nu += e >= 0.0f;
-      if (e >= 0.0f) atomicAdd(&hist[__float_as_uint(e + 0.0f) >> 24], 1u);
+      const unsigned bal = __ballot_sync(0xffffffffu, e >= 0.0f);
+      if (bal) {
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&s_nu, __popc(bal));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & lanemask_lt());
+        if (e >= 0.0f && at < KCAP)
+          ukey[at] = ((unsigned long long)__float_as_uint(e + 0.0f) << 32) | (0xffffffffu - (unsigned)i);
+      }
     }
-    nu = bsum_i(nu, red_i);
+    __syncthreads();
+    const int nu = s_nu;
     if (s_err) break;
     if (nu == 0) {
       if (deleted == 0) status = 0;
       break;
     }
-    int nb = max(1, (int)ceil(0.02 * (double)np_bound));
-    nb = min(nu, nb);
-    // radix select of the nb largest energies among the unbound members:
-    // key = bits of (E + 0) (E >= 0, so the bits order like the values)
-    unsigned prefix = 0, mask = 0;
-    int need = nb, n_eq = 0;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-      if (shift != 24) {  // the top digit's histogram came with the energies
+    const int nb = min(nu, max(1, (int)ceil(0.02 * (double)np_bound)));
+    int need = nb;
+    if (nu <= KCAP) {
+      // the nb largest keys, digit by digit from the top, until the keys of
+      // the last digit's bin are all taken (the keys are distinct)
+      unsigned long long prefix = 0, mask = 0;
+      for (int shift = 56; shift >= 0; shift -= 8) {
         for (int t = threadIdx.x; t < 256; t += IBLK) hist[t] = 0;
         __syncthreads();
-        for (int64_t i = threadIdx.x; i < np; i += IBLK) {
+        for (int t = threadIdx.x; t < nu; t += IBLK) {
+          const unsigned long long key = ukey[t];
+          if ((key & mask) == prefix) atomicAdd(&hist[(unsigned)(key >> shift) & 255u], 1u);
+        }
+        __syncthreads();
+        int above, count;
+        const int digit = digit_of(hist, need, above, count);
+        __syncthreads();
+        need -= above;
+        prefix |= (unsigned long long)digit << shift;
+        mask |= 255ull << shift;
+        if (need == count) break;
+      }
+      for (int t = threadIdx.x; t < nu; t += IBLK) {
+        const unsigned long long key = ukey[t];
+        if (key >= prefix) remove((int)(0xffffffffu - (unsigned)key));
+      }
+    } else {
+      // radix select of the nb largest energies among the unbound members:
+      // key = bits of (E + 0) (E >= 0, so the bits order like the values)
+      unsigned prefix = 0, mask = 0;
+      int n_eq = 0;
+      for (int shift = 24; shift >= 0; shift -= 8) {
+        for (int t = threadIdx.x; t < 256; t += IBLK) hist[t] = 0;
+        __syncthreads();
+        for (int i = threadIdx.x; i < np; i += IBLK) {
           const int64_t k = b0 + i;
           if (!keep[k]) continue;
           const float e = en[k];
           if (!(e >= 0.0f)) continue;
           const unsigned key = __float_as_uint(e + 0.0f);
-          if ((key & mask) != prefix) continue;
-          atomicAdd(&hist[(key >> shift) & 255u], 1u);
+          if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
         }
         __syncthreads();
+        int above;
+        const int digit = digit_of(hist, need, above, n_eq);
+        __syncthreads();
+        need -= above;
+        prefix |= (unsigned)digit << shift;
+        mask |= 255u << shift;
       }
-      // digit holding the need-th largest key
-      int digit = 255, above = 0;
-      for (; digit >= 0; --digit) {
-        const int c = (int)hist[digit];
-        if (above + c >= need) {
-          n_eq = c;  // at shift 0: the members whose key equals the threshold
-          break;
-        }
-        above += c;
-      }
-      __syncthreads();
-      need -= above;
-      prefix |= (unsigned)digit << shift;
-      mask |= 255u << shift;
-    }
-    // delete every key > threshold and the `need` lowest indices among
-    // key == threshold (equal energies: lower index first)
-    const unsigned thr = prefix;
-    if (need == n_eq) {
-      // every member at the threshold goes: no index order needed
-      for (int64_t i = threadIdx.x; i < np; i += IBLK) {
+      // delete every key > threshold and the `need` lowest indices among
+      // key == threshold (equal energies: lower index first)
+      const unsigned thr = prefix;
+      int taken_eq = 0;
+      for (int base = 0; base < np; base += IBLK) {
+        const int i = base + threadIdx.x;
         const int64_t k = b0 + i;
-        if (!keep[k]) continue;
-        const float e = en[k];
-        if (e >= 0.0f && __float_as_uint(e + 0.0f) >= thr) {
-          keep[k] = 0;
-          rflag[epos[k]] = 1;
+        bool del_gt = false, is_eq = false;
+        if (i < np && keep[k]) {
+          const float e = en[k];
+          if (e >= 0.0f) {
+            const unsigned key = __float_as_uint(e + 0.0f);
+            del_gt = key > thr;
+            is_eq = key == thr;
+          }
         }
-      }
-      __syncthreads();
-    }
-    int taken_eq = 0;
-    for (int64_t base = 0; base < (need == n_eq ? 0 : np); base += IBLK) {
-      const int64_t i = base + threadIdx.x;
-      int64_t k = b0 + i;
-      bool del_gt = false, is_eq = false;
-      if (i < np && keep[k]) {
-        const float e = en[k];
-        if (e >= 0.0f) {
-          const unsigned key = __float_as_uint(e + 0.0f);
-          del_gt = key > thr;
-          is_eq = key == thr;
+        int before = taken_eq;
+        if (need != n_eq) {  // ordered rank of is_eq within this chunk
+          const unsigned bal = __ballot_sync(0xffffffffu, is_eq);
+          const int warp = threadIdx.x >> 5;
+          __syncthreads();
+          if (lane == 0) red_i[warp] = __popc(bal);
+          __syncthreads();
+          for (int w = 0; w < warp; ++w) before += red_i[w];
+          before += __popc(bal & lanemask_lt());
+          for (int w = 0; w < IBLK / 32; ++w) taken_eq += red_i[w];
         }
+        if (del_gt || (is_eq && (need == n_eq || before < need))) remove(i);
       }
-      // ordered rank of is_eq within this chunk
-      const unsigned bal = __ballot_sync(0xffffffffu, is_eq);
-      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-      __syncthreads();
-      if (lane == 0) red_i[warp] = __popc(bal);
-      __syncthreads();
-      int before = taken_eq;
-      for (int w = 0; w < warp; ++w) before += red_i[w];
-      before += __popc(bal & ((1u << lane) - 1u));
-      int chunk_eq = 0;
-      for (int w = 0; w < IBLK / 32; ++w) chunk_eq += red_i[w];
-      if (i < np && (del_gt || (is_eq && before < need))) {
-        keep[k] = 0;
-        rflag[epos[k]] = 1;
-      }
-      taken_eq += chunk_eq;
-      __syncthreads();
     }
+    __syncthreads();
     np_bound -= nb;
     deleted += nb;
     if (np_bound < nmin) { status = 1; break; }

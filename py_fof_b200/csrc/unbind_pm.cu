@@ -17,6 +17,7 @@
 // gathers all of them.  R = float is the product path, R = double the plain
 // FP64 path.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <functional>
@@ -202,6 +203,7 @@ struct PmHalo {      // device copy of one PM halo's parameters
   float spacing;
   float origin[3];
   int64_t cell_off;  // first C2 cell
+  int64_t e0;        // first member in cell order (the halo's members are consecutive)
   int32_t nc[3];     // C2 cells per axis
   double u_min[3];   // C2 cell origin (q/spacing units)
   double mkeep;      // kept mass at the start of the pass (FP64)
@@ -220,56 +222,66 @@ struct TlRegion {
   float u0[3];         // inner grid origin
 };
 
-// TSC weights and self potential (bound_fortran.f90:2562-2602).  FP32
-// weights as in the reference; the self term accumulates in FP64.
-template <typename R>
-__global__ void pm_setup_kernel(const Members m, const PmHalo *__restrict__ H,
-                                const int32_t *__restrict__ mhalo, int64_t M,
-                                const R *const *__restrict__ selfs, int3 *__restrict__ first,
-                                float *__restrict__ wt, R *__restrict__ selfv, int32_t *flags) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < M;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int h = mhalo[k];
-    if (h < 0) continue;
-    const PmHalo &p = H[h];
-    float w9[9];
-    int f[3];
-    bool bad = false;
+// Nearest node f and TSC weights of one coordinate t (grid units): FP32 as in
+// the reference (bound_fortran.f90:2562-2576).
+__device__ __forceinline__ int tsc_axis(float t, float *w3) {
+  const int nearest = (int)lroundf(t);
+  const float dl = __fsub_rn(t, (float)nearest);
+  const float a = __fsub_rn(0.5f, dl), b = __fadd_rn(0.5f, dl);
+  w3[0] = __fmul_rn(0.5f, __fmul_rn(a, a));
+  w3[1] = __fsub_rn(0.75f, __fmul_rn(dl, dl));
+  w3[2] = __fmul_rn(0.5f, __fmul_rn(b, b));
+  return nearest;
+}
+
+// The same for a member at q on its halo's grid.  Returns false outside the
+// source domain.
+__device__ __forceinline__ bool pm_tsc(const PmHalo &p, float4 q, int *f, float *w9) {
+  const float x[3] = {q.x, q.y, q.z};
+  bool ok = true;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const float t = __fdiv_rn(__fsub_rn(m.q[d][k], p.origin[d]), p.spacing);
-      if (!isfinite(t)) bad = true;
-      if (!(t >= 0.0f) || t >= (float)(p.n / 2 - 1)) bad = true;
-      const int nearest = (int)lroundf(t);
-      const float dl = __fsub_rn(t, (float)nearest);
-      const float a = __fsub_rn(0.5f, dl), b = __fadd_rn(0.5f, dl);
-      w9[3 * d + 0] = __fmul_rn(0.5f, __fmul_rn(a, a));
-      w9[3 * d + 1] = __fsub_rn(0.75f, __fmul_rn(dl, dl));
-      w9[3 * d + 2] = __fmul_rn(0.5f, __fmul_rn(b, b));
-      f[d] = nearest;
-    }
-    if (bad) {
+  for (int d = 0; d < 3; ++d) {
+    const float t = __fdiv_rn(__fsub_rn(x[d], p.origin[d]), p.spacing);
+    if (!(t >= 0.0f) || t >= (float)(p.n / 2 - 1)) ok = false;
+    f[d] = tsc_axis(t, w9 + 3 * d);
+  }
+  return ok;
+}
+
+// Self potential of a TSC cloud on a grid (bound_fortran.f90:2577-2602): FP32
+// products, FP64 sum.
+template <typename R>
+__device__ __forceinline__ R tsc_self(const float *w9, const R *__restrict__ sp) {
+  double acc = 0.0;
+  for (int sz = 0; sz < 3; ++sz)
+    for (int sy = 0; sy < 3; ++sy)
+      for (int sx = 0; sx < 3; ++sx) {
+        const float sw = __fmul_rn(__fmul_rn(w9[sx], w9[3 + sy]), w9[6 + sz]);
+        for (int tz = 0; tz < 3; ++tz)
+          for (int ty = 0; ty < 3; ++ty)
+            for (int tx = 0; tx < 3; ++tx) {
+              const float tw = __fmul_rn(__fmul_rn(w9[tx], w9[3 + ty]), w9[6 + tz]);
+              acc += (double)__fmul_rn(sw, tw) *
+                     (double)sp[((tz - sz + 2) * 5 + (ty - sy + 2)) * 5 + (tx - sx + 2)];
+            }
+      }
+  return (R)acc;
+}
+
+// Domain check and self potential of every PM member, in cell order.
+template <typename R>
+__global__ void pm_setup_kernel(const float4 *__restrict__ src4, const uint32_t *__restrict__ cmem, int64_t n,
+                                const PmHalo *__restrict__ H, const int32_t *__restrict__ mhalo,
+                                const R *const *__restrict__ selfs, R *__restrict__ selfe, int32_t *flags) {
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
+    const int h = mhalo[cmem[e]];
+    int f[3];
+    float w9[9];
+    if (!pm_tsc(H[h], src4[e], f, w9)) {
       atomicCAS(&flags[FLAG_ERR], 0, kInvalid);
       continue;
     }
-    const R *sp = selfs[h];
-    double acc = 0.0;
-    for (int sz = 0; sz < 3; ++sz)
-      for (int sy = 0; sy < 3; ++sy)
-        for (int sx = 0; sx < 3; ++sx) {
-          const float sw = __fmul_rn(__fmul_rn(w9[sx], w9[3 + sy]), w9[6 + sz]);
-          for (int tz = 0; tz < 3; ++tz)
-            for (int ty = 0; ty < 3; ++ty)
-              for (int tx = 0; tx < 3; ++tx) {
-                const float tw = __fmul_rn(__fmul_rn(w9[tx], w9[3 + ty]), w9[6 + tz]);
-                acc += (double)__fmul_rn(sw, tw) *
-                       (double)sp[((tz - sz + 2) * 5 + (ty - sy + 2)) * 5 + (tx - sx + 2)];
-              }
-        }
-    selfv[k] = (R)acc;
-    first[k] = make_int3(f[0], f[1], f[2]);
-#pragma unroll
-    for (int j = 0; j < 9; ++j) wt[9 * k + j] = w9[j];
+    selfe[e] = tsc_self<R>(w9, selfs[h]);
   }
 }
 
@@ -430,73 +442,162 @@ __device__ __forceinline__ int seg_of(const uint32_t *__restrict__ off, int n, u
   return lo;
 }
 
+// The deposits and gathers run a block per chunk of up to kDepChunk members
+// consecutive in cell order, so that a block's members are close together:
+// bpre = prefix of the chunk counts of a batch's grids.
+constexpr int kDepChunk = BLK;
+constexpr int kDepNodes = 4096;
+
+struct DepositTile {
+  unsigned lo[kDepNodes], hi[kDepNodes];
+  int box[6];
+};
+
+// Adds one member's 27 contributions per thread (act: the thread has one; f,
+// w9, wk its node, weights and mass) to the grid g with rows of nx and planes
+// of ny rows.  The members of a chunk share most of their nodes, and the adds
+// are bound by the rate of 64-bit atomics in L2 (about 2e11 a second), so they
+// are summed in shared memory over the box of the chunk's nodes where it has
+// at most kDepNodes (two 32-bit words and a carry per node), and each node
+// goes out once.  Neighbour threads start at different nodes: in a cusp all
+// of them add to the same 27.
+__device__ __forceinline__ void deposit_chunk(bool act, const int (&f)[3], const float (&w9)[9], float wk, double sc,
+                                              unsigned long long *__restrict__ g, int nx, int ny, DepositTile &S) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid < 6) S.box[tid] = tid < 3 ? INT_MAX : INT_MIN;
+  __syncthreads();
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int mn = __reduce_min_sync(FULL, act ? f[d] : INT_MAX), mx = __reduce_max_sync(FULL, act ? f[d] : INT_MIN);
+    if (lane == 0) {
+      atomicMin(&S.box[d], mn);
+      atomicMax(&S.box[3 + d], mx);
+    }
+  }
+  __syncthreads();
+  if (S.box[0] > S.box[3]) return;  // nothing to add
+  const int x0 = S.box[0] - 1, y0 = S.box[1] - 1, z0 = S.box[2] - 1;
+  const int bx = S.box[3] - x0 + 2, by = S.box[4] - y0 + 2, bz = S.box[5] - z0 + 2;
+  const int64_t vol = (int64_t)bx * by * bz;
+  const bool tile = vol <= kDepNodes;
+  if (tile) {
+    for (int i = tid; i < (int)vol; i += BLK) S.lo[i] = S.hi[i] = 0;
+    __syncthreads();
+  }
+  if (act) {
+    // this thread's order of the three nodes of each axis
+    const int r[3] = {lane % 3, (lane / 3) % 3, (lane / 9) % 3};
+    int o[3][3];
+    float w[3][3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const int k = j + r[d] < 3 ? j + r[d] : j + r[d] - 3;
+        o[d][j] = k;
+        w[d][j] = k == 0 ? w9[3 * d] : (k == 1 ? w9[3 * d + 1] : w9[3 * d + 2]);
+      }
+    const int row = tile ? bx : nx, plane = tile ? bx * by : nx * ny;
+    const int64_t at = tile ? (f[0] - 1 - x0) + (int64_t)row * (f[1] - 1 - y0) + (int64_t)plane * (f[2] - 1 - z0)
+                            : (f[0] - 1) + (int64_t)row * (f[1] - 1) + (int64_t)plane * (f[2] - 1);
+#pragma unroll
+    for (int jz = 0; jz < 3; ++jz)
+#pragma unroll
+      for (int jy = 0; jy < 3; ++jy)
+#pragma unroll
+        for (int jx = 0; jx < 3; ++jx) {
+          const float v = __fmul_rn(__fmul_rn(__fmul_rn(wk, w[0][jx]), w[1][jy]), w[2][jz]);
+          const unsigned long long u = fx_quantum(v, sc);
+          const int64_t i = at + o[0][jx] + row * o[1][jy] + (int64_t)plane * o[2][jz];
+          if (tile) {
+            const unsigned l = (unsigned)u, old = atomicAdd(&S.lo[i], l);
+            const unsigned hi = (unsigned)(u >> 32) + (old + l < l ? 1u : 0u);
+            if (hi) atomicAdd(&S.hi[i], hi);
+          } else {
+            atomicAdd(&g[i], u);
+          }
+        }
+  }
+  if (tile) {
+    __syncthreads();
+    for (int i = tid; i < (int)vol; i += BLK) {
+      const unsigned long long u = ((unsigned long long)S.hi[i] << 32) | S.lo[i];
+      if (!u) continue;
+      const int z = i / (bx * by), rem = i - z * (bx * by), y = rem / bx, x = rem - y * bx;
+      atomicAdd(&g[(x0 + x) + (int64_t)nx * ((y0 + y) + (int64_t)ny * (z0 + z))], u);
+    }
+  }
+}
+
 // Deposit of the kept members of a batch of halos (batch[j] = halo of
-// grid j, boxes[j] its support box, bpre = prefix of their member counts),
-// flat over the batch's members in their stored order (coalesced member
-// reads).  Each of a member's 27 contributions is one 64-bit integer atomic
-// add.  Block 0 also writes the grids' inverse scales inv[j] = 2^(e - 61).
-__global__ void __launch_bounds__(BLK) pm_deposit_kernel(const Members m, const PmHalo *__restrict__ H,
+// grid j, boxes[j] its support box).  Block 0 also writes the grids' inverse
+// scales inv[j] = 2^(e - 61).
+__global__ void __launch_bounds__(BLK) pm_deposit_kernel(const float4 *__restrict__ src4,
+                                                         const uint32_t *__restrict__ cmem,
+                                                         const PmHalo *__restrict__ H,
                                                          const ConvBox *__restrict__ boxes,
                                                          const int32_t *__restrict__ batch,
                                                          const uint32_t *__restrict__ bpre, int nb,
                                                          const uint8_t *__restrict__ keep,
-                                                         const int3 *__restrict__ first,
-                                                         const float *__restrict__ wt,
                                                          unsigned long long *__restrict__ acc,
                                                          double *__restrict__ inv) {
+  __shared__ DepositTile S;
   if (blockIdx.x == 0)
     for (int j = threadIdx.x; j < nb; j += blockDim.x) inv[j] = scalbn(1.0, fx_exp(H[batch[j]].mkeep) - 61);
-  const uint32_t total = bpre[nb];
-  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-    const int j = seg_of(bpre, nb, idx);
-    const PmHalo &p = H[batch[j]];
-    const int64_t k = p.off + (idx - bpre[j]);
-    if (!keep[k]) continue;
-    const double sc = scalbn(1.0, 61 - fx_exp(p.mkeep));
-    const int3 f = first[k];
-    const float *w9 = wt + 9 * k;
-    const float wk = m.w[k];
-    const int nx = boxes[j].in[0], ny = boxes[j].in[1];
-    unsigned long long *g = acc + boxes[j].in_off + (((int64_t)(f.z - 1) * ny + (f.y - 1)) * nx + (f.x - 1));
-    for (int sz = 0; sz < 3; ++sz)
-      for (int sy = 0; sy < 3; ++sy)
-        for (int sx = 0; sx < 3; ++sx) {
-          const float v = __fmul_rn(__fmul_rn(__fmul_rn(wk, w9[sx]), w9[3 + sy]), w9[6 + sz]);
-          atomicAdd(&g[((int64_t)sz * ny + sy) * nx + sx], fx_quantum(v, sc));
-        }
+  const int j = seg_of(bpre, nb, blockIdx.x);
+  const PmHalo &p = H[batch[j]];
+  const int64_t i = (int64_t)(blockIdx.x - bpre[j]) * kDepChunk + threadIdx.x;
+  const bool act = i < p.np && keep[cmem[p.e0 + i]];
+  int f[3] = {0, 0, 0};
+  float w9[9] = {}, wk = 0.f;
+  if (act) {
+    const float4 q = src4[p.e0 + i];
+    pm_tsc(p, q, f, w9);
+    wk = q.w;
   }
+  deposit_chunk(act, f, w9, wk, scalbn(1.0, 61 - fx_exp(p.mkeep)), acc + boxes[j].in_off, boxes[j].in[0],
+                boxes[j].in[1], S);
+}
+
+// Value of the convolved grid g (rows of nx, planes of ny rows) at a TSC cloud.
+template <typename R>
+__device__ __forceinline__ R tsc_gather(const R *__restrict__ g, int nx, int ny, const float (&w9)[9]) {
+  R raw = 0;
+  for (int sz = 0; sz < 3; ++sz)
+    for (int sy = 0; sy < 3; ++sy)
+      for (int sx = 0; sx < 3; ++sx)
+        raw += g[((int64_t)sz * ny + sy) * nx + sx] * (R)w9[sx] * (R)w9[3 + sy] * (R)w9[6 + sz];
+  return raw;
 }
 
 // TSC gather and the C1 potential (bound_fortran.f90:2681-2703) at the kept
 // members of a batch; grid j holds the potential of halo batch[j].
 template <typename R>
-__global__ void pm_gather_kernel(const Members m, const PmHalo *__restrict__ H, const ConvBox *__restrict__ boxes,
-                                 const int32_t *__restrict__ batch, const uint32_t *__restrict__ bpre, int nb,
-                                 const uint8_t *__restrict__ keep, const int3 *__restrict__ first,
-                                 const float *__restrict__ wt, const R *__restrict__ selfv,
-                                 const R *__restrict__ rho, double a_val, R *__restrict__ phi_c1) {
-  const uint32_t total = bpre[nb];
-  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-    const int j = seg_of(bpre, nb, idx);
-    const PmHalo &p = H[batch[j]];
-    const int64_t k = p.off + (idx - bpre[j]);
-    if (!keep[k]) continue;
-    const int3 f = first[k];
-    const int nx = boxes[j].out[0], ny = boxes[j].out[1];  // the window starts at node 0
-    const R *g = rho + boxes[j].out_off + (((int64_t)(f.z - 1) * ny + (f.y - 1)) * nx + (f.x - 1));
-    const float *w9 = wt + 9 * k;
-    R raw = 0;
-    for (int sz = 0; sz < 3; ++sz)
-      for (int sy = 0; sy < 3; ++sy)
-        for (int sx = 0; sx < 3; ++sx)
-          raw += g[((int64_t)sz * ny + sy) * nx + sx] * (R)w9[sx] * (R)w9[3 + sy] * (R)w9[6 + sz];
-    const R wk = (R)m.w[k];
-    const double rest = p.mkeep - (double)m.w[k];
-    const R radius = (R)p.n / (R)2;
-    const R dz0 = (R)(rest > 0.0 ? rest : 0.0) / radius;
-    const R pref = (R)(a_val / (6.0 * kPi * (double)p.spacing));
-    phi_c1[k] = pref * ((raw - wk * selfv[k]) - dz0);
-  }
+__global__ void __launch_bounds__(BLK) pm_gather_kernel(
+    const float4 *__restrict__ src4, const uint32_t *__restrict__ cmem, const PmHalo *__restrict__ H,
+    const ConvBox *__restrict__ boxes, const int32_t *__restrict__ batch, const uint32_t *__restrict__ bpre, int nb,
+    const uint8_t *__restrict__ keep, const R *__restrict__ selfe, const R *__restrict__ rho, double a_val,
+    R *__restrict__ phi_c1) {
+  const int j = seg_of(bpre, nb, blockIdx.x);
+  const PmHalo &p = H[batch[j]];
+  const int64_t i = (int64_t)(blockIdx.x - bpre[j]) * kDepChunk + threadIdx.x;
+  if (i >= p.np) return;
+  const int64_t e = p.e0 + i, k = cmem[e];
+  if (!keep[k]) return;
+  const float4 q = src4[e];
+  int f[3];
+  float w9[9];
+  pm_tsc(p, q, f, w9);
+  const int nx = boxes[j].out[0], ny = boxes[j].out[1];  // the window starts at node 0
+  const R raw = tsc_gather<R>(rho + boxes[j].out_off + (((int64_t)(f[2] - 1) * ny + (f[1] - 1)) * nx + (f[0] - 1)), nx,
+                              ny, w9);
+  const R wk = (R)q.w;
+  const double rest = p.mkeep - (double)q.w;
+  const R radius = (R)p.n / (R)2;
+  const R dz0 = (R)(rest > 0.0 ? rest : 0.0) / radius;
+  const R pref = (R)(a_val / (6.0 * kPi * (double)p.spacing));
+  phi_c1[k] = pref * ((raw - wk * selfe[e]) - dz0);
 }
 
 // bound_depth_continuous / bound_c2_delta_depth (:3080-3117)
@@ -977,10 +1078,10 @@ __global__ void sr_removed_fill_kernel(uint32_t *__restrict__ flag, const uint32
 
 // One refined region: halo h, region b (8x8x8 regions of 16 grid cells),
 // ratio r, inner grid n_in (bound_two_level_build_halo, :614-823).
-__device__ __forceinline__ void tl_t(const Members &m, const PmHalo &p, int64_t k, float *t) {
+__device__ __forceinline__ void tl_t(const PmHalo &p, float x, float y, float z, float *t) {
+  const float q[3] = {x, y, z};
 #pragma unroll
-  for (int d = 0; d < 3; ++d)
-    t[d] = (float)(((double)m.q[d][k] - (double)p.origin[d]) / (double)p.spacing);
+  for (int d = 0; d < 3; ++d) t[d] = (float)(((double)q[d] - (double)p.origin[d]) / (double)p.spacing);
 }
 
 __device__ __forceinline__ int tl_region(const float *t, int *bxyz) {
@@ -998,206 +1099,187 @@ __device__ __forceinline__ bool tl_tsc(const TlRegion &R, const float *t, int *f
   bool ok = true;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const float tf = __fmul_rn(__fsub_rn(t[d], R.u0[d]), (float)R.r);
-    const int nearest = (int)lroundf(tf);
-    const float dl = __fsub_rn(tf, (float)nearest);
-    const float a = __fsub_rn(0.5f, dl), b = __fadd_rn(0.5f, dl);
-    w9[3 * d + 0] = __fmul_rn(0.5f, __fmul_rn(a, a));
-    w9[3 * d + 1] = __fsub_rn(0.75f, __fmul_rn(dl, dl));
-    w9[3 * d + 2] = __fmul_rn(0.5f, __fmul_rn(b, b));
-    f[d] = nearest;
-    if (nearest < 1 || nearest + 2 > R.n_in / 2) ok = false;
+    f[d] = tsc_axis(__fmul_rn(__fsub_rn(t[d], R.u0[d]), (float)R.r), w9 + 3 * d);
+    if (f[d] < 1 || f[d] + 2 > R.n_in / 2) ok = false;
   }
   return ok;
 }
 
+// Refinement ratio of every member (1 without refinement).
 __global__ void tl_particle_kernel(const Members m, const PmHalo *__restrict__ H,
                                    const int32_t *__restrict__ mhalo, int64_t M,
-                                   const uint8_t *__restrict__ region_r,
-                                   const int32_t *__restrict__ act_of, uint8_t *__restrict__ pr,
-                                   int32_t *__restrict__ preg) {
+                                   const uint8_t *__restrict__ region_r, uint8_t *__restrict__ pr) {
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < M;
        k += (int64_t)gridDim.x * blockDim.x) {
     const int h = mhalo[k];
     if (h < 0) continue;
     const PmHalo &p = H[h];
-    if (!p.two_level) { pr[k] = 1; preg[k] = -1; continue; }
+    if (!p.two_level) { pr[k] = 1; continue; }
     float t[3];
     int bx[3];
-    tl_t(m, p, k, t);
-    const int b = tl_region(t, bx);
-    pr[k] = region_r[(int64_t)h * 512 + b];
-    preg[k] = act_of[(int64_t)h * 512 + b];
+    tl_t(p, m.q[0][k], m.q[1][k], m.q[2][k], t);
+    pr[k] = region_r[(int64_t)h * 512 + tl_region(t, bx)];
   }
 }
 
-// Sources of every refined region: members inside the region box widened
-// by 3.5 + 3/r grid cells (:685-745).  pass 0 counts, pass 1 fills.
-__global__ void tl_source_kernel(const Members m, const PmHalo *__restrict__ H,
-                                 const int32_t *__restrict__ mhalo, int64_t M,
-                                 const int32_t *__restrict__ act_of, const TlRegion *__restrict__ A,
-                                 uint32_t *__restrict__ cnt, uint32_t *__restrict__ src, int fill) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < M;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int h = mhalo[k];
-    if (h < 0 || !H[h].two_level) continue;
-    float t[3];
-    int bx[3];
-    tl_t(m, H[h], k, t);
-    tl_region(t, bx);
-    for (int dz = -1; dz <= 1; ++dz)
-      for (int dy = -1; dy <= 1; ++dy)
-        for (int dx = -1; dx <= 1; ++dx) {
-          const int x = bx[0] + dx, y = bx[1] + dy, z = bx[2] + dz;
-          if (x < 0 || x > 7 || y < 0 || y > 7 || z < 0 || z > 7) continue;
-          const int a = act_of[(int64_t)h * 512 + x + 8 * y + 64 * z];
-          if (a < 0) continue;
-          const TlRegion &R = A[a];
-          bool in = true;
+// A region's sources are the members inside its box widened by 3.5 + 3/r grid
+// cells (:685-745), its targets the members inside it.  Neither is listed:
+// the bricks that the (widened) box touches are whole rows of consecutive
+// members in cell order, cut into chunks of kDepChunk, and a chunk's members
+// test the box themselves.  A warp per region counts its chunks (fill = 0:
+// cnt[a]) or writes them (fill = 1: from start[a] on); widen = 0 for targets.
+__global__ void __launch_bounds__(BLK) tl_chunk_kernel(const PmHalo *__restrict__ H, const TlRegion *__restrict__ A,
+                                                       int na, int widen, const uint32_t *__restrict__ cstart,
+                                                       uint32_t *__restrict__ cnt, const uint32_t *__restrict__ start,
+                                                       uint2 *__restrict__ chunk, int fill) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  for (int a = (int)(((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5); a < na; a += (int)((gridDim.x * BLK) >> 5)) {
+    const TlRegion &Rg = A[a];
+    const PmHalo &p = H[Rg.h];
+    int b0[3], nbk[3];
 #pragma unroll
-          for (int d = 0; d < 3; ++d)
-            in = in && t[d] >= __fsub_rn(R.lo[d], R.bo) && t[d] <= __fadd_rn(R.hi[d], R.bo);
-          if (!in) continue;
-          const uint32_t pos = atomicAdd(&cnt[a], 1u);
-          if (fill) src[pos] = (uint32_t)k;
-        }
+    for (int d = 0; d < 3; ++d) {
+      const double mrg = widen ? (double)Rg.bo : 0.0, off = (double)p.origin[d] / (double)p.spacing - p.u_min[d];
+      // (the FP32 grid units of a member are within 1e-5 of these)
+      const double gl = ((double)Rg.lo[d] - mrg + off) / p.cw_u - 1e-3;
+      const double gh = ((double)Rg.lo[d] + 16.0 + mrg + off) / p.cw_u + 1e-3;
+      const int top = p.nc[d] - 1;
+      const int c0 = gl <= 0.0 ? 0 : (gl >= (double)top ? top : (int)gl);
+      const int c1 = gh <= 0.0 ? 0 : (gh >= (double)top ? top : (int)gh);
+      b0[d] = c0 >> 2;
+      nbk[d] = (c1 >> 2) - b0[d] + 1;
+    }
+    uint32_t run = 0;
+    const int rows = nbk[1] * nbk[2];
+    for (int r0 = 0; r0 < rows; r0 += 32) {
+      const int r = r0 + lane;
+      uint32_t e0 = 0, e1 = 0;
+      if (r < rows) {
+        const int y = b0[1] + r % nbk[1], z = b0[2] + r / nbk[1];
+        e0 = cstart[sr_cell(p, 4 * b0[0], 4 * y, 4 * z)];
+        e1 = cstart[sr_cell(p, 4 * (b0[0] + nbk[0] - 1), 4 * y, 4 * z) + 64];
+      }
+      const uint32_t n = (e1 - e0 + kDepChunk - 1) / kDepChunk;
+      uint32_t incl = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (fill)
+        for (uint32_t i = 0; i < n; ++i)
+          chunk[start[a] + run + incl - n + i] =
+              make_uint2(e0 + kDepChunk * i, min((uint32_t)kDepChunk, e1 - e0 - kDepChunk * i));
+      run += __shfl_sync(FULL, incl, 31);
+    }
+    if (!fill && lane == 0) cnt[a] = run;
   }
 }
 
-// Targets of every refined region: its own members (pass 0 counts, 1 fills)
-__global__ void tl_target_kernel(const int32_t *__restrict__ preg, int64_t M,
-                                 uint32_t *__restrict__ cnt, uint32_t *__restrict__ tgt, int fill) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < M;
-       k += (int64_t)gridDim.x * blockDim.x) {
-    const int a = preg[k];
-    if (a < 0) continue;
-    const uint32_t pos = atomicAdd(&cnt[a], 1u);
-    if (fill) tgt[pos] = (uint32_t)k;
-  }
+// Whether a member at t is a target of region R.
+__device__ __forceinline__ bool tl_is_target(const TlRegion &R, const float *t) {
+  int bx[3];
+  return tl_region(t, bx) == R.b;
 }
 
-// Node range checks of sources and targets, and the inner self term of
-// every target (:729-800).
-// Set-up of the refined regions, flat over all their sources and targets:
-// every source must fall inside its region's inner grid, and every target
-// gets its inner self term.
-__global__ void tl_check_kernel(const Members m, const PmHalo *__restrict__ H,
-                                const TlRegion *__restrict__ A, int na,
-                                const uint32_t *__restrict__ src_start, const uint32_t *__restrict__ src,
-                                int32_t *flags) {
-  const uint32_t total = src_start[na];
-  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-    const int a = seg_of(src_start, na, e);
-    const TlRegion &Rg = A[a];
-    float t[3], w9[9];
-    int f[3];
-    tl_t(m, H[Rg.h], src[e], t);
-    if (!tl_tsc(Rg, t, f, w9)) atomicCAS(&flags[FLAG_ERR], 0, kInvalid);
-  }
-}
-
+// Inner self term of every target (:772-800); a block per target chunk.
 template <typename R>
-__global__ void tl_self_kernel(const Members m, const PmHalo *__restrict__ H,
-                               const TlRegion *__restrict__ A, int na,
-                               const uint32_t *__restrict__ tgt_start, const uint32_t *__restrict__ tgt,
-                               const R *__restrict__ self2, const R *__restrict__ self4,
-                               R *__restrict__ self_in, int32_t *flags) {
-  const uint32_t total = tgt_start[na];
-  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-    const int a = seg_of(tgt_start, na, e);
-    const TlRegion &Rg = A[a];
-    const R *sp = Rg.r == 2 ? self2 : self4;
-    const int64_t k = tgt[e];
-    float t[3], w9[9];
-    int f[3];
-    tl_t(m, H[Rg.h], k, t);
-    if (!tl_tsc(Rg, t, f, w9)) { atomicCAS(&flags[FLAG_ERR], 0, kInvalid); continue; }
-    double acc = 0.0;
-    for (int sz = 0; sz < 3; ++sz)
-      for (int sy = 0; sy < 3; ++sy)
-        for (int sx = 0; sx < 3; ++sx) {
-          const float sw = __fmul_rn(__fmul_rn(w9[sx], w9[3 + sy]), w9[6 + sz]);
-          for (int tz = 0; tz < 3; ++tz)
-            for (int ty = 0; ty < 3; ++ty)
-              for (int tx = 0; tx < 3; ++tx) {
-                const float tw = __fmul_rn(__fmul_rn(w9[tx], w9[3 + ty]), w9[6 + tz]);
-                acc += (double)__fmul_rn(sw, tw) *
-                       (double)sp[((tz - sz + 2) * 5 + (ty - sy + 2)) * 5 + (tx - sx + 2)];
-              }
-        }
-    self_in[k] = (R)acc;
+__global__ void __launch_bounds__(BLK) tl_self_kernel(const float4 *__restrict__ src4, const PmHalo *__restrict__ H,
+                                                      const TlRegion *__restrict__ A, int na,
+                                                      const uint32_t *__restrict__ start,
+                                                      const uint2 *__restrict__ chunk, const R *__restrict__ self2,
+                                                      const R *__restrict__ self4, R *__restrict__ self_in,
+                                                      int32_t *flags) {
+  const TlRegion &Rg = A[seg_of(start, na, blockIdx.x)];
+  const uint2 c = chunk[blockIdx.x];
+  if (threadIdx.x >= c.y) return;
+  const int64_t e = (int64_t)c.x + threadIdx.x;
+  const float4 q = src4[e];
+  float t[3], w9[9];
+  int f[3];
+  tl_t(H[Rg.h], q.x, q.y, q.z, t);
+  if (!tl_is_target(Rg, t)) return;
+  if (!tl_tsc(Rg, t, f, w9)) {
+    atomicCAS(&flags[FLAG_ERR], 0, kInvalid);
+    return;
   }
+  self_in[e] = tsc_self<R>(w9, Rg.r == 2 ? self2 : self4);
 }
 
 // Inner PM of a batch of refined regions of one inner grid size
-// (bound_two_level_run_pm, :825-942): deposit of the kept sources ...
-__global__ void tl_deposit_kernel(const Members m, const PmHalo *__restrict__ H,
-                                  const TlRegion *__restrict__ A, const ConvBox *__restrict__ boxes,
-                                  const int32_t *__restrict__ batch, const uint32_t *__restrict__ bpre, int nb,
-                                  const uint32_t *__restrict__ src_start, const uint32_t *__restrict__ src,
-                                  const uint8_t *__restrict__ keep, unsigned long long *__restrict__ acc,
-                                  double *__restrict__ inv) {
+// (bound_two_level_run_pm, :825-942): deposit of the kept sources, a block per
+// source chunk ...
+__global__ void __launch_bounds__(BLK) tl_deposit_kernel(const float4 *__restrict__ src4,
+                                                         const uint32_t *__restrict__ cmem,
+                                                         const PmHalo *__restrict__ H, const TlRegion *__restrict__ A,
+                                                         const ConvBox *__restrict__ boxes,
+                                                         const int32_t *__restrict__ batch,
+                                                         const uint32_t *__restrict__ bpre, int nb,
+                                                         const uint32_t *__restrict__ start,
+                                                         const uint2 *__restrict__ chunk,
+                                                         const uint8_t *__restrict__ keep,
+                                                         unsigned long long *__restrict__ acc,
+                                                         double *__restrict__ inv) {
+  __shared__ DepositTile S;
   if (blockIdx.x == 0)
     for (int j = threadIdx.x; j < nb; j += blockDim.x) inv[j] = scalbn(1.0, fx_exp(H[A[batch[j]].h].mkeep) - 61);
-  // flat over the sources of the batch: bpre[j] = first index of region j;
-  // fixed-point integer adds as pm_deposit_kernel (order-independent)
-  const uint32_t total = bpre[nb];
-  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-    const int j = seg_of(bpre, nb, idx);
-    const int a = batch[j];
-    const TlRegion &Rg = A[a];
-    const PmHalo &p = H[Rg.h];
-    const int64_t k = src[src_start[a] + (idx - bpre[j])];
-    if (!keep[k]) continue;
-    const double sc = scalbn(1.0, 61 - fx_exp(p.mkeep));
-    float t[3], w9[9];
-    int f[3];
-    tl_t(m, p, k, t);
-    tl_tsc(Rg, t, f, w9);
-    const float wk = m.w[k];
-    const int nx = boxes[j].in[0], ny = boxes[j].in[1];
-    unsigned long long *g = acc + boxes[j].in_off + (((int64_t)(f[2] - 1) * ny + (f[1] - 1)) * nx + (f[0] - 1));
-    for (int sz = 0; sz < 3; ++sz)
-      for (int sy = 0; sy < 3; ++sy)
-        for (int sx = 0; sx < 3; ++sx) {
-          const float v = __fmul_rn(__fmul_rn(__fmul_rn(wk, w9[sx]), w9[3 + sy]), w9[6 + sz]);
-          atomicAdd(&g[((int64_t)sz * ny + sy) * nx + sx], fx_quantum(v, sc));
-        }
+  const int j = seg_of(bpre, nb, blockIdx.x);
+  const int a = batch[j];
+  const TlRegion &Rg = A[a];
+  const PmHalo &p = H[Rg.h];
+  const uint2 c = chunk[start[a] + (blockIdx.x - bpre[j])];
+  int f[3] = {0, 0, 0};
+  float w9[9] = {}, wk = 0.f;
+  bool act = false;
+  if (threadIdx.x < c.y) {
+    const float4 q = src4[c.x + threadIdx.x];
+    float t[3];
+    tl_t(p, q.x, q.y, q.z, t);
+    act = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      act = act && t[d] >= __fsub_rn(Rg.lo[d], Rg.bo) && t[d] <= __fadd_rn(Rg.hi[d], Rg.bo);
+    act = act && keep[cmem[c.x + threadIdx.x]];
+    // (a source inside the widened box is inside the inner grid's half)
+    if (act) act = tl_tsc(Rg, t, f, w9);
+    wk = q.w;
   }
+  deposit_chunk(act, f, w9, wk, scalbn(1.0, 61 - fx_exp(p.mkeep)), acc + boxes[j].in_off, boxes[j].in[0],
+                boxes[j].in[1], S);
 }
 
 // ... and gather at the kept targets: phi_in = a r/(6 pi sp) (raw - w self_in)
 template <typename R>
-__global__ void tl_gather_kernel(const Members m, const PmHalo *__restrict__ H,
-                                 const TlRegion *__restrict__ A, const ConvBox *__restrict__ boxes,
-                                 const int32_t *__restrict__ batch, const uint32_t *__restrict__ bpre, int nb,
-                                 const uint32_t *__restrict__ tgt_start, const uint32_t *__restrict__ tgt,
-                                 const uint8_t *__restrict__ keep, const R *__restrict__ self_in,
-                                 const R *__restrict__ rho, double a_val, R *__restrict__ phi_in) {
-  const uint32_t total = bpre[nb];
-  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-    const int j = seg_of(bpre, nb, idx);
-    const int a = batch[j];
-    const TlRegion &Rg = A[a];
-    const PmHalo &p = H[Rg.h];
-    const int64_t k = tgt[tgt_start[a] + (idx - bpre[j])];
-    if (!keep[k]) continue;
-    const R pref = (R)(a_val * (double)Rg.r / (6.0 * kPi * (double)p.spacing));
-    float t[3], w9[9];
-    int f[3];
-    tl_t(m, p, k, t);
-    tl_tsc(Rg, t, f, w9);
-    const ConvBox &bx = boxes[j];
-    const int nx = bx.out[0], ny = bx.out[1];
-    const R *g = rho + bx.out_off +
-                 (((int64_t)(f[2] - 1 - bx.out0[2]) * ny + (f[1] - 1 - bx.out0[1])) * nx + (f[0] - 1 - bx.out0[0]));
-    R raw = 0;
-    for (int sz = 0; sz < 3; ++sz)
-      for (int sy = 0; sy < 3; ++sy)
-        for (int sx = 0; sx < 3; ++sx)
-          raw += g[((int64_t)sz * ny + sy) * nx + sx] * (R)w9[sx] * (R)w9[3 + sy] * (R)w9[6 + sz];
-    phi_in[k] = pref * (raw - (R)m.w[k] * self_in[k]);
-  }
+__global__ void __launch_bounds__(BLK) tl_gather_kernel(
+    const float4 *__restrict__ src4, const uint32_t *__restrict__ cmem, const PmHalo *__restrict__ H,
+    const TlRegion *__restrict__ A, const ConvBox *__restrict__ boxes, const int32_t *__restrict__ batch,
+    const uint32_t *__restrict__ bpre, int nb, const uint32_t *__restrict__ start, const uint2 *__restrict__ chunk,
+    const uint8_t *__restrict__ keep, const R *__restrict__ self_in, const R *__restrict__ rho, double a_val,
+    R *__restrict__ phi_in) {
+  const int j = seg_of(bpre, nb, blockIdx.x);
+  const int a = batch[j];
+  const TlRegion &Rg = A[a];
+  const PmHalo &p = H[Rg.h];
+  const uint2 c = chunk[start[a] + (blockIdx.x - bpre[j])];
+  if (threadIdx.x >= c.y) return;
+  const int64_t e = (int64_t)c.x + threadIdx.x;
+  const float4 q = src4[e];
+  float t[3], w9[9];
+  int f[3];
+  tl_t(p, q.x, q.y, q.z, t);
+  if (!tl_is_target(Rg, t)) return;
+  const int64_t k = cmem[e];
+  if (!keep[k]) return;
+  tl_tsc(Rg, t, f, w9);
+  const ConvBox &bx = boxes[j];
+  const int nx = bx.out[0], ny = bx.out[1];
+  const R raw = tsc_gather<R>(rho + bx.out_off +
+                                  (((int64_t)(f[2] - 1 - bx.out0[2]) * ny + (f[1] - 1 - bx.out0[1])) * nx +
+                                   (f[0] - 1 - bx.out0[0])),
+                              nx, ny, w9);
+  const R pref = (R)(a_val * (double)Rg.r / (6.0 * kPi * (double)p.spacing));
+  phi_in[k] = pref * (raw - (R)q.w * self_in[e]);
 }
 
 // ---------------------------------------------------------------- removal
@@ -1909,16 +1991,14 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   int32_t *dlist = W.carve<int32_t>(nh);
   const R **dselfs = W.carve<const R *>(nh);
   int32_t *mhalo = W.carve<int32_t>(M);
-  int3 *first = W.carve<int3>(M);
-  float *wt = W.carve<float>(9 * (size_t)M);
-  R *selfv = W.carve<R>(M), *c1 = W.carve<R>(M), *c2 = W.carve<R>(M);
+  R *selfe = W.carve<R>(M), *c1 = W.carve<R>(M), *c2 = W.carve<R>(M);
   float *phi = W.carve<float>(M), *en = W.carve<float>(M);
   R *tl_self_in = nullptr;
   uint32_t *epos = W.carve<uint32_t>(M);  // positions in cell order (PM members)
   if (!epos) { set_error("workspace exhausted (cell positions)"); return kAlloc; }
   double *ext = W.carve<double>(6 * (size_t)nh);
   int32_t *dsup = W.carve<int32_t>(3 * (size_t)nh);
-  if (!dH || !dlist || !dselfs || !mhalo || !first || !wt || !selfv || !c1 || !c2 || !phi || !en || !ext || !dsup) {
+  if (!dH || !dlist || !dselfs || !mhalo || !selfe || !c1 || !c2 || !phi || !en || !ext || !dsup) {
     set_error("workspace exhausted (PM members)");
     return kAlloc;
   }
@@ -1930,12 +2010,9 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   PYFOF_CHECK_LAUNCH();
   pm_mark_halo_kernel<<<nh, BLK, 0, s>>>(dH, nh, mhalo, keep);
   PYFOF_CHECK_LAUNCH();
-  pm_setup_kernel<R><<<gM, BLK, 0, s>>>(m, dH, mhalo, M, dselfs, first, wt, selfv, ctx.d_flags);
-  PYFOF_CHECK_LAUNCH();
   // two-level refinement of dense 16-cell regions of 256-grid halos
   // (bound_two_level_setup_ratios / build_halo, bound_fortran.f90:551-823)
   std::vector<TlRegion> act;
-  std::vector<int32_t> act_of((size_t)nh * 512, -1);
   std::vector<uint8_t> region_r((size_t)nh * 512, 1);
   {
     uint32_t *rc = W.carve<uint32_t>((size_t)nh * 512);
@@ -1978,7 +2055,6 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
           Rg.hi[d] = std::min(Rg.lo[d] + 16.0f, 127.0f);
           Rg.u0[d] = ((Rg.lo[d] - Rg.bo) - (1.0f / (float)r)) + (0.0f / (float)r);
         }
-        act_of[(size_t)h * 512 + b] = (int32_t)act.size();
         act.push_back(Rg);
       }
     }
@@ -2009,10 +2085,12 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   PYFOF_CUDA(cudaMemcpyAsync(hext.data(), ext, sizeof(double) * 6 * nh, cudaMemcpyDeviceToHost, s));
   PYFOF_CUDA(cudaMemcpyAsync(hsup.data(), dsup, sizeof(int32_t) * 3 * nh, cudaMemcpyDeviceToHost, s));
   PYFOF_CUDA(cudaStreamSynchronize(s));
-  int64_t ncell = 0;
+  int64_t ncell = 0, first_e = 0;
   for (int h = 0; h < nh; ++h) {
     PmHalo &p = H[h];
     p.cell_off = ncell;
+    p.e0 = first_e;
+    first_e += p.np;
     p.cw_u = p.two_level ? 3.5 / (double)p.r_max : 3.5;
     int64_t c = 1;
     for (int d = 0; d < 3; ++d) {
@@ -2074,6 +2152,8 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   const unsigned gP = (unsigned)std::min<int64_t>(ceil_div(std::max<uint32_t>(npm, 1), BLK), 148 * 16);
   sr_pack_kernel<<<gP, BLK, 0, s>>>(m, cmem, npm, src4, epos);
   PYFOF_CHECK_LAUNCH();
+  pm_setup_kernel<R><<<gP, BLK, 0, s>>>(src4, cmem, npm, dH, mhalo, dselfs, selfe, ctx.d_flags);
+  PYFOF_CHECK_LAUNCH();
   sr_chunk_fill_kernel<<<gC, BLK, 0, s>>>(cstart, chcnt, nbrick, chspan);
   PYFOF_CHECK_LAUNCH();
   // persistent blocks: those that fit on the GPU at once, if there is work for them
@@ -2081,23 +2161,21 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   // per-member refinement ratio, refined-region sources and targets
   const int na = (int)act.size();
   uint8_t *pr = W.carve<uint8_t>(M);
-  int32_t *preg = W.carve<int32_t>(M);
   R *phi_in = W.carve<R>(M);
-  if (!pr || !preg || !phi_in) { set_error("workspace exhausted (two-level)"); return kAlloc; }
+  if (!pr || !phi_in) { set_error("workspace exhausted (two-level)"); return kAlloc; }
   PYFOF_CUDA(cudaMemsetAsync(phi_in, 0, sizeof(R) * M, s));
   PYFOF_CUDA(cudaMemsetAsync(pr, 1, M, s));
-  PYFOF_CUDA(cudaMemsetAsync(preg, 0xff, sizeof(int32_t) * M, s));  // -1: no refined region
   TlRegion *dA = nullptr;
-  uint32_t *src_start = nullptr, *src = nullptr, *tgt_start = nullptr, *tgt = nullptr;
+  // source and target chunks of the refined regions (tl_chunk_kernel)
+  uint32_t *src_start = nullptr, *tgt_start = nullptr;
+  uint2 *src = nullptr, *tgt = nullptr;
   std::vector<uint32_t> hsrc, htgt;
   std::shared_ptr<GreenTable> g_r2, g_r4;
   {
     uint8_t *dregr = W.carve<uint8_t>((size_t)nh * 512);
-    int32_t *dact_of = W.carve<int32_t>((size_t)nh * 512);
-    if (!dregr || !dact_of) { set_error("workspace exhausted (two-level)"); return kAlloc; }
+    if (!dregr) { set_error("workspace exhausted (two-level)"); return kAlloc; }
     PYFOF_TRY(upload(ctx, dregr, region_r.data(), (size_t)nh * 512, s));
-    PYFOF_TRY(upload(ctx, dact_of, act_of.data(), sizeof(int32_t) * nh * 512, s));
-    tl_particle_kernel<<<gM, BLK, 0, s>>>(m, dH, mhalo, M, dregr, dact_of, pr, preg);
+    tl_particle_kernel<<<gM, BLK, 0, s>>>(m, dH, mhalo, M, dregr, pr);
     PYFOF_CHECK_LAUNCH();
     {
       // chunk records, then most sources first (a stable sort on a 16-bit key)
@@ -2124,47 +2202,37 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
       tgt_start = W.carve<uint32_t>(na + 1);
       if (!dA || !cnt || !src_start || !tgt_start) { set_error("workspace exhausted (two-level)"); return kAlloc; }
       PYFOF_TRY(upload(ctx, dA, act.data(), sizeof(TlRegion) * na, s));
-      // sources
-      PYFOF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (na + 1), s));
-      tl_source_kernel<<<gM, BLK, 0, s>>>(m, dH, mhalo, M, dact_of, dA, cnt, nullptr, 0);
-      PYFOF_CHECK_LAUNCH();
-      PYFOF_TRY(exclusive_scan_u32(cnt, src_start, na + 1, nullptr, W, s));
-      hsrc.resize(na + 1);
-      PYFOF_CUDA(cudaMemcpyAsync(hsrc.data(), src_start, sizeof(uint32_t) * (na + 1), cudaMemcpyDeviceToHost, s));
+      const unsigned gA = (unsigned)std::min<int64_t>(ceil_div((int64_t)na * 32, BLK), 148 * 8);
+      for (int w = 0; w < 2; ++w) {  // sources (the widened box), then targets
+        uint32_t *st = w == 0 ? src_start : tgt_start;
+        std::vector<uint32_t> &hs = w == 0 ? hsrc : htgt;
+        PYFOF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (na + 1), s));
+        tl_chunk_kernel<<<gA, BLK, 0, s>>>(dH, dA, na, w == 0, cstart, cnt, nullptr, nullptr, 0);
+        PYFOF_CHECK_LAUNCH();
+        PYFOF_TRY(exclusive_scan_u32(cnt, st, na + 1, nullptr, W, s));
+        hs.resize(na + 1);
+        PYFOF_CUDA(cudaMemcpyAsync(hs.data(), st, sizeof(uint32_t) * (na + 1), cudaMemcpyDeviceToHost, s));
+      }
       PYFOF_CUDA(cudaStreamSynchronize(s));
-      src = W.carve<uint32_t>(std::max<uint32_t>(hsrc[na], 1));
-      if (!src) { set_error("workspace exhausted (two-level sources)"); return kAlloc; }
-      PYFOF_CUDA(cudaMemcpyAsync(cnt, src_start, sizeof(uint32_t) * (na + 1), cudaMemcpyDeviceToDevice, s));
-      tl_source_kernel<<<gM, BLK, 0, s>>>(m, dH, mhalo, M, dact_of, dA, cnt, src, 1);
+      src = W.carve<uint2>(std::max<uint32_t>(hsrc[na], 1));
+      tgt = W.carve<uint2>(std::max<uint32_t>(htgt[na], 1));
+      if (!src || !tgt) { set_error("workspace exhausted (two-level chunks)"); return kAlloc; }
+      tl_chunk_kernel<<<gA, BLK, 0, s>>>(dH, dA, na, 1, cstart, cnt, src_start, src, 1);
       PYFOF_CHECK_LAUNCH();
-      // targets
-      PYFOF_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (na + 1), s));
-      tl_target_kernel<<<gM, BLK, 0, s>>>(preg, M, cnt, nullptr, 0);
-      PYFOF_CHECK_LAUNCH();
-      PYFOF_TRY(exclusive_scan_u32(cnt, tgt_start, na + 1, nullptr, W, s));
-      htgt.resize(na + 1);
-      PYFOF_CUDA(cudaMemcpyAsync(htgt.data(), tgt_start, sizeof(uint32_t) * (na + 1), cudaMemcpyDeviceToHost, s));
-      PYFOF_CUDA(cudaStreamSynchronize(s));
-      tgt = W.carve<uint32_t>(std::max<uint32_t>(htgt[na], 1));
-      if (!tgt) { set_error("workspace exhausted (two-level targets)"); return kAlloc; }
-      PYFOF_CUDA(cudaMemcpyAsync(cnt, tgt_start, sizeof(uint32_t) * (na + 1), cudaMemcpyDeviceToDevice, s));
-      tl_target_kernel<<<gM, BLK, 0, s>>>(preg, M, cnt, tgt, 1);
+      tl_chunk_kernel<<<gA, BLK, 0, s>>>(dH, dA, na, 0, cstart, cnt, tgt_start, tgt, 1);
       PYFOF_CHECK_LAUNCH();
       bool need2 = false, need4 = false;
       for (auto &Rg : act) { need2 |= Rg.r == 2; need4 |= Rg.r == 4; }
       if (need2) PYFOF_TRY(get_green<R>(ctx, 128, 3.5, 7.0, 0, &g_r2));
       if (need4) PYFOF_TRY(get_green<R>(ctx, 216, 3.5, 14.0, 0, &g_r4));
-      R *self_in = c1;  // reuse: c1 is rewritten every pass, self_in must persist -> own array
-      self_in = W.carve<R>(M);
+      R *self_in = W.carve<R>(M);
       if (!self_in) { set_error("workspace exhausted (two-level self)"); return kAlloc; }
-      const unsigned gs = (unsigned)std::min<int64_t>(ceil_div(std::max<uint32_t>(hsrc[na], 1), BLK), 148 * 16);
-      tl_check_kernel<<<gs, BLK, 0, s>>>(m, dH, dA, na, src_start, src, ctx.d_flags);
-      PYFOF_CHECK_LAUNCH();
-      const unsigned gt = (unsigned)std::min<int64_t>(ceil_div(std::max<uint32_t>(htgt[na], 1), BLK), 148 * 16);
-      tl_self_kernel<R><<<gt, BLK, 0, s>>>(m, dH, dA, na, tgt_start, tgt,
-                                           g_r2 ? (const R *)g_r2->self : nullptr,
-                                           g_r4 ? (const R *)g_r4->self : nullptr, self_in, ctx.d_flags);
-      PYFOF_CHECK_LAUNCH();
+      if (htgt[na] > 0) {
+        tl_self_kernel<R><<<htgt[na], BLK, 0, s>>>(src4, dH, dA, na, tgt_start, tgt,
+                                                   g_r2 ? (const R *)g_r2->self : nullptr,
+                                                   g_r4 ? (const R *)g_r4->self : nullptr, self_in, ctx.d_flags);
+        PYFOF_CHECK_LAUNCH();
+      }
       tl_self_in = self_in;
     }
   }
@@ -2182,7 +2250,7 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   auto waves = [&](int n) { return a.tiles.conv_waves[kGridIndex(n)]; };
   // the box of a halo's own grid, and of a region's inner grid: its sources
   // lie within 3.5 + 3/r grid cells of the region, its targets inside it
-  // (tl_source_kernel, tl_particle_kernel), one node of slack each side
+  // (tl_deposit_kernel, tl_gather_kernel), one node of slack each side
   auto halo_box = [&](int h) {
     ConvBox b{};
     for (int d = 0; d < 3; ++d) b.in[d] = b.out[d] = H[h].sup[d];
@@ -2253,7 +2321,7 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
     const ConvBox *dbox;
     const int32_t *did;
     const uint32_t *dpre0, *dpre1;
-    uint32_t n0, n1;  // members: sources and targets (the same for a halo's own grid)
+    uint32_t n0, n1;  // chunks of sources and of targets (the same for a halo's own grid)
   };
   // takes grids from items[at..] while they fit, and uploads the tables
   std::vector<unsigned char> meta;
@@ -2278,7 +2346,7 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
         p0.push_back(p0.back() + (hsrc[items[at] + 1] - hsrc[items[at]]));
         p1.push_back(p1.back() + (htgt[items[at] + 1] - htgt[items[at]]));
       } else {
-        p0.push_back(p0.back() + (uint32_t)H[items[at]].np);
+        p0.push_back(p0.back() + (uint32_t)ceil_div(H[items[at]].np, kDepChunk));
       }
     }
     const size_t nb = B.ids.size(), ob = sizeof(ConvBox) * nb, oi = ob + 4 * nb, op = oi + 4 * (nb + 1);
@@ -2297,9 +2365,6 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
     ctx.last_pm_solves += (int64_t)nb;
     PYFOF_CUDA(cudaMemsetAsync(scratch, 0, B.acc, s));
     return kOk;
-  };
-  auto flat_grid = [&](uint32_t n) {
-    return (unsigned)std::min<int64_t>(ceil_div(std::max<uint32_t>(n, 1), BLK), 148 * 16);
   };
   unsigned long long *const acc = reinterpret_cast<unsigned long long *>(scratch);
   R *const rho = reinterpret_cast<R *>(scratch);  // the convolved grids overwrite acc
@@ -2374,16 +2439,15 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
       for (size_t at = 0; at < grp.size();) {
         PYFOF_TRY(next_batch(grp, at, n, false, B));
         const int nb = (int)B.ids.size();
-        const unsigned gb = flat_grid(B.n0);
-        pm_deposit_kernel<<<gb, BLK, 0, s>>>(m, dH, B.dbox, B.did, B.dpre0, nb, keep, first, wt, acc, dinv);
+        pm_deposit_kernel<<<B.n0, BLK, 0, s>>>(src4, cmem, dH, B.dbox, B.did, B.dpre0, nb, keep, acc, dinv);
         PYFOF_CHECK_LAUNCH();
         if (ctx.timing) ctx.conv_timer.begin(s);
         PYFOF_TRY(pm_convolve_batch<R>(acc, dinv, rho, reinterpret_cast<cplx_t<R> *>(scratch + B.acc),
                                        (const R *)green_of[n]->g, (const cplx_t<R> *)green_of[n]->tw, n, B.dbox,
                                        B.ext, nb, s, waves(n)));
         if (ctx.timing) ctx.conv_timer.end(s);
-        pm_gather_kernel<R><<<gb, BLK, 0, s>>>(m, dH, B.dbox, B.did, B.dpre0, nb, keep, first, wt, selfv, rho,
-                                               a.a_val, c1);
+        pm_gather_kernel<R><<<B.n0, BLK, 0, s>>>(src4, cmem, dH, B.dbox, B.did, B.dpre0, nb, keep, selfe, rho,
+                                                 a.a_val, c1);
         PYFOF_CHECK_LAUNCH();
       }
     }
@@ -2397,17 +2461,19 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
       for (size_t at = 0; at < regs.size();) {
         PYFOF_TRY(next_batch(regs, at, nin, true, B));
         const int nb = (int)B.ids.size();
-        tl_deposit_kernel<<<flat_grid(B.n0), BLK, 0, s>>>(m, dH, dA, B.dbox, B.did, B.dpre0, nb, src_start, src,
-                                                          keep, acc, dinv);
+        tl_deposit_kernel<<<B.n0, BLK, 0, s>>>(src4, cmem, dH, dA, B.dbox, B.did, B.dpre0, nb, src_start, src, keep,
+                                               acc, dinv);
         PYFOF_CHECK_LAUNCH();
         if (ctx.timing) ctx.conv_timer.begin(s);
         PYFOF_TRY(pm_convolve_batch<R>(acc, dinv, rho, reinterpret_cast<cplx_t<R> *>(scratch + B.acc),
                                        (const R *)gin->g, (const cplx_t<R> *)gin->tw, nin, B.dbox, B.ext, nb, s,
                                        waves(nin)));
         if (ctx.timing) ctx.conv_timer.end(s);
-        tl_gather_kernel<R><<<flat_grid(B.n1), BLK, 0, s>>>(m, dH, dA, B.dbox, B.did, B.dpre1, nb, tgt_start, tgt,
-                                                            keep, tl_self_in, rho, a.a_val, phi_in);
-        PYFOF_CHECK_LAUNCH();
+        if (B.n1 > 0) {
+          tl_gather_kernel<R><<<B.n1, BLK, 0, s>>>(src4, cmem, dH, dA, B.dbox, B.did, B.dpre1, nb, tgt_start, tgt,
+                                                   keep, tl_self_in, rho, a.a_val, phi_in);
+          PYFOF_CHECK_LAUNCH();
+        }
       }
     }
     PYFOF_CUDA(cudaMemsetAsync(sr_next, 0, 2 * sizeof(unsigned), s));

@@ -205,12 +205,24 @@ constexpr size_t smem_lines_bytes() {
   return sizeof(cplx_t<R>) * (size_t)(N + (kW<R> + 1) * N);
 }
 
-// Shared memory of the fused z pass: the tile plus two staging buffers of
-// N/2+1 rows for the next halo's input.
+// Shared memory of the fused z pass: the tile plus a staging buffer of `rows`
+// rows for the next grid's input.
 template <typename R, int N>
-constexpr size_t smem_conv_bytes() {
-  return smem_lines_bytes<R, N>() + sizeof(cplx_t<R>) * (size_t)(2 * (N / 2 + 1) * kW<R>);
+constexpr size_t smem_conv_bytes(int rows) {
+  return smem_lines_bytes<R, N>() + sizeof(cplx_t<R>) * (size_t)(rows * kW<R>);
 }
+
+// Blocks per SM the registers of a line kernel are limited for.  The FP64 z
+// pass is bound by FP64 issue and the latency between dependent operations,
+// so a few more warps help until the registers spill (256: 2.97 ms a call of
+// the 256^3 box at 3 blocks, 3.28 at 4; 216: 6.7 -> 4.5 ms of the NFW list at
+// 3 instead of 2).  The y passes go without a staging buffer: with one their
+// registers left 2 blocks per SM and they ran a quarter slower.
+template <typename R, int N, bool CONV>
+constexpr int kMinBlocks = 0;  // the compiler's choice
+template <> constexpr int kMinBlocks<double, 256, true> = 3;
+template <> constexpr int kMinBlocks<double, 216, true> = 3;
+template <> constexpr int kMinBlocks<double, 128, true> = 7;
 
 // 16-byte asynchronous copy global -> shared (completion by wait_group)
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
@@ -438,7 +450,7 @@ enum { kYForward = 0, kZConv = 1, kYInverse = 2, kZInverse = 3 };
 // kYInverse: lines (kx, z of the output window), all N in, its y out.
 // kZInverse: lines (kx, ky), all N in and out (the self kernel).
 template <typename R, int N, int PASS>
-__global__ void __launch_bounds__(Cfg<R, N>::T) k_lines(cplx_t<R> *__restrict__ spec, const R *__restrict__ green,
+__global__ void __launch_bounds__(Cfg<R, N>::T, kMinBlocks<R, N, PASS == kZConv>) k_lines(cplx_t<R> *__restrict__ spec, const R *__restrict__ green,
                                                         const cplx_t<R> *__restrict__ twt,
                                                         const ConvBox *__restrict__ boxes, int nhp, int ntiles,
                                                         int nbb, int batch) {
@@ -483,25 +495,24 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_lines(cplx_t<R> *__restrict__ 
     return spec + boxes[b].spec_off + o * nhp + kx0;
   };
   // CONV: the input rows of the next grid are copied into a staging buffer
-  // while the current one is transformed (two buffers of N/2+1 rows of W
-  // complex)
-  constexpr int SROWS = N / 2 + 1, CPR = (int)(W * sizeof(C) / 16);
-  C *const stage0 = buf0 + WP * N;
-  auto prefetch = [&](int b, int slot) {
+  // while the current one is transformed, from the end of its stage A (which
+  // empties the buffer) on
+  constexpr int CPR = (int)(W * sizeof(C) / 16);
+  C *const stg = buf0 + WP * N;
+  auto prefetch = [&](int b) {
     const C *src = tile_base(b);
     const int rows = boxes[b].in[2];
-    C *dst = stage0 + slot * (SROWS * W);
     for (int c = threadIdx.x; c < rows * CPR; c += T) {
       const int e = c / CPR, part = c - e * CPR;
-      cp_async16(reinterpret_cast<char *>(dst + e * W) + 16 * part,
+      cp_async16(reinterpret_cast<char *>(stg + e * W) + 16 * part,
                  reinterpret_cast<const char *>(src + (int64_t)e * estride) + 16 * part);
     }
     cp_async_commit();
   };
   if constexpr (CONV) {
-    if (b0 < b1) prefetch(b0, 0);
+    if (b0 < b1) prefetch(b0);
   }
-  for (int b = b0, i = 0; b < b1; ++b, ++i) {
+  for (int b = b0; b < b1; ++b) {
     C *const base = tile_base(b);
     const ConvBox &bx = boxes[b];
     const int in_lim = CONV ? bx.in[2] : (PASS == kYForward ? bx.in[1] : N);
@@ -509,14 +520,8 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_lines(cplx_t<R> *__restrict__ 
     const int lo = CONV ? bx.out0[2] : (PASS == kYInverse ? bx.out0[1] : 0);
     const unsigned cnt = CONV ? bx.out[2] : (PASS == kYInverse ? bx.out[1] : N);
     C *bA = buf0;
-    const C *stg = stage0 + (i & 1) * (SROWS * W);
     if constexpr (CONV) {
-      if (b + 1 < b1) {
-        prefetch(b + 1, (i + 1) & 1);
-        cp_async_wait<1>();
-      } else {
-        cp_async_wait<0>();
-      }
+      cp_async_wait<0>();
       __syncthreads();
     }
     // stage A: input -> registers -> DFT over q -> twiddle -> shared
@@ -542,6 +547,9 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_lines(cplx_t<R> *__restrict__ 
       }
     }
     __syncthreads();
+    if constexpr (CONV) {
+      if (b + 1 < b1) prefetch(b + 1);
+    }
     // stage B: DFT over s (and for CONV: Green, inverse DFT over k2, twiddle,
     // written back in place: unit (li, k1) reads and rewrites only its own
     // elements li + WP (k1 + N1 s))
@@ -634,7 +642,7 @@ int32_t prepare() {
     if (r == kOk) r = allow_smem(k_lines<R, N, kYForward>, sm);
     if (r == kOk) r = allow_smem(k_lines<R, N, kYInverse>, sm);
     if (r == kOk) r = allow_smem(k_lines<R, N, kZInverse>, sm);
-    if (r == kOk) r = allow_smem(k_lines<R, N, kZConv>, smem_conv_bytes<R, N>());
+    if (r == kOk) r = allow_smem(k_lines<R, N, kZConv>, smem_conv_bytes<R, N>(N / 2 + 1));
     status = r;
   });
   return status;
@@ -658,19 +666,16 @@ int32_t convolve_n(const unsigned long long *acc, const double *inv_scale, R *ph
   PYFOF_CHECK_LAUNCH();
   // z: grids split into chunks so that the launch is at least `waves` full waves
   const int64_t per = (int64_t)ntiles * N;
-  static int conv_blocks_per_sm = 0;
-  if (!conv_blocks_per_sm) {
-    int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_lines<R, N, kZConv>, T, smem_conv_bytes<R, N>()) !=
-            cudaSuccess || b < 1)
-      b = 1;
-    conv_blocks_per_sm = b;
-  }
+  const size_t smc = smem_conv_bytes<R, N>(ext.in_z);
+  int conv_blocks_per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&conv_blocks_per_sm, k_lines<R, N, kZConv>, T, smc) !=
+          cudaSuccess || conv_blocks_per_sm < 1)
+    conv_blocks_per_sm = 1;
   const int64_t slots = (int64_t)conv_blocks_per_sm * kNumSMs;
   const int nchunk = (int)std::max<int64_t>(1, std::min<int64_t>(batch, ceil_div((int64_t)waves * slots, per)));
   const int nbb = (int)ceil_div(batch, nchunk);
   const int nchunk_used = (int)ceil_div(batch, nbb);
-  k_lines<R, N, kZConv><<<dim3((unsigned)per, (unsigned)nchunk_used), T, smem_conv_bytes<R, N>(), s>>>(
+  k_lines<R, N, kZConv><<<dim3((unsigned)per, (unsigned)nchunk_used), T, smc, s>>>(
       spec, green, tw, boxes, nhp, ntiles, nbb, batch);
   PYFOF_CHECK_LAUNCH();
   k_lines<R, N, kYInverse><<<dim3((unsigned)(ntiles * ext.out_z), (unsigned)batch), T, sm, s>>>(

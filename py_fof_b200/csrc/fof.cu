@@ -1282,16 +1282,26 @@ __global__ void __launch_bounds__(BLK) fof_vd_intra_kernel(
 // a neighbour very dense cell; pairs of cells from the lower cell, in one
 // cell B > A) whose grid boxes come within `reach` are joined when any of
 // their pairs passes the exact test.  The pairs are tested only while the
-// two roots differ, 32 members of A at a time against each member of B
-// inside A's widened box, up to the first link: sub-cells already joined
-// cost two root look-ups, and linking one pair joins the whole of both.
-// A warp per sub-cell A, a block per dense cell.
+// two roots differ, 32 members of A at a time against the members of B
+// inside A's widened box, up to the first link: linking one pair joins the
+// whole of both.  A warp per sub-cell A, a block per dense cell.  The
+// sub-cells B of all neighbour cells are looked up 32 at a time, a lane each:
+// most are joined to A already, and their tables and roots are chains of
+// dependent loads (one after the other they were most of the kernel).
+struct VdCell {
+  const uint32_t *tab;
+  uint32_t b;           // first particle
+  float wl[3], wh[3];   // A's widened box
+  int slo[3], nx, ny, s0, s01, own;
+};
+
 __global__ void __launch_bounds__(BLK) fof_vd_inter_kernel(
     const uint32_t *__restrict__ list, const uint32_t *__restrict__ cs, const RegionDev *__restrict__ R,
     const uint64_t *__restrict__ cell_off, int nreg, int stride, const uint32_t *__restrict__ tab,
     const uint32_t *__restrict__ rank, const float4 *__restrict__ dpos, int *parent, LinkParams P,
     float reach, int32_t *flags) {
   constexpr unsigned FULL = 0xffffffffu;
+  __shared__ VdCell nb_cells[BLK / 32][27];
   const uint32_t c = list[blockIdx.x];
   const int64_t base = cs[c];
   const int64_t n = (int64_t)cs[c + 1] - base;
@@ -1301,6 +1311,7 @@ __global__ void __launch_bounds__(BLK) fof_vd_inter_kernel(
   const int S = g.s[0] * g.s[1] * g.s[2];
   const uint32_t *t = tab + (int64_t)blockIdx.x * stride;
   const int lane = threadIdx.x & 31;
+  VdCell *cells = nb_cells[threadIdx.x >> 5];
   const int64_t local = (int64_t)c - (int64_t)r.cell_off;
   const int64_t Nd[3] = {r.N[0], r.N[1], r.N[2]};
   const int64_t ixyz[3] = {local % Nd[0], (local / Nd[0]) % Nd[1], local / (Nd[0] * Nd[1])};
@@ -1322,72 +1333,118 @@ __global__ void __launch_bounds__(BLK) fof_vd_inter_kernel(
         lo[d] = fminf(lo[d], __shfl_xor_sync(FULL, lo[d], o));
         hi[d] = fmaxf(hi[d], __shfl_xor_sync(FULL, hi[d], o));
       }
-    const int leadA = __float_as_int(dpos[a0].w);
-    for (int nb = 0; nb < 27; ++nb) {
-      const int off[3] = {nb % 3 - 1, (nb / 3) % 3 - 1, nb / 9 - 1};
+    // neighbour cells, a lane each
+    uint32_t nsub = 0;
+    if (lane < 27) {
+      const int off[3] = {lane % 3 - 1, (lane / 3) % 3 - 1, lane / 9 - 1};
+      VdCell &v = cells[lane];
       int64_t jcoord[3];
-      float sh[3] = {0.f, 0.f, 0.f};
       bool ok = true;
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
         int64_t j = ixyz[d] + off[d];
+        float sh = 0.f;
         if ((r.pdim >> d) & 1) {
-          if (j < 0) { j += Nd[d]; sh[d] = (float)P.L; } else if (j >= Nd[d]) { j -= Nd[d]; sh[d] = -(float)P.L; }
+          if (j < 0) { j += Nd[d]; sh = (float)P.L; } else if (j >= Nd[d]) { j -= Nd[d]; sh = -(float)P.L; }
         } else if (j < 0 || j >= Nd[d]) ok = false;
         jcoord[d] = j;
+        v.wl[d] = __fsub_rn(__fadd_rn(lo[d], sh), reach);
+        v.wh[d] = __fadd_rn(__fadd_rn(hi[d], sh), reach);
       }
-      if (!ok) continue;
       const int64_t jl = jcoord[0] + Nd[0] * (jcoord[1] + Nd[1] * jcoord[2]);
-      if (jl < local) continue;
-      const uint64_t jc = r.cell_off + (uint64_t)jl;
-      const int64_t jb = cs[jc], nj = (int64_t)cs[jc + 1] - jb;
-      if (!is_vd(r, nj)) continue;
-      const SubGrid gj = dense_sub(r, nj);
-      const uint32_t *tj = tab + (int64_t)rank[jc] * stride;
-      float wl[3], wh[3];
-      int slo[3], shi[3];
+      if (ok && jl >= local) {
+        const uint64_t jc = r.cell_off + (uint64_t)jl;
+        const uint32_t jb = cs[jc], nj = cs[jc + 1] - jb;
+        if (is_vd(r, nj)) {
+          const SubGrid gj = dense_sub(r, nj);
+          int shi[3];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        wl[d] = __fsub_rn(__fadd_rn(lo[d], sh[d]), reach);
-        wh[d] = __fadd_rn(__fadd_rn(hi[d], sh[d]), reach);
-        const float cl = cell_lower(r, d, jcoord[d]);
-        slo[d] = sub_of(wl[d], cl, gj.inv[d], gj.s[d]);
-        shi[d] = sub_of(wh[d], cl, gj.inv[d], gj.s[d]);
+          for (int d = 0; d < 3; ++d) {
+            const float cl = cell_lower(r, d, jcoord[d]);
+            v.slo[d] = sub_of(v.wl[d], cl, gj.inv[d], gj.s[d]);
+            shi[d] = sub_of(v.wh[d], cl, gj.inv[d], gj.s[d]);
+          }
+          v.tab = tab + (int64_t)rank[jc] * stride;
+          v.b = jb;
+          v.nx = shi[0] - v.slo[0] + 1;
+          v.ny = shi[1] - v.slo[1] + 1;
+          v.s0 = gj.s[0];
+          v.s01 = gj.s[0] * gj.s[1];
+          v.own = jl == local;
+          nsub = (uint32_t)(v.nx * v.ny * (shi[2] - v.slo[2] + 1));
+        }
       }
-      for (int bz = slo[2]; bz <= shi[2]; ++bz)
-        for (int by = slo[1]; by <= shi[1]; ++by)
-          for (int bx = slo[0]; bx <= shi[0]; ++bx) {
-            const int B = bx + gj.s[0] * (by + gj.s[1] * bz);
-            if (jl == local && B <= A) continue;
-            const int64_t b0 = jb + tj[B], b1 = jb + tj[B + 1];
-            if (b1 == b0) continue;
-            int same = 0;
-            if (lane == 0) same = dsu_find(parent, leadA) == dsu_find(parent, __float_as_int(dpos[b0].w));
-            if (__shfl_sync(FULL, same, 0)) continue;
-            bool done = false;
-            for (int64_t ka = a0; ka < a1 && !done; ka += 32) {
-              const int64_t k = ka + lane;
-              const bool valid = k < a1;
-              const float4 me = valid ? dpos[k] : make_float4(0.f, 0.f, 0.f, 0.f);
-              for (int64_t kb = b0; kb < b1; ++kb) {
-                const float4 o = dpos[kb];
-                if (!(o.x >= wl[0] && o.x <= wh[0] && o.y >= wl[1] && o.y <= wh[1] && o.z >= wl[2] &&
-                      o.z <= wh[2]))
-                  continue;
-                const bool lk = valid && (per ? linked_pbc(me, o, P) : linked_open(me, o, P.rp2_open));
-                const unsigned m = __ballot_sync(FULL, lk);
-                if (m) {
-                  if (lane == __ffs(m) - 1) {
-                    int rp = -1;
-                    link_pair(parent, __float_as_int(me.w), __float_as_int(o.w), rp, flags);
-                  }
-                  done = true;
-                  break;
-                }
-              }
+    }
+    uint32_t sub_end = nsub;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(FULL, sub_end, o);
+      if (lane >= o) sub_end += v;
+    }
+    const uint32_t total = __shfl_sync(FULL, sub_end, 31);
+    __syncwarp();
+    int ra = dsu_find(parent, __float_as_int(dpos[a0].w));  // the same on every lane
+    ra = __shfl_sync(FULL, ra, 0);
+    for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+      const uint32_t k = t0 + (uint32_t)lane;
+      int cell = 0;
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const uint32_t v = __shfl_sync(FULL, sub_end, cell + step - 1);
+        if (v <= k) cell += step;
+      }
+      cell &= 31;
+      const uint32_t k0 = __shfl_sync(FULL, sub_end - nsub, cell);
+      uint32_t b0 = 0, b1 = 0;
+      int hb = -1;  // root of B's set; -1: no candidate
+      if (k < total) {
+        const VdCell &v = cells[cell];
+        const int q = (int)(k - k0), z = q / (v.nx * v.ny), rem = q - z * (v.nx * v.ny), y = rem / v.nx,
+                  x = rem - y * v.nx;
+        const int B = (v.slo[0] + x) + v.s0 * (v.slo[1] + y) + v.s01 * (v.slo[2] + z);
+        if (!(v.own && B <= A)) {
+          b0 = v.b + v.tab[B];
+          b1 = v.b + v.tab[B + 1];
+          if (b1 > b0) hb = dsu_find(parent, __float_as_int(dpos[b0].w));
+        }
+      }
+      unsigned mask = __ballot_sync(FULL, hb >= 0 && hb != ra);
+      while (mask) {
+        const int src = __ffs(mask) - 1;
+        mask &= mask - 1;
+        const int hs = __shfl_sync(FULL, hb, src);
+        const uint32_t s0 = __shfl_sync(FULL, b0, src), s1 = __shfl_sync(FULL, b1, src);
+        const VdCell &v = cells[__shfl_sync(FULL, cell, src)];
+        bool linked = false;
+        for (int64_t ka = a0; ka < a1 && !linked; ka += 32) {
+          const bool valid = ka + lane < a1;
+          const float4 me = valid ? dpos[ka + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (uint32_t kb = s0; kb < s1 && !linked; kb += 32) {
+            const float4 o = kb + lane < s1 ? dpos[kb + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+            unsigned in = __ballot_sync(FULL, kb + lane < s1 && o.x >= v.wl[0] && o.x <= v.wh[0] && o.y >= v.wl[1] &&
+                                                  o.y <= v.wh[1] && o.z >= v.wl[2] && o.z <= v.wh[2]);
+            while (in && !linked) {
+              const int j = __ffs(in) - 1;
+              in &= in - 1;
+              float4 so;
+              so.x = __shfl_sync(FULL, o.x, j);
+              so.y = __shfl_sync(FULL, o.y, j);
+              so.z = __shfl_sync(FULL, o.z, j);
+              so.w = 0.f;
+              linked = __any_sync(FULL, valid && (per ? linked_pbc(me, so, P) : linked_open(me, so, P.rp2_open)));
             }
           }
+        }
+        if (!linked) continue;
+        int joined = 0;
+        if (lane == 0) joined = dsu_join(parent, ra, hs, flags);
+        joined = __shfl_sync(FULL, joined, 0);
+        if (hb == hs || hb == ra) hb = joined;
+        ra = joined;
+        mask &= __ballot_sync(FULL, hb >= 0 && hb != ra);
+      }
     }
+    __syncwarp();
   }
 }
 

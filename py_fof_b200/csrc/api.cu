@@ -62,6 +62,7 @@ Context::~Context() {
   if (h_flags) cudaFreeHost(h_flags);
   if (h_stage) cudaFreeHost(h_stage);
   for (uint8_t *p : stage_retired) cudaFreeHost(p);
+  copy_ring.release();
 }
 
 // dst[i] = src[i], src in mapped host memory at a 16-byte aligned address
@@ -529,9 +530,6 @@ static int32_t run_host(Context &ctx, const double *xp, const double *vp, const 
   // are converted after their check, inside the call
   ctx.timing = g_timing != 0;
   if (ctx.timing) cudaEventRecord(ctx.ev[5], s);
-  PYFOF_CUDA(cudaMemcpyAsync(xd, xp, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s));
-  if (u.x_div != 1.0) PYFOF_TRY(divide_inplace(xd, (int64_t)(3 * n), u.x_div, s));
-  if (ctx.timing) cudaEventRecord(ctx.ev[6], s);
   if (side) {
     // the other inputs follow the positions on the host link (the copies
     // share its bandwidth, so the positions, which the linking needs, go
@@ -540,23 +538,57 @@ static int32_t run_host(Context &ctx, const double *xp, const double *vp, const 
     PYFOF_CUDA(cudaEventRecord(ctx.ev_alloc, s));
     PYFOF_CUDA(cudaStreamWaitEvent(ctx.aux_stream, ctx.ev_alloc, 0));
   }
-  if (mp) {
-    PYFOF_CUDA(cudaMemcpyAsync(md, mp, sizeof(double) * n, cudaMemcpyHostToDevice, ctx.aux_stream));
-    a.m_div = u.m_div;
-  } else if (fill_m) {
-    PYFOF_TRY(fill_value(md, (int64_t)n, u.m_const, ctx.aux_stream));
+  // large pageable inputs: issued by worker threads, positions first; the
+  // destructor ends them before any buffer goes away
+  StagedCopy copies;
+  int seg_x = -1, seg_m = -1, seg_v = -1;
+  {
+    const size_t total = sizeof(double) * n * (3 + (vp ? 3 : 0) + (mp ? 1 : 0));
+    if (total >= StagedCopy::kMinBytes && StagedCopy::pageable(xp)) {
+      seg_x = copies.add(xd, xp, sizeof(double) * 3 * n, s);
+      if (mp) seg_m = copies.add(md, mp, sizeof(double) * n, ctx.aux_stream);
+      if (vp) seg_v = copies.add(vd, vp, sizeof(double) * 3 * n, ctx.aux_stream);
+      if (!copies.start(ctx.copy_ring, ctx.device)) seg_x = seg_m = seg_v = -1;
+    }
   }
-  if (mp || fill_m) {
-    PYFOF_CUDA(cudaEventRecord(ctx.ev_masses, ctx.aux_stream));
-    a.masses_ready = ctx.ev_masses;
+  const bool staged = seg_x >= 0;
+  if (staged) copies.wait(seg_x);
+  else PYFOF_CUDA(cudaMemcpyAsync(xd, xp, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s));
+  if (u.x_div != 1.0) PYFOF_TRY(divide_inplace(xd, (int64_t)(3 * n), u.x_div, s));
+  if (ctx.timing) cudaEventRecord(ctx.ev[6], s);
+  // the rest of the inputs: now, or (staged) when the call first waits for them
+  auto issue_masses = [&]() -> int32_t {
+    if (mp) {
+      if (staged) copies.wait(seg_m);
+      else PYFOF_CUDA(cudaMemcpyAsync(md, mp, sizeof(double) * n, cudaMemcpyHostToDevice, ctx.aux_stream));
+    } else if (fill_m) {
+      PYFOF_TRY(fill_value(md, (int64_t)n, u.m_const, ctx.aux_stream));
+    }
+    if (mp || fill_m) PYFOF_CUDA(cudaEventRecord(ctx.ev_masses, ctx.aux_stream));
+    return kOk;
+  };
+  auto issue_velocities = [&]() -> int32_t {
+    if (vp) {
+      if (staged) copies.wait(seg_v);
+      else PYFOF_CUDA(cudaMemcpyAsync(vd, vp, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx.aux_stream));
+      if (u.v_mul != 1.0) PYFOF_TRY(multiply_inplace(vd, (int64_t)(3 * n), u.v_mul, ctx.aux_stream));
+    }
+    if (side) {
+      if (ctx.timing) cudaEventRecord(ctx.ev[8], ctx.aux_stream);
+      PYFOF_CUDA(cudaEventRecord(ctx.ev_inputs, ctx.aux_stream));
+    }
+    return kOk;
+  };
+  if (staged) {
+    a.issue_masses = issue_masses;
+    a.issue_inputs = issue_velocities;
+  } else {
+    PYFOF_TRY(issue_masses());
+    PYFOF_TRY(issue_velocities());
   }
-  if (vp) {
-    PYFOF_CUDA(cudaMemcpyAsync(vd, vp, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx.aux_stream));
-    if (u.v_mul != 1.0) PYFOF_TRY(multiply_inplace(vd, (int64_t)(3 * n), u.v_mul, ctx.aux_stream));
-  }
+  if (mp) a.m_div = u.m_div;
+  if (mp || fill_m) a.masses_ready = ctx.ev_masses;
   if (side) {
-    if (ctx.timing) cudaEventRecord(ctx.ev[8], ctx.aux_stream);
-    PYFOF_CUDA(cudaEventRecord(ctx.ev_inputs, ctx.aux_stream));
     a.inputs_ready = ctx.ev_inputs;
     a.input_stream = ctx.aux_stream;
   }
@@ -609,6 +641,13 @@ static int32_t run_host(Context &ctx, const double *xp, const double *vp, const 
   }
   // an early failure may leave the side copies in flight: their buffers are
   // released in the order of stream s, after them
+  {
+    const cudaError_t ce = copies.join();
+    if (r == kOk && ce != cudaSuccess) {
+      set_error("CUDA failure in an input copy: %s", cudaGetErrorString(ce));
+      r = kCuda;
+    }
+  }
   if (side) {
     // everything the call queued on the input stream (its copies and the
     // velocity pack of the unbinding)

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "hostcopy.cuh"
 
 namespace pyfof {
 
@@ -101,6 +102,7 @@ struct Context {
   size_t stage_cap = 0, stage_used = 0;
   std::vector<uint8_t *> stage_retired;
   void stage_reset() { stage_used = 0; }
+  CopyRing copy_ring;  // pinned chunks of pageable inputs (StagedCopy)
   ~Context();
 };
 

@@ -2235,10 +2235,12 @@ int32_t fof_run(Context &ctx, const FofArgs &a) {
   if (ctx.timing) cudaEventRecord(ctx.ev[2], ctx.stream);
   PYFOF_TRY(fof_link_stage(ctx, a, st));
   PYFOF_TRY(fof_candidates_stage(ctx, a, st, !a.bound_check));
+  if (a.issue_masses) PYFOF_TRY(a.issue_masses());
   if (a.masses_ready) PYFOF_CUDA(cudaStreamWaitEvent(ctx.stream, a.masses_ready, 0));
   if (a.mp) PYFOF_TRY(check_masses(ctx, a.mp, a.total_np, a.m_div));
   if (ctx.timing) cudaEventRecord(ctx.ev[3], ctx.stream);
   if (!a.bound_check) {
+    if (a.issue_inputs) PYFOF_TRY(a.issue_inputs());
     if (a.inputs_ready) PYFOF_CUDA(cudaStreamWaitEvent(ctx.stream, a.inputs_ready, 0));
     PYFOF_TRY(fof_plain_angmom(ctx, a, st));
   } else {

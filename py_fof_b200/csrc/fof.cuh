@@ -1,6 +1,8 @@
 // Friends-of-friends pipeline on one device.
 #pragma once
 
+#include <functional>
+
 #include "common.cuh"
 
 namespace pyfof {
@@ -53,6 +55,10 @@ struct FofArgs {
   // already on the device
   cudaEvent_t masses_ready = nullptr, inputs_ready = nullptr;
   cudaStream_t input_stream = nullptr;
+  // called before the events are waited for: pageable inputs are still being
+  // issued by other threads then (StagedCopy), and the events are recorded
+  // behind them
+  std::function<int32_t()> issue_masses, issue_inputs;
   // outputs (device): in_halo, halo_id (N int32); ang_mom host (3,nhalo) F-order
   int32_t *in_halo = nullptr, *halo_id = nullptr;
   double *ang_mom = nullptr;

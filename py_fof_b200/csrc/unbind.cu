@@ -530,6 +530,7 @@ int32_t unbind_stage(Context &ctx, const FofArgs &a, FofState &st) {
     }
   } velocity_join{ctx, s};
   if (a.inputs_ready && a.input_stream) {
+    if (a.issue_inputs) PYFOF_TRY(a.issue_inputs());
     PYFOF_CUDA(cudaEventRecord(ctx.ev_pack, s));
     PYFOF_CUDA(cudaStreamWaitEvent(a.input_stream, ctx.ev_pack, 0));
     PYFOF_CUDA(cudaStreamWaitEvent(a.input_stream, a.inputs_ready, 0));

@@ -43,6 +43,7 @@ Context::~Context() {
     cudaStreamSynchronize(stream);
     work.release();
     cudaStreamSynchronize(stream);
+    work.destroy();
   }
   if (own_stream) cudaStreamDestroy(own_stream);
   if (aux_stream) cudaStreamDestroy(aux_stream);
@@ -518,9 +519,10 @@ static int32_t run_host(Context &ctx, const double *xp, const double *vp, const 
   a.xp = xd;
   a.vp = vd;
   a.mp = md;
-  a.in_halo = ctx.work.carve<int32_t>(n);
+  // (in_halo is halo_id > 0: an array of its own only for a caller that wants one)
+  a.in_halo = in_halo ? ctx.work.carve<int32_t>(n) : nullptr;
   a.halo_id = ctx.work.carve<int32_t>(n);
-  if (!xd || (vp && !vd) || ((mp || fill_m) && !md) || !a.in_halo || !a.halo_id) {
+  if (!xd || (vp && !vd) || ((mp || fill_m) && !md) || (in_halo && !a.in_halo) || !a.halo_id) {
     ctx.work.release();
     set_error("device allocation failed for %zu particles", n);
     return kAlloc;
@@ -592,7 +594,7 @@ static int32_t run_host(Context &ctx, const double *xp, const double *vp, const 
     a.inputs_ready = ctx.ev_inputs;
     a.input_stream = ctx.aux_stream;
   }
-  PYFOF_CUDA(cudaMemsetAsync(a.in_halo, 0, sizeof(int32_t) * n, s));
+  if (a.in_halo) PYFOF_CUDA(cudaMemsetAsync(a.in_halo, 0, sizeof(int32_t) * n, s));
   PYFOF_CUDA(cudaMemsetAsync(a.halo_id, 0, sizeof(int32_t) * n, s));
   a.soa = layout == PYFOF_LAYOUT_SOA ? 1 : 0;
   a.np_halo = np_halo;

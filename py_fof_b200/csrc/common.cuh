@@ -58,12 +58,19 @@ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 constexpr int kNumSMs = 148;
 
-// Per-call device allocator.  carve() takes memory from the device's
-// stream-ordered pool (cudaMallocAsync on the call's stream; the pool keeps
-// freed blocks cached, so steady-state calls do not reach the driver) and
-// release() returns everything at the end of the call.
+// Per-call device allocator.  Blocks of at most kSmall bytes are cut from a
+// slab that the arena keeps between calls (its calls run one after the other
+// on one stream, each synchronised before the next); what does not fit, and
+// larger blocks, come from the device's stream-ordered pool (cudaMallocAsync
+// on the call's stream; the pool keeps freed blocks cached).  A call of a few
+// thousand particles makes about 60 allocations: at a microsecond or two each
+// to allocate and to free they were a quarter of its time.  release() returns
+// everything at the end of the call.
 struct Arena {
+  static constexpr size_t kSlab = (size_t)16 << 20, kSmall = (size_t)1 << 20;
   cudaStream_t stream = nullptr;
+  uint8_t *slab = nullptr;
+  size_t slab_used = 0;
   std::vector<void *> ptrs;
   std::vector<size_t> sizes;
   size_t bytes = 0;      // held by this call
@@ -72,8 +79,16 @@ struct Arena {
   template <class T>
   T *carve(size_t count) {
     void *p = nullptr;
-    size_t b = (count ? count : 1) * sizeof(T);
-    if (cudaMallocAsync(&p, b, stream) != cudaSuccess) {
+    const size_t b = (count ? count : 1) * sizeof(T);
+    const size_t r = (b + 255) & ~(size_t)255;
+    if (b <= kSmall && !slab && cudaMalloc(reinterpret_cast<void **>(&slab), kSlab) != cudaSuccess) {
+      cudaGetLastError();
+      slab = nullptr;
+    }
+    if (b <= kSmall && slab && slab_used + r <= kSlab) {
+      p = slab + slab_used;
+      slab_used += r;
+    } else if (cudaMallocAsync(&p, b, stream) != cudaSuccess) {
       cudaGetLastError();
       last_fail = b;
       return nullptr;
@@ -89,11 +104,17 @@ struct Arena {
   size_t mark() const { return ptrs.size(); }
   void release_to(size_t m) {
     while (ptrs.size() > m) {
-      cudaFreeAsync(ptrs.back(), stream);
+      uint8_t *p = static_cast<uint8_t *>(ptrs.back());
+      if (slab && p >= slab && p < slab + kSlab) slab_used = (size_t)(p - slab);
+      else cudaFreeAsync(p, stream);
       bytes -= sizes.back();
       ptrs.pop_back();
       sizes.pop_back();
     }
+  }
+  void destroy() {  // after release(), with the stream idle
+    if (slab) cudaFree(slab);
+    slab = nullptr;
   }
 };
 

@@ -40,7 +40,10 @@ namespace pyfof {
 
 namespace {
 
-constexpr int TILE = 4096;  // particles per block of the bbox, key and scatter kernels (16 per thread)
+// particles per block of the bbox, key and scatter kernels: 16 per thread, 4
+// where few blocks would leave most SMs idle
+constexpr int TILE = 4096, TILE_SMALL = 1024;
+constexpr int64_t kTileSmallUpTo = 1 << 19;
 constexpr int LU = 4;       // particles whose loads a thread has in flight there
 constexpr int BLK = 256;
 
@@ -1502,6 +1505,7 @@ __global__ void __launch_bounds__(BLK) fof_cand_count_kernel(const uint32_t *__r
     uint32_t t = 0;
     for (int w = 0; w < BLK / 32; ++w) t += red[w];
     cnt[blockIdx.x] = t;
+    if (blockIdx.x == 0) cnt[gridDim.x] = 0;
   }
 }
 
@@ -1588,7 +1592,7 @@ __global__ void fof_member_kernel(const int *lab, const uint32_t *gsize,
     pcand[p] = c;
     if (write_out && c >= 0) {
       const int i = __float_as_int(pos[p].w);
-      in_halo[i] = 1;
+      if (in_halo) in_halo[i] = 1;
       halo_id[i] = c + 1;
     }
   }
@@ -1779,6 +1783,7 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
   // --- region table and tiles (host)
   std::vector<RegionDev> reg(nreg);
   std::vector<Tile> tiles;
+  const int64_t tile = n <= kTileSmallUpTo ? TILE_SMALL : TILE;
   int64_t start = 0;
   for (int r = 0; r < nreg; ++r) {
     RegionDev &R = reg[r];
@@ -1786,8 +1791,8 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
     R.start = start;
     R.np = a.np_halo[r];
     R.active = (R.np >= a.np_halo_min && R.np > 0) ? 1 : 0;
-    for (int64_t b = start; b < start + R.np; b += TILE)
-      tiles.push_back(Tile{r, 0, b, std::min<int64_t>(start + R.np, b + TILE)});
+    for (int64_t b = start; b < start + R.np; b += tile)
+      tiles.push_back(Tile{r, 0, b, std::min<int64_t>(start + R.np, b + tile)});
     start += R.np;
   }
   if (start != n) {
@@ -1795,32 +1800,39 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
     return kInvalid;
   }
   const int64_t ntiles = (int64_t)tiles.size();
-  RegionDev *dR = W.carve<RegionDev>(nreg);
-  Tile *dT = W.carve<Tile>(std::max<int64_t>(ntiles, 1));
-  unsigned long long *dbb = W.carve<unsigned long long>(6 * (size_t)nreg);
-  if (!dR || !dT || !dbb) { set_error("workspace exhausted (regions)"); return kAlloc; }
-  PYFOF_TRY(upload(ctx, dR, reg.data(), sizeof(RegionDev) * nreg, s));
-  PYFOF_TRY(upload(ctx, dT, tiles.data(), sizeof(Tile) * ntiles, s));
-  {
-    std::vector<unsigned long long> init(6 * (size_t)nreg);
-    for (int r = 0; r < nreg; ++r)
-      for (int d = 0; d < 3; ++d) { init[6 * r + d] = ~0ull; init[6 * r + 3 + d] = 0ull; }
-    PYFOF_TRY(upload(ctx, dbb, init.data(), sizeof(unsigned long long) * init.size(), s));
-  }
+  // one block of tables: regions, cell offsets, bounding boxes, an error
+  // word, tiles; uploaded together, the boxes and the error word read back
+  // together, regions and offsets uploaded again with the geometry
+  const size_t o_off = sizeof(RegionDev) * nreg, o_bb = o_off + sizeof(uint64_t) * (nreg + 1),
+               o_err = o_bb + 6 * sizeof(uint64_t) * nreg, o_tile = o_err + sizeof(uint64_t),
+               tab_bytes = o_tile + sizeof(Tile) * ntiles;
+  static_assert(sizeof(RegionDev) % 8 == 0, "the tables that follow hold 64-bit values");
+  uint8_t *dtab = W.carve<uint8_t>(tab_bytes);
+  if (!dtab) { set_error("workspace exhausted (regions)"); return kAlloc; }
+  RegionDev *dR = reinterpret_cast<RegionDev *>(dtab);
+  uint64_t *dcoff = reinterpret_cast<uint64_t *>(dtab + o_off);
+  unsigned long long *dbb = reinterpret_cast<unsigned long long *>(dtab + o_bb);
+  int32_t *derr = reinterpret_cast<int32_t *>(dtab + o_err);
+  Tile *dT = reinterpret_cast<Tile *>(dtab + o_tile);
+  std::vector<uint64_t> tab((tab_bytes + 7) / 8, 0);
+  uint8_t *htab = reinterpret_cast<uint8_t *>(tab.data());
+  memcpy(htab, reg.data(), sizeof(RegionDev) * nreg);
+  for (int r = 0; r < nreg; ++r)
+    for (int d = 0; d < 3; ++d) tab[o_bb / 8 + 6 * (size_t)r + d] = ~0ull;  // minima; maxima start at 0
+  if (ntiles) memcpy(htab + o_tile, tiles.data(), sizeof(Tile) * ntiles);
+  PYFOF_TRY(upload(ctx, dtab, htab, tab_bytes, s));
   PYFOF_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(int32_t) * FLAG_COUNT, s));
   if (ntiles) {
-    fof_bbox_kernel<<<(unsigned)ntiles, BLK, 0, s>>>(xp, dR, dT, L, half, dbb, ctx.d_flags);
+    fof_bbox_kernel<<<(unsigned)ntiles, BLK, 0, s>>>(xp, dR, dT, L, half, dbb, derr);
     PYFOF_CHECK_LAUNCH();
   }
-  std::vector<unsigned long long> bb(6 * (size_t)nreg);
+  std::vector<unsigned long long> bb(6 * (size_t)nreg + 1);
   PYFOF_CUDA(cudaMemcpyAsync(bb.data(), dbb, sizeof(unsigned long long) * bb.size(),
                              cudaMemcpyDeviceToHost, s));
-  PYFOF_CUDA(cudaMemcpyAsync(ctx.h_flags, ctx.d_flags, sizeof(int32_t) * FLAG_COUNT,
-                             cudaMemcpyDeviceToHost, s));
   PYFOF_CUDA(cudaStreamSynchronize(s));
-  if (ctx.h_flags[FLAG_ERR]) {
+  if (const int32_t err = (int32_t)bb[6 * (size_t)nreg]) {
     set_error("non-finite particle coordinates");
-    return ctx.h_flags[FLAG_ERR];
+    return err;
   }
 
   // --- reference geometry per region (host)
@@ -1851,15 +1863,15 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
   st.total_cells = total_cells;
   ctx.last_cells = (int64_t)total_cells;
   ctx.last_active = n_active;
-  PYFOF_TRY(upload(ctx, dR, reg.data(), sizeof(RegionDev) * nreg, s));
-  uint64_t *dcoff = W.carve<uint64_t>(nreg + 1);
+  memcpy(htab, reg.data(), sizeof(RegionDev) * nreg);
+  memcpy(htab + o_off, cell_off.data(), sizeof(uint64_t) * (nreg + 1));
+  PYFOF_TRY(upload(ctx, dtab, htab, o_bb, s));
   uint32_t *keys = W.carve<uint32_t>(std::max<int64_t>(n, 1));
   uint32_t *cstart = W.carve<uint32_t>(total_cells + 2);
-  if (!dcoff || !keys || !cstart) {
+  if (!keys || !cstart) {
     set_error("workspace exhausted (keys)");
     return kAlloc;
   }
-  PYFOF_TRY(upload(ctx, dcoff, cell_off.data(), sizeof(uint64_t) * (nreg + 1), s));
   PYFOF_CUDA(cudaMemsetAsync(cstart, 0, sizeof(uint32_t) * (total_cells + 2), s));
   // the particles' slots within their cells (sort scratch in the sorted modes)
   uint32_t *slot = W.carve<uint32_t>(std::max<int64_t>(n, 1));
@@ -1881,8 +1893,7 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
   uint32_t *drank = W.carve<uint32_t>(total_cells + 1);
   DenseChunk *dchunks = W.carve<DenseChunk>((size_t)n_active / 32 + dense_cap);
   if (!list || !drank || !dchunks) { set_error("workspace exhausted (dense cells)"); return kAlloc; }
-  uint32_t *dcells = reinterpret_cast<uint32_t *>(ctx.d_flags + FLAG_COUNT_A);  // A, B, C
-  PYFOF_CUDA(cudaMemsetAsync(dcells, 0, 3 * sizeof(uint32_t), s));
+  uint32_t *dcells = reinterpret_cast<uint32_t *>(ctx.d_flags + FLAG_COUNT_A);  // A, B, C (zero)
   if (total_cells > 0) {
     const unsigned cgrid = (unsigned)std::min<int64_t>(ceil_div((int64_t)total_cells, (int64_t)BLK), (int64_t)kNumSMs * 16);
     fof_cells_kernel<<<cgrid, BLK, 0, s>>>(cstart, (int64_t)total_cells, dcells, list, drank, dchunks, skey);
@@ -1997,7 +2008,6 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
     // dense-cell particles and the rest as two launches: the long pair loops
     // of the dense part do not hold back blocks of the short sparse work
     if (ctx.timing) cudaEventRecord(ctx.ev[0], s);
-    PYFOF_CUDA(cudaMemsetAsync(ctx.d_flags + FLAG_VD, 0, sizeof(int32_t), s));
     if (ctx.last_dense > 0 && any_vd) {
       fof_vd_intra_kernel<<<(unsigned)ctx.last_dense, BLK, 0, s>>>(list, cstart, dR, dcoff, nreg, D.stride,
                                                                    D.tab, D.dpos, parent, ctx.d_flags);
@@ -2007,8 +2017,6 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
                                                                    ctx.d_flags);
       PYFOF_CHECK_LAUNCH();
     }
-    PYFOF_CUDA(cudaMemcpyAsync(ctx.h_flags + FLAG_VD, ctx.d_flags + FLAG_VD, sizeof(int32_t),
-                               cudaMemcpyDeviceToHost, s));
     if (ndense_chunks > 0) {
       const unsigned dgrid = (unsigned)std::min<int64_t>(ceil_div(ndense_chunks * 32, BLK), (int64_t)kNumSMs * 24);
       fof_link_dense_kernel<<<dgrid, BLK, 0, s>>>(pos, prid, dR, cstart, parent, dchunks, ndense_chunks, P, D,
@@ -2048,12 +2056,10 @@ int32_t fof_candidates_stage(Context &ctx, const FofArgs &a, FofState &st, bool 
     st.lab = reinterpret_cast<int *>(st.keys_free);  // keys are dead after the scatter
     fof_root_kernel<<<grid, BLK, 0, s>>>(st.parent, st.lab, st.gsize, na);
     PYFOF_CHECK_LAUNCH();
-    PYFOF_CUDA(cudaMemsetAsync(toff + ntile, 0, sizeof(uint32_t), s));
     fof_cand_count_kernel<<<(unsigned)ntile, BLK, 0, s>>>(st.gsize, na, nmin, toff);
     PYFOF_CHECK_LAUNCH();
-    PYFOF_TRY(exclusive_scan_u32(toff, toff, ntile + 1, nullptr, W, s));
-    PYFOF_CUDA(cudaMemcpyAsync(ctx.d_flags + FLAG_COUNT_A, toff + ntile, sizeof(uint32_t), cudaMemcpyDeviceToDevice,
-                               s));
+    PYFOF_TRY(exclusive_scan_u32(toff, toff, ntile + 1, reinterpret_cast<uint32_t *>(ctx.d_flags + FLAG_COUNT_A), W,
+                                 s));
     PYFOF_CUDA(cudaMemcpyAsync(ctx.h_flags, ctx.d_flags, sizeof(int32_t) * FLAG_COUNT,
                                cudaMemcpyDeviceToHost, s));
     PYFOF_CUDA(cudaStreamSynchronize(s));
@@ -2068,12 +2074,12 @@ int32_t fof_candidates_stage(Context &ctx, const FofArgs &a, FofState &st, bool 
   st.pcand = pcand;
   const int64_t nc = std::max<int64_t>(st.ncand, 1);
   st.cand_anchor = W.carve<int64_t>(nc);
-  st.cand_region = W.carve<int32_t>(nc);
-  st.cand_np = W.carve<int32_t>(nc);
-  st.cand_root = W.carve<int32_t>(nc);
+  st.cand_np = W.carve<int32_t>(3 * nc);
+  st.cand_region = st.cand_np + nc;
+  st.cand_root = st.cand_np + 2 * nc;
   int32_t *root = W.carve<int32_t>(nc);
   uint32_t *first = W.carve<uint32_t>(nc);
-  if (!st.cand_anchor || !st.cand_region || !st.cand_np || !st.cand_root || !root || !first) {
+  if (!st.cand_anchor || !st.cand_np || !root || !first) {
     set_error("workspace exhausted (candidates)");
     return kAlloc;
   }
@@ -2103,11 +2109,10 @@ int32_t fof_plain_angmom(Context &ctx, const FofArgs &a, FofState &st) {
   std::vector<double> am_host(3 * (size_t)nreg, 0.0);
   if (st.ncand > 0 && a.vp) {
     const int64_t na = st.n_active, nc = st.ncand;
-    double *acc = W.carve<double>(7 * (size_t)nc);
-    double *am = W.carve<double>(3 * (size_t)nc);
-    if (!acc || !am) { set_error("workspace exhausted (ang_mom)"); return kAlloc; }
-    PYFOF_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * 7 * nc, s));
-    PYFOF_CUDA(cudaMemsetAsync(am, 0, sizeof(double) * 3 * nc, s));
+    double *acc = W.carve<double>(10 * (size_t)nc);
+    if (!acc) { set_error("workspace exhausted (ang_mom)"); return kAlloc; }
+    double *am = acc + 7 * (size_t)nc;
+    PYFOF_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * 10 * nc, s));
     Coords xp{a.xp, a.total_np, a.soa}, vp{a.vp, a.total_np, a.soa};
     const unsigned grid = (unsigned)std::min<int64_t>(ceil_div(na, BLK), (int64_t)kNumSMs * 16);
     fof_com_kernel<<<grid, BLK, 0, s>>>(xp, vp, a.mp, st.pos, st.pcand, st.cand_anchor, na,
@@ -2117,10 +2122,10 @@ int32_t fof_plain_angmom(Context &ctx, const FofArgs &a, FofState &st) {
                                            na, a.L_Box, 0.5 * a.L_Box, am);
     PYFOF_CHECK_LAUNCH();
     std::vector<double> amc(3 * (size_t)nc);
-    std::vector<int32_t> creg(nc);
+    std::vector<int32_t> creg(nc, 0);
     PYFOF_CUDA(cudaMemcpyAsync(amc.data(), am, sizeof(double) * 3 * nc, cudaMemcpyDeviceToHost, s));
-    PYFOF_CUDA(cudaMemcpyAsync(creg.data(), st.cand_region, sizeof(int32_t) * nc,
-                               cudaMemcpyDeviceToHost, s));
+    if (nreg > 1)
+      PYFOF_CUDA(cudaMemcpyAsync(creg.data(), st.cand_region, sizeof(int32_t) * nc, cudaMemcpyDeviceToHost, s));
     PYFOF_CUDA(cudaStreamSynchronize(s));
     for (int64_t c = 0; c < nc; ++c)
       for (int d = 0; d < 3; ++d) am_host[3 * (size_t)creg[c] + d] += amc[3 * c + d];

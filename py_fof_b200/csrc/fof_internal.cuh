@@ -67,7 +67,7 @@ struct FofState {
   int32_t *pcand = nullptr;   // candidate of each sorted particle or -1
   uint32_t ncand = 0;
   int64_t *cand_anchor = nullptr;  // original index of each candidate's first member in the reference's order
-  int32_t *cand_region = nullptr, *cand_np = nullptr, *cand_root = nullptr;
+  int32_t *cand_np = nullptr, *cand_region = nullptr, *cand_root = nullptr;  // one block, in this order
   float *phi_out = nullptr;   // optional: final potential of every packed member
 };
 

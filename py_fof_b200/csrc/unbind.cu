@@ -195,7 +195,7 @@ __global__ void ub_write_kernel(const uint32_t *__restrict__ mcand, const Member
     const uint32_t c = mcand[k];
     if (valid[c] && keep[k]) {
       const int32_t i = m.pid[k];
-      in_halo[i] = 1;
+      if (in_halo) in_halo[i] = 1;
       halo_id[i] = (int32_t)vrank[c] + 1;
     }
   }
@@ -495,9 +495,11 @@ int32_t unbind_stage(Context &ctx, const FofArgs &a, FofState &st) {
   uint32_t *mcand, *midx;
   PYFOF_TRY(radix_sort_pairs(cand_of, nullptr, n, bits_for((uint64_t)ncand), ka, va, kb, vb, &mcand,
                              &midx, W, s));
-  std::vector<int32_t> cnp(ncand);
-  PYFOF_CUDA(cudaMemcpyAsync(cnp.data(), st.cand_np, sizeof(int32_t) * ncand, cudaMemcpyDeviceToHost, s));
+  // member counts and regions (adjacent, FofState)
+  std::vector<int32_t> cnp(2 * (size_t)ncand);
+  PYFOF_CUDA(cudaMemcpyAsync(cnp.data(), st.cand_np, sizeof(int32_t) * 2 * ncand, cudaMemcpyDeviceToHost, s));
   PYFOF_CUDA(cudaStreamSynchronize(s));
+  const int32_t *creg = cnp.data() + ncand;
   std::vector<int64_t> hoff(ncand + 1, 0);
   for (int c = 0; c < ncand; ++c) hoff[c + 1] = hoff[c] + cnp[c];
   const int64_t M = hoff[ncand];
@@ -511,9 +513,13 @@ int32_t unbind_stage(Context &ctx, const FofArgs &a, FofState &st) {
   m.w = W.carve<float>(M);
   m.pid = W.carve<int32_t>(M);
   float *lo = W.carve<float>(3 * (size_t)ncand), *span = W.carve<float>(ncand);
-  HaloResult *res = W.carve<HaloResult>(ncand);
+  // per candidate: angular momentum, result, copied back together; the sums
+  // (am and the centre sums acc before it) are zeroed together
+  double *acc = W.carve<double>(11 * (size_t)ncand), *am = acc + 7 * (size_t)ncand;
+  HaloResult *res = reinterpret_cast<HaloResult *>(am + 3 * (size_t)ncand);
+  static_assert(sizeof(HaloResult) == sizeof(double), "acc, am and res share a block");
   uint8_t *keep = W.carve<uint8_t>(M);
-  if (!m.w || !m.pid || !lo || !span || !res || !keep) { set_error("workspace exhausted (xv)"); return kAlloc; }
+  if (!m.w || !m.pid || !lo || !span || !acc || !keep) { set_error("workspace exhausted (xv)"); return kAlloc; }
   const unsigned grid_m = (unsigned)std::min<int64_t>(ceil_div(M, BLK), (int64_t)kNumSMs * 16);
   ub_pack_kernel<<<grid_m, BLK, 0, s>>>(xp, a.mp, mcand, midx, st.cand_anchor, M, L, half, m);
   PYFOF_CHECK_LAUNCH();
@@ -707,30 +713,24 @@ int32_t unbind_stage(Context &ctx, const FofArgs &a, FofState &st) {
 
   // 4. outputs
   uint32_t *valid = W.carve<uint32_t>(ncand + 1), *vrank = W.carve<uint32_t>(ncand + 1);
-  double *acc = W.carve<double>(7 * (size_t)ncand), *am = W.carve<double>(3 * (size_t)ncand);
-  if (!valid || !vrank || !acc || !am) { set_error("workspace exhausted (outputs)"); return kAlloc; }
+  if (!valid || !vrank) { set_error("workspace exhausted (outputs)"); return kAlloc; }
   const unsigned grid_c = (unsigned)std::min<int64_t>(ceil_div(ncand, BLK), (int64_t)kNumSMs * 8);
   ub_valid_kernel<<<grid_c, BLK, 0, s>>>(res, ncand, a.np_halo_min, valid);
   PYFOF_CHECK_LAUNCH();
   PYFOF_TRY(exclusive_scan_u32(valid, vrank, ncand, nullptr, W, s));
   ub_write_kernel<<<grid_m, BLK, 0, s>>>(mcand, m, keep, valid, vrank, M, a.in_halo, a.halo_id);
   PYFOF_CHECK_LAUNCH();
-  PYFOF_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * 7 * ncand, s));
-  PYFOF_CUDA(cudaMemsetAsync(am, 0, sizeof(double) * 3 * ncand, s));
+  PYFOF_CUDA(cudaMemsetAsync(acc, 0, sizeof(double) * 10 * ncand, s));
   ub_com_kernel<<<grid_m, BLK, 0, s>>>(xp, vp, a.mp, mcand, m, keep, valid, st.cand_anchor, M, L,
                                        half, acc);
   PYFOF_CHECK_LAUNCH();
   ub_angmom_kernel<<<grid_m, BLK, 0, s>>>(xp, vp, a.mp, mcand, m, keep, valid, st.cand_anchor,
                                           acc, M, L, half, am);
   PYFOF_CHECK_LAUNCH();
-  std::vector<double> amc(3 * (size_t)ncand);
-  std::vector<int32_t> creg(ncand);
-  std::vector<HaloResult> hres(ncand);
-  PYFOF_CUDA(cudaMemcpyAsync(amc.data(), am, sizeof(double) * 3 * ncand, cudaMemcpyDeviceToHost, s));
-  PYFOF_CUDA(cudaMemcpyAsync(creg.data(), st.cand_region, sizeof(int32_t) * ncand,
-                             cudaMemcpyDeviceToHost, s));
-  PYFOF_CUDA(cudaMemcpyAsync(hres.data(), res, sizeof(HaloResult) * ncand, cudaMemcpyDeviceToHost, s));
+  std::vector<double> amc(4 * (size_t)ncand);
+  PYFOF_CUDA(cudaMemcpyAsync(amc.data(), am, sizeof(double) * 4 * ncand, cudaMemcpyDeviceToHost, s));
   PYFOF_CUDA(cudaStreamSynchronize(s));
+  const HaloResult *hres = reinterpret_cast<const HaloResult *>(amc.data() + 3 * (size_t)ncand);
   int64_t nvalid = 0, nmax = 0;
   for (int c = 0; c < ncand; ++c) {
     for (int d = 0; d < 3; ++d) am_host[3 * (size_t)creg[c] + d] += amc[3 * c + d];

@@ -600,28 +600,6 @@ __global__ void __launch_bounds__(BLK) pm_gather_kernel(
   phi_c1[k] = pref * ((raw - wk * selfe[e]) - dz0);
 }
 
-// bound_depth_continuous / bound_c2_delta_depth (:3080-3117)
-template <typename T>
-__device__ __forceinline__ T depth_c(T r, T h) {
-  if (r <= (T)0) return (T)208 / ((T)70 * h);
-  if (r >= h) return (T)1 / r;
-  const T e = (T)2 * r / h;
-  if (e <= (T)1) {
-    const T prim = e * e * ((T)112 + e * e * ((T)-56 + e * ((T)14 + e * ((T)8 - (T)3 * e))));
-    return ((T)208 - prim) / ((T)70 * h);
-  }
-  const T prim = e * e * ((T)448 + e * ((T)-280 + e * ((T)56 + e * ((T)14 + e * ((T)-8 + e))))) -
-                 (T)224 * e - (T)12 / e;
-  return ((T)128 - prim) / ((T)70 * h);
-}
-
-template <typename T>
-__device__ __forceinline__ T c2_delta(T r, T ht, T hs) {
-  if (r <= (T)0) return ((T)208 / (T)70) * ((T)1 / ht - (T)1 / hs);
-  if (r >= ht && r >= hs) return (T)0;
-  return depth_c<T>(r, ht) - depth_c<T>(r, hs);
-}
-
 // Short-range residual of every kept member: the spline-softened kernel
 // minus the split kernel its potential already contains, over the kept
 // members within the member's own cutoff a_i = 3.5 spacing / r_i, where
@@ -634,9 +612,9 @@ __device__ __forceinline__ T c2_delta(T r, T ht, T hs) {
 // bound_two_level_pp_update :1345-1498): UPDATE sums over those sources only
 // and subtracts.
 //
-// FP32 product path: the spline-softened 1/r of depth_c with its divisions
-// replaced by products with per-h reciprocals and 1/r from rsqrtf (a few
-// ulps).  FP32 sums are compensated (Kahan); FP64 sums are plain, which
+// FP32 product path: the spline-softened 1/r, D(r, h) (bound_depth_continuous,
+// :3080-3102), with its divisions replaced by products with per-h reciprocals
+// and 1/r from rsqrtf (a few ulps).  FP32 sums are compensated (Kahan); FP64 sums are plain, which
 // keeps the dependent chain per pair to one add.
 struct DepthConst {
   float h, two_over_h, inv70h, six_h;
@@ -657,30 +635,65 @@ __device__ __forceinline__ float depth_fast(float r, float rinv, const DepthCons
   return (128.0f - prim) * c.inv70h;
 }
 
-// FP64 path of the same kernel without divisions or branches on the spline
-// piece.  With e = 2r/h the two pieces and the 1/r beyond them are one
-// expression in truncated powers (expand it to get depth_c's polynomials):
-//     r D(r, h) = 1 - S(e) / 140,
-//     S(e) = (2-e)_+^6 (e^2 + 4e + 2) + 4 (1-e)_+^7 (3 + e),
-// so a pair's term D(r, a) - D(r, eps) is (S(2r/eps) - S(2r/a)) / (140 r).
-// Its rounding error is that of 1/r, above the softened kernel's own
-// once r is far below eps: pairs closer than eps/20 keep depth_c.  1/r: an
-// FP32 reciprocal square root seed y (relative error about 2^-22) and one step
-// of the binomial series 1/sqrt(r2) = y (1 - g)^(-1/2) = y (1 + g/2 + 3 g^2/8
-// + ..), g = 1 - r2 y^2 (|g| about 2^-21, so the dropped cubic term is 2^-65).
-__device__ __forceinline__ double rsqrt_series64(double r2) {
-  const double y = (double)rsqrtf((float)r2);
+// FP64 path: a pair's term D(r, a) - D(r, eps) as one polynomial.  Between the
+// break points h/2 and h of the two kernels each is a polynomial in r, or that
+// plus a multiple of 1/r (the outer piece's 12/e is 6 h / r), and so
+// is their difference: k / r + c0 + c1 r + .. + c7 r^7, with the coefficients
+// of the zone the pair is in.  Where both are on the same piece the 1/r
+// cancels.  A table per halo and refinement ratio (SrSpline) holds the four
+// zones; the pieces join smoothly, so an FP32 distance is enough to pick one.
+// (Two splines per pair took 45 FP64 operations, this takes 22.)
+struct alignas(16) SrSpline {
+  double c[4][10];  // per zone: c0..c7, k, 0
+  float b2[4];      // squared distances at which zones 1, 2, 3 begin
+};
+
+__device__ __forceinline__ void spline_piece(double h, double mid, double *c) {
+  const double s = 2.0 / h, u = 1.0 / (70.0 * h);
+  const double inner[8] = {208.0, 0.0, -112.0, 0.0, 56.0, -14.0, -8.0, 3.0};
+  const double outer[8] = {128.0, 224.0, -448.0, 280.0, -56.0, -14.0, 8.0, -1.0};
+  double p = u;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    c[j] = mid >= h ? 0.0 : (mid < 0.5 * h ? inner[j] : outer[j]) * p;
+    p *= s;
+  }
+  c[8] = mid >= h ? 1.0 : (mid < 0.5 * h ? 0.0 : 6.0 / 70.0);
+}
+
+// A thread per (halo, ratio 1, 2, 4).
+__global__ void sr_spline_kernel(const PmHalo *__restrict__ H, int nh, double app, SrSpline *__restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 3 * nh) return;
+  const double eps = (double)(float)app, a = 3.5 * (double)H[i / 3].spacing / (double)(1 << (i % 3));
+  double b[4] = {0.5 * eps, 0.5 * a, eps, a};  // ascending below
+  for (int j = 0; j < 3; ++j)
+    for (int k = j + 1; k < 4; ++k)
+      if (b[k] < b[j]) {
+        const double t = b[j];
+        b[j] = b[k];
+        b[k] = t;
+      }
+  SrSpline &S = out[i];
+  for (int z = 0; z < 4; ++z) {
+    const double mid = 0.5 * ((z ? b[z - 1] : 0.0) + b[z]);
+    double ca[9], ce[9];
+    spline_piece(a, mid, ca);
+    spline_piece(eps, mid, ce);
+    for (int j = 0; j < 9; ++j) S.c[z][j] = ca[j] - ce[j];
+    S.c[z][9] = 0.0;
+    S.b2[z] = z < 3 ? (float)(b[z] * b[z]) : 0.0f;
+  }
+}
+
+// 1/r: an FP32 reciprocal square root seed y (relative error about 2^-22) and
+// one step of the binomial series 1/sqrt(r2) = y (1 - g)^(-1/2) = y (1 + g/2 +
+// 3 g^2/8 + ..), g = 1 - r2 y^2 (|g| about 2^-21, so the dropped cubic term is
+// 2^-64).
+__device__ __forceinline__ double rsqrt_series64(double r2, float seed) {
+  const double y = (double)seed;
   const double g = fma(-(r2 * y), y, 1.0);
   return fma(y * g, fma(0.375, g, 0.5), y);
-}
-// S(e) for 0 <= e <= 2
-__device__ __forceinline__ double spline_s64(double e) {
-  const double u = 2.0 - e, v = 1.0 - e;
-  const int neg = __double2hiint(v) >> 31;  // all ones when e > 1
-  const double vp = __hiloint2double(__double2hiint(v) & ~neg, __double2loint(v) & ~neg);
-  const double u2 = u * u, v2 = vp * vp;
-  const double u6 = u2 * u2 * u2, v7 = v2 * v2 * v2 * (4.0 * vp);
-  return fma(v7, 3.0 + e, u6 * fma(e, e + 4.0, 2.0));
 }
 
 // A target chunk: up to 32 members of one brick, consecutive in cell order
@@ -815,8 +828,8 @@ struct SrTarget {
   float a2f;      // FP32 bound of the pair test, a little above a2; < 0: no target
   R a2;
   bool tl;
-  DepthConst eps, ai;  // FP32 path
-  double two_over_eps, two_over_ai, eps64, r2_min;  // FP64 path
+  DepthConst eps, ai;      // FP32 path
+  const SrSpline *spline;  // FP64 path: the halo's table of this target's ratio
   R acc, comp;
 };
 
@@ -849,11 +862,12 @@ __device__ __forceinline__ void sr_pairs(const float4 *__restrict__ buf, const u
     const int j = __ffs(mask) - 1;
     mask &= mask - 1;
     const float4 s = buf[j];
+    const float fx = s.x - t.me.x, fy = s.y - t.me.y, fz = s.z - t.me.z;
     R dx, dy, dz;
     if (t.tl) {
       dx = (R)s.x - (R)t.me.x; dy = (R)s.y - (R)t.me.y; dz = (R)s.z - (R)t.me.z;
     } else {
-      dx = (R)__fsub_rn(s.x, t.me.x); dy = (R)__fsub_rn(s.y, t.me.y); dz = (R)__fsub_rn(s.z, t.me.z);
+      dx = (R)fx; dy = (R)fy; dz = (R)fz;
     }
     const R r2 = dx * dx + dy * dy + dz * dz;
     if (!(r2 < t.a2)) continue;
@@ -863,15 +877,23 @@ __device__ __forceinline__ void sr_pairs(const float4 *__restrict__ buf, const u
       const float v = t.acc + y;
       t.comp = (v - t.acc) - y;
       t.acc = v;
-    } else if (r2 > t.r2_min) {
-      const double rinv = rsqrt_series64(r2), d = r2 * rinv;
-      double sd = -spline_s64(d * t.two_over_ai);
-      const double ee = d * t.two_over_eps;
-      if (ee < 2.0) sd += spline_s64(ee);
-      t.acc = fma((double)s.w * rinv, sd, t.acc);
     } else {
-      const R d = sqrt(r2);
-      t.acc += (R)140 * (R)s.w * (depth_c<R>(d, sqrt(t.a2)) - depth_c<R>(d, t.eps64));
+      const float r2f = fx * fx + fy * fy + fz * fz;
+      const SrSpline &S = *t.spline;
+      const int z = (r2f >= S.b2[0]) + (r2f >= S.b2[1]) + (r2f >= S.b2[2]);
+      const double2 *c = reinterpret_cast<const double2 *>(S.c[z]);
+      // (coincident members: a finite 1/r with coefficient 0, r = 0)
+      const double rinv = rsqrt_series64(r2, rsqrtf(fmaxf(r2f, 1e-30f))), r = r2 * rinv;
+      const double2 c67 = c[3], c45 = c[2], c23 = c[1], c01 = c[0];
+      double v = fma(c67.y, r, c67.x);
+      v = fma(v, r, c45.y);
+      v = fma(v, r, c45.x);
+      v = fma(v, r, c23.y);
+      v = fma(v, r, c23.x);
+      v = fma(v, r, c01.y);
+      v = fma(v, r, c01.x);
+      v = fma(S.c[z][8], rinv, v);
+      t.acc = fma((double)s.w, v, t.acc);
     }
   }
 }
@@ -964,7 +986,7 @@ __device__ __forceinline__ void sr_chunk_sum(const SrChunk &C, const PmHalo &p, 
   }
 }
 
-// Bound by FP64 arithmetic per interacting pair (about 45 operations) once
+// Bound by instruction issue per interacting pair (FP64 and conversions) once
 // enough warps have work.  Persistent blocks: first the heavy chunks, a
 // block each (eight warps take the source batches in turn and their sums
 // are added in warp order), then the others, a warp each; both most sources
@@ -974,23 +996,21 @@ __global__ void __launch_bounds__(32 * kSrWarps, sizeof(R) == 4 ? 4 : 3) sr_gath
     const PmHalo *__restrict__ H, const uint8_t *__restrict__ keep, const uint8_t *__restrict__ pr,
     const SrChunk *__restrict__ chunks, uint32_t nchunks, const uint32_t *__restrict__ nheavy_p,
     const uint32_t *__restrict__ cstart, const uint32_t *__restrict__ cmem, const float4 *__restrict__ src4,
-    const uint32_t *__restrict__ rpos, const uint32_t *__restrict__ rsrc, double a_val, double app,
-    R *__restrict__ phi_sr, unsigned *__restrict__ next) {
+    const uint32_t *__restrict__ rpos, const uint32_t *__restrict__ rsrc, const SrSpline *__restrict__ splines,
+    double a_val, double app, R *__restrict__ phi_sr, unsigned *__restrict__ next) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ float4 buf[kSrWarps][64];
   __shared__ uint32_t idx[kSrWarps][64];
   __shared__ R part[kSrWarps][32];
   __shared__ unsigned s_ch;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // the spline tables of the halo in hand (FP64), one copy per warp
+  __shared__ SrSpline tables[sizeof(R) == 8 ? kSrWarps : 1][3];
+  int table_h = -1;
   const uint32_t nheavy = nheavy_p[UPDATE ? 1 : 0];
-  const R eps = (R)(double)(float)app;
-  // FP64 sums carry the 140 of S(e)
-  const R fac = (R)(a_val / (6.0 * kPi) / (sizeof(R) == 8 ? 140.0 : 1.0));
+  const R fac = (R)(a_val / (6.0 * kPi));
   SrTarget<R> t;
-  t.eps = depth_const((float)eps);
-  t.eps64 = (double)eps;
-  t.two_over_eps = 2.0 / (double)eps;
-  t.r2_min = fmax(2.5e-3 * (double)eps * (double)eps, 1e-30);
+  t.eps = depth_const((float)(double)(float)app);
   // the chunk's targets; false when it has nothing to do
   auto begin = [&](const SrChunk &C, const PmHalo &p, int64_t &k) -> bool {
     if (!p.pending) return false;
@@ -1006,7 +1026,17 @@ __global__ void __launch_bounds__(32 * kSrWarps, sizeof(R) == 4 ? 4 : 3) sr_gath
     // the FP32 distance of a pair is within 1e-6 of the exact one
     t.a2f = active ? (float)t.a2 * 1.00001f + 1e-37f : -1.0f;
     t.ai = depth_const((float)ai);
-    t.two_over_ai = 2.0 / (double)ai;
+    if constexpr (sizeof(R) == 8) {
+      if (C.h != table_h) {
+        __syncwarp();
+        const uint4 *from = reinterpret_cast<const uint4 *>(splines + 3 * (int64_t)C.h);
+        uint4 *to = reinterpret_cast<uint4 *>(tables[warp]);
+        for (int i = lane; i < (int)(3 * sizeof(SrSpline) / 16); i += 32) to[i] = from[i];
+        __syncwarp();
+        table_h = C.h;
+      }
+      t.spline = &tables[warp][ri == 4 ? 2 : ri - 1];
+    }
     t.tl = p.two_level != 0;
     t.acc = t.comp = (R)0;
     if (!active) k = -1;
@@ -2156,6 +2186,13 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   PYFOF_CHECK_LAUNCH();
   sr_chunk_fill_kernel<<<gC, BLK, 0, s>>>(cstart, chcnt, nbrick, chspan);
   PYFOF_CHECK_LAUNCH();
+  SrSpline *splines = W.carve<SrSpline>(3 * (size_t)nh);
+  if (!splines) { set_error("workspace exhausted (C2 splines)"); return kAlloc; }
+  static_assert(sizeof(SrSpline) % 16 == 0, "copied as 16-byte words");
+  if (sizeof(R) == 8) {
+    sr_spline_kernel<<<(unsigned)ceil_div(3 * (int64_t)nh, 128), 128, 0, s>>>(dH, nh, a.softening, splines);
+    PYFOF_CHECK_LAUNCH();
+  }
   // persistent blocks: those that fit on the GPU at once, if there is work for them
   const unsigned gS = (unsigned)std::min<int64_t>(std::max<uint32_t>(nchunk, 1), 148 * (sizeof(R) == 4 ? 4 : 3));
   // per-member refinement ratio, refined-region sources and targets
@@ -2479,16 +2516,16 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
     PYFOF_CUDA(cudaMemsetAsync(sr_next, 0, 2 * sizeof(unsigned), s));
     if (pass == 1) {
       sr_gather_kernel<R, false><<<gS, 32 * kSrWarps, 0, s>>>(dH, keep, pr, chunks, nchunk, sr_next + 2, cstart,
-                                                              cmem, src4, nullptr, nullptr, a.a_val, a.softening,
-                                                              c2, sr_next);
+                                                              cmem, src4, nullptr, nullptr, splines, a.a_val,
+                                                              a.softening, c2, sr_next);
       PYFOF_CHECK_LAUNCH();
     } else {
       PYFOF_TRY(exclusive_scan_u32(rflag, rpos, (int64_t)npm + 1, nullptr, W, s));
       sr_removed_fill_kernel<<<gP, BLK, 0, s>>>(rflag, rpos, npm, rsrc);
       PYFOF_CHECK_LAUNCH();
       sr_gather_kernel<R, true><<<gS, 32 * kSrWarps, 0, s>>>(dH, keep, pr, chunks, nchunk, sr_next + 2, cstart,
-                                                             cmem, src4, rpos, rsrc, a.a_val, a.softening, c2,
-                                                             sr_next);
+                                                             cmem, src4, rpos, rsrc, splines, a.a_val, a.softening,
+                                                             c2, sr_next);
       PYFOF_CHECK_LAUNCH();
     }
     if (!pend_small.empty()) {

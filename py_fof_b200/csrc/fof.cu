@@ -930,14 +930,16 @@ __device__ __forceinline__ void link_batch(ChunkPair &c, float4 o, int q, int hq
 __global__ void __launch_bounds__(BLK, 4) fof_link_dense_kernel(
     const float4 *__restrict__ pos, const uint32_t *__restrict__ prid, const RegionDev *__restrict__ R,
     const uint32_t *__restrict__ cell_start, int *parent, const DenseChunk *__restrict__ chunks,
-    int64_t nchunks, LinkParams P, DenseIndex D, int32_t *flags) {
+    int64_t nchunks, int lg_parts, LinkParams P, DenseIndex D, int32_t *flags) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ NbCell nb_cells[BLK / 32][27];
   const int lane = threadIdx.x & 31;
   NbCell *cells = nb_cells[threadIdx.x >> 5];
   const int64_t nw = ((int64_t)gridDim.x * BLK) >> 5;
-  for (int64_t ch = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5; ch < nchunks; ch += nw) {
-    const DenseChunk C = chunks[ch];
+  for (int64_t w = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5; w < nchunks << lg_parts; w += nw) {
+    const DenseChunk C = chunks[w >> lg_parts];
+    const uint32_t part = (uint32_t)w & ((1u << lg_parts) - 1);
+    uint32_t turn = 0;  // batches so far
     const int64_t cb = cell_start[C.cell];
     const int64_t cn = (int64_t)cell_start[C.cell + 1] - cb;
     const int64_t k = (int64_t)C.e0 + lane;
@@ -1077,6 +1079,7 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_dense_kernel(
       const uint32_t T = __shfl_sync(FULL, incl, 31);
       const uint32_t at = first - (incl - cnt);  // source of batch index g: at + g
       for (uint32_t g0 = 0; g0 < T; g0 += 32) {
+        if ((turn++ & ((1u << lg_parts) - 1)) != part) continue;
         // --- a source per lane
         const uint32_t g = g0 + (uint32_t)lane;
         int owner = 0;
@@ -1223,14 +1226,21 @@ __global__ void __launch_bounds__(BLK) fof_dense_build_kernel(
     atomicAdd(&hist[sx + g.s[0] * (sy + g.s[1] * sz)], 1u);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x < 32) {
     uint32_t run = 0;
-    for (int k = 0; k < S; ++k) {
-      const uint32_t h = hist[k];
-      cur[k] = run;
-      run += h;
+    for (int k0 = 0; k0 < S; k0 += 32) {
+      const int k = k0 + (int)threadIdx.x;
+      const uint32_t h = k < S ? hist[k] : 0;
+      uint32_t incl = h;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((int)threadIdx.x >= o) incl += v;
+      }
+      if (k < S) cur[k] = run + incl - h;
+      run += __shfl_sync(0xffffffffu, incl, 31);
     }
-    cur[S] = run;
+    if (threadIdx.x == 0) cur[S] = run;
   }
   __syncthreads();
   uint32_t *t = tab + (int64_t)blockIdx.x * stride;
@@ -2018,8 +2028,12 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
       PYFOF_CHECK_LAUNCH();
     }
     if (ndense_chunks > 0) {
-      const unsigned dgrid = (unsigned)std::min<int64_t>(ceil_div(ndense_chunks * 32, BLK), (int64_t)kNumSMs * 24);
-      fof_link_dense_kernel<<<dgrid, BLK, 0, s>>>(pos, prid, dR, cstart, parent, dchunks, ndense_chunks, P, D,
+      // warps per chunk: up to 8 while the blocks all fit on the chip at once
+      int lg = 0;
+      while (lg < 3 && ndense_chunks << (lg + 1) <= (int64_t)kNumSMs * 4 * (BLK / 32)) ++lg;
+      const unsigned dgrid = (unsigned)std::min<int64_t>(ceil_div((ndense_chunks << lg) * 32, BLK),
+                                                         (int64_t)kNumSMs * 24);
+      fof_link_dense_kernel<<<dgrid, BLK, 0, s>>>(pos, prid, dR, cstart, parent, dchunks, ndense_chunks, lg, P, D,
                                                   ctx.d_flags);
       PYFOF_CHECK_LAUNCH();
     }

@@ -440,19 +440,29 @@ static int32_t launch_direct_loop(bool fp64, int threads, unsigned nb, int cap, 
 static int32_t direct_first_pass(Context &ctx, bool fp64, const Members &m, const int64_t *off, const int32_t *dl,
                                  const std::vector<int32_t> &list, const std::vector<HaloTask> &tasks,
                                  const direct::DirectParams &P, double *phi1, cudaStream_t s) {
-  const int pt = fp64 ? direct::kPhi1Targets<true> : direct::kPhi1Targets<false>;
+  // lanes per target (ub_direct_phi1_kernel): more than one while a lane each
+  // would leave the chip's thread slots empty
+  int64_t targets = 0;
+  for (int32_t c : list) targets += tasks[c].np;
+  int sms = 0, per_sm = 0;
+  PYFOF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx.device));
+  PYFOF_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxThreadsPerMultiProcessor, ctx.device));
+  const bool wide = fp64 && targets < (int64_t)sms * per_sm;
+  const int pt = wide ? direct::kPhi1Targets<direct::kPhi1Lanes> : direct::kPhi1Targets<1>;
   std::vector<int2> tl;
   for (size_t e = 0; e < list.size(); ++e)
     for (int t0 = 0; t0 < tasks[list[e]].np; t0 += pt) tl.push_back(make_int2((int)e, t0));
   int2 *dtl = ctx.work.carve<int2>(tl.size());
   if (!dtl) { set_error("workspace exhausted (direct potentials)"); return kAlloc; }
   PYFOF_TRY(upload(ctx, dtl, tl.data(), sizeof(int2) * tl.size(), s));
-  if (fp64)
-    direct::ub_direct_phi1_kernel<true><<<(unsigned)tl.size(), direct::kPhi1Threads<true>, 0, s>>>(m, off, dl, dtl, P,
-                                                                                                  phi1);
+  const unsigned nb = (unsigned)tl.size();
+  constexpr int L = direct::kPhi1Lanes;
+  if (wide)
+    direct::ub_direct_phi1_kernel<true, L><<<nb, direct::kPhi1Targets<L> * L, 0, s>>>(m, off, dl, dtl, P, phi1);
+  else if (fp64)
+    direct::ub_direct_phi1_kernel<true, 1><<<nb, direct::kPhi1Targets<1>, 0, s>>>(m, off, dl, dtl, P, phi1);
   else
-    direct::ub_direct_phi1_kernel<false><<<(unsigned)tl.size(), direct::kPhi1Threads<false>, 0, s>>>(m, off, dl, dtl,
-                                                                                                    P, phi1);
+    direct::ub_direct_phi1_kernel<false, 1><<<nb, direct::kPhi1Targets<1>, 0, s>>>(m, off, dl, dtl, P, phi1);
   PYFOF_CHECK_LAUNCH();
   return kOk;
 }

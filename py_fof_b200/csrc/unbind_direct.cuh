@@ -98,36 +98,41 @@ __device__ __forceinline__ double pair_depth64(float xj, float yj, float zj, flo
 // every lane of the group: a serial sum whose terms were computed in parallel.
 template <int G>
 __device__ __forceinline__ void add_in_order(double &acc, double t, int n, unsigned group) {
+  if constexpr (G == 1) {
+    acc = __dadd_rn(acc, t);
+  } else {
 #pragma unroll
-  for (int u = 0; u < G; ++u) {
-    const double v = __shfl_sync(group, t, u, G);
-    if (u < n) acc = __dadd_rn(acc, v);
+    for (int u = 0; u < G; ++u) {
+      const double v = __shfl_sync(group, t, u, G);
+      if (u < n) acc = __dadd_rn(acc, v);
+    }
   }
 }
 
 // The first-pass potentials of many direct-summation halos, spread over the
-// whole GPU: block b takes the kPhi1Targets targets tiles[b] = (entry of list, first
+// whole GPU: block b takes the kPhi1Targets<G> targets tiles[b] = (entry of list, first
 // target) of one halo and streams the halo's members through shared memory
 // in ascending order.  Each target adds its sources in ascending index,
 // skipping itself: the reference's accumulation order (bound_fortran.f90:
 // 2619-2640; its i<j loop adds each pair term to both ends) with the
 // operations of the in-kernel first pass of ub_direct_kernel, so the results
 // are the same bits; the removal loop then starts from phi1.
-// FP64: latency-bound (a square root and a division per term in one
-// dependent chain per target), so G = 8 lanes share a target: they compute
-// eight terms at once and add them in order (add_in_order).  A halo of 450
-// members took 184 us with a lane per target.  FP32: a lane per target (its
-// terms are as short as the ordered adds would be).
-constexpr int kPhi1Lanes64 = 8;
-template <bool FP64>
-constexpr int kPhi1Targets = FP64 ? 32 : 64;
-template <bool FP64>
-constexpr int kPhi1Threads = FP64 ? 32 * kPhi1Lanes64 : 64;
-template <bool FP64>
-__global__ void __launch_bounds__(kPhi1Threads<FP64>) ub_direct_phi1_kernel(
+// G lanes share a target: they compute G terms at once and add them in order
+// (add_in_order).  An FP64 term is a square root and a division in one
+// dependent chain per target, so a few targets (fewer than the chip has
+// thread slots) are latency-bound and take G = 8: a halo of 450 members takes
+// 41 us, with a lane per target 184.  With more targets the chains hide one
+// another and the ordered adds are only extra work, so G = 1: 20,000 halos of
+// 20 to 1000 members 2.6 ms, with eight lanes 3.7.  FP32 terms are as short
+// as the ordered adds: always G = 1.
+constexpr int kPhi1Lanes = 8;
+template <int G>
+constexpr int kPhi1Targets = G == 1 ? 64 : 32;
+template <bool FP64, int G>
+__global__ void __launch_bounds__(kPhi1Targets<G> * G) ub_direct_phi1_kernel(
     Members m, const int64_t *__restrict__ off, const int32_t *__restrict__ list, const int2 *__restrict__ tiles,
     DirectParams P, double *__restrict__ phi1) {
-  constexpr int G = FP64 ? kPhi1Lanes64 : 1, NT = kPhi1Threads<FP64>;
+  constexpr int NT = kPhi1Targets<G> * G;
   __shared__ float4 src[NT];
   const int2 t = tiles[blockIdx.x];
   const int c = list[t.x];
@@ -215,7 +220,7 @@ __global__ void __launch_bounds__(NT) ub_direct_kernel(Members m, const int64_t 
   unsigned long long *ukey = reinterpret_cast<unsigned long long *>(jdel + cap);
   double *phid = reinterpret_cast<double *>(ukey + cap);
   unsigned char *keep = reinterpret_cast<unsigned char *>(phid + cap);
-  constexpr int G = FP64 ? kPhi1Lanes64 : 1;
+  constexpr int G = FP64 ? kPhi1Lanes : 1;
   __shared__ int red_i[NT / 32];
   __shared__ double red_d[7][NT / 32];
   __shared__ double s_sum[7];

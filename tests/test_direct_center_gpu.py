@@ -61,3 +61,25 @@ def test_first_pass_is_the_static_path(n):
         b, ierr = _native.halo_potential_direct_static(q, w, fp64=fp64)
         assert meth == 0 and ierr == 0
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("fp64", [1, 0])
+def test_first_pass_of_many_halos_is_that_of_few(fp64):
+    """More direct-summation members in a call than the chip has thread slots
+    (a lane per target) against the same halos in two calls that stay below
+    (eight lanes per target in FP64): the same bits."""
+    rng = np.random.default_rng(5)
+    sizes = rng.integers(700, 1000, 480)
+    xs = [rng.standard_normal((3, n)) * 0.25 + rng.uniform(50, 450, (3, 1)) for n in sizes]
+    vs = [rng.standard_normal((3, n)) * np.sqrt(0.02 * n) for n in sizes]
+    kw = dict(L_Box=512.0, linking_length=0.5, np_halo_min=5, bound_check=True)
+    h = len(sizes) // 2
+    assert sizes.sum() > 148 * 2048 > max(sizes[:h].sum(), sizes[h:].sum())
+    with _native.options(unbind_fp64=fp64):
+        g = P._fof_core(xs, vp_list=vs, **kw)
+        assert _native.get_stat("direct_halos") >= len(sizes)
+        parts = [P._fof_core(xs[a:b], vp_list=vs[a:b], **kw) for a, b in ((0, h), (h, len(sizes)))]
+    in_halo, halo_id = np.asarray(g[0]), np.asarray(g[1])
+    assert 0.1 < in_halo.mean() < 0.999
+    assert np.array_equal(in_halo, np.concatenate([q[0] for q in parts]))
+    assert np.array_equal(halo_id > 0, np.concatenate([q[1] for q in parts]) > 0)

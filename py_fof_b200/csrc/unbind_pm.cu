@@ -1351,30 +1351,54 @@ __device__ __forceinline__ double bsum_d(double v, double *red) {
   return t;
 }
 
-// Seven block sums at once: each value is reduced in the same order as by
+// Seven block sums at once, for 32 warps or fewer: each is reduced as by
 // bsum_d (warp butterfly, then the warp partials in warp order), so the
-// results are bit-identical, with 2 barriers instead of 21.
-__device__ __forceinline__ void bsum7_d(double *v, double *red) {
-  constexpr int NW = IBLK / 32;
+// results are bit-identical.  The butterfly's first three steps exchange
+// halves: at each a lane hands over the values it does not go on with (18
+// shuffles instead of 70), and one lane per value adds the partials, not
+// every thread all of them.  Afterwards lane j of warp 0 holds sum j (j < 7);
+// the other threads hold nothing.  red: 7 * 33 doubles.
+__device__ __forceinline__ double block_sum7(const double *a, double *red) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double v[4];
 #pragma unroll
-  for (int j = 0; j < 7; ++j)
-    for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0)
-#pragma unroll
-    for (int j = 0; j < 7; ++j) red[j * NW + (threadIdx.x >> 5)] = v[j];
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < 7; ++j) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[j * NW + w];
-    v[j] = t;
+  for (int j = 0; j < 4; ++j) {
+    const double hi = j < 3 ? a[j + 4] : 0.0;
+    const double got = __shfl_xor_sync(FULL, lane & 16 ? a[j] : hi, 16);
+    v[j] = (lane & 16 ? hi : a[j]) + got;
   }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const double got = __shfl_xor_sync(FULL, lane & 8 ? v[j] : v[j + 2], 8);
+    v[j] = (lane & 8 ? v[j + 2] : v[j]) + got;
+  }
+  const double got = __shfl_xor_sync(FULL, lane & 4 ? v[0] : v[1], 4);
+  double t = (lane & 4 ? v[1] : v[0]) + got;
+  t += __shfl_xor_sync(FULL, t, 2);
+  t += __shfl_xor_sync(FULL, t, 1);
+  const int j = (lane & 16) / 4 + (lane & 8) / 4 + (lane & 4) / 4;
+  if ((lane & 3) == 0 && j < 7) red[33 * j + warp] = t;
+  __syncthreads();
+  t = 0.0;
+  if (warp == 0 && lane < 7) {
+#pragma unroll 8
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[33 * lane + w];
+  }
+  return t;
+}
+
+// Centre and mean velocity from the seven sums in the lanes of warp 0, to
+// c6[6].  All threads of warp 0 call it.
+__device__ __forceinline__ void centre_of(double t, float *c6) {
+  const int lane = threadIdx.x & 31;
+  const double w = __shfl_sync(0xffffffffu, t, 0);
+  if (lane >= 1 && lane < 7) c6[lane - 1] = __double2float_rn(t / w);
 }
 
 // The digit of the need-th largest key, from a 256-bin histogram of one digit
-// of the keys: bins are summed from the top.  Every warp does it alone (eight
-// bins per lane, a suffix scan over the lanes).  Returns the digit; above =
+// of the keys: bins are summed from the top by one warp (eight bins per lane, a suffix
+// scan over the lanes).  Returns the digit; above =
 // keys in higher bins, count = keys in it.
 __device__ __forceinline__ int digit_of(const unsigned *hist, int need, int &above, int &count) {
   constexpr unsigned FULL = 0xffffffffu;
@@ -1409,16 +1433,78 @@ __device__ __forceinline__ int digit_of(const unsigned *hist, int need, int &abo
   return __shfl_sync(FULL, digit, src);
 }
 
+// The unbound members leave most energetic first; equal energies: lower index
+// first.  As one 64-bit key (the bits of E + 0, which order like E >= 0,
+// then ~index) they are distinct; 0 is no key.
+__device__ __forceinline__ unsigned long long removal_key(float e, uint32_t i) {
+  return ((unsigned long long)__float_as_uint(e + 0.0f) << 32) | (0xffffffffu - i);
+}
+
+// The need-th largest of the keys key(0) .. key(nu - 1) up to the digits that
+// do not matter: exactly `need` keys are at or above the value returned.
+// Radix select by the block, from the exponent down, until the keys of the
+// last digit's bin are all taken (three digits, usually).  Energies have few
+// exponents, so that digit is counted per warp first.  hist: 2 x 256.
+template <typename Key>
+__device__ __forceinline__ unsigned long long nth_largest(Key key, int nu, int need, unsigned (*hist)[256],
+                                                          int *s_digit) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nt = (int)blockDim.x;
+  unsigned long long prefix = 0, mask = 0;
+  for (int t = threadIdx.x; t < 512; t += nt) (&hist[0][0])[t] = 0;
+  __syncthreads();
+  for (int step = 0; step < 8; ++step) {
+    // bits 62..55, 54..47, .., 14..7, 6..0
+    const int shift = step < 7 ? 55 - 8 * step : 0;
+    const unsigned dm = step < 7 ? 255u : 127u;
+    unsigned *h = hist[step & 1];
+    if (step == 0) {
+      for (int t0 = 32 * warp; t0 < nu; t0 += nt) {
+        const unsigned long long k = t0 + lane < nu ? key(t0 + lane) : 0;
+        const unsigned d = k ? (unsigned)(k >> 55) & 255u : 256u;
+        const unsigned same = __match_any_sync(FULL, d);
+        if (k && lane == __ffs(same) - 1) atomicAdd(&h[d], (unsigned)__popc(same));
+      }
+    } else {
+#pragma unroll 4
+      for (int t = threadIdx.x; t < nu; t += nt) {
+        const unsigned long long k = key(t);
+        if (k && (k & mask) == prefix) atomicAdd(&h[(unsigned)(k >> shift) & dm], 1u);
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      int above, count;
+      const int digit = digit_of(h, need, above, count);
+      if (lane == 0) {
+        s_digit[0] = digit;
+        s_digit[1] = need - above;
+        s_digit[2] = count;
+      }
+    } else if (step > 0) {  // the previous step's bins, for the next step
+      for (int t = threadIdx.x - 32; t < 256; t += nt - 32) hist[(step + 1) & 1][t] = 0;
+    }
+    __syncthreads();
+    need = s_digit[1];
+    prefix |= (unsigned long long)s_digit[0] << shift;
+    mask |= (unsigned long long)dm << shift;
+    if (need == s_digit[2]) break;
+  }
+  return prefix;
+}
+
 // One block per pending halo: combine the potential, then the inner
 // removal loop of bound_check_grid (:2739-2855).  Leaves status -1 when the
 // potential must be refreshed (next pass).
 //
 // A chain of sweeps over the members with a barrier between them, bound by
-// latency.  An iteration sweeps all members twice (centre, energies); the
-// unbound ones go as 64-bit keys (energy, then ~index, so the order is total)
-// to shared memory, and the nb-th largest key is found by a radix select over
-// that list.  Only when more than KCAP are unbound are the energies selected
-// from memory, by sweeps over all members.
+// latency.  An iteration sweeps all members twice (centre, energies) with the
+// loads of four members in flight; the unbound ones go as removal keys to
+// shared memory, where the nb-th largest is found.  Only when more than KCAP
+// are unbound are the keys made again from memory, by sweeps over all members.
+// (256^3 box, 17 passes: 1.79 ms with every thread adding all warps' partial
+// sums, dividing for the centre and looking for the digit, 1.23 ms with one
+// warp doing so.)
 constexpr int KCAP = 4096;
 
 template <typename R>
@@ -1436,11 +1522,11 @@ __global__ void __launch_bounds__(IBLK) pm_inner_kernel(const Members m, PmHalo 
   const int h = list[blockIdx.x];
   PmHalo &p = H[h];
   if (!p.pending) return;
-  __shared__ double red7[7 * (IBLK / 32)];
-  __shared__ int red_i[IBLK / 32];
-  __shared__ unsigned hist[256];
+  __shared__ double red7[7 * 33];
+  __shared__ unsigned hist[2][256];
   __shared__ unsigned long long ukey[KCAP];
-  __shared__ int s_err, s_nu;
+  __shared__ float s_c[6];
+  __shared__ int s_err, s_nu, s_digit[3];
   const int64_t b0 = p.off;
   const int np = p.np;
   const int lane = threadIdx.x & 31;
@@ -1473,42 +1559,45 @@ __global__ void __launch_bounds__(IBLK) pm_inner_kernel(const Members m, PmHalo 
   for (;;) {
     double a7[7] = {0, 0, 0, 0, 0, 0, 0};
     if (threadIdx.x == 0) s_nu = 0;
-#pragma unroll 2
+#pragma unroll 4
     for (int i = threadIdx.x; i < np; i += IBLK) {
       const int64_t k = b0 + i;
-      if (!keep[k]) continue;
+      const bool in = keep[k];
       const double wi = (double)m.w[k];
-      a7[0] += wi;
-      for (int d = 0; d < 3; ++d) { a7[1 + d] += wi * (double)m.q[d][k]; a7[4 + d] += wi * (double)m.v[d][k]; }
+      a7[0] += in ? wi : 0.0;
+      for (int d = 0; d < 3; ++d) {
+        const double q = wi * (double)m.q[d][k], v = wi * (double)m.v[d][k];
+        a7[1 + d] += in ? q : 0.0;
+        a7[4 + d] += in ? v : 0.0;
+      }
     }
-    bsum7_d(a7, red7);
-    float qc[3], vc[3];
-    for (int d = 0; d < 3; ++d) {
-      qc[d] = __double2float_rn(a7[1 + d] / a7[0]);
-      vc[d] = __double2float_rn(a7[4 + d] / a7[0]);
-    }
-#pragma unroll 2
+    const double sum = block_sum7(a7, red7);
+    if (threadIdx.x < 32) centre_of(sum, s_c);
+    __syncthreads();
+    const float qc[3] = {s_c[0], s_c[1], s_c[2]}, vc[3] = {s_c[3], s_c[4], s_c[5]};
+#pragma unroll 4
     for (int i0 = threadIdx.x - lane; i0 < np; i0 += IBLK) {
       const int i = i0 + lane;
-      const int64_t k = b0 + i;
-      float e = -1.0f;
-      if (i < np && keep[k]) {
-        float s = 0.f;
-        for (int d = 0; d < 3; ++d) {
-          const float dv = __fadd_rn(__fsub_rn(m.v[d][k], vc[d]), __fmul_rn(b_val, __fsub_rn(m.q[d][k], qc[d])));
-          s = d == 0 ? __fmul_rn(dv, dv) : __fadd_rn(s, __fmul_rn(dv, dv));
-        }
-        e = __fadd_rn(__fdiv_rn(s, 2.0f), phi[k]);
+      const int64_t k = b0 + min(i, np - 1);
+      const bool in = i < np && keep[k];
+      float s = 0.f;
+      for (int d = 0; d < 3; ++d) {
+        const float dv = __fadd_rn(__fsub_rn(m.v[d][k], vc[d]), __fmul_rn(b_val, __fsub_rn(m.q[d][k], qc[d])));
+        s = d == 0 ? __fmul_rn(dv, dv) : __fadd_rn(s, __fmul_rn(dv, dv));
+      }
+      float e = __fadd_rn(__fdiv_rn(s, 2.0f), phi[k]);
+      if (in) {
         if (!isfinite(e)) s_err = kInvalid;
         en[k] = e;
+      } else {
+        e = -1.0f;
       }
       const unsigned bal = __ballot_sync(0xffffffffu, e >= 0.0f);
       if (bal) {
         int at = 0;
         if (lane == 0) at = atomicAdd(&s_nu, __popc(bal));
         at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & lanemask_lt());
-        if (e >= 0.0f && at < KCAP)
-          ukey[at] = ((unsigned long long)__float_as_uint(e + 0.0f) << 32) | (0xffffffffu - (unsigned)i);
+        if (e >= 0.0f && at < KCAP) ukey[at] = removal_key(e, (uint32_t)i);
       }
     }
     __syncthreads();
@@ -1519,83 +1608,22 @@ __global__ void __launch_bounds__(IBLK) pm_inner_kernel(const Members m, PmHalo 
       break;
     }
     const int nb = min(nu, max(1, (int)ceil(0.02 * (double)np_bound)));
-    int need = nb;
     if (nu <= KCAP) {
-      // the nb largest keys, digit by digit from the top, until the keys of
-      // the last digit's bin are all taken (the keys are distinct)
-      unsigned long long prefix = 0, mask = 0;
-      for (int shift = 56; shift >= 0; shift -= 8) {
-        for (int t = threadIdx.x; t < 256; t += IBLK) hist[t] = 0;
-        __syncthreads();
-        for (int t = threadIdx.x; t < nu; t += IBLK) {
-          const unsigned long long key = ukey[t];
-          if ((key & mask) == prefix) atomicAdd(&hist[(unsigned)(key >> shift) & 255u], 1u);
-        }
-        __syncthreads();
-        int above, count;
-        const int digit = digit_of(hist, need, above, count);
-        __syncthreads();
-        need -= above;
-        prefix |= (unsigned long long)digit << shift;
-        mask |= 255ull << shift;
-        if (need == count) break;
-      }
+      const unsigned long long least = nth_largest([&](int t) { return ukey[t]; }, nu, nb, hist, s_digit);
       for (int t = threadIdx.x; t < nu; t += IBLK) {
         const unsigned long long key = ukey[t];
-        if (key >= prefix) remove((int)(0xffffffffu - (unsigned)key));
+        if (key >= least) remove((int)(0xffffffffu - (unsigned)key));
       }
     } else {
-      // radix select of the nb largest energies among the unbound members:
-      // key = bits of (E + 0) (E >= 0, so the bits order like the values)
-      unsigned prefix = 0, mask = 0;
-      int n_eq = 0;
-      for (int shift = 24; shift >= 0; shift -= 8) {
-        for (int t = threadIdx.x; t < 256; t += IBLK) hist[t] = 0;
-        __syncthreads();
-        for (int i = threadIdx.x; i < np; i += IBLK) {
-          const int64_t k = b0 + i;
-          if (!keep[k]) continue;
-          const float e = en[k];
-          if (!(e >= 0.0f)) continue;
-          const unsigned key = __float_as_uint(e + 0.0f);
-          if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
-        }
-        __syncthreads();
-        int above;
-        const int digit = digit_of(hist, need, above, n_eq);
-        __syncthreads();
-        need -= above;
-        prefix |= (unsigned)digit << shift;
-        mask |= 255u << shift;
-      }
-      // delete every key > threshold and the `need` lowest indices among
-      // key == threshold (equal energies: lower index first)
-      const unsigned thr = prefix;
-      int taken_eq = 0;
-      for (int base = 0; base < np; base += IBLK) {
-        const int i = base + threadIdx.x;
+      auto key = [&](int i) -> unsigned long long {
         const int64_t k = b0 + i;
-        bool del_gt = false, is_eq = false;
-        if (i < np && keep[k]) {
-          const float e = en[k];
-          if (e >= 0.0f) {
-            const unsigned key = __float_as_uint(e + 0.0f);
-            del_gt = key > thr;
-            is_eq = key == thr;
-          }
-        }
-        int before = taken_eq;
-        if (need != n_eq) {  // ordered rank of is_eq within this chunk
-          const unsigned bal = __ballot_sync(0xffffffffu, is_eq);
-          const int warp = threadIdx.x >> 5;
-          __syncthreads();
-          if (lane == 0) red_i[warp] = __popc(bal);
-          __syncthreads();
-          for (int w = 0; w < warp; ++w) before += red_i[w];
-          before += __popc(bal & lanemask_lt());
-          for (int w = 0; w < IBLK / 32; ++w) taken_eq += red_i[w];
-        }
-        if (del_gt || (is_eq && (need == n_eq || before < need))) remove(i);
+        const float e = keep[k] ? en[k] : -1.0f;
+        return e >= 0.0f ? removal_key(e, (uint32_t)i) : 0ull;
+      };
+      const unsigned long long least = nth_largest(key, np, nb, hist, s_digit);
+      for (int i = threadIdx.x; i < np; i += IBLK) {
+        const unsigned long long v = key(i);
+        if (v && v >= least) remove(i);
       }
     }
     __syncthreads();
@@ -1620,12 +1648,18 @@ __global__ void __launch_bounds__(IBLK) pm_inner_kernel(const Members m, PmHalo 
 // Halos above kBigNp members run the same removal loop as pm_inner_kernel,
 // but spread over the whole GPU: their members are cut into chunks of
 // kChunk, every sweep is a grid of chunk blocks, and the per-halo decisions
-// (centre, selection, stop conditions) are small kernels between sweeps,
+// (selection, stop conditions) are small kernels between sweeps,
 // driven by a host loop.  The unbound members of an iteration are compacted
-// into a per-halo list, so the radix select runs over that list only.
+// into a per-halo list of removal keys, so the selection runs over that list
+// only.
+// Bound by the latency of three small launches per iteration: one halo of
+// 0.6 M members 29 us, in four launches with the centre by one thread and
+// half as many blocks per sweep 62 us.
 
 constexpr int64_t kBigNp = 32768;  // default; option "unbind_big_np" overrides
 constexpr int kChunk = 8192;
+// blocks per chunk of the sweeps that sum nothing
+constexpr int kBigSplit = 4;
 
 struct BigHalo {
   int32_t h;          // index into the PM halo table
@@ -1634,8 +1668,6 @@ struct BigHalo {
   int64_t uoff;       // first slot of the halo's unbound list
   int32_t chunk0, nchunk;
   int32_t np_bound, deleted, n_source, status;
-  int32_t nu, nb;
-  float qc[3], vc[3];
 };
 
 struct BigChunk {
@@ -1649,11 +1681,14 @@ __global__ void big_phi_kernel(const BigChunk *__restrict__ ch, int nch, const B
                                const uint8_t *__restrict__ keep, const R *__restrict__ c1,
                                const R *__restrict__ in, const R *__restrict__ c2, float *__restrict__ phi,
                                int32_t *flags) {
-  const BigChunk c = ch[blockIdx.x];
+  const BigChunk c = ch[blockIdx.x / kBigSplit];
   const BigHalo &bh = B[c.b];
   if (!bh.active) return;
   bool bad = false;
-  for (int64_t k = c.start + threadIdx.x; k < c.end; k += blockDim.x) {
+  const int64_t k0 = c.start + (int64_t)(blockIdx.x % kBigSplit) * (kChunk / kBigSplit);
+  const int64_t k1 = min(c.end, k0 + kChunk / kBigSplit);
+#pragma unroll 4
+  for (int64_t k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
     if (!keep[k]) continue;
     float v = (float)((c1[k] + in[k]) + c2[k]);
     if (bh.np_bound == 1 || bh.n_source == 1) v = 0.0f;
@@ -1669,77 +1704,72 @@ __global__ void big_com_kernel(const Members m, const BigChunk *__restrict__ ch,
   const BigChunk c = ch[blockIdx.x];
   if (!B[c.b].active) return;
   double a7[7] = {0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 4
   for (int64_t k = c.start + threadIdx.x; k < c.end; k += blockDim.x) {
-    if (!keep[k]) continue;
+    const bool in = keep[k];
     const double wi = (double)m.w[k];
-    a7[0] += wi;
-    for (int d = 0; d < 3; ++d) { a7[1 + d] += wi * (double)m.q[d][k]; a7[4 + d] += wi * (double)m.v[d][k]; }
+    a7[0] += in ? wi : 0.0;
+    for (int d = 0; d < 3; ++d) {
+      const double q = wi * (double)m.q[d][k], v = wi * (double)m.v[d][k];
+      a7[1 + d] += in ? q : 0.0;
+      a7[4 + d] += in ? v : 0.0;
+    }
   }
-  __shared__ double red[32];
-  for (int j = 0; j < 7; ++j) {
-    const double t = bsum_d(a7[j], red);
-    if (threadIdx.x == 0) part[7 * (int64_t)blockIdx.x + j] = t;
-  }
+  __shared__ double red[7 * 33];
+  const double t = block_sum7(a7, red);
+  if (threadIdx.x < 7) part[7 * (int64_t)blockIdx.x + threadIdx.x] = t;
 }
 
-// per big halo: centre from the chunk sums (in chunk order)
-__global__ void big_center_kernel(BigHalo *__restrict__ B, int nbig, const double *__restrict__ part,
-                                  int32_t *__restrict__ ucount) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nbig) return;
-  BigHalo &bh = B[b];
-  ucount[b] = 0;
-  if (!bh.active) return;
-  double a7[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int c = bh.chunk0; c < bh.chunk0 + bh.nchunk; ++c)
-    for (int j = 0; j < 7; ++j) a7[j] += part[7 * (int64_t)c + j];
-  for (int d = 0; d < 3; ++d) {
-    bh.qc[d] = __double2float_rn(a7[1 + d] / a7[0]);
-    bh.vc[d] = __double2float_rn(a7[4 + d] / a7[0]);
-  }
-}
-
-// energies of the kept members; the unbound ones join the halo's list
+// Energies of the kept members; the unbound ones join the halo's list.  Every
+// block adds up the halo's chunk sums (in chunk order) for the centre itself.
 __global__ void big_energy_kernel(const Members m, const BigChunk *__restrict__ ch, const BigHalo *__restrict__ B,
                                   const uint8_t *__restrict__ keep, const float *__restrict__ phi,
-                                  float *__restrict__ en, float b_val, int32_t *__restrict__ ucount,
-                                  uint32_t *__restrict__ ulist, int32_t *flags) {
-  const BigChunk c = ch[blockIdx.x];
+                                  const double *__restrict__ part, float b_val, int32_t *__restrict__ ucount,
+                                  unsigned long long *__restrict__ ulist, int32_t *flags) {
+  const BigChunk c = ch[blockIdx.x / kBigSplit];
   const BigHalo &bh = B[c.b];
   if (!bh.active) return;
-  bool bad = false;
   const int lane = threadIdx.x & 31;
-  for (int64_t base = c.start; base < c.end; base += blockDim.x) {
-    const int64_t k = base + threadIdx.x;
-    bool unb = false;
-    if (k < c.end && keep[k]) {
-      float s = 0.f;
-      for (int d = 0; d < 3; ++d) {
-        const float dv = __fadd_rn(__fsub_rn(m.v[d][k], bh.vc[d]), __fmul_rn(b_val, __fsub_rn(m.q[d][k], bh.qc[d])));
-        s = d == 0 ? __fmul_rn(dv, dv) : __fadd_rn(s, __fmul_rn(dv, dv));
-      }
-      const float e = __fadd_rn(__fdiv_rn(s, 2.0f), phi[k]);
-      bad |= !isfinite(e);
-      en[k] = e;
-      unb = e >= 0.0f;
+  __shared__ float s_c[6];
+  if (threadIdx.x < 32) {
+    double t = 0.0;
+    if (lane < 7) {
+#pragma unroll 8
+      for (int j = bh.chunk0; j < bh.chunk0 + bh.nchunk; ++j) t += part[7 * (int64_t)j + lane];
     }
+    centre_of(t, s_c);
+  }
+  __syncthreads();
+  const float qc[3] = {s_c[0], s_c[1], s_c[2]}, vc[3] = {s_c[3], s_c[4], s_c[5]};
+  bool bad = false;
+  const int64_t k0 = c.start + (int64_t)(blockIdx.x % kBigSplit) * (kChunk / kBigSplit);
+  const int64_t k1 = min(c.end, k0 + kChunk / kBigSplit);
+#pragma unroll 4
+  for (int64_t base = k0; base < k1; base += blockDim.x) {
+    const int64_t i = base + threadIdx.x, k = min(i, k1 - 1);
+    const bool in = i < k1 && keep[k];
+    float s = 0.f;
+    for (int d = 0; d < 3; ++d) {
+      const float dv = __fadd_rn(__fsub_rn(m.v[d][k], vc[d]), __fmul_rn(b_val, __fsub_rn(m.q[d][k], qc[d])));
+      s = d == 0 ? __fmul_rn(dv, dv) : __fadd_rn(s, __fmul_rn(dv, dv));
+    }
+    const float e = __fadd_rn(__fdiv_rn(s, 2.0f), phi[k]);
+    if (in) bad |= !isfinite(e);
+    const bool unb = in && e >= 0.0f;
     // warp-aggregated append
     const unsigned bal = __ballot_sync(0xffffffffu, unb);
-    int basepos = 0;
-    if (lane == 0 && bal) basepos = atomicAdd(&ucount[c.b], __popc(bal));
-    basepos = __shfl_sync(0xffffffffu, basepos, 0);
-    if (unb) ulist[bh.uoff + basepos + __popc(bal & ((1u << lane) - 1u))] = (uint32_t)(k - bh.off);
+    int at = 0;
+    if (lane == 0 && bal) at = atomicAdd(&ucount[c.b], __popc(bal));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (unb) ulist[bh.uoff + at + __popc(bal & lanemask_lt())] = removal_key(e, (uint32_t)(k - bh.off));
   }
   if (__syncthreads_or(bad) && threadIdx.x == 0) atomicCAS(&flags[FLAG_ERR], 0, kInvalid);
 }
 
-// per big halo, one block: the nb most unbound members leave (radix select
-// over the compact list; equal energies: lower index first), then the stop
-// conditions of the inner loop
-__global__ void __launch_bounds__(IBLK) big_select_kernel(BigHalo *__restrict__ B, const int32_t *__restrict__ ucount,
-                                                          const uint32_t *__restrict__ ulist,
-                                                          uint32_t *__restrict__ eqbuf,
-                                                          const float *__restrict__ en,
+// per big halo, one block: the nb most unbound members leave, then the stop
+// conditions of the inner loop; the count starts again
+__global__ void __launch_bounds__(IBLK) big_select_kernel(BigHalo *__restrict__ B, int32_t *__restrict__ ucount,
+                                                          const unsigned long long *__restrict__ ulist,
                                                           uint8_t *__restrict__ keep,
                                                           const uint32_t *__restrict__ epos,
                                                           uint32_t *__restrict__ rflag,
@@ -1747,9 +1777,8 @@ __global__ void __launch_bounds__(IBLK) big_select_kernel(BigHalo *__restrict__ 
                                                           const int32_t *flags) {
   BigHalo &bh = B[blockIdx.x];
   if (!bh.active) return;
-  __shared__ unsigned hist[IBLK / 32][64];  // per-warp 6-bit digit histograms
-  __shared__ unsigned tot[64];
-  __shared__ int s_digit, s_above, s_neq;
+  __shared__ unsigned hist[2][256];
+  __shared__ int s_digit[3];
   if (flags[FLAG_ERR]) {  // a sweep failed: stop, the host reports it
     if (threadIdx.x == 0) { bh.active = 0; atomicSub(nactive, 1); }
     return;
@@ -1764,72 +1793,19 @@ __global__ void __launch_bounds__(IBLK) big_select_kernel(BigHalo *__restrict__ 
     return;
   }
   const int nb = min(nu, max(1, (int)ceil(0.02 * (double)bh.np_bound)));
-  const uint32_t *L = ulist + bh.uoff;
-  const float *E = en + bh.off;
-  const int warp = threadIdx.x >> 5;
-  unsigned prefix = 0, mask = 0;
-  int need = nb;
-  // 32-bit keys in digits of 6 bits from the top: 2 + 5 x 6
-  for (int shift = 30; shift >= 0; shift -= 6) {
-    const int bits = shift == 30 ? 2 : 6;
-    const unsigned dm = (1u << bits) - 1u;
-    for (int t = threadIdx.x; t < (IBLK / 32) * 64; t += IBLK) (&hist[0][0])[t] = 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < nu; i += IBLK) {
-      const unsigned key = __float_as_uint(E[L[i]] + 0.0f);
-      if ((key & mask) != prefix) continue;
-      atomicAdd(&hist[warp][(key >> shift) & dm], 1u);
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < 64; t += IBLK) {
-      unsigned s = 0;
-      for (int w = 0; w < IBLK / 32; ++w) s += hist[w][t];
-      tot[t] = s;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int digit = (int)dm, above = 0;
-      for (; digit >= 0; --digit) {
-        const int c = (int)tot[digit];
-        if (above + c >= need) break;
-        above += c;
-      }
-      s_digit = digit;
-      s_above = above;
-    }
-    __syncthreads();
-    need -= s_above;
-    prefix |= (unsigned)s_digit << shift;
-    mask |= dm << shift;
-    __syncthreads();
-  }
-  const unsigned thr = prefix;
-  if (threadIdx.x == 0) s_neq = 0;
-  __syncthreads();
-  uint32_t *EQ = eqbuf + bh.uoff;
-  for (int i = threadIdx.x; i < nu; i += IBLK) {
-    const uint32_t li = L[i];
-    const unsigned key = __float_as_uint(E[li] + 0.0f);
-    if (key > thr) {
-      keep[bh.off + li] = 0;
-      rflag[epos[bh.off + li]] = 1;
-    } else if (key == thr) {
-      EQ[atomicAdd(&s_neq, 1)] = li;
-    }
-  }
-  __syncthreads();
-  const int neq = s_neq;
-  for (int i = threadIdx.x; i < neq; i += IBLK) {
-    const uint32_t li = EQ[i];
-    int rank = 0;
-    for (int j = 0; j < neq; ++j) rank += EQ[j] < li;
-    if (rank < need) {
-      keep[bh.off + li] = 0;
-      rflag[epos[bh.off + li]] = 1;
-    }
+  const unsigned long long *L = ulist + bh.uoff;
+  const unsigned long long least = nth_largest([&](int t) { return L[t]; }, nu, nb, hist, s_digit);
+#pragma unroll 4
+  for (int t = threadIdx.x; t < nu; t += IBLK) {
+    const unsigned long long key = L[t];
+    if (key < least) continue;
+    const int64_t k = bh.off + (0xffffffffu - (unsigned)key);
+    keep[k] = 0;
+    rflag[epos[k]] = 1;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
+    ucount[blockIdx.x] = 0;
     bh.np_bound -= nb;
     bh.deleted += nb;
     if (bh.np_bound < nmin) {
@@ -1857,10 +1833,11 @@ __global__ void big_finish_kernel(const BigHalo *__restrict__ B, int nbig, PmHal
 
 // start of a pass: the pending big halos enter the inner loop
 __global__ void big_start_kernel(BigHalo *__restrict__ B, int nbig, const PmHalo *__restrict__ H, int phi_only,
-                                 int32_t *__restrict__ nactive) {
+                                 int32_t *__restrict__ nactive, int32_t *__restrict__ ucount) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nbig) return;
   BigHalo &bh = B[b];
+  ucount[b] = 0;
   const PmHalo &p = H[bh.h];
   bh.active = p.pending ? 1 : 0;
   bh.np_bound = p.np_bound;
@@ -1886,8 +1863,11 @@ __global__ void big_mass_kernel(const Members m, const BigChunk *__restrict__ ch
   const BigChunk c = ch[blockIdx.x];
   if (!H[B[c.b].h].pending) return;
   double s = 0.0;
-  for (int64_t k = c.start + threadIdx.x; k < c.end; k += blockDim.x)
-    if (keep[k]) s += (double)m.w[k];
+#pragma unroll 8
+  for (int64_t k = c.start + threadIdx.x; k < c.end; k += blockDim.x) {
+    const double w = (double)m.w[k];
+    s += keep[k] ? w : 0.0;
+  }
   __shared__ double red[32];
   s = bsum_d(s, red);
   if (threadIdx.x == 0) part[7 * (int64_t)blockIdx.x] = s;
@@ -1911,9 +1891,11 @@ __global__ void pm_mkeep_kernel(const Members m, PmHalo *__restrict__ H, const i
   PmHalo &p = H[h];
   if (!p.pending) return;
   double s = 0.0;
+#pragma unroll 8
   for (int64_t i = threadIdx.x; i < p.np; i += blockDim.x) {
     const int64_t k = p.off + i;
-    if (keep[k]) s += (double)m.w[k];
+    const double w = (double)m.w[k];
+    s += keep[k] ? w : 0.0;
   }
   __shared__ double red[32];
   s = bsum_d(s, red);
@@ -1976,14 +1958,13 @@ int bits_for(uint64_t v) {
 template <typename R>
 int32_t big_removal(Context &ctx, const Members &m, BigHalo *dB, int nbig, const BigChunk *dCh, int nchb,
                     PmHalo *dH, uint8_t *keep, const uint32_t *epos, uint32_t *rflag, const R *c1, const R *phi_in, const R *c2,
-                    float *phi, float *en, double *part, int32_t *ucount, uint32_t *ulist, uint32_t *eqbuf,
-                    int32_t *nactive, float b_val, int nmin, int phi_only) {
+                    float *phi, double *part, int32_t *ucount, unsigned long long *ulist, int32_t *nactive, float b_val, int nmin, int phi_only) {
   cudaStream_t s = ctx.stream;
   const unsigned gb = (unsigned)ceil_div(nbig, 128);
   PYFOF_CUDA(cudaMemsetAsync(nactive, 0, sizeof(int32_t), s));
-  big_start_kernel<<<gb, 128, 0, s>>>(dB, nbig, dH, phi_only, nactive);
+  big_start_kernel<<<gb, 128, 0, s>>>(dB, nbig, dH, phi_only, nactive, ucount);
   PYFOF_CHECK_LAUNCH();
-  big_phi_kernel<R><<<nchb, 256, 0, s>>>(dCh, nchb, dB, keep, c1, phi_in, c2, phi, ctx.d_flags);
+  big_phi_kernel<R><<<nchb * kBigSplit, 256, 0, s>>>(dCh, nchb, dB, keep, c1, phi_in, c2, phi, ctx.d_flags);
   PYFOF_CHECK_LAUNCH();
   if (phi_only) {
     big_phi_only_kernel<<<gb, 128, 0, s>>>(dB, nbig);
@@ -1997,12 +1978,10 @@ int32_t big_removal(Context &ctx, const Members &m, BigHalo *dB, int nbig, const
       for (int j = 0; j < 4; ++j) {
         big_com_kernel<<<nchb, 256, 0, s>>>(m, dCh, dB, keep, part);
         PYFOF_CHECK_LAUNCH();
-        big_center_kernel<<<gb, 128, 0, s>>>(dB, nbig, part, ucount);
+        big_energy_kernel<<<nchb * kBigSplit, 256, 0, s>>>(m, dCh, dB, keep, phi, part, b_val, ucount, ulist,
+                                                           ctx.d_flags);
         PYFOF_CHECK_LAUNCH();
-        big_energy_kernel<<<nchb, 256, 0, s>>>(m, dCh, dB, keep, phi, en, b_val, ucount, ulist, ctx.d_flags);
-        PYFOF_CHECK_LAUNCH();
-        big_select_kernel<<<nbig, IBLK, 0, s>>>(dB, ucount, ulist, eqbuf, en, keep, epos, rflag, nmin, nactive,
-                                                ctx.d_flags);
+        big_select_kernel<<<nbig, IBLK, 0, s>>>(dB, ucount, ulist, keep, epos, rflag, nmin, nactive, ctx.d_flags);
         PYFOF_CHECK_LAUNCH();
       }
       PYFOF_CUDA(cudaMemcpyAsync(ctx.h_flags + FLAG_COUNT_B, nactive, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
@@ -2456,16 +2435,15 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   BigChunk *dCh = nullptr;
   double *bpart = nullptr;
   int32_t *bucount = nullptr;
-  uint32_t *bulist = nullptr, *beq = nullptr;
+  unsigned long long *bulist = nullptr;
   int32_t *nactive = ctx.d_flags + FLAG_COUNT_B;
   if (nbig) {
     dB = W.carve<BigHalo>(nbig);
     dCh = W.carve<BigChunk>(nchb);
     bpart = W.carve<double>(7 * (size_t)nchb);
     bucount = W.carve<int32_t>(nbig);
-    bulist = W.carve<uint32_t>(ubig);
-    beq = W.carve<uint32_t>(ubig);
-    if (!dB || !dCh || !bpart || !bucount || !bulist || !beq) {
+    bulist = W.carve<unsigned long long>(ubig);
+    if (!dB || !dCh || !bpart || !bucount || !bulist) {
       set_error("workspace exhausted (large halos)");
       return kAlloc;
     }
@@ -2562,10 +2540,8 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
                                                                      ctx.d_flags);
       PYFOF_CHECK_LAUNCH();
     }
-    if (nbig) PYFOF_TRY(big_removal<R>(ctx, m, dB, nbig, dCh, nchb, dH, keep, epos, rflag, c1, phi_in, c2, phi, en,
-                                       bpart,
-                                       bucount, bulist, beq, nactive, (float)a.b_val, a.np_halo_min,
-                                       phi_only));
+    if (nbig) PYFOF_TRY(big_removal<R>(ctx, m, dB, nbig, dCh, nchb, dH, keep, epos, rflag, c1, phi_in, c2, phi, bpart,
+                                       bucount, bulist, nactive, (float)a.b_val, a.np_halo_min, phi_only));
     if (ctx.timing) ctx.gap_timer.begin(s);
     PYFOF_CUDA(cudaMemcpyAsync(H.data(), dH, sizeof(PmHalo) * nh, cudaMemcpyDeviceToHost, s));
     PYFOF_CUDA(cudaMemcpyAsync(ctx.h_flags, ctx.d_flags, sizeof(int32_t), cudaMemcpyDeviceToHost, s));

@@ -448,8 +448,14 @@ __device__ __forceinline__ int seg_of(const uint32_t *__restrict__ off, int n, u
 constexpr int kDepChunk = BLK;
 constexpr int kDepNodes = 4096;
 
+constexpr int kDepWords = 11;  // (odd: members' words fall in different banks)
 struct DepositTile {
-  unsigned lo[kDepNodes], hi[kDepNodes];
+  union {
+    struct {
+      unsigned lo[kDepNodes], hi[kDepNodes];
+    };
+    float member[BLK][kDepWords];  // weights, mass and first node of the block's members
+  };
   int box[6];
 };
 
@@ -485,6 +491,28 @@ __device__ __forceinline__ void deposit_chunk(bool act, const int (&f)[3], const
     for (int i = tid; i < (int)vol; i += BLK) S.lo[i] = S.hi[i] = 0;
     __syncthreads();
   }
+  if (!tile) {
+    // a row of three nodes by three lanes: the adds of a warp instruction that
+    // fall in one 32-byte sector go to L2 as one request
+    float *mine = S.member[tid];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) mine[j] = w9[j];
+    mine[9] = wk;
+    mine[10] = __int_as_float(act ? (f[0] - 1) + nx * ((f[1] - 1) + ny * (f[2] - 1)) : -1);
+    __syncwarp();
+    const float(*members)[kDepWords] = &S.member[tid - lane];
+#pragma unroll 3
+    for (int k = 0; k < 27; ++k) {
+      const int t = 32 * k + lane, i = t / 27, node = t - 27 * i, jz = node / 9, jy = node / 3 - 3 * jz;
+      const int jx = node - 9 * jz - 3 * jy;
+      const float *c = members[i];
+      const int at = __float_as_int(c[10]);
+      if (at < 0) continue;
+      const float v = __fmul_rn(__fmul_rn(__fmul_rn(c[9], c[jx]), c[3 + jy]), c[6 + jz]);
+      atomicAdd(&g[at + jx + nx * (jy + ny * jz)], fx_quantum(v, sc));
+    }
+    return;
+  }
   if (act) {
     // this thread's order of the three nodes of each axis
     const int r[3] = {lane % 3, (lane / 3) % 3, (lane / 9) % 3};
@@ -498,9 +526,7 @@ __device__ __forceinline__ void deposit_chunk(bool act, const int (&f)[3], const
         o[d][j] = k;
         w[d][j] = k == 0 ? w9[3 * d] : (k == 1 ? w9[3 * d + 1] : w9[3 * d + 2]);
       }
-    const int row = tile ? bx : nx, plane = tile ? bx * by : nx * ny;
-    const int64_t at = tile ? (f[0] - 1 - x0) + (int64_t)row * (f[1] - 1 - y0) + (int64_t)plane * (f[2] - 1 - z0)
-                            : (f[0] - 1) + (int64_t)row * (f[1] - 1) + (int64_t)plane * (f[2] - 1);
+    const int plane = bx * by, at = (f[0] - 1 - x0) + bx * (f[1] - 1 - y0) + plane * (f[2] - 1 - z0);
 #pragma unroll
     for (int jz = 0; jz < 3; ++jz)
 #pragma unroll
@@ -509,24 +535,18 @@ __device__ __forceinline__ void deposit_chunk(bool act, const int (&f)[3], const
         for (int jx = 0; jx < 3; ++jx) {
           const float v = __fmul_rn(__fmul_rn(__fmul_rn(wk, w[0][jx]), w[1][jy]), w[2][jz]);
           const unsigned long long u = fx_quantum(v, sc);
-          const int64_t i = at + o[0][jx] + row * o[1][jy] + (int64_t)plane * o[2][jz];
-          if (tile) {
-            const unsigned l = (unsigned)u, old = atomicAdd(&S.lo[i], l);
-            const unsigned hi = (unsigned)(u >> 32) + (old + l < l ? 1u : 0u);
-            if (hi) atomicAdd(&S.hi[i], hi);
-          } else {
-            atomicAdd(&g[i], u);
-          }
+          const int i = at + o[0][jx] + bx * o[1][jy] + plane * o[2][jz];
+          const unsigned l = (unsigned)u, old = atomicAdd(&S.lo[i], l);
+          const unsigned hi = (unsigned)(u >> 32) + (old + l < l ? 1u : 0u);
+          if (hi) atomicAdd(&S.hi[i], hi);
         }
   }
-  if (tile) {
-    __syncthreads();
-    for (int i = tid; i < (int)vol; i += BLK) {
-      const unsigned long long u = ((unsigned long long)S.hi[i] << 32) | S.lo[i];
-      if (!u) continue;
-      const int z = i / (bx * by), rem = i - z * (bx * by), y = rem / bx, x = rem - y * bx;
-      atomicAdd(&g[(x0 + x) + (int64_t)nx * ((y0 + y) + (int64_t)ny * (z0 + z))], u);
-    }
+  __syncthreads();
+  for (int i = tid; i < (int)vol; i += BLK) {
+    const unsigned long long u = ((unsigned long long)S.hi[i] << 32) | S.lo[i];
+    if (!u) continue;
+    const int z = i / (bx * by), rem = i - z * (bx * by), y = rem / bx, x = rem - y * bx;
+    atomicAdd(&g[(x0 + x) + (int64_t)nx * ((y0 + y) + (int64_t)ny * (z0 + z))], u);
   }
 }
 

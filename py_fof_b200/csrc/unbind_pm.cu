@@ -770,7 +770,10 @@ struct SrChunk {
 
 // Chunks whose nodes hold this many members or more are summed by the eight
 // warps of a block together.  The rule looks at the chunk alone, so the order
-// of its sum does not depend on what else is in the call.
+// of its sum does not depend on what else is in the call.  Where the line
+// lies: a full chip likes it higher (20,000 halos: 21.2 ms at 512, 20.6 at
+// 1024, 19.9 at 2048), a call of middle-sized halos lower, since its last
+// chunks run alone (1000 halos: 0.67, 0.79, 0.92 ms).
 // Update passes sum over the removed members only, a few per cent of them.
 constexpr uint32_t kSrHeavy = 1024, kSrHeavyUpdate = 16384;
 constexpr int kSrWarps = 8;
@@ -915,65 +918,81 @@ __device__ __forceinline__ void sr_pairs(const float4 *__restrict__ buf, const u
       if (__shfl_sync(0xffffffffu, own, j) == (uint32_t)lane) mask &= ~(1u << j);
     }
   }
+  const int none = __ffs(mask) - 1;  // a mark to stand in for a missing second one
   while (mask) {
-    const int j = __ffs(mask) - 1;
+    // two pairs at a time, for their dependent chains to overlap
+    int j[2];
+    j[0] = __ffs(mask) - 1;
     mask &= mask - 1;
-    const float4 s = buf[j];
-    const float fx = s.x - t.me.x, fy = s.y - t.me.y, fz = s.z - t.me.z;
-    R dx, dy, dz;
-    if (t.tl) {
-      dx = (R)s.x - (R)t.me.x; dy = (R)s.y - (R)t.me.y; dz = (R)s.z - (R)t.me.z;
-    } else {
-      dx = (R)fx; dy = (R)fy; dz = (R)fz;
+    const bool two = mask != 0;
+    j[1] = two ? __ffs(mask) - 1 : none;
+    mask &= mask - 1;
+    R v[2], w[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float4 s = buf[j[e]];
+      const float fx = s.x - t.me.x, fy = s.y - t.me.y, fz = s.z - t.me.z;
+      R dx, dy, dz;
+      if (t.tl) {
+        dx = (R)s.x - (R)t.me.x; dy = (R)s.y - (R)t.me.y; dz = (R)s.z - (R)t.me.z;
+      } else {
+        dx = (R)fx; dy = (R)fy; dz = (R)fz;
+      }
+      const R r2 = dx * dx + dy * dy + dz * dz;
+      w[e] = r2 < t.a2 && (e == 0 || two) ? (R)s.w : (R)0;
+      if constexpr (sizeof(R) == 4) {
+        const float rinv = rsqrtf(r2), d = r2 * rinv;
+        v[e] = depth_fast(d, rinv, t.eps) - depth_fast(d, rinv, t.ai);
+      } else {
+        const float r2f = fx * fx + fy * fy + fz * fz;
+        const SrSpline &S = *t.spline;
+        const int z = (r2f >= S.b2[0]) + (r2f >= S.b2[1]) + (r2f >= S.b2[2]);
+        const double2 *c = reinterpret_cast<const double2 *>(S.c[z]);
+        // (coincident members: a finite 1/r with coefficient 0, u = -m)
+        const double rinv = rsqrt_series64(r2, rsqrtf(fmaxf(r2f, 1e-30f)));
+        const double2 km = c[4], c67 = c[3], c45 = c[2], c23 = c[1], c01 = c[0];
+        const double u = fma(r2, rinv, -km.y);
+        double f = fma(c67.y, u, c67.x);
+        f = fma(f, u, c45.y);
+        f = fma(f, u, c45.x);
+        f = fma(f, u, c23.y);
+        f = fma(f, u, c23.x);
+        f = fma(f, u, c01.y);
+        f = fma(f, u, c01.x);
+        v[e] = fma(km.x, rinv, f);
+      }
     }
-    const R r2 = dx * dx + dy * dy + dz * dz;
-    if (!(r2 < t.a2)) continue;
-    if constexpr (sizeof(R) == 4) {  // compensated sum of the negated terms
-      const float rinv = rsqrtf(r2), d = r2 * rinv;
-      const float y = -(s.w * (depth_fast(d, rinv, t.eps) - depth_fast(d, rinv, t.ai))) - t.comp;
-      const float v = t.acc + y;
-      t.comp = (v - t.acc) - y;
-      t.acc = v;
-    } else {
-      const float r2f = fx * fx + fy * fy + fz * fz;
-      const SrSpline &S = *t.spline;
-      const int z = (r2f >= S.b2[0]) + (r2f >= S.b2[1]) + (r2f >= S.b2[2]);
-      const double2 *c = reinterpret_cast<const double2 *>(S.c[z]);
-      // (coincident members: a finite 1/r with coefficient 0, u = -m)
-      const double rinv = rsqrt_series64(r2, rsqrtf(fmaxf(r2f, 1e-30f)));
-      const double2 km = c[4], c67 = c[3], c45 = c[2], c23 = c[1], c01 = c[0];
-      const double u = fma(r2, rinv, -km.y);
-      double v = fma(c67.y, u, c67.x);
-      v = fma(v, u, c45.y);
-      v = fma(v, u, c45.x);
-      v = fma(v, u, c23.y);
-      v = fma(v, u, c23.x);
-      v = fma(v, u, c01.y);
-      v = fma(v, u, c01.x);
-      v = fma(km.x, rinv, v);
-      t.acc = fma((double)s.w, v, t.acc);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      if constexpr (sizeof(R) == 4) {  // compensated sum of the negated terms
+        if (w[e] == 0.0f) continue;
+        const float y = -(w[e] * v[e]) - t.comp;
+        const float sum = t.acc + y;
+        t.comp = (sum - t.acc) - y;
+        t.acc = sum;
+      } else {
+        t.acc = fma(w[e], v[e], t.acc);
+      }
     }
   }
 }
-
-// The sum of one chunk, or every nparts-th batch of its sources.  Nodes are
-// taken 32 at a time: a lane loads one node's member range, the ranges are
-// concatenated by a warp prefix sum and read in batches of 32 (a lane finds
+// The sum of one chunk by a warp.  Nodes are taken 32 at a time: a lane loads
+// one node's member range, the ranges are concatenated by a warp prefix sum and read in batches of 32 (a lane finds
 // its source's node by a binary search over the prefix); sources within the
 // largest cutoff of the targets' bounding box are staged, and every 32
 // staged sources go to sr_pairs.
 template <typename R, bool UPDATE>
-__device__ __forceinline__ void sr_chunk_sum(const SrChunk &C, const PmHalo &p, int part, int nparts,
-                                             const uint32_t *__restrict__ cstart, const float4 *__restrict__ src4,
-                                             const uint32_t *__restrict__ rpos, const uint32_t *__restrict__ rsrc,
-                                             float4 *buf, uint32_t *idx, SrTarget<R> &t) {
+__device__ __forceinline__ void sr_chunk_sum(const SrChunk &C, const PmHalo &p, const uint32_t *__restrict__ cstart,
+                                             const float4 *__restrict__ src4, const uint32_t *__restrict__ rpos,
+                                             const uint32_t *__restrict__ rsrc, float4 *buf, uint32_t *idx,
+                                             SrTarget<R> &t) {
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt = lanemask_lt();
   const float amax2 = C.amax * C.amax;
   const int w0 = C.nx[0], w1 = C.nx[1], nodes = w0 * w1 * C.nx[2];
   int fill = 0, n0 = -32;
-  uint32_t T = 0, g0 = 0, incl = 0, first = 0, turn = 0;  // the 32 nodes in hand; batches so far
+  uint32_t T = 0, g0 = 0, incl = 0, first = 0;  // the 32 nodes in hand
   for (;;) {
     bool more = true;
     while (fill < 32) {
@@ -1003,7 +1022,6 @@ __device__ __forceinline__ void sr_chunk_sum(const SrChunk &C, const PmHalo &p, 
       }
       const uint32_t g = g0 + (uint32_t)lane;
       g0 += 32;
-      if (nparts > 1 && (turn++ & (uint32_t)(nparts - 1)) != (uint32_t)part) continue;
       int owner = 0;
 #pragma unroll
       for (int step = 16; step > 0; step >>= 1) {
@@ -1044,11 +1062,99 @@ __device__ __forceinline__ void sr_chunk_sum(const SrChunk &C, const PmHalo &p, 
   }
 }
 
+// The sum of a heavy chunk by a block: the ranges of 256 nodes at a time are
+// loaded and concatenated by all threads, and every warp takes the source
+// batches of 32 in turn.
+struct SrNodes {
+  uint32_t incl[32 * kSrWarps], first[32 * kSrWarps], total[kSrWarps];
+};
+
+template <typename R, bool UPDATE>
+__device__ __forceinline__ void sr_block_sum(const SrChunk &C, const PmHalo &p, const uint32_t *__restrict__ cstart,
+                                             const float4 *__restrict__ src4, const uint32_t *__restrict__ rpos,
+                                             const uint32_t *__restrict__ rsrc, SrNodes &N, float4 *buf,
+                                             uint32_t *idx, SrTarget<R> &t) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int NT = 32 * kSrWarps;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float amax2 = C.amax * C.amax;
+  const int w0 = C.nx[0], w1 = C.nx[1], nodes = w0 * w1 * C.nx[2];
+  int fill = 0;
+  for (int n0 = 0; n0 < nodes; n0 += NT) {
+    const int j = n0 + (int)threadIdx.x;
+    uint32_t s0 = 0, cnt = 0;
+    if (j < nodes) {
+      uint2 r = sr_node_range(p, cstart, C.x0[0] + j % w0, C.x0[1] + (j / w0) % w1, C.x0[2] + j / (w0 * w1), C.level);
+      if (UPDATE && r.y > r.x) r = make_uint2(rpos[r.x], rpos[r.y]);
+      s0 = r.x;
+      cnt = r.y - r.x;
+    }
+    uint32_t incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) N.total[warp] = incl;
+    __syncthreads();
+    uint32_t T = 0;
+#pragma unroll
+    for (int w = 0; w < kSrWarps; ++w) {
+      if (w == warp) incl += T;
+      T += N.total[w];
+    }
+    N.incl[threadIdx.x] = incl;
+    N.first[threadIdx.x] = s0 - (incl - cnt);  // source of batch index g: first + g
+    __syncthreads();
+    for (uint32_t g0 = 32 * (uint32_t)warp; g0 < T; g0 += NT) {
+      const uint32_t g = g0 + (uint32_t)lane;
+      int owner = 0;  // nodes that end at or before g
+#pragma unroll
+      for (int step = NT / 2; step > 0; step >>= 1)
+        if (N.incl[owner + step - 1] <= g) owner += step;
+      uint32_t se = 0;
+      float4 sv = make_float4(0.f, 0.f, 0.f, 0.f);
+      bool cand = false;
+      if (g < T) {
+        const uint32_t e = N.first[owner] + g;
+        se = UPDATE ? rsrc[e] : e;
+        sv = src4[se];
+        const float bx = fmaxf(fmaxf(C.lo[0] - sv.x, sv.x - C.hi[0]), 0.f);
+        const float by = fmaxf(fmaxf(C.lo[1] - sv.y, sv.y - C.hi[1]), 0.f);
+        const float bz = fmaxf(fmaxf(C.lo[2] - sv.z, sv.z - C.hi[2]), 0.f);
+        cand = bx * bx + by * by + bz * bz <= amax2;
+      }
+      const unsigned m = __ballot_sync(FULL, cand);
+      if (cand) {
+        const int q = fill + __popc(m & lanemask_lt());
+        buf[q] = sv;
+        idx[q] = se;
+      }
+      fill += __popc(m);
+      __syncwarp();
+      if (fill < 32) continue;
+      sr_pairs<R, UPDATE>(buf, idx, 32, t);
+      __syncwarp();
+      fill -= 32;
+      if (lane < fill) {
+        buf[lane] = buf[32 + lane];
+        idx[lane] = idx[32 + lane];
+      }
+      __syncwarp();
+    }
+    __syncthreads();
+  }
+  if (fill) sr_pairs<R, UPDATE>(buf, idx, fill, t);
+  __syncwarp();
+}
+
 // Bound by instruction issue per interacting pair (FP64 and conversions) once
 // enough warps have work.  Persistent blocks: first the heavy chunks, a
-// block each (eight warps take the source batches in turn and their sums
-// are added in warp order), then the others, a warp each; both most sources
-// first, fetched from a counter.
+// block each (the node ranges are found once for its eight warps, which take
+// the source batches in turn; their sums are added in warp order), then the
+// others, a warp each; both most sources first, fetched from a counter.  Two
+// pairs in flight per lane and the shared node ranges: 1 M zoom region 3.72 ->
+// 3.37 ms, 20,000 halos 22.6 -> 20.6 ms.
 template <typename R, bool UPDATE>
 __global__ void __launch_bounds__(32 * kSrWarps, sizeof(R) == 4 ? 4 : 3) sr_gather_kernel(
     const PmHalo *__restrict__ H, const uint8_t *__restrict__ keep, const uint8_t *__restrict__ pr,
@@ -1060,6 +1166,7 @@ __global__ void __launch_bounds__(32 * kSrWarps, sizeof(R) == 4 ? 4 : 3) sr_gath
   __shared__ float4 buf[kSrWarps][64];
   __shared__ uint32_t idx[kSrWarps][64];
   __shared__ R part[kSrWarps][32];
+  __shared__ SrNodes nodes;
   __shared__ unsigned s_ch;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // the spline tables of the halo in hand (FP64), one copy per warp
@@ -1120,11 +1227,13 @@ __global__ void __launch_bounds__(32 * kSrWarps, sizeof(R) == 4 ? 4 : 3) sr_gath
     const PmHalo &p = H[C.h];
     int64_t k;
     const bool some = begin(C, p, k);
-    if (some)
-      sr_chunk_sum<R, UPDATE>(C, p, heavy ? warp : 0, heavy ? kSrWarps : 1, cstart, src4, rpos, rsrc, buf[warp],
-                              idx[warp], t);
-    if (heavy) {
-      if (some) part[warp][lane] = t.acc;
+    if (!heavy) {
+      if (some) sr_chunk_sum<R, UPDATE>(C, p, cstart, src4, rpos, rsrc, buf[warp], idx[warp], t);
+    } else {
+      if (some) {  // the same for every warp
+        sr_block_sum<R, UPDATE>(C, p, cstart, src4, rpos, rsrc, nodes, buf[warp], idx[warp], t);
+        part[warp][lane] = t.acc;
+      }
       __syncthreads();
       if (warp != 0 || !some) continue;
 #pragma unroll
@@ -2230,8 +2339,12 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
     sr_spline_kernel<<<(unsigned)ceil_div(3 * (int64_t)nh, 128), 128, 0, s>>>(dH, nh, a.softening, splines);
     PYFOF_CHECK_LAUNCH();
   }
-  // persistent blocks: those that fit on the GPU at once, if there is work for them
-  const unsigned gS = (unsigned)std::min<int64_t>(std::max<uint32_t>(nchunk, 1), 148 * (sizeof(R) == 4 ? 4 : 3));
+  // persistent blocks: those that fit on the GPU at once, if there is work for
+  // them; with fewer chunks than the warps of two blocks per SM, no more than
+  // two (one halo of 30,000 members: 0.32 ms against 0.39 with three, where
+  // most blocks take two chunks and some a third)
+  const int per_sm = nchunk <= 148 * 2 * kSrWarps ? 2 : (sizeof(R) == 4 ? 4 : 3);
+  const unsigned gS = (unsigned)std::min<int64_t>(std::max<uint32_t>(nchunk, 1), 148 * per_sm);
   // per-member refinement ratio, refined-region sources and targets
   const int na = (int)act.size();
   uint8_t *pr = W.carve<uint8_t>(M);

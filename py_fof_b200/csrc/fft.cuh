@@ -2,7 +2,8 @@
 // isolated particle-mesh convolution (replaces FFTW3f at
 // bound_fortran.f90:2166-2169, :2675-2677, :894-906).
 //
-// Grids: n points per axis, n = 2^a 3^b <= 256 (48, 64, 128, 216, 256).
+// Grids: n points per axis, n = 2^a 3^b 5^c <= 256 (48, 64, 128, 216, 256; in
+// FP64 also 96, 108, 144, 160, 180, 192, 240).
 // Every grid of a batch comes with its support box (ConvBox): the density is
 // nonzero only on the nodes [0, in) of the zero-padded half of the isolated
 // convolution, and the potential is wanted only on the nodes
@@ -41,6 +42,33 @@ constexpr int64_t spec_elems(int n, int nz) {
   return spec_row<R>(n) * n * nz;
 }
 
+// Lengths a convolution on the n-point grid may run at, ascending, n last.
+// The grid is a zero-padded one: between the nodes of a box a convolution only
+// meets the lags |d| <= reach, so any transform of 2 reach + 1 points or more
+// gives the same potential, with the kernel cut to the lags of its length.
+// A 256-point grid whose halo fills half of what it may costs a sixth at 128
+// points; calls: 256^3 box 27.7 -> 25.5 ms, 20,000 halos 108.6 -> 93.7 ms, 1 M
+// zoom region 19.4 -> 16.7 ms.  The list is coarse, since every length in a call is five more launches.  A
+// halo's length follows from its own box alone, so its bits do not depend on
+// what else is in the call.  FP32 stays at n: there the rounding of another
+// length (1e-7) could show in who is bound.
+inline const int *conv_lengths(int n, bool fp64) {
+  static const int own[5][2] = {{48, 0}, {64, 0}, {128, 0}, {216, 0}, {256, 0}};
+  static const int l64[] = {48, 64, 0}, l128[] = {96, 108, 128, 0}, l216[] = {180, 216, 0};
+  static const int l256[] = {128, 144, 160, 180, 192, 216, 240, 256, 0};
+  if (fp64) {
+    if (n == 64) return l64;
+    if (n == 128) return l128;
+    if (n == 216) return l216;
+    if (n == 256) return l256;
+  }
+  return own[n == 48 ? 0 : n == 64 ? 1 : n == 128 ? 2 : n == 216 ? 3 : 4];
+}
+
+// Nonzero input nodes per axis that a transform of n points takes (a refined
+// region's sources reach beyond half of its 96 or 180 points).
+__host__ __device__ constexpr int conv_in_max(int n) { return n == 96 || n == 180 ? 5 * n / 8 : n / 2 + 1; }
+
 // One grid of a batch (see above).  Offsets in elements; out0 + out <= in.
 struct ConvBox {
   int64_t in_off;    // density (64-bit fixed-point nodes)
@@ -50,6 +78,20 @@ struct ConvBox {
   int32_t out0[3], out[3];
   int32_t pad;
 };
+
+// Transform length for a box on the n-point grid.
+inline int conv_length(int n, bool fp64, const ConvBox &b) {
+  int reach = 0, in = 0;
+  for (int d = 0; d < 3; ++d) {
+    const int back = b.in[d] - 1 - b.out0[d], ahead = b.out0[d] + b.out[d] - 1;
+    reach = back > reach ? back : reach;
+    reach = ahead > reach ? ahead : reach;
+    in = b.in[d] > in ? b.in[d] : in;
+  }
+  const int *l = conv_lengths(n, fp64);
+  while (*l < n && (*l < 2 * reach + 1 || conv_in_max(*l) < in)) ++l;
+  return *l;
+}
 
 // Bytes the five passes of one grid's convolution read and write (x, y,
 // fused z, y, x), each line once.
@@ -63,9 +105,11 @@ inline double conv_bytes(int n, const ConvBox &b) {
 
 // Largest extents over the boxes of a batch (launch shapes).
 struct ConvExtent {
-  int in_y = 0, in_z = 0, out_y = 0, out_z = 0;
+  int in_x = 0, in_y = 0, in_z = 0, out_x = 0, out_y = 0, out_z = 0;
   int64_t in_lines = 0, out_lines = 0;
   void add(const ConvBox &b) {
+    in_x = b.in[0] > in_x ? b.in[0] : in_x;
+    out_x = b.out[0] > out_x ? b.out[0] : out_x;
     in_y = b.in[1] > in_y ? b.in[1] : in_y;
     in_z = b.in[2] > in_z ? b.in[2] : in_z;
     out_y = b.out[1] > out_y ? b.out[1] : out_y;
@@ -84,7 +128,8 @@ int32_t fill_twiddles(cplx_t<R> *tw, int n, cudaStream_t s);
 //   acc, inv_scale  the densities as 64-bit fixed-point nodes (value of grid
 //         j = acc * inv_scale[j])
 //   phi   the potentials divided by n^3 in R precision (as the reference's
-//         rho/real(n**3)); may alias acc when every out_off is at its grid's
+//         rho/real(n**3)), or as they are where the table holds the factor
+//         (scaled); may alias acc when every out_off is at its grid's
 //         in_off or below it in bytes
 //   boxes, ext  the batch's boxes (device) and their largest extents
 //   spec  half spectra (scratch)
@@ -96,7 +141,7 @@ int32_t fill_twiddles(cplx_t<R> *tw, int n, cudaStream_t s);
 template <typename R>
 int32_t pm_convolve_batch(const unsigned long long *acc, const double *inv_scale, R *phi, cplx_t<R> *spec,
                           const R *green, const cplx_t<R> *tw, int n, const ConvBox *boxes, const ConvExtent &ext,
-                          int batch, cudaStream_t s, int waves = 4);
+                          int batch, bool scaled, cudaStream_t s, int waves = 4);
 
 // FFTW-style c2r of a real half-spectrum table (the Green's function) into a
 // full n^3 real grid (unnormalised); used once per table to extract the

@@ -124,14 +124,45 @@ __global__ void self_extract_kernel(const R *__restrict__ grid, int n, R *__rest
   self[t] = grid[((int64_t)z * n + y) * n + x] / n3;
 }
 
+// The kernel on the m^3 lags of a shorter transform, as a half-spectrum shaped
+// table (h[(z m + y)(m/2+1) + x]), from the n^3 grid of c2r_full.  Lag m/2
+// stands for both signs and is never met.
+__global__ void lag_crop_kernel(const double *__restrict__ grid, int n, double *__restrict__ h, int m) {
+  const int mh = m / 2 + 1;
+  const int64_t total = (int64_t)mh * m * m;
+  const double n3 = (double)n * n * n;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const int x = (int)(t % mh), y = (int)((t / mh) % m), z = (int)(t / ((int64_t)mh * m));
+    const int ly = y <= m / 2 ? y : n - m + y, lz = z <= m / 2 ? z : n - m + z;
+    h[t] = grid[((int64_t)lz * n + ly) * n + x] / n3;
+  }
+}
+
+// The half of an m^3 grid that a table holds, with the 1/m^3 of a transform
+// and its inverse.
+__global__ void half_table_kernel(const double *__restrict__ grid, int m, double *__restrict__ g) {
+  const int mh = m / 2 + 1;
+  const int64_t total = (int64_t)mh * m * m;
+  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+       t += (int64_t)gridDim.x * blockDim.x)
+    g[t] = grid[(t / mh) * m + t % mh] / ((double)m * m * m);
+}
+
 }  // namespace
 
 struct GreenTable {
-  int n = 0;
+  int n = 0;             // transform length
   void *g = nullptr;     // half-spectrum table (R)
   void *self = nullptr;  // 125 self-kernel values (R), device
   void *tw = nullptr;    // the transforms' twiddles (complex R), device
-  bool fp64 = false;
+  bool fp64 = false, scaled = false;  // scaled: holds the transforms' 1/n^3
+  std::vector<std::shared_ptr<GreenTable>> shorter;  // the same kernel at other conv_lengths (no self)
+  const GreenTable *at(int m) const {
+    for (const auto &t : shorter)
+      if (t->n == m) return t.get();
+    return this;
+  }
   ~GreenTable() {
     if (g) cudaFree(g);
     if (self) cudaFree(self);
@@ -140,6 +171,49 @@ struct GreenTable {
 };
 
 namespace {
+
+inline unsigned table_grid(int64_t n) { return (unsigned)std::min<int64_t>(ceil_div(n, 256), 148 * 16); }
+
+// The tables of the n-point kernel (its real-space values in `grid`, n^3) at
+// its shorter transform lengths.  The kernel is even along every axis, so its
+// forward transform is the inverse one that c2r_full runs.  Once per process
+// and grid size: about a millisecond for 256 points, all lengths together.
+int32_t shorter_tables(GreenTable &t, const double *grid, double2 *spec, ConvBox *dbox, cudaStream_t s) {
+  double *h = nullptr, *out = nullptr;
+  int32_t r = kOk;
+  auto one = [&](int m) -> int32_t {
+    const int64_t cnt = (int64_t)(m / 2 + 1) * m * m;
+    auto q = std::make_shared<GreenTable>();
+    q->n = m;
+    q->fp64 = q->scaled = true;
+    PYFOF_CUDA(cudaMalloc(&q->g, sizeof(double) * cnt));
+    PYFOF_CUDA(cudaMalloc(&q->tw, sizeof(double2) * m));
+    PYFOF_TRY(fill_twiddles<double>((double2 *)q->tw, m, s));
+    ConvBox box{};
+    for (int d = 0; d < 3; ++d) box.in[d] = box.out[d] = m;
+    PYFOF_CUDA(cudaMemcpyAsync(dbox, &box, sizeof(ConvBox), cudaMemcpyHostToDevice, s));
+    lag_crop_kernel<<<table_grid(cnt), 256, 0, s>>>(grid, t.n, h, m);
+    PYFOF_CHECK_LAUNCH();
+    PYFOF_TRY(c2r_full<double>(h, spec, out, (const double2 *)q->tw, dbox, m, s));
+    half_table_kernel<<<table_grid(cnt), 256, 0, s>>>(out, m, (double *)q->g);
+    PYFOF_CHECK_LAUNCH();
+    t.shorter.push_back(std::move(q));
+    return kOk;
+  };
+  const int64_t n = t.n;
+  const int *l = conv_lengths(t.n, true);
+  if (*l == t.n) return kOk;
+  if (cudaMallocAsync(&h, sizeof(double) * n * n * n, s) != cudaSuccess ||
+      cudaMallocAsync(&out, sizeof(double) * n * n * n, s) != cudaSuccess) {
+    cudaGetLastError();
+    set_error("device allocation failed (kernel tables)");
+    r = kAlloc;
+  }
+  for (; r == kOk && *l < t.n; ++l) r = one(*l);
+  if (h) cudaFreeAsync(h, s);
+  if (out) cudaFreeAsync(out, s);
+  return r;
+}
 
 // Green table of grid n for (soft, range, truncated), cached per context.
 template <typename R>
@@ -177,6 +251,7 @@ int32_t get_green(Context &ctx, int n, double soft, double range, int truncated,
   if (r == kOk) {
     self_extract_kernel<R><<<1, 128, 0, s>>>(grid, n, (R *)t->self);
     PYFOF_CHECK_LAUNCH();
+    if constexpr (sizeof(R) == 8) r = shorter_tables(*t, grid, spec, dbox, s);
   }
   cudaFreeAsync(grid, s);
   cudaFreeAsync(spec, s);
@@ -2430,11 +2505,17 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
     return ctx.h_flags[FLAG_ERR];
   }
 
-  // grid batches per class, bounded by a spectrum budget; one scratch area,
-  // sized for the largest batch, serves every batch of every pass
-  const size_t budget = ctx.pm_budget;
+  // One batch deposits and gathers grids of every class together, and runs
+  // the convolutions of each class and transform length (a run) one after the
+  // other.  The grids have an area each and the runs share one for their
+  // spectra, both bounded by half the budget and reused by every pass.
+  const size_t budget = std::max<size_t>(ctx.pm_budget / 2, 1);
   auto round256 = [](size_t b) { return (b + 255) & ~(size_t)255; };
   auto waves = [&](int n) { return a.tiles.conv_waves[kGridIndex(n)]; };
+  auto run_cap = [&](int n) {
+    const int cap = a.tiles.pm_batch[kGridIndex(n)];
+    return (size_t)(cap > 0 ? std::min(cap, 65535) : 65535);
+  };
   // the box of a halo's own grid, and of a region's inner grid: its sources
   // lie within 3.5 + 3/r grid cells of the region, its targets inside it
   // (tl_deposit_kernel, tl_gather_kernel), one node of slack each side
@@ -2459,38 +2540,53 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
     return round256(sizeof(unsigned long long) * b.in[0] * (size_t)b.in[1] * b.in[2]);
   };
   auto spec_bytes = [&](int n, const ConvBox &b) { return sizeof(cplx_t<R>) * (size_t)spec_elems<R>(n, b.in[2]); };
-  size_t scratch_bytes = 256;
-  int64_t nbat = 1;
-  {
-    std::vector<size_t> sizes;
-    auto room = [&](int n) {
-      if (sizes.empty()) return;
-      std::sort(sizes.begin(), sizes.end(), std::greater<size_t>());
-      const int cap = a.tiles.pm_batch[kGridIndex(n)];
-      size_t need = 0;
-      for (size_t i = 0; i < sizes.size() && (cap <= 0 || i < (size_t)cap); ++i) need += sizes[i];
-      scratch_bytes = std::max(scratch_bytes, std::min(need, std::max(budget, sizes[0])));
-      nbat = std::max<int64_t>(nbat, (int64_t)sizes.size());
-    };
-    for (int n : {48, 64, 128, 256}) {
-      sizes.clear();
-      for (int h = 0; h < nh; ++h)
-        if (H[h].n == n) {
-          const ConvBox b = halo_box(h);
-          sizes.push_back(acc_bytes(b) + spec_bytes(n, b));
-        }
-      room(n);
+  // grids in batch order: class, length, boxes of similar size together (a
+  // launch is shaped by the largest)
+  struct Grid {
+    ConvBox box;
+    int32_t id, n, len;
+  };
+  auto order = [](std::vector<Grid> &g) {
+    std::stable_sort(g.begin(), g.end(), [](const Grid &x, const Grid &y) {
+      if (x.n != y.n) return x.n < y.n;
+      if (x.len != y.len) return x.len < y.len;
+      return (int64_t)x.box.in[1] * x.box.in[2] > (int64_t)y.box.in[1] * y.box.in[2];
+    });
+  };
+  std::vector<Grid> hgrid, rgrid;
+  for (int h = 0; h < nh; ++h) {
+    const ConvBox b = halo_box(h);
+    hgrid.push_back(Grid{b, h, H[h].n, conv_length(H[h].n, sizeof(R) == 8, b)});
+  }
+  for (int ia = 0; ia < na; ++ia) {
+    const ConvBox b = region_box(ia);
+    rgrid.push_back(Grid{b, ia, act[ia].n_in, conv_length(act[ia].n_in, sizeof(R) == 8, b)});
+  }
+  order(hgrid);
+  order(rgrid);
+  size_t acc_cap = 256, spec_cap = 256;
+  for (const auto *gs : {&hgrid, &rgrid}) {
+    size_t need = 0, largest = 0;
+    for (size_t i = 0; i < gs->size(); ++i) {
+      const size_t ab = acc_bytes((*gs)[i].box);
+      need += ab;
+      largest = std::max(largest, ab);
     }
-    for (int n : {128, 216}) {
-      sizes.clear();
-      for (int ia = 0; ia < na; ++ia)
-        if (act[ia].n_in == n) {
-          const ConvBox b = region_box(ia);
-          sizes.push_back(acc_bytes(b) + spec_bytes(n, b));
-        }
-      room(n);
+    acc_cap = std::max(acc_cap, std::min(need, std::max(budget, largest)));
+    for (size_t i = 0; i < gs->size();) {
+      const Grid &g = (*gs)[i];
+      std::vector<size_t> sizes;
+      for (; i < gs->size() && (*gs)[i].n == g.n && (*gs)[i].len == g.len; ++i)
+        sizes.push_back(spec_bytes(g.len, (*gs)[i].box));
+      std::sort(sizes.begin(), sizes.end(), std::greater<size_t>());
+      size_t sum = 0;
+      for (size_t j = 0; j < sizes.size() && j < run_cap(g.n); ++j) sum += sizes[j];
+      spec_cap = std::max(spec_cap, std::min(sum, std::max(budget, sizes[0])));
     }
   }
+  acc_cap = round256(acc_cap);
+  const size_t scratch_bytes = acc_cap + spec_cap;
+  const int64_t nbat = std::max<int64_t>(nh, na);
   unsigned char *scratch = W.carve<unsigned char>(scratch_bytes);
   int32_t *dpend = W.carve<int32_t>(nh);
   // a batch's tables, uploaded together: boxes, ids, member prefixes
@@ -2500,11 +2596,15 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
     set_error("workspace exhausted (PM grids)");
     return kAlloc;
   }
+  struct Run {  // grids [first, first + count) of a batch
+    int n, len, first, count;
+    ConvExtent ext;
+  };
   struct Batch {
     std::vector<int32_t> ids;
     std::vector<ConvBox> boxes;
-    ConvExtent ext;
-    size_t acc = 0, spec = 0;  // bytes
+    std::vector<Run> runs;
+    size_t acc = 0;  // bytes
     const ConvBox *dbox;
     const int32_t *did;
     const uint32_t *dpre0, *dpre1;
@@ -2512,28 +2612,35 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   };
   // takes grids from items[at..] while they fit, and uploads the tables
   std::vector<unsigned char> meta;
-  auto next_batch = [&](const std::vector<int32_t> &items, size_t &at, int n, bool region, Batch &B) -> int32_t {
+  auto next_batch = [&](const std::vector<const Grid *> &items, size_t &at, bool region, Batch &B) -> int32_t {
     B = Batch();
-    const int cap = a.tiles.pm_batch[kGridIndex(n)];
     std::vector<uint32_t> p0(1, 0), p1(1, 0);
-    for (; at < items.size() && (cap <= 0 || (int)B.ids.size() < cap) && B.ids.size() < 65535; ++at) {
-      ConvBox b = region ? region_box(items[at]) : halo_box(items[at]);
-      const size_t ab = acc_bytes(b), sb = spec_bytes(n, b);
-      if (!B.ids.empty() && B.acc + B.spec + ab + sb > scratch_bytes) break;
+    size_t spec = 0;
+    for (; at < items.size(); ++at) {
+      const Grid &g = *items[at];
+      ConvBox b = g.box;
+      const size_t ab = acc_bytes(b), sb = spec_bytes(g.len, b);
+      if (!B.ids.empty() && B.acc + ab > acc_cap) break;
+      if (B.runs.empty() || B.runs.back().n != g.n || B.runs.back().len != g.len || spec + sb > spec_cap ||
+          (size_t)B.runs.back().count >= run_cap(g.n)) {
+        B.runs.push_back(Run{g.n, g.len, (int)B.ids.size(), 0, ConvExtent()});
+        spec = 0;
+      }
       b.in_off = (int64_t)(B.acc / sizeof(unsigned long long));
       b.out_off = (int64_t)(B.acc / sizeof(R));
-      b.spec_off = (int64_t)(B.spec / sizeof(cplx_t<R>));
+      b.spec_off = (int64_t)(spec / sizeof(cplx_t<R>));
       B.acc += ab;
-      B.spec += sb;
-      B.ext.add(b);
-      ctx.last_pm_fft_bytes += conv_bytes<R>(n, b);
-      B.ids.push_back(items[at]);
+      spec += sb;
+      B.runs.back().ext.add(b);
+      ++B.runs.back().count;
+      ctx.last_pm_fft_bytes += conv_bytes<R>(g.len, b);
+      B.ids.push_back(g.id);
       B.boxes.push_back(b);
       if (region) {
-        p0.push_back(p0.back() + (hsrc[items[at] + 1] - hsrc[items[at]]));
-        p1.push_back(p1.back() + (htgt[items[at] + 1] - htgt[items[at]]));
+        p0.push_back(p0.back() + (hsrc[g.id + 1] - hsrc[g.id]));
+        p1.push_back(p1.back() + (htgt[g.id + 1] - htgt[g.id]));
       } else {
-        p0.push_back(p0.back() + (uint32_t)ceil_div(H[items[at]].np, kDepChunk));
+        p0.push_back(p0.back() + (uint32_t)ceil_div(H[g.id].np, kDepChunk));
       }
     }
     const size_t nb = B.ids.size(), ob = sizeof(ConvBox) * nb, oi = ob + 4 * nb, op = oi + 4 * (nb + 1);
@@ -2555,6 +2662,17 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   };
   unsigned long long *const acc = reinterpret_cast<unsigned long long *>(scratch);
   R *const rho = reinterpret_cast<R *>(scratch);  // the convolved grids overwrite acc
+  auto convolve = [&](const Batch &B, auto &&table) -> int32_t {
+    if (ctx.timing) ctx.conv_timer.begin(s);
+    for (const Run &r : B.runs) {
+      const GreenTable *g = table(r.n)->at(r.len);
+      PYFOF_TRY(pm_convolve_batch<R>(acc, dinv + r.first, rho, reinterpret_cast<cplx_t<R> *>(scratch + acc_cap),
+                                     (const R *)g->g, (const cplx_t<R> *)g->tw, r.len, B.dbox + r.first, r.ext,
+                                     r.count, g->scaled, s, waves(r.n)));
+    }
+    if (ctx.timing) ctx.conv_timer.end(s);
+    return kOk;
+  };
   // halos above kBigNp members: chunked removal loop
   std::vector<BigHalo> hbig;
   std::vector<BigChunk> hch;
@@ -2615,51 +2733,34 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
       PYFOF_CHECK_LAUNCH();
     }
     Batch B;
-    for (int n : {48, 64, 128, 256}) {
-      std::vector<int32_t> grp;
-      for (int h : pend) if (H[h].n == n) grp.push_back(h);
-      // boxes of similar size together: a launch is shaped by the largest
-      std::stable_sort(grp.begin(), grp.end(), [&](int x, int y) {
-        return (int64_t)H[x].sup[1] * H[x].sup[2] > (int64_t)H[y].sup[1] * H[y].sup[2];
-      });
-      for (size_t at = 0; at < grp.size();) {
-        PYFOF_TRY(next_batch(grp, at, n, false, B));
-        const int nb = (int)B.ids.size();
-        pm_deposit_kernel<<<B.n0, BLK, 0, s>>>(src4, cmem, dH, B.dbox, B.did, B.dpre0, nb, keep, acc, dinv);
-        PYFOF_CHECK_LAUNCH();
-        if (ctx.timing) ctx.conv_timer.begin(s);
-        PYFOF_TRY(pm_convolve_batch<R>(acc, dinv, rho, reinterpret_cast<cplx_t<R> *>(scratch + B.acc),
-                                       (const R *)green_of[n]->g, (const cplx_t<R> *)green_of[n]->tw, n, B.dbox,
-                                       B.ext, nb, s, waves(n)));
-        if (ctx.timing) ctx.conv_timer.end(s);
-        pm_gather_kernel<R><<<B.n0, BLK, 0, s>>>(src4, cmem, dH, B.dbox, B.did, B.dpre0, nb, keep, selfe, rho,
-                                                 a.a_val, c1);
-        PYFOF_CHECK_LAUNCH();
-      }
+    std::vector<const Grid *> todo;
+    for (const Grid &g : hgrid)
+      if (H[g.id].pending) todo.push_back(&g);
+    for (size_t at = 0; at < todo.size();) {
+      PYFOF_TRY(next_batch(todo, at, false, B));
+      const int nb = (int)B.ids.size();
+      pm_deposit_kernel<<<B.n0, BLK, 0, s>>>(src4, cmem, dH, B.dbox, B.did, B.dpre0, nb, keep, acc, dinv);
+      PYFOF_CHECK_LAUNCH();
+      PYFOF_TRY(convolve(B, [&](int n) { return green_of[n].get(); }));
+      pm_gather_kernel<R><<<B.n0, BLK, 0, s>>>(src4, cmem, dH, B.dbox, B.did, B.dpre0, nb, keep, selfe, rho,
+                                               a.a_val, c1);
+      PYFOF_CHECK_LAUNCH();
     }
-    // refined regions of pending halos, batched per inner grid size
-    for (int r : {2, 4}) {
-      std::vector<int32_t> regs;
-      for (int ia = 0; ia < na; ++ia)
-        if (act[ia].r == r && H[act[ia].h].pending) regs.push_back(ia);
-      const int nin = r == 2 ? 128 : 216;
-      const GreenTable *gin = (r == 2 ? g_r2 : g_r4).get();
-      for (size_t at = 0; at < regs.size();) {
-        PYFOF_TRY(next_batch(regs, at, nin, true, B));
-        const int nb = (int)B.ids.size();
-        tl_deposit_kernel<<<B.n0, BLK, 0, s>>>(src4, cmem, dH, dA, B.dbox, B.did, B.dpre0, nb, src_start, src, keep,
-                                               acc, dinv);
+    // refined regions of pending halos
+    todo.clear();
+    for (const Grid &g : rgrid)
+      if (H[act[g.id].h].pending) todo.push_back(&g);
+    for (size_t at = 0; at < todo.size();) {
+      PYFOF_TRY(next_batch(todo, at, true, B));
+      const int nb = (int)B.ids.size();
+      tl_deposit_kernel<<<B.n0, BLK, 0, s>>>(src4, cmem, dH, dA, B.dbox, B.did, B.dpre0, nb, src_start, src, keep,
+                                             acc, dinv);
+      PYFOF_CHECK_LAUNCH();
+      PYFOF_TRY(convolve(B, [&](int n) { return (n == 128 ? g_r2 : g_r4).get(); }));
+      if (B.n1 > 0) {
+        tl_gather_kernel<R><<<B.n1, BLK, 0, s>>>(src4, cmem, dH, dA, B.dbox, B.did, B.dpre1, nb, tgt_start, tgt,
+                                                 keep, tl_self_in, rho, a.a_val, phi_in);
         PYFOF_CHECK_LAUNCH();
-        if (ctx.timing) ctx.conv_timer.begin(s);
-        PYFOF_TRY(pm_convolve_batch<R>(acc, dinv, rho, reinterpret_cast<cplx_t<R> *>(scratch + B.acc),
-                                       (const R *)gin->g, (const cplx_t<R> *)gin->tw, nin, B.dbox, B.ext, nb, s,
-                                       waves(nin)));
-        if (ctx.timing) ctx.conv_timer.end(s);
-        if (B.n1 > 0) {
-          tl_gather_kernel<R><<<B.n1, BLK, 0, s>>>(src4, cmem, dH, dA, B.dbox, B.did, B.dpre1, nb, tgt_start, tgt,
-                                                   keep, tl_self_in, rho, a.a_val, phi_in);
-          PYFOF_CHECK_LAUNCH();
-        }
       }
     }
     PYFOF_CUDA(cudaMemsetAsync(sr_next, 0, 2 * sizeof(unsigned), s));

@@ -748,15 +748,15 @@ __device__ __forceinline__ float depth_fast(float r, float rinv, const DepthCons
 // is their difference: k / r + c0 + c1 u + .. + c7 u^7, u = r - m, with the
 // coefficients and the middle m of the zone the pair is in.  Where both are on
 // the same piece the 1/r cancels.  A table per halo and refinement ratio
-// (SrSpline) holds the four zones; the pieces join smoothly, so an FP32
-// distance is enough to pick one.  About the middle the terms do not cancel:
+// (SrSpline) holds the four zones; the pieces join smoothly, so the upper half
+// of the squared distance is enough to pick one.  About the middle the terms do not cancel:
 // the largest error against quadruple precision over d < a, for a = 1.2 to 17
 // eps and eps = 0.05, is 1.1e-14 on values up to 56 (splines evaluated in
 // e = 2 r / h, as the oracle's formula is written: 1.0e-13).  Two splines per
 // pair took 45 FP64 operations, this takes 22.
 struct alignas(16) SrSpline {
   double c[4][10];  // per zone: c0..c7, k, m
-  float b2[4];      // squared distances at which zones 1, 2, 3 begin
+  int b2[4];        // squared distances at which zones 1, 2, 3 begin (upper halves)
 };
 
 // a b + c with a and c as unevaluated sums of two doubles.
@@ -814,16 +814,18 @@ __global__ void sr_spline_kernel(const PmHalo *__restrict__ H, int nh, double ap
     spline_piece(eps, mid, ce);
     for (int j = 0; j < 9; ++j) S.c[z][j] = ca[j] - ce[j];
     S.c[z][9] = mid;
-    S.b2[z] = z < 3 ? (float)(b[z] * b[z]) : 0.0f;
+    S.b2[z] = z < 3 ? __double2hiint(b[z] * b[z]) : 0;
   }
 }
 
-// 1/r: an FP32 reciprocal square root seed y (relative error about 2^-22) and
-// one step of the binomial series 1/sqrt(r2) = y (1 - g)^(-1/2) = y (1 + g/2 +
-// 3 g^2/8 + ..), g = 1 - r2 y^2 (|g| about 2^-21, so the dropped cubic term is
-// 2^-64).
-__device__ __forceinline__ double rsqrt_series64(double r2, float seed) {
-  const double y = (double)seed;
+// 1/r: the hardware's reciprocal square root of a double's upper half as the
+// seed y and one step of the binomial series 1/sqrt(r2) = y (1 - g)^(-1/2) =
+// y (1 + g/2 + 3 g^2/8 + ..), g = 1 - r2 y^2.  The argument is kept above
+// 2^-199, for a finite 1/r of coincident members.
+__device__ __forceinline__ double rsqrt_series64(double r2) {
+  const double a = __hiloint2double(max(__double2hiint(r2), 0x33800000), __double2loint(r2));
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
   const double g = fma(-(r2 * y), y, 1.0);
   return fma(y * g, fma(0.375, g, 0.5), y);
 }
@@ -968,6 +970,66 @@ struct SrTarget {
   R acc, comp;
 };
 
+// A warp's 32 sources in FP64, converted once for all its targets.
+struct SrWide {
+  double2 xy[32], zw[32];
+};
+
+// The terms of a target's marked sources.  The conversion units were the
+// busiest part of a pair (59 %: three coordinates, the weight and both ways
+// around the seed of 1/r): with sources converted once per warp and a seed from
+// the FP64 word they do one operation per pair of a two-level halo
+// (DIFF64: differences in FP64) and four where the differences are FP32's.
+template <bool DIFF64>
+__device__ __forceinline__ void sr_marked64(const float4 *__restrict__ buf, const SrWide &wide, unsigned mask,
+                                            SrTarget<double> &t) {
+  const SrSpline &S = *t.spline;
+  const double mx = (double)t.me.x, my = (double)t.me.y, mz = (double)t.me.z;
+  const int none = __ffs(mask) - 1;  // a mark to stand in for a missing second one
+  while (mask) {
+    // two pairs at a time, for their dependent chains to overlap
+    int j[2];
+    j[0] = __ffs(mask) - 1;
+    mask &= mask - 1;
+    const bool two = mask != 0;
+    j[1] = two ? __ffs(mask) - 1 : none;
+    mask &= mask - 1;
+    double v[2], w[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      double dx, dy, dz;
+      if (DIFF64) {
+        const double2 xy = wide.xy[j[e]], zw = wide.zw[j[e]];
+        dx = xy.x - mx; dy = xy.y - my; dz = zw.x - mz;
+        w[e] = zw.y;
+      } else {
+        const float4 s = buf[j[e]];
+        dx = (double)(s.x - t.me.x); dy = (double)(s.y - t.me.y); dz = (double)(s.z - t.me.z);
+        w[e] = wide.zw[j[e]].y;
+      }
+      const double r2 = dx * dx + dy * dy + dz * dz;
+      if (!(r2 < t.a2 && (e == 0 || two))) w[e] = 0.0;
+      const int r2h = __double2hiint(r2);
+      const int z = (r2h >= S.b2[0]) + (r2h >= S.b2[1]) + (r2h >= S.b2[2]);
+      const double2 *c = reinterpret_cast<const double2 *>(S.c[z]);
+      // (coincident members: a finite 1/r with coefficient 0, u = -m)
+      const double rinv = rsqrt_series64(r2);
+      const double2 km = c[4], c67 = c[3], c45 = c[2], c23 = c[1], c01 = c[0];
+      const double u = fma(r2, rinv, -km.y);
+      double f = fma(c67.y, u, c67.x);
+      f = fma(f, u, c45.y);
+      f = fma(f, u, c45.x);
+      f = fma(f, u, c23.y);
+      f = fma(f, u, c23.x);
+      f = fma(f, u, c01.y);
+      f = fma(f, u, c01.x);
+      v[e] = fma(km.x, rinv, f);
+    }
+    t.acc = fma(w[0], v[0], t.acc);
+    t.acc = fma(w[1], v[1], t.acc);
+  }
+}
+
 // Up to 32 staged sources against the warp's 32 targets.  Every lane first
 // marks the sources inside its own cutoff with an FP32 test (the box filter
 // in front of it keeps a chunk's union, of which a target needs a third or
@@ -975,7 +1037,7 @@ struct SrTarget {
 // interacting pairs only, in ascending source order per target.
 template <typename R, bool UPDATE>
 __device__ __forceinline__ void sr_pairs(const float4 *__restrict__ buf, const uint32_t *__restrict__ idx, int cnt,
-                                         SrTarget<R> &t) {
+                                         SrWide *wide, SrTarget<R> &t) {
   unsigned mask = 0;
 #pragma unroll 8
   for (int j = 0; j < cnt; ++j) {
@@ -993,64 +1055,45 @@ __device__ __forceinline__ void sr_pairs(const float4 *__restrict__ buf, const u
       if (__shfl_sync(0xffffffffu, own, j) == (uint32_t)lane) mask &= ~(1u << j);
     }
   }
-  const int none = __ffs(mask) - 1;  // a mark to stand in for a missing second one
-  while (mask) {
-    // two pairs at a time, for their dependent chains to overlap
-    int j[2];
-    j[0] = __ffs(mask) - 1;
-    mask &= mask - 1;
-    const bool two = mask != 0;
-    j[1] = two ? __ffs(mask) - 1 : none;
-    mask &= mask - 1;
-    R v[2], w[2];
+  if constexpr (sizeof(R) == 8) {
+    const float4 s = buf[threadIdx.x & 31];
+    wide->xy[threadIdx.x & 31] = make_double2((double)s.x, (double)s.y);
+    wide->zw[threadIdx.x & 31] = make_double2((double)s.z, (double)s.w);
+    __syncwarp();
+    if (t.tl) sr_marked64<true>(buf, *wide, mask, t);
+    else sr_marked64<false>(buf, *wide, mask, t);
+  } else {
+    const int none = __ffs(mask) - 1;  // a mark to stand in for a missing second one
+    while (mask) {
+      // two pairs at a time, for their dependent chains to overlap
+      int j[2];
+      j[0] = __ffs(mask) - 1;
+      mask &= mask - 1;
+      const bool two = mask != 0;
+      j[1] = two ? __ffs(mask) - 1 : none;
+      mask &= mask - 1;
+      R v[2], w[2];
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const float4 s = buf[j[e]];
-      const float fx = s.x - t.me.x, fy = s.y - t.me.y, fz = s.z - t.me.z;
-      R dx, dy, dz;
-      if (t.tl) {
-        dx = (R)s.x - (R)t.me.x; dy = (R)s.y - (R)t.me.y; dz = (R)s.z - (R)t.me.z;
-      } else {
-        dx = (R)fx; dy = (R)fy; dz = (R)fz;
-      }
-      const R r2 = dx * dx + dy * dy + dz * dz;
-      w[e] = r2 < t.a2 && (e == 0 || two) ? (R)s.w : (R)0;
-      if constexpr (sizeof(R) == 4) {
+      for (int e = 0; e < 2; ++e) {
+        const float4 s = buf[j[e]];
+        const R dx = s.x - t.me.x, dy = s.y - t.me.y, dz = s.z - t.me.z;
+        const R r2 = dx * dx + dy * dy + dz * dz;
+        w[e] = r2 < t.a2 && (e == 0 || two) ? s.w : (R)0;
         const float rinv = rsqrtf(r2), d = r2 * rinv;
         v[e] = depth_fast(d, rinv, t.eps) - depth_fast(d, rinv, t.ai);
-      } else {
-        const float r2f = fx * fx + fy * fy + fz * fz;
-        const SrSpline &S = *t.spline;
-        const int z = (r2f >= S.b2[0]) + (r2f >= S.b2[1]) + (r2f >= S.b2[2]);
-        const double2 *c = reinterpret_cast<const double2 *>(S.c[z]);
-        // (coincident members: a finite 1/r with coefficient 0, u = -m)
-        const double rinv = rsqrt_series64(r2, rsqrtf(fmaxf(r2f, 1e-30f)));
-        const double2 km = c[4], c67 = c[3], c45 = c[2], c23 = c[1], c01 = c[0];
-        const double u = fma(r2, rinv, -km.y);
-        double f = fma(c67.y, u, c67.x);
-        f = fma(f, u, c45.y);
-        f = fma(f, u, c45.x);
-        f = fma(f, u, c23.y);
-        f = fma(f, u, c23.x);
-        f = fma(f, u, c01.y);
-        f = fma(f, u, c01.x);
-        v[e] = fma(km.x, rinv, f);
       }
-    }
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      if constexpr (sizeof(R) == 4) {  // compensated sum of the negated terms
+      for (int e = 0; e < 2; ++e) {  // compensated sum of the negated terms
         if (w[e] == 0.0f) continue;
         const float y = -(w[e] * v[e]) - t.comp;
         const float sum = t.acc + y;
         t.comp = (sum - t.acc) - y;
         t.acc = sum;
-      } else {
-        t.acc = fma(w[e], v[e], t.acc);
       }
     }
   }
 }
+
 // The sum of one chunk by a warp.  Nodes are taken 32 at a time: a lane loads
 // one node's member range, the ranges are concatenated by a warp prefix sum and read in batches of 32 (a lane finds
 // its source's node by a binary search over the prefix); sources within the
@@ -1060,7 +1103,7 @@ template <typename R, bool UPDATE>
 __device__ __forceinline__ void sr_chunk_sum(const SrChunk &C, const PmHalo &p, const uint32_t *__restrict__ cstart,
                                              const float4 *__restrict__ src4, const uint32_t *__restrict__ rpos,
                                              const uint32_t *__restrict__ rsrc, float4 *buf, uint32_t *idx,
-                                             SrTarget<R> &t) {
+                                             SrWide *wide, SrTarget<R> &t) {
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const unsigned lt = lanemask_lt();
@@ -1125,7 +1168,7 @@ __device__ __forceinline__ void sr_chunk_sum(const SrChunk &C, const PmHalo &p, 
       fill += __popc(m);
       __syncwarp();
     }
-    if (fill) sr_pairs<R, UPDATE>(buf, idx, min(fill, 32), t);
+    if (fill) sr_pairs<R, UPDATE>(buf, idx, min(fill, 32), wide, t);
     __syncwarp();
     if (!more) break;
     fill -= 32;
@@ -1148,7 +1191,7 @@ template <typename R, bool UPDATE>
 __device__ __forceinline__ void sr_block_sum(const SrChunk &C, const PmHalo &p, const uint32_t *__restrict__ cstart,
                                              const float4 *__restrict__ src4, const uint32_t *__restrict__ rpos,
                                              const uint32_t *__restrict__ rsrc, SrNodes &N, float4 *buf,
-                                             uint32_t *idx, SrTarget<R> &t) {
+                                             uint32_t *idx, SrWide *wide, SrTarget<R> &t) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int NT = 32 * kSrWarps;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1208,7 +1251,7 @@ __device__ __forceinline__ void sr_block_sum(const SrChunk &C, const PmHalo &p, 
       fill += __popc(m);
       __syncwarp();
       if (fill < 32) continue;
-      sr_pairs<R, UPDATE>(buf, idx, 32, t);
+      sr_pairs<R, UPDATE>(buf, idx, 32, wide, t);
       __syncwarp();
       fill -= 32;
       if (lane < fill) {
@@ -1219,7 +1262,7 @@ __device__ __forceinline__ void sr_block_sum(const SrChunk &C, const PmHalo &p, 
     }
     __syncthreads();
   }
-  if (fill) sr_pairs<R, UPDATE>(buf, idx, fill, t);
+  if (fill) sr_pairs<R, UPDATE>(buf, idx, fill, wide, t);
   __syncwarp();
 }
 
@@ -1246,6 +1289,8 @@ __global__ void __launch_bounds__(32 * kSrWarps, sizeof(R) == 4 ? 4 : 3) sr_gath
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // the spline tables of the halo in hand (FP64), one copy per warp
   __shared__ SrSpline tables[sizeof(R) == 8 ? kSrWarps : 1][3];
+  __shared__ SrWide wides[sizeof(R) == 8 ? kSrWarps : 1];
+  SrWide *const w64 = &wides[sizeof(R) == 8 ? warp : 0];
   int table_h = -1;
   const uint32_t nheavy = nheavy_p[UPDATE ? 1 : 0];
   const R fac = (R)(a_val / (6.0 * kPi));
@@ -1303,10 +1348,10 @@ __global__ void __launch_bounds__(32 * kSrWarps, sizeof(R) == 4 ? 4 : 3) sr_gath
     int64_t k;
     const bool some = begin(C, p, k);
     if (!heavy) {
-      if (some) sr_chunk_sum<R, UPDATE>(C, p, cstart, src4, rpos, rsrc, buf[warp], idx[warp], t);
+      if (some) sr_chunk_sum<R, UPDATE>(C, p, cstart, src4, rpos, rsrc, buf[warp], idx[warp], w64, t);
     } else {
       if (some) {  // the same for every warp
-        sr_block_sum<R, UPDATE>(C, p, cstart, src4, rpos, rsrc, nodes, buf[warp], idx[warp], t);
+        sr_block_sum<R, UPDATE>(C, p, cstart, src4, rpos, rsrc, nodes, buf[warp], idx[warp], w64, t);
         part[warp][lane] = t.acc;
       }
       __syncthreads();

@@ -691,22 +691,34 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
             link_range(pos, me, ip, b, e, r.periodic, P, parent, flags);
           }
         };
-        // the sparse cells among c0..c1, positions from `from` on
+        // the sparse cells among c0..c1, positions from `from` on; neighbours
+        // in cell order are one range
         auto add_cells = [&](uint32_t c0, uint32_t c1, uint32_t from) {
+          uint32_t run = cs[c0], end = run;
 #pragma unroll 1
           for (uint32_t c = c0; c <= c1; ++c) {
-            const uint32_t cb = cs[c], ce = cs[c + 1];
-            if (ce - cb <= (uint32_t)DENSE_T) add(max(cb, from), ce);
+            const uint32_t ce = cs[c + 1];
+            if (ce - end > (uint32_t)DENSE_T) {
+              add(max(run, from), end);
+              run = ce;
+            }
+            end = ce;
           }
+          add(max(run, from), end);
         };
         const bool px = r.pdim & 1;
-        if (N0 >= 3 && iy > 0 && iy < N1 - 1 && iz > 0 && iz < N2 - 1) {
+        // rows by steps of the cell number wherever no row wraps around; at an
+        // open face the rows outside the box are left out (a list of 20,000
+        // small regions is mostly faces: 3.97 -> 2.45 ms with neighbouring sparse cells as one range)
+        if ((!px || N0 >= 3) && (!(r.pdim & 2) || (iy > 0 && iy < N1 - 1)) &&
+            (!(r.pdim & 4) || (iz > 0 && iz < N2 - 1))) {
           // x neighbours: a run of cells, and the cell around the box's edge
           const int x0 = below[0] && ix > 0 ? -1 : 0, x1 = above[0] && ix < N0 - 1 ? 1 : 0;
           const bool lo_wrap = px && below[0] && ix == 0, hi_wrap = px && above[0] && ix == N0 - 1;
+          const bool up_y = above[1] && iy < N1 - 1, dn_y = below[1] && iy > 0, up_z = above[2] && iz < N2 - 1;
           // the rows to visit: own, then (y, z) = (+1, 0), (-1, +1), (0, +1),
           // (+1, +1); all their bounds are loaded before the first is used
-          const bool need[5] = {true, above[1], above[2] && below[1], above[2], above[2] && above[1]};
+          const bool need[5] = {true, up_y, up_z && dn_y, up_z, up_z && up_y};
           const int step[5] = {0, N0, N0 * (N1 - 1), N0 * N1, N0 * (N1 + 1)};
           uint32_t rb[5], re[5];
 #pragma unroll
@@ -729,7 +741,7 @@ __global__ void __launch_bounds__(BLK, 4) fof_link_kernel(
 #pragma unroll 1
             for (int i = lo_wrap ? 0 : 1; i < 5; ++i) {
               const int dz = i > 1 ? 1 : 0, dy = i > 1 ? i - 3 : i;
-              if ((dz && !above[2]) || (dy > 0 && !above[1]) || (dy < 0 && !below[1])) continue;
+              if ((dz && !up_z) || (dy > 0 && !up_y) || (dy < 0 && !dn_y)) continue;
               const uint32_t c = cell + (uint32_t)(N0 * (dy + N1 * dz)) + (lo_wrap ? N0 - 1 : 1 - N0);
               add_cells(c, c, 0);
             }
@@ -1273,17 +1285,19 @@ __global__ void __launch_bounds__(BLK) fof_dense_build_kernel(
 
 // Very dense cells, step 1: every particle of a merge sub-cell joins the
 // sub-cell's first particle (every pair inside one passes the exact test,
-// see region_geometry).  One block per dense cell; the others return.
+// see region_geometry).  One block per dense cell; the others return.  The
+// very dense cells and their regions are listed for step 2 (in any order).
 __global__ void __launch_bounds__(BLK) fof_vd_intra_kernel(
     const uint32_t *__restrict__ list, const uint32_t *__restrict__ cs, const RegionDev *__restrict__ R,
     const uint64_t *__restrict__ cell_off, int nreg, int stride, const uint32_t *__restrict__ tab,
-    const float4 *__restrict__ dpos, int *parent, int32_t *flags) {
+    const float4 *__restrict__ dpos, int *parent, int2 *__restrict__ vd, int32_t *flags) {
   const uint32_t c = list[blockIdx.x];
   const int64_t base = cs[c];
   const int64_t n = (int64_t)cs[c + 1] - base;
-  const RegionDev &r = R[nreg == 1 ? 0 : region_of_key(cell_off, nreg, (uint64_t)c)];
+  const int ri = nreg == 1 ? 0 : region_of_key(cell_off, nreg, (uint64_t)c);
+  const RegionDev &r = R[ri];
   if (!is_vd(r, n)) return;
-  if (threadIdx.x == 0) atomicAdd(&flags[FLAG_VD], 1);
+  if (threadIdx.x == 0) vd[atomicAdd(&flags[FLAG_VD], 1)] = make_int2((int)blockIdx.x, ri);
   const SubGrid g = dense_sub(r, n);
   const int S = g.s[0] * g.s[1] * g.s[2];
   const uint32_t *t = tab + (int64_t)blockIdx.x * stride;
@@ -1303,7 +1317,9 @@ __global__ void __launch_bounds__(BLK) fof_vd_intra_kernel(
 // their pairs passes the exact test.  The pairs are tested only while the
 // two roots differ, 32 members of A at a time against the members of B
 // inside A's widened box, up to the first link: linking one pair joins the
-// whole of both.  A warp per sub-cell A, a block per dense cell.  The
+// whole of both.  A warp per sub-cell A, taken in turn by the warps of a full
+// grid (with a block per cell, the few cells that hold most of the members of
+// a cluster left most of the chip idle: 1 M zoom region 2.23 -> 1.75 ms).  The
 // sub-cells B of all neighbour cells are looked up 32 at a time, a lane each:
 // most are joined to A already, and their tables and roots are chains of
 // dependent loads (one after the other they were most of the kernel).
@@ -1316,28 +1332,29 @@ struct VdCell {
 
 __global__ void __launch_bounds__(BLK) fof_vd_inter_kernel(
     const uint32_t *__restrict__ list, const uint32_t *__restrict__ cs, const RegionDev *__restrict__ R,
-    const uint64_t *__restrict__ cell_off, int nreg, int stride, const uint32_t *__restrict__ tab,
+    const int2 *__restrict__ vd, int smax, int stride, const uint32_t *__restrict__ tab,
     const uint32_t *__restrict__ rank, const float4 *__restrict__ dpos, int *parent, LinkParams P,
     float reach, int32_t *flags) {
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ VdCell nb_cells[BLK / 32][27];
-  const uint32_t c = list[blockIdx.x];
-  const int64_t base = cs[c];
-  const int64_t n = (int64_t)cs[c + 1] - base;
-  const RegionDev &r = R[nreg == 1 ? 0 : region_of_key(cell_off, nreg, (uint64_t)c)];
-  if (!is_vd(r, n)) return;
-  const SubGrid g = dense_sub(r, n);
-  const int S = g.s[0] * g.s[1] * g.s[2];
-  const uint32_t *t = tab + (int64_t)blockIdx.x * stride;
   const int lane = threadIdx.x & 31;
   VdCell *cells = nb_cells[threadIdx.x >> 5];
-  const int64_t local = (int64_t)c - (int64_t)r.cell_off;
-  const int64_t Nd[3] = {r.N[0], r.N[1], r.N[2]};
-  const int64_t ixyz[3] = {local % Nd[0], (local / Nd[0]) % Nd[1], local / (Nd[0] * Nd[1])};
-  const bool per = r.periodic != 0;
-  for (int A = threadIdx.x >> 5; A < S; A += BLK / 32) {
+  const int64_t items = (int64_t)flags[FLAG_VD] * smax;
+  for (int64_t item = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5; item < items;
+       item += ((int64_t)gridDim.x * BLK) >> 5) {
+    const int2 e = vd[item / smax];
+    const int A = (int)(item % smax);
+    const RegionDev &r = R[e.y];
+    const uint32_t c = list[e.x];
+    const int64_t base = cs[c];
+    const uint32_t *t = tab + (int64_t)e.x * stride;
+    if (A >= r.vd_k[0] * r.vd_k[1] * r.vd_k[2]) continue;
     const int64_t a0 = base + t[A], a1 = base + t[A + 1];
     if (a1 == a0) continue;
+    const int64_t local = (int64_t)c - (int64_t)r.cell_off;
+    const int64_t Nd[3] = {r.N[0], r.N[1], r.N[2]};
+    const int64_t ixyz[3] = {local % Nd[0], (local / Nd[0]) % Nd[1], local / (Nd[0] * Nd[1])};
+    const bool per = r.periodic != 0;
     // A's bounding box from its members
     float lo[3] = {3e38f, 3e38f, 3e38f}, hi[3] = {-3e38f, -3e38f, -3e38f};
     for (int64_t k = a0 + lane; k < a1; k += 32) {
@@ -2025,12 +2042,17 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
     // of the dense part do not hold back blocks of the short sparse work
     if (ctx.timing) cudaEventRecord(ctx.ev[0], s);
     if (ctx.last_dense > 0 && any_vd) {
+      int2 *vd = W.carve<int2>(ctx.last_dense);
+      if (!vd) { set_error("workspace exhausted (very dense cells)"); return kAlloc; }
+      int vd_max = 1;
+      for (int r = 0; r < nreg; ++r)
+        if (reg[r].active) vd_max = std::max(vd_max, reg[r].vd_k[0] * reg[r].vd_k[1] * reg[r].vd_k[2]);
       fof_vd_intra_kernel<<<(unsigned)ctx.last_dense, BLK, 0, s>>>(list, cstart, dR, dcoff, nreg, D.stride,
-                                                                   D.tab, D.dpos, parent, ctx.d_flags);
+                                                                   D.tab, D.dpos, parent, vd, ctx.d_flags);
       PYFOF_CHECK_LAUNCH();
-      fof_vd_inter_kernel<<<(unsigned)ctx.last_dense, BLK, 0, s>>>(list, cstart, dR, dcoff, nreg, D.stride,
-                                                                   D.tab, D.rank, D.dpos, parent, P, D.reach,
-                                                                   ctx.d_flags);
+      const int64_t vd_blocks = ceil_div((int64_t)ctx.last_dense * vd_max, BLK / 32);
+      fof_vd_inter_kernel<<<(unsigned)std::min<int64_t>(vd_blocks, kNumSMs * 5), BLK, 0, s>>>(
+          list, cstart, dR, vd, vd_max, D.stride, D.tab, D.rank, D.dpos, parent, P, D.reach, ctx.d_flags);
       PYFOF_CHECK_LAUNCH();
     }
     if (ndense_chunks > 0) {

@@ -124,26 +124,41 @@ __device__ __forceinline__ C twc(C v) {
 }
 
 // In-register DFT of length M: v[k] <- sum_e v[e] exp(SIGN 2 pi i e k / M).
-template <int M, int SIGN, typename C>
+// Only the first NI inputs are read, the others are zero.  (Outputs nobody
+// reads cost nothing: the compiler drops their arithmetic.)
+template <int M, int SIGN, int NI = M, typename C>
 __device__ __forceinline__ void dft(C (&v)[M]) {
   using R = decltype(v[0].x);
-  if constexpr (M == 1) {
+  static_assert(NI >= 1 && NI <= M, "nonzero inputs");
+  if constexpr (NI == 1) {
+#pragma unroll
+    for (int k = 1; k < M; ++k) v[k] = v[0];
   } else if constexpr (M == 2) {
     const C a = v[0], b = v[1];
     v[0] = cadd(a, b);
     v[1] = csub(a, b);
   } else if constexpr (M == 3) {
     const R h = (R)0.866025403784438646763723170752936183;  // sqrt(3)/2
-    const C t1 = cadd(v[1], v[2]);
+    C t1 = v[1], d = v[1];
+    if constexpr (NI == 3) {
+      t1 = cadd(v[1], v[2]);
+      d = csub(v[1], v[2]);
+    }
     const C t2 = mk<C>(v[0].x - (R)0.5 * t1.x, v[0].y - (R)0.5 * t1.y);
-    const C d = csub(v[1], v[2]);
     const C t3 = SIGN < 0 ? mk<C>(h * d.y, -h * d.x) : mk<C>(-h * d.y, h * d.x);
     v[0] = cadd(v[0], t1);
     v[1] = cadd(t2, t3);
     v[2] = csub(t2, t3);
   } else if constexpr (M == 4) {
-    const C t0 = cadd(v[0], v[2]), t1 = csub(v[0], v[2]);
-    const C t2 = cadd(v[1], v[3]), d = csub(v[1], v[3]);
+    C t0 = v[0], t1 = v[0], t2 = v[1], d = v[1];
+    if constexpr (NI >= 3) {
+      t0 = cadd(v[0], v[2]);
+      t1 = csub(v[0], v[2]);
+    }
+    if constexpr (NI == 4) {
+      t2 = cadd(v[1], v[3]);
+      d = csub(v[1], v[3]);
+    }
     const C t3 = SIGN < 0 ? mk<C>(d.y, -d.x) : mk<C>(-d.y, d.x);
     v[0] = cadd(t0, t2);
     v[1] = cadd(t1, t3);
@@ -152,14 +167,30 @@ __device__ __forceinline__ void dft(C (&v)[M]) {
   } else if constexpr (M == 5) {
     constexpr CosSin w1 = turn(1, 5), w2 = turn(2, 5);
     constexpr R c1 = (R)w1.c, c2 = (R)w2.c, s1 = (R)w1.s, s2 = (R)w2.s;
-    const C a1 = cadd(v[1], v[4]), a2 = cadd(v[2], v[3]);
-    const C d1 = csub(v[1], v[4]), d2 = csub(v[2], v[3]);
-    const C e1 = mk<C>(v[0].x + c1 * a1.x + c2 * a2.x, v[0].y + c1 * a1.y + c2 * a2.y);
-    const C e2 = mk<C>(v[0].x + c2 * a1.x + c1 * a2.x, v[0].y + c2 * a1.y + c1 * a2.y);
-    // SIGN i times the odd parts
-    const C o1 = mk<C>((R)-SIGN * (s1 * d1.y + s2 * d2.y), (R)SIGN * (s1 * d1.x + s2 * d2.x));
-    const C o2 = mk<C>((R)-SIGN * (s2 * d1.y - s1 * d2.y), (R)SIGN * (s2 * d1.x - s1 * d2.x));
-    v[0] = cadd(v[0], cadd(a1, a2));
+    C a1 = v[1], d1 = v[1], a2 = mk<C>(0, 0), d2 = a2;
+    if constexpr (NI == 5) {
+      a1 = cadd(v[1], v[4]);
+      d1 = csub(v[1], v[4]);
+    }
+    if constexpr (NI == 3) a2 = d2 = v[2];
+    if constexpr (NI >= 4) {
+      a2 = cadd(v[2], v[3]);
+      d2 = csub(v[2], v[3]);
+    }
+    C e1, e2, o1, o2;  // o1, o2: SIGN i times the odd parts
+    if constexpr (NI >= 3) {
+      e1 = mk<C>(v[0].x + c1 * a1.x + c2 * a2.x, v[0].y + c1 * a1.y + c2 * a2.y);
+      e2 = mk<C>(v[0].x + c2 * a1.x + c1 * a2.x, v[0].y + c2 * a1.y + c1 * a2.y);
+      o1 = mk<C>((R)-SIGN * (s1 * d1.y + s2 * d2.y), (R)SIGN * (s1 * d1.x + s2 * d2.x));
+      o2 = mk<C>((R)-SIGN * (s2 * d1.y - s1 * d2.y), (R)SIGN * (s2 * d1.x - s1 * d2.x));
+      v[0] = cadd(v[0], cadd(a1, a2));
+    } else {
+      e1 = mk<C>(v[0].x + c1 * a1.x, v[0].y + c1 * a1.y);
+      e2 = mk<C>(v[0].x + c2 * a1.x, v[0].y + c2 * a1.y);
+      o1 = mk<C>((R)-SIGN * (s1 * d1.y), (R)SIGN * (s1 * d1.x));
+      o2 = mk<C>((R)-SIGN * (s2 * d1.y), (R)SIGN * (s2 * d1.x));
+      v[0] = cadd(v[0], a1);
+    }
     v[1] = cadd(e1, o1);
     v[2] = cadd(e2, o2);
     v[3] = csub(e2, o2);
@@ -168,22 +199,23 @@ __device__ __forceinline__ void dft(C (&v)[M]) {
     // decimation in time: e = p + P q, k = k' + Q j
     constexpr int P = (M % 4 == 0) ? 4 : ((M % 2 == 0) ? 2 : (M % 3 == 0) ? 3 : 5);
     constexpr int Q = M / P;
+    constexpr int NP = NI < P ? NI : P;  // nonzero sub-transforms
     static_assert(P * Q == M, "DFT length must be 2^a 3^b 5^c");
     C sub[P][Q];
-#pragma unroll
-    for (int p = 0; p < P; ++p) {
+    sfor<NP>([&](auto pc) {
+      constexpr int p = decltype(pc)::value;
 #pragma unroll
       for (int q = 0; q < Q; ++q) sub[p][q] = v[p + P * q];
-      dft<Q, SIGN>(sub[p]);
-    }
+      dft<Q, SIGN, (NI - p + P - 1) / P>(sub[p]);
+    });
     sfor<Q>([&](auto kc) {
       constexpr int k = decltype(kc)::value;
       C t[P];
-      sfor<P>([&](auto pc) {
+      sfor<NP>([&](auto pc) {
         constexpr int p = decltype(pc)::value;
         t[p] = twc<SIGN, p * k, M>(sub[p][k]);
       });
-      dft<P, SIGN>(t);
+      dft<P, SIGN, NP>(t);
 #pragma unroll
       for (int j = 0; j < P; ++j) v[k + Q * j] = t[j];
     });
@@ -216,6 +248,19 @@ template <> struct Cfg<double, 192> { static constexpr int N1 = 16, N2 = 12, T =
 template <> struct Cfg<double, 216> { static constexpr int N1 = 12, N2 = 18, T = 144; };
 template <> struct Cfg<double, 240> { static constexpr int N1 = 16, N2 = 15, T = 128; };
 template <> struct Cfg<double, 256> { static constexpr int N1 = 16, N2 = 16, T = 128; };
+
+// What of a line a convolution can read and write: stage A's nonzero inputs
+// (e = s + N2 q < conv_in_max) and the elements that stage A' (e = s + N2 q)
+// and stage B (e = k1 + N1 k2) of the inverse transforms produce (e <
+// conv_out_end), out of N1, N1 and N2.  About half of each; leaving out the
+// rest took 5 to 13 % off the FP64 passes (fused z pass of 180 points, 282
+// refined regions: 3.37 -> 2.96 ms; 96 points: 3.92 -> 3.63 ms).  FP32 keeps all of them (and with them its bits).
+template <typename R, int N>
+constexpr int kInA = sizeof(R) == 8 ? (conv_in_max(N) + Cfg<R, N>::N2 - 1) / Cfg<R, N>::N2 : Cfg<R, N>::N1;
+template <typename R, int N>
+constexpr int kOutA = sizeof(R) == 8 ? (conv_out_end(N) + Cfg<R, N>::N2 - 1) / Cfg<R, N>::N2 : Cfg<R, N>::N1;
+template <typename R, int N>
+constexpr int kOutB = sizeof(R) == 8 ? (conv_out_end(N) + Cfg<R, N>::N1 - 1) / Cfg<R, N>::N1 : Cfg<R, N>::N2;
 
 // Threads of the fused z pass: as above, but 216 points do better with two
 // rounds of stage A than with fewer registers (18.7 us a grid against 23; the
@@ -283,7 +328,7 @@ __device__ __forceinline__ void load_twiddles(cplx_t<R> *tw, const cplx_t<R> *__
 // Stage A in place on `buf`: every thread first reads all the elements of
 // its units into registers, then (after a barrier) writes the results over
 // the tile.
-template <typename R, int N, int SIGN>
+template <typename R, int N, int SIGN, int NI>
 __device__ __forceinline__ void stage_a_inplace(cplx_t<R> *buf, const cplx_t<R> *tw, int in_lim) {
   using C = cplx_t<R>;
   constexpr int N1 = Cfg<R, N>::N1, N2 = Cfg<R, N>::N2, T = Cfg<R, N>::T;
@@ -294,7 +339,7 @@ __device__ __forceinline__ void stage_a_inplace(cplx_t<R> *buf, const cplx_t<R> 
     const int u = threadIdx.x + it * T;
     const int li = u % W, s = u / W;
 #pragma unroll
-    for (int q = 0; q < N1; ++q) {
+    for (int q = 0; q < NI; ++q) {
       const int e = s + N2 * q;
       v[it][q] = (u < UA && e < in_lim) ? buf[li + WP * e] : mk<C>(0, 0);
     }
@@ -305,7 +350,7 @@ __device__ __forceinline__ void stage_a_inplace(cplx_t<R> *buf, const cplx_t<R> 
     const int u = threadIdx.x + it * T;
     if (u < UA) {
       const int li = u % W, s = u / W;
-      dft<N1, SIGN>(v[it]);
+      dft<N1, SIGN, NI>(v[it]);
 #pragma unroll
       for (int k1 = 0; k1 < N1; ++k1)
         buf[li + WP * (k1 + N1 * s)] = SIGN < 0 ? cmul(v[it][k1], tw[s * k1]) : cmulc(v[it][k1], tw[s * k1]);
@@ -315,8 +360,8 @@ __device__ __forceinline__ void stage_a_inplace(cplx_t<R> *buf, const cplx_t<R> 
 
 // Stage B from `src` (stage A layout) into tile layout `dst` (li + (W+1) k).
 // Unit (li, k1) reads and writes only the elements li + (W+1) (k1 + N1 j),
-// so src may equal dst.
-template <typename R, int N, int SIGN>
+// so src may equal dst.  The outputs k2 < NO are written.
+template <typename R, int N, int SIGN, int NO>
 __device__ __forceinline__ void stage_b_smem(const cplx_t<R> *src, cplx_t<R> *dst) {
   using C = cplx_t<R>;
   constexpr int N1 = Cfg<R, N>::N1, N2 = Cfg<R, N>::N2, T = Cfg<R, N>::T;
@@ -331,7 +376,7 @@ __device__ __forceinline__ void stage_b_smem(const cplx_t<R> *src, cplx_t<R> *ds
       for (int s = 0; s < N2; ++s) v[s] = src[li + WP * (k1 + N1 * s)];
       dft<N2, SIGN>(v);
 #pragma unroll
-      for (int k2 = 0; k2 < N2; ++k2) dst[li + WP * (k1 + N1 * k2)] = v[k2];
+      for (int k2 = 0; k2 < NO; ++k2) dst[li + WP * (k1 + N1 * k2)] = v[k2];
     }
   }
 }
@@ -388,9 +433,9 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_x_r2c(const unsigned long long
     }
   }
   __syncthreads();
-  stage_a_inplace<R, N, -1>(t0, tw, sx);
+  stage_a_inplace<R, N, -1, kInA<R, N>>(t0, tw, sx);
   __syncthreads();
-  stage_b_smem<R, N, -1>(t0, t0);
+  stage_b_smem<R, N, -1, Cfg<R, N>::N2>(t0, t0);
   __syncthreads();
 #pragma unroll
   for (int it = 0; it < (2 * W * NH + T - 1) / T; ++it) {
@@ -449,9 +494,9 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_x_c2r(const cplx_t<R> *__restr
     }
   }
   __syncthreads();
-  stage_a_inplace<R, N, +1>(t0, tw, N);
+  stage_a_inplace<R, N, +1, Cfg<R, N>::N1>(t0, tw, N);
   __syncthreads();
-  stage_b_smem<R, N, +1>(t0, t0);
+  stage_b_smem<R, N, +1, SUP == N ? Cfg<R, N>::N2 : kOutB<R, N>>(t0, t0);
   __syncthreads();
   R *dst = phi + bx.out_off + (int64_t)L0 * ox;
   // a power of two divides exactly as its reciprocal multiplies
@@ -472,7 +517,7 @@ __global__ void __launch_bounds__(Cfg<R, N>::T) k_x_c2r(const cplx_t<R> *__restr
 }
 
 // Strided passes over tiles of W consecutive kx.
-enum { kYForward = 0, kZConv = 1, kYInverse = 2, kZInverse = 3 };
+enum { kYForward = 0, kZConv = 1, kYInverse = 2, kZInverse = 3, kYInverseAll = 4 };
 
 // kYForward: lines (kx, z < in[2]), values y < in[1] in, all N out.
 // kZConv: lines (kx, ky), values z < in[2] in, forward transform,
@@ -480,7 +525,8 @@ enum { kYForward = 0, kZConv = 1, kYInverse = 2, kZInverse = 3 };
 //   inverse transform, the output window's z out; a block handles the grids
 //   [b0, b0 + nbb) of the batch with its Green values in registers.
 // kYInverse: lines (kx, z of the output window), all N in, its y out.
-// kZInverse: lines (kx, ky), all N in and out (the self kernel).
+// kZInverse: lines (kx, ky), all N in and out, kYInverseAll: lines (kx, z) of
+//   all z, all N in and out (c2r_full).
 template <typename R, int N, int PASS>
 __global__ void __launch_bounds__(PASS == kZConv ? kConvT<R, N> : Cfg<R, N>::T, kMinBlocks<R, N, PASS == kZConv>) k_lines(cplx_t<R> *__restrict__ spec, const R *__restrict__ green,
                                                         const cplx_t<R> *__restrict__ twt,
@@ -492,6 +538,8 @@ __global__ void __launch_bounds__(PASS == kZConv ? kConvT<R, N> : Cfg<R, N>::T, 
   constexpr int W = kW<R>, WP = W + 1, NH = N / 2 + 1;
   constexpr int UA = W * N2, UB = W * N1;
   constexpr int IA = (UA + T - 1) / T, IB = (UB + T - 1) / T;
+  constexpr int NI = FWD ? kInA<R, N> : N1;
+  constexpr int NOA = kOutA<R, N>, NOB = PASS == kYInverse ? kOutB<R, N> : N2;
   const int tile = (int)(blockIdx.x % (unsigned)ntiles);
   const int other = (int)(blockIdx.x / (unsigned)ntiles);
   const int kx0 = tile * W;
@@ -565,12 +613,12 @@ __global__ void __launch_bounds__(PASS == kZConv ? kConvT<R, N> : Cfg<R, N>::T, 
         const bool col = kx0 + li < NH;
         C v[N1];
 #pragma unroll
-        for (int q = 0; q < N1; ++q) {
+        for (int q = 0; q < NI; ++q) {
           const int e = s + N2 * q;
           if constexpr (CONV) v[q] = (col && e < in_lim) ? stg[e * W + li] : mk<C>(0, 0);
           else v[q] = (col && e < in_lim) ? base[(int64_t)e * estride + li] : mk<C>(0, 0);
         }
-        dft<N1, FWD ? -1 : +1>(v);
+        dft<N1, FWD ? -1 : +1, NI>(v);
 #pragma unroll
         for (int k1 = 0; k1 < N1; ++k1) {
           const C w = tw[s * k1];
@@ -607,7 +655,7 @@ __global__ void __launch_bounds__(PASS == kZConv ? kConvT<R, N> : Cfg<R, N>::T, 
         } else {
           if (kx0 + li < NH) {
 #pragma unroll
-            for (int k2 = 0; k2 < N2; ++k2) {
+            for (int k2 = 0; k2 < NOB; ++k2) {
               const int e = k1 + N1 * k2;
               if ((unsigned)(e - lo) < cnt) base[(int64_t)e * estride + li] = v[k2];
             }
@@ -629,7 +677,7 @@ __global__ void __launch_bounds__(PASS == kZConv ? kConvT<R, N> : Cfg<R, N>::T, 
           dft<N1, +1>(v);
           if (kx0 + li < NH) {
 #pragma unroll
-            for (int q = 0; q < N1; ++q) {
+            for (int q = 0; q < NOA; ++q) {
               const int e = s + N2 * q;
               if ((unsigned)(e - lo) < cnt) base[(int64_t)e * estride + li] = v[q];
             }
@@ -673,6 +721,7 @@ int32_t prepare() {
     if (r == kOk) r = allow_smem(k_x_c2r<R, N, N>, sm);
     if (r == kOk) r = allow_smem(k_lines<R, N, kYForward>, sm);
     if (r == kOk) r = allow_smem(k_lines<R, N, kYInverse>, sm);
+    if (r == kOk) r = allow_smem(k_lines<R, N, kYInverseAll>, sm);
     if (r == kOk) r = allow_smem(k_lines<R, N, kZInverse>, sm);
     if (r == kOk) r = allow_smem(k_lines<R, N, kZConv>, smem_conv_bytes<R, N>(conv_in_max(N)));
     status = r;
@@ -732,7 +781,7 @@ int32_t c2r_full_n(const R *green, cplx_t<R> *spec, R *out, const cplx_t<R> *tw,
   // z inverse over all ky, then y inverse over all z
   k_lines<R, N, kZInverse><<<(unsigned)(ntiles * N), T, sm, s>>>(spec, nullptr, tw, box, nhp, ntiles, 1, 1);
   PYFOF_CHECK_LAUNCH();
-  k_lines<R, N, kYInverse><<<(unsigned)(ntiles * N), T, sm, s>>>(spec, nullptr, tw, box, nhp, ntiles, 1, 1);
+  k_lines<R, N, kYInverseAll><<<(unsigned)(ntiles * N), T, sm, s>>>(spec, nullptr, tw, box, nhp, ntiles, 1, 1);
   PYFOF_CHECK_LAUNCH();
   k_x_c2r<R, N, N><<<(unsigned)ceil_div((int64_t)N * N, 2 * W), T, sm, s>>>(spec, out, tw, box, nhp, (R)1);
   PYFOF_CHECK_LAUNCH();
@@ -752,9 +801,9 @@ template <typename R>
 int32_t pm_convolve_batch(const unsigned long long *acc, const double *inv_scale, R *phi, cplx_t<R> *spec,
                           const R *green, const cplx_t<R> *tw, int n, const ConvBox *boxes, const ConvExtent &ext,
                           int batch, bool scaled, cudaStream_t s, int waves) {
-  const int in_max = conv_in_max(n), out_max = n / 2 + 1;
+  const int in_max = conv_in_max(n), out_max = conv_out_end(n);
   if (batch < 1 || batch > 65535 || ext.in_lines < 1 || ext.out_lines < 1 || ext.in_x > in_max ||
-      ext.in_y > in_max || ext.in_z > in_max || ext.out_x > out_max || ext.out_y > out_max || ext.out_z > out_max) {
+      ext.in_y > in_max || ext.in_z > in_max || ext.out_end > out_max) {
     set_error("invalid convolution batch (n %d, batch %d)", n, batch);
     return kInvalid;
   }

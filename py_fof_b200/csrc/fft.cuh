@@ -65,9 +65,15 @@ inline const int *conv_lengths(int n, bool fp64) {
   return own[n == 48 ? 0 : n == 64 ? 1 : n == 128 ? 2 : n == 216 ? 3 : 4];
 }
 
-// Nonzero input nodes per axis that a transform of n points takes (a refined
-// region's sources reach beyond half of its 96 or 180 points).
-__host__ __device__ constexpr int conv_in_max(int n) { return n == 96 || n == 180 ? 5 * n / 8 : n / 2 + 1; }
+// Nonzero input nodes per axis that a transform of n points takes, and the end
+// of the nodes it can put out.  A box that fits a shorter transform is at most
+// half of it; a whole grid's may have one node more, a refined region's sources
+// reach beyond half of its 96 or 180 points.
+__host__ __device__ constexpr bool conv_shorter(int n) {
+  return n == 96 || n == 108 || n == 144 || n == 160 || n == 180 || n == 192 || n == 240;
+}
+__host__ __device__ constexpr int conv_out_end(int n) { return conv_shorter(n) ? n / 2 : n / 2 + 1; }
+__host__ __device__ constexpr int conv_in_max(int n) { return n == 96 ? 56 : n == 180 ? 108 : conv_out_end(n); }
 
 // One grid of a batch (see above).  Offsets in elements; out0 + out <= in.
 struct ConvBox {
@@ -81,15 +87,16 @@ struct ConvBox {
 
 // Transform length for a box on the n-point grid.
 inline int conv_length(int n, bool fp64, const ConvBox &b) {
-  int reach = 0, in = 0;
+  int reach = 0, in = 0, end = 0;
   for (int d = 0; d < 3; ++d) {
     const int back = b.in[d] - 1 - b.out0[d], ahead = b.out0[d] + b.out[d] - 1;
     reach = back > reach ? back : reach;
     reach = ahead > reach ? ahead : reach;
     in = b.in[d] > in ? b.in[d] : in;
+    end = ahead + 1 > end ? ahead + 1 : end;
   }
   const int *l = conv_lengths(n, fp64);
-  while (*l < n && (*l < 2 * reach + 1 || conv_in_max(*l) < in)) ++l;
+  while (*l < n && (*l < 2 * reach + 1 || conv_in_max(*l) < in || conv_out_end(*l) < end)) ++l;
   return *l;
 }
 
@@ -105,11 +112,11 @@ inline double conv_bytes(int n, const ConvBox &b) {
 
 // Largest extents over the boxes of a batch (launch shapes).
 struct ConvExtent {
-  int in_x = 0, in_y = 0, in_z = 0, out_x = 0, out_y = 0, out_z = 0;
+  int in_x = 0, in_y = 0, in_z = 0, out_y = 0, out_z = 0, out_end = 0;
   int64_t in_lines = 0, out_lines = 0;
   void add(const ConvBox &b) {
     in_x = b.in[0] > in_x ? b.in[0] : in_x;
-    out_x = b.out[0] > out_x ? b.out[0] : out_x;
+    for (int d = 0; d < 3; ++d) out_end = b.out0[d] + b.out[d] > out_end ? b.out0[d] + b.out[d] : out_end;
     in_y = b.in[1] > in_y ? b.in[1] : in_y;
     in_z = b.in[2] > in_z ? b.in[2] : in_z;
     out_y = b.out[1] > out_y ? b.out[1] : out_y;

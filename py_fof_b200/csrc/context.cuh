@@ -102,6 +102,15 @@ struct Context {
   size_t stage_cap = 0, stage_used = 0;
   std::vector<uint8_t *> stage_retired;
   void stage_reset() { stage_used = 0; }
+  // Host side of a call's region table, kept for the next one: the pages of a
+  // fresh table cost more than filling it (20,000 regions: 7.5 MB, three
+  // copies of it).  Tables above 64 MB are the call's own.
+  std::vector<uint64_t> h_words;
+  uint64_t *host_words(size_t n, std::vector<uint64_t> &own) {
+    std::vector<uint64_t> &v = n <= ((size_t)64 << 20) / 8 ? h_words : own;
+    if (v.size() < n) v.resize(n);
+    return v.data();
+  }
   CopyRing copy_ring;  // pinned chunks of pageable inputs (StagedCopy)
   ~Context();
 };

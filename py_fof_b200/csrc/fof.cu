@@ -1814,25 +1814,16 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
   Coords xp{a.xp, n, a.soa};
 
   // --- region table and tiles (host)
-  std::vector<RegionDev> reg(nreg);
-  std::vector<Tile> tiles;
   const int64_t tile = n <= kTileSmallUpTo ? TILE_SMALL : TILE;
-  int64_t start = 0;
+  int64_t total = 0, ntiles = 0;
   for (int r = 0; r < nreg; ++r) {
-    RegionDev &R = reg[r];
-    memset(&R, 0, sizeof(R));
-    R.start = start;
-    R.np = a.np_halo[r];
-    R.active = (R.np >= a.np_halo_min && R.np > 0) ? 1 : 0;
-    for (int64_t b = start; b < start + R.np; b += tile)
-      tiles.push_back(Tile{r, 0, b, std::min<int64_t>(start + R.np, b + tile)});
-    start += R.np;
+    total += a.np_halo[r];
+    ntiles += a.np_halo[r] > 0 ? ceil_div(a.np_halo[r], tile) : 0;
   }
-  if (start != n) {
-    set_error("sum(np_halo)=%lld != total_np=%lld", (long long)start, (long long)n);
+  if (total != n) {
+    set_error("sum(np_halo)=%lld != total_np=%lld", (long long)total, (long long)n);
     return kInvalid;
   }
-  const int64_t ntiles = (int64_t)tiles.size();
   // one block of tables: regions, cell offsets, bounding boxes, an error
   // word, tiles; uploaded together, the boxes and the error word read back
   // together, regions and offsets uploaded again with the geometry
@@ -1847,21 +1838,31 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
   unsigned long long *dbb = reinterpret_cast<unsigned long long *>(dtab + o_bb);
   int32_t *derr = reinterpret_cast<int32_t *>(dtab + o_err);
   Tile *dT = reinterpret_cast<Tile *>(dtab + o_tile);
-  std::vector<uint64_t> tab((tab_bytes + 7) / 8, 0);
-  uint8_t *htab = reinterpret_cast<uint8_t *>(tab.data());
-  memcpy(htab, reg.data(), sizeof(RegionDev) * nreg);
-  for (int r = 0; r < nreg; ++r)
-    for (int d = 0; d < 3; ++d) tab[o_bb / 8 + 6 * (size_t)r + d] = ~0ull;  // minima; maxima start at 0
-  if (ntiles) memcpy(htab + o_tile, tiles.data(), sizeof(Tile) * ntiles);
+  std::vector<uint64_t> large_tab;
+  uint64_t *tab = ctx.host_words((tab_bytes + 7) / 8, large_tab);
+  uint8_t *htab = reinterpret_cast<uint8_t *>(tab);
+  RegionDev *reg = reinterpret_cast<RegionDev *>(htab);
+  uint64_t *cell_off = tab + o_off / 8, *bb = tab + o_bb / 8;
+  Tile *tiles = reinterpret_cast<Tile *>(htab + o_tile);
+  memset(htab, 0, o_tile);
+  int64_t start = 0;
+  for (int r = 0; r < nreg; ++r) {
+    RegionDev &R = reg[r];
+    R.start = start;
+    R.np = a.np_halo[r];
+    R.active = (R.np >= a.np_halo_min && R.np > 0) ? 1 : 0;
+    for (int64_t b = start; b < start + R.np; b += tile)
+      *tiles++ = Tile{r, 0, b, std::min<int64_t>(start + R.np, b + tile)};
+    start += R.np;
+    for (int d = 0; d < 3; ++d) bb[6 * (size_t)r + d] = ~0ull;  // minima; maxima start at 0
+  }
   PYFOF_TRY(upload(ctx, dtab, htab, tab_bytes, s));
   PYFOF_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(int32_t) * FLAG_COUNT, s));
   if (ntiles) {
     fof_bbox_kernel<<<(unsigned)ntiles, BLK, 0, s>>>(xp, dR, dT, L, half, dbb, derr);
     PYFOF_CHECK_LAUNCH();
   }
-  std::vector<unsigned long long> bb(6 * (size_t)nreg + 1);
-  PYFOF_CUDA(cudaMemcpyAsync(bb.data(), dbb, sizeof(unsigned long long) * bb.size(),
-                             cudaMemcpyDeviceToHost, s));
+  PYFOF_CUDA(cudaMemcpyAsync(bb, dbb, sizeof(uint64_t) * (6 * (size_t)nreg + 1), cudaMemcpyDeviceToHost, s));
   PYFOF_CUDA(cudaStreamSynchronize(s));
   if (const int32_t err = (int32_t)bb[6 * (size_t)nreg]) {
     set_error("non-finite particle coordinates");
@@ -1871,7 +1872,6 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
   // --- reference geometry per region (host)
   uint64_t total_cells = 0;
   int64_t n_active = 0;
-  std::vector<uint64_t> cell_off(nreg + 1);
   for (int r = 0; r < nreg; ++r) {
     RegionDev &R = reg[r];
     cell_off[r] = total_cells;
@@ -1896,8 +1896,6 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
   st.total_cells = total_cells;
   ctx.last_cells = (int64_t)total_cells;
   ctx.last_active = n_active;
-  memcpy(htab, reg.data(), sizeof(RegionDev) * nreg);
-  memcpy(htab + o_off, cell_off.data(), sizeof(uint64_t) * (nreg + 1));
   PYFOF_TRY(upload(ctx, dtab, htab, o_bb, s));
   uint32_t *keys = W.carve<uint32_t>(std::max<int64_t>(n, 1));
   uint32_t *cstart = W.carve<uint32_t>(total_cells + 2);
@@ -2077,7 +2075,6 @@ int32_t fof_link_stage(Context &ctx, const FofArgs &a, FofState &st) {
   st.gsize = gsize;
   st.cell_start = cstart;
   st.keys_free = keys;
-  st.reg = reg;
   return kOk;
 }
 

@@ -55,7 +55,6 @@ struct FofState {
   int64_t n = 0, n_active = 0;
   int nreg = 0;
   uint64_t total_cells = 0;
-  std::vector<RegionDev> reg;
   RegionDev *dR = nullptr;
   float4 *pos = nullptr;      // sorted FP32 coordinates, .w = original index bits
   uint32_t *prid = nullptr;   // region of each sorted particle (null: one region)

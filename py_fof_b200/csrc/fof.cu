@@ -1360,7 +1360,8 @@ __global__ void __launch_bounds__(BLK) fof_vd_intra_kernel(
 // inside A's widened box, up to the first link: linking one pair joins the
 // whole of both.  A warp per sub-cell A, taken in turn by the warps of a full
 // grid (with a block per cell, the few cells that hold most of the members of
-// a cluster left most of the chip idle: 1 M zoom region 2.23 -> 1.75 ms).  The
+// a cluster left most of the chip idle: 1 M zoom region 2.23 -> 1.0 to 1.75 ms,
+// by the order the joins come in).  The
 // sub-cells B of all neighbour cells are looked up 32 at a time, a lane each:
 // most are joined to A already, and their tables and roots are chains of
 // dependent loads (one after the other they were most of the kernel).

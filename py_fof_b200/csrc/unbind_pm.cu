@@ -8,13 +8,12 @@
 //       gather, self term and the far-field constant (:2657-2703);
 //   C2: short-range residual between the spline-softened kernel and the C1
 //       split kernel for pairs closer than 3.5 grid cells (:3403-3552),
-//       evaluated over 3.5-cell neighbour lists, recomputed over the kept set
-//       each pass (the reference updates it incrementally; the sum is the
-//       same set of pair terms);
+//       evaluated over nodes of 3.5-cell neighbour cells: the kept set on the
+//       first pass, the members removed since on the later ones;
 //   removal: the inner loop of the direct path, with the top-2% selection
 //       done by an in-block radix select (only the deleted set matters here).
-// Halos of one grid class are batched: one launch deposits, transforms and
-// gathers all of them.  R = float is the product path, R = double the plain
+// Halos are batched: one launch deposits and one gathers all of them, the
+// transforms run per grid class and transform length.  R = float is the product path, R = double the plain
 // FP64 path.
 #include <algorithm>
 #include <climits>
@@ -200,11 +199,12 @@ int32_t shorter_tables(GreenTable &t, const double *grid, double2 *spec, ConvBox
     t.shorter.push_back(std::move(q));
     return kOk;
   };
-  const int64_t n = t.n;
   const int *l = conv_lengths(t.n, true);
   if (*l == t.n) return kOk;
-  if (cudaMallocAsync(&h, sizeof(double) * n * n * n, s) != cudaSuccess ||
-      cudaMallocAsync(&out, sizeof(double) * n * n * n, s) != cudaSuccess) {
+  int64_t top = 0;  // the longest of them
+  for (const int *k = l; *k < t.n; ++k) top = *k;
+  if (cudaMallocAsync(&h, sizeof(double) * (top / 2 + 1) * top * top, s) != cudaSuccess ||
+      cudaMallocAsync(&out, sizeof(double) * top * top * top, s) != cudaSuccess) {
     cudaGetLastError();
     set_error("device allocation failed (kernel tables)");
     r = kAlloc;

@@ -324,21 +324,36 @@ __device__ __forceinline__ bool pm_tsc(const PmHalo &p, float4 q, int *f, float 
 }
 
 // Self potential of a TSC cloud on a grid (bound_fortran.f90:2577-2602): FP32
-// products, FP64 sum.
+// products, FP64 sum over the 27 x 27 pairs of its nodes, offset by offset.  The
+// product of a pair is the same both ways round, so the two kernel values of
+// an offset and its opposite are added and half the pairs are left.  Bound by
+// the conversions of the products (71 % of the conversion units with all of
+// them): 20,000 halos 1.14 -> 0.57 ms (refined regions 0.76 -> 0.34 ms), 256^3
+// box 277 -> 139 us, FP32 203^3 box 199 -> 88 us.
 template <typename R>
 __device__ __forceinline__ R tsc_self(const float *w9, const R *__restrict__ sp) {
+  float w[27];
+#pragma unroll
+  for (int j = 0; j < 27; ++j) w[j] = __fmul_rn(__fmul_rn(w9[j % 3], w9[3 + j / 3 % 3]), w9[6 + j / 9]);
   double acc = 0.0;
-  for (int sz = 0; sz < 3; ++sz)
-    for (int sy = 0; sy < 3; ++sy)
-      for (int sx = 0; sx < 3; ++sx) {
-        const float sw = __fmul_rn(__fmul_rn(w9[sx], w9[3 + sy]), w9[6 + sz]);
-        for (int tz = 0; tz < 3; ++tz)
-          for (int ty = 0; ty < 3; ++ty)
-            for (int tx = 0; tx < 3; ++tx) {
-              const float tw = __fmul_rn(__fmul_rn(w9[tx], w9[3 + ty]), w9[6 + tz]);
-              acc += (double)__fmul_rn(sw, tw) *
-                     (double)sp[((tz - sz + 2) * 5 + (ty - sy + 2)) * 5 + (tx - sx + 2)];
-            }
+#pragma unroll
+  for (int j = 0; j < 27; ++j) acc += (double)__fmul_rn(w[j], w[j]);
+  acc *= (double)sp[62];
+#pragma unroll
+  for (int dz = 0; dz < 3; ++dz)
+#pragma unroll
+    for (int dy = -2; dy < 3; ++dy)
+#pragma unroll
+      for (int dx = -2; dx < 3; ++dx) {
+        if (dz == 0 && (dy < 0 || (dy == 0 && dx <= 0))) continue;  // the opposite offset
+        double t = 0.0;
+#pragma unroll
+        for (int j = 0; j < 27; ++j) {
+          const int x = j % 3 + dx, y = j / 3 % 3 + dy, z = j / 9 + dz;
+          if (x >= 0 && x < 3 && y >= 0 && y < 3 && z < 3) t += (double)__fmul_rn(w[j], w[x + 3 * (y + 3 * z)]);
+        }
+        const int k = ((dz + 2) * 5 + (dy + 2)) * 5 + (dx + 2);
+        acc += t * ((double)sp[k] + (double)sp[124 - k]);
       }
   return (R)acc;
 }

@@ -787,14 +787,21 @@ __device__ __forceinline__ Two two_fma(Two a, double b, Two c) {
 }
 
 // The piece of D(., h) around distance m: Taylor coefficients of its
-// polynomial about m, and the factor of 1/r.
+// polynomial about m, and the factor of 1/r.  At and beyond h (always, for
+// h = 0) it is 1/r alone.
 __device__ __forceinline__ void spline_piece(double h, double m, double *c) {
+  if (m >= h) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) c[j] = 0.0;
+    c[8] = 1.0;
+    return;
+  }
   const double s = 2.0 / h, u = 1.0 / (70.0 * h), e0 = s * m;
   const double inner[8] = {208.0, 0.0, -112.0, 0.0, 56.0, -14.0, -8.0, 3.0};
   const double outer[8] = {128.0, 224.0, -448.0, 280.0, -56.0, -14.0, 8.0, -1.0};
   Two d[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) d[j] = Two{m >= h ? 0.0 : (m < 0.5 * h ? inner[j] : outer[j]), 0.0};
+  for (int j = 0; j < 8; ++j) d[j] = Two{m < 0.5 * h ? inner[j] : outer[j], 0.0};
 #pragma unroll
   for (int i = 0; i < 7; ++i)
 #pragma unroll
@@ -805,15 +812,18 @@ __device__ __forceinline__ void spline_piece(double h, double m, double *c) {
     c[j] = d[j].hi * p;
     p *= s;
   }
-  c[8] = m >= h ? 1.0 : (m < 0.5 * h ? 0.0 : 6.0 / 70.0);
+  c[8] = m < 0.5 * h ? 0.0 : 6.0 / 70.0;
 }
 
-// A thread per (halo, ratio 1, 2, 4).
+// A thread per (halo, ratio 1, 2, 4).  A softening of 0 has no zones of its
+// own: the first one then holds distance 0 only, where D(0, h) = 208 / (70 h)
+// is infinite.
 __global__ void sr_spline_kernel(const PmHalo *__restrict__ H, int nh, double app, SrSpline *__restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 3 * nh) return;
   const double eps = (double)(float)app, a = 3.5 * (double)H[i / 3].spacing / (double)(1 << (i % 3));
-  double b[4] = {0.5 * eps, 0.5 * a, eps, a};  // ascending below
+  const double soft = eps > 0.0 ? eps : 0.0;
+  double b[4] = {0.5 * soft, 0.5 * a, soft, a};  // ascending below
   for (int j = 0; j < 3; ++j)
     for (int k = j + 1; k < 4; ++k)
       if (b[k] < b[j]) {
@@ -828,17 +838,22 @@ __global__ void sr_spline_kernel(const PmHalo *__restrict__ H, int nh, double ap
     spline_piece(a, mid, ca);
     spline_piece(eps, mid, ce);
     for (int j = 0; j < 9; ++j) S.c[z][j] = ca[j] - ce[j];
+    if (b[z] == 0.0) {  // distance 0
+      S.c[z][0] = 208.0 / (70.0 * a) - 208.0 / (70.0 * eps);
+      S.c[z][8] = 0.0;
+    }
     S.c[z][9] = mid;
-    S.b2[z] = z < 3 ? __double2hiint(b[z] * b[z]) : 0;
+    S.b2[z] = z < 3 ? max(__double2hiint(b[z] * b[z]), 1) : 0;
   }
 }
 
 // 1/r: the hardware's reciprocal square root of a double's upper half as the
 // seed y and one step of the binomial series 1/sqrt(r2) = y (1 - g)^(-1/2) =
 // y (1 + g/2 + 3 g^2/8 + ..), g = 1 - r2 y^2.  The argument is kept above
-// 2^-199, for a finite 1/r of coincident members.
+// 2^-300, for a finite 1/r of coincident members; distinct FP32 coordinates
+// are at least 2^-149 apart.
 __device__ __forceinline__ double rsqrt_series64(double r2) {
-  const double a = __hiloint2double(max(__double2hiint(r2), 0x33800000), __double2loint(r2));
+  const double a = __hiloint2double(max(__double2hiint(r2), 0x2d300000), __double2loint(r2));
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
   const double g = fma(-(r2 * y), y, 1.0);

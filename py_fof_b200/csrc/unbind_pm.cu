@@ -215,7 +215,9 @@ int32_t shorter_tables(GreenTable &t, const double *grid, double2 *spec, ConvBox
   return r;
 }
 
-// Green table of grid n for (soft, range, truncated), cached per context.
+// Green table of grid n for (soft, range, truncated), cached per device.  Its
+// kernel has a status word of its own: the call's is being written by other
+// streams (direct-summation halos) and may hold an error already.
 template <typename R>
 int32_t get_green(Context &ctx, int n, double soft, double range, int truncated,
                   std::shared_ptr<GreenTable> *out) {
@@ -234,18 +236,21 @@ int32_t get_green(Context &ctx, int n, double soft, double range, int truncated,
   PYFOF_CUDA(cudaMalloc(&t->self, sizeof(R) * 125));
   PYFOF_CUDA(cudaMalloc(&t->tw, sizeof(cplx_t<R>) * n));
   PYFOF_TRY(fill_twiddles<R>((cplx_t<R> *)t->tw, n, s));
-  PYFOF_CUDA(cudaMemsetAsync(ctx.d_flags, 0, sizeof(int32_t), s));
-  green_kernel<R><<<(unsigned)std::min<int64_t>(ceil_div(cnt, 128), 148 * 64), 128, 0, s>>>(
-      (R *)t->g, n, soft, range, truncated, ctx.d_flags);
-  PYFOF_CHECK_LAUNCH();
   R *grid = nullptr;
   cplx_t<R> *spec = nullptr;
   ConvBox *dbox = nullptr;
+  int32_t *status = nullptr;  // FLAG_ERR of the tables' kernel
   ConvBox box{};
   for (int d = 0; d < 3; ++d) box.in[d] = box.out[d] = n;
   PYFOF_CUDA(cudaMallocAsync(&grid, sizeof(R) * (size_t)n * n * n, s));
   PYFOF_CUDA(cudaMallocAsync(&spec, sizeof(cplx_t<R>) * spec_elems<R>(n, n), s));
   PYFOF_CUDA(cudaMallocAsync(&dbox, sizeof(ConvBox), s));
+  PYFOF_CUDA(cudaMallocAsync(&status, sizeof(int32_t), s));
+  static_assert(FLAG_ERR == 0, "the status word stands for the flags");
+  PYFOF_CUDA(cudaMemsetAsync(status, 0, sizeof(int32_t), s));
+  green_kernel<R><<<(unsigned)std::min<int64_t>(ceil_div(cnt, 128), 148 * 64), 128, 0, s>>>(
+      (R *)t->g, n, soft, range, truncated, status);
+  PYFOF_CHECK_LAUNCH();
   PYFOF_CUDA(cudaMemcpyAsync(dbox, &box, sizeof(ConvBox), cudaMemcpyHostToDevice, s));
   int32_t r = c2r_full<R>((const R *)t->g, spec, grid, (const cplx_t<R> *)t->tw, dbox, n, s);
   if (r == kOk) {
@@ -253,13 +258,15 @@ int32_t get_green(Context &ctx, int n, double soft, double range, int truncated,
     PYFOF_CHECK_LAUNCH();
     if constexpr (sizeof(R) == 8) r = shorter_tables(*t, grid, spec, dbox, s);
   }
+  int32_t bad = 0;
+  PYFOF_CUDA(cudaMemcpyAsync(&bad, status, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
   cudaFreeAsync(grid, s);
   cudaFreeAsync(spec, s);
   cudaFreeAsync(dbox, s);
-  PYFOF_CUDA(cudaMemcpyAsync(ctx.h_flags, ctx.d_flags, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  cudaFreeAsync(status, s);
   PYFOF_CUDA(cudaStreamSynchronize(s));
   if (r != kOk) return r;
-  if (ctx.h_flags[FLAG_ERR]) {
+  if (bad) {
     set_error("Green's function: zero assignment response");
     return kInvalid;
   }

@@ -1158,7 +1158,8 @@ __device__ __forceinline__ void sr_pairs(const float4 *__restrict__ buf, const u
         const R dx = s.x - t.me.x, dy = s.y - t.me.y, dz = s.z - t.me.z;
         const R r2 = dx * dx + dy * dy + dz * dz;
         w[e] = r2 < t.a2 && (e == 0 || two) ? s.w : (R)0;
-        const float rinv = rsqrtf(r2), d = r2 * rinv;
+        // (coincident members: 1/r is infinite, and not needed within a softening)
+        const float rinv = rsqrtf(r2), d = r2 > 0.0f ? r2 * rinv : 0.0f;
         v[e] = depth_fast(d, rinv, t.eps) - depth_fast(d, rinv, t.ai);
       }
 #pragma unroll

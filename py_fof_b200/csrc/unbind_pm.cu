@@ -1349,9 +1349,10 @@ __device__ __forceinline__ void sr_block_sum(const SrChunk &C, const PmHalo &p, 
 // Bound by instruction issue per interacting pair (FP64 and conversions) once
 // enough warps have work.  Persistent blocks: first the heavy chunks, a
 // block each (the node ranges are found once for its eight warps, which take
-// the source batches in turn; their sums are added in warp order), then the
-// others, a warp each; both most sources first, fetched from a counter.  Two
-// pairs in flight per lane and the shared node ranges: 1 M zoom region 3.72 ->
+// the source batches in turn; their sums are added in warp order, the FP32
+// ones compensated like the sums themselves), then the others, a warp each;
+// both most sources first, fetched from a counter.  Two pairs in flight per
+// lane and the shared node ranges: 1 M zoom region 3.72 ->
 // 3.37 ms, 20,000 halos 22.6 -> 20.6 ms.
 template <typename R, bool UPDATE>
 __global__ void __launch_bounds__(32 * kSrWarps, sizeof(R) == 4 ? 4 : 3) sr_gather_kernel(
@@ -1363,7 +1364,7 @@ __global__ void __launch_bounds__(32 * kSrWarps, sizeof(R) == 4 ? 4 : 3) sr_gath
   constexpr unsigned FULL = 0xffffffffu;
   __shared__ float4 buf[kSrWarps][64];
   __shared__ uint32_t idx[kSrWarps][64];
-  __shared__ R part[kSrWarps][32];
+  __shared__ R part[kSrWarps][32], pcomp[sizeof(R) == 4 ? kSrWarps : 1][32];
   __shared__ SrNodes nodes;
   __shared__ unsigned s_ch;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1432,11 +1433,25 @@ __global__ void __launch_bounds__(32 * kSrWarps, sizeof(R) == 4 ? 4 : 3) sr_gath
       if (some) {  // the same for every warp
         sr_block_sum<R, UPDATE>(C, p, cstart, src4, rpos, rsrc, nodes, buf[warp], idx[warp], &stages[warp], t);
         part[warp][lane] = t.acc;
+        if (sizeof(R) == 4) pcomp[warp][lane] = t.comp;
       }
       __syncthreads();
       if (warp != 0 || !some) continue;
+      if constexpr (sizeof(R) == 8) {
 #pragma unroll
-      for (int w = 1; w < kSrWarps; ++w) t.acc += part[w][lane];
+        for (int w = 1; w < kSrWarps; ++w) t.acc += part[w][lane];
+      } else {
+        // the warps' sums with what they left out (comp: the excess of a sum)
+        // and what each addition here leaves out
+        R low = -t.comp;
+#pragma unroll
+        for (int w = 1; w < kSrWarps; ++w) {
+          const R x = part[w][lane], sum = __fadd_rn(t.acc, x), bb = __fsub_rn(sum, t.acc);
+          low += __fadd_rn(__fsub_rn(t.acc, __fsub_rn(sum, bb)), __fsub_rn(x, bb)) - pcomp[w][lane];
+          t.acc = sum;
+        }
+        t.acc += low;
+      }
     }
     if (some && k >= 0) {
       const R v = fac * t.acc;

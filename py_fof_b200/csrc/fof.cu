@@ -1611,40 +1611,115 @@ __global__ void __launch_bounds__(BLK) fof_cand_fill_kernel(const uint32_t *__re
 // First member of every candidate in the reference's order (cell, then
 // ascending original index): the root is the lowest position, so it lies in
 // the group's first cell, and the first member is the lowest index among the
-// group's members there (they follow the root).  A warp per candidate.
+// group's members there (they follow the root).  A warp per candidate, where
+// at most kAnchorScan positions follow: 128 steps.  A cell with more of them
+// would be walked by each of its candidates, so its positions are queued
+// once, in pieces (`piece`, flags[FLAG_PIECES]), for
+// fof_cand_anchor_large_kernel.  flags[FLAG_RUN]: more than kCandRun
+// candidates share a cell; they are then sorted instead of counted (all after
+// the linking, 1,000 counted take 0.17 ms, 1,728 0.27, sorted 0.14).  With a
+// walk and a count by every candidate 64,000 groups of one cell took 9.4 ms and
+// 512,000 270 ms, now 0.23 and 0.44 ms; one group of 10^6 members in a cell
+// 1.86 -> 0.13 ms.
+constexpr int kAnchorScan = 4096, kCandRun = 1024;
+
 __global__ void __launch_bounds__(BLK) fof_cand_anchor_kernel(const int32_t *__restrict__ root, int64_t ncand,
                                                               const int *__restrict__ lab,
                                                               const uint32_t *__restrict__ skey,
                                                               const uint32_t *__restrict__ cs,
                                                               const float4 *__restrict__ pos,
-                                                              uint32_t *__restrict__ first) {
+                                                              uint32_t *__restrict__ first,
+                                                              uint32_t *__restrict__ crank,
+                                                              uint2 *__restrict__ piece, int32_t *__restrict__ flags) {
   const int lane = threadIdx.x & 31;
   for (int64_t c = ((int64_t)blockIdx.x * BLK + threadIdx.x) >> 5; c < ncand; c += ((int64_t)gridDim.x * BLK) >> 5) {
     const int r = root[c];
-    const int64_t e = cs[skey[r] + 1];
+    const uint32_t cell = skey[r];
+    const int64_t e = cs[cell + 1];
     uint32_t m = 0xffffffffu;
-    for (int64_t q = (int64_t)r + lane; q < e; q += 32)
-      if (lab[q] == r) m = min(m, (uint32_t)__float_as_int(pos[q].w));
-    m = __reduce_min_sync(0xffffffffu, m);
-    if (lane == 0) first[c] = m;
+    if (e - r <= kAnchorScan) {
+      for (int64_t q = (int64_t)r + lane; q < e; q += 32)
+        if (lab[q] == r) m = min(m, (uint32_t)__float_as_int(pos[q].w));
+      m = __reduce_min_sync(0xffffffffu, m);
+    } else if (c == 0 || skey[root[c - 1]] != cell) {  // the cell's first candidate
+      const uint32_t k = (uint32_t)((e - r + kAnchorScan - 1) / kAnchorScan);
+      uint32_t at = 0;
+      if (lane == 0) at = (uint32_t)atomicAdd(&flags[FLAG_PIECES], (int32_t)k);
+      at = __shfl_sync(0xffffffffu, at, 0);
+      for (uint32_t i = lane; i < k; i += 32) {
+        const uint32_t b = (uint32_t)r + i * kAnchorScan;
+        piece[at + i] = make_uint2(b, min((uint32_t)e, b + kAnchorScan));
+      }
+    }
+    if (lane == 0) {
+      first[c] = m;
+      crank[r] = (uint32_t)c;
+      if (c + kCandRun < ncand && skey[root[c + kCandRun]] == cell) flags[FLAG_RUN] = 1;
+    }
   }
 }
 
+// The first members of the candidates that were not walked, position by
+// position: a block per queued piece.  A warp whose positions all belong to one
+// group adds one minimum.
+__global__ void __launch_bounds__(BLK) fof_cand_anchor_large_kernel(
+    const uint2 *__restrict__ piece, const int32_t *__restrict__ flags, const int *__restrict__ lab,
+    const uint32_t *__restrict__ skey, const uint32_t *__restrict__ cs, const uint32_t *__restrict__ gsize,
+    uint32_t nmin, const float4 *__restrict__ pos, const uint32_t *__restrict__ crank,
+    uint32_t *__restrict__ first) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, np = flags[FLAG_PIECES];
+  for (int i = blockIdx.x; i < np; i += gridDim.x) {
+    const uint2 p = piece[i];
+    const uint32_t cell = skey[p.x];
+    const int64_t begin = cs[cell], end = cs[cell + 1];
+    for (uint32_t q0 = p.x + threadIdx.x - lane; q0 < p.y; q0 += BLK) {
+      const uint32_t q = q0 + lane;
+      const int r = q < p.y ? lab[q] : -1;
+      // a root of this cell, of a group large enough, and not walked
+      const bool mine = r >= begin && end - r > kAnchorScan && gsize[r] >= nmin;
+      const uint32_t idx = mine ? (uint32_t)__float_as_int(pos[q].w) : 0xffffffffu;
+      const int r0 = __shfl_sync(FULL, r, 0);
+      if (__all_sync(FULL, r == r0)) {
+        const uint32_t m = __reduce_min_sync(FULL, idx);
+        if (mine && lane == 0) atomicMin(&first[crank[r]], m);
+      } else if (mine) {
+        uint32_t *f = &first[crank[r]];
+        if (idx < __ldcg(f)) atomicMin(f, idx);
+      }
+    }
+  }
+}
+
+// Cells of the candidates in `order`.
+__global__ void fof_cand_cell_kernel(const uint32_t *__restrict__ order, int64_t ncand,
+                                     const int32_t *__restrict__ root, const uint32_t *__restrict__ skey,
+                                     uint32_t *__restrict__ cell) {
+  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncand; c += (int64_t)gridDim.x * blockDim.x)
+    cell[c] = skey[root[order[c]]];
+}
+
 // Candidate ids: position order, and by first member among candidates whose
-// roots share a cell.
+// roots share a cell: counted among them or, where more than kCandRun do,
+// taken from the candidates sorted that way (`order`).
 __global__ void fof_cand_info_kernel(const int32_t *__restrict__ root, int64_t ncand,
-                                     const uint32_t *__restrict__ first, const uint32_t *__restrict__ skey,
+                                     const uint32_t *__restrict__ first, const uint32_t *__restrict__ order,
+                                     const uint32_t *__restrict__ skey,
                                      const uint32_t *__restrict__ prid, const uint32_t *__restrict__ gsize,
                                      uint32_t *__restrict__ crank, int64_t *__restrict__ cand_anchor,
                                      int32_t *__restrict__ cand_region, int32_t *__restrict__ cand_np,
                                      int32_t *__restrict__ cand_root) {
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncand;
-       c += (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < ncand;
+       j += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t c = order ? order[j] : j;
     const int r = root[c];
-    const uint32_t cell = skey[r], f = first[c];
-    int64_t id = c;
-    for (int64_t k = c - 1; k >= 0 && skey[root[k]] == cell; --k) id -= first[k] > f;
-    for (int64_t k = c + 1; k < ncand && skey[root[k]] == cell; ++k) id += first[k] < f;
+    const uint32_t f = first[c];
+    int64_t id = j;
+    if (!order) {
+      const uint32_t cell = skey[r];
+      for (int64_t k = c - 1; k >= 0 && skey[root[k]] == cell; --k) id -= first[k] > f;
+      for (int64_t k = c + 1; k < ncand && skey[root[k]] == cell; ++k) id += first[k] < f;
+    }
     crank[r] = (uint32_t)id;
     cand_anchor[id] = f;
     cand_region[id] = prid ? (int32_t)prid[r] : 0;
@@ -2166,12 +2241,48 @@ int32_t fof_candidates_stage(Context &ctx, const FofArgs &a, FofState &st, bool 
     fof_cand_fill_kernel<<<(unsigned)ntile, BLK, 0, s>>>(st.gsize, na, nmin, toff, root);
     PYFOF_CHECK_LAUNCH();
     const unsigned gw = (unsigned)std::min<int64_t>(ceil_div(nc * 32, (int64_t)BLK), (int64_t)kNumSMs * 16);
-    fof_cand_anchor_kernel<<<gw, BLK, 0, s>>>(root, nc, st.lab, st.skey, st.cell_start, st.pos, first);
-    PYFOF_CHECK_LAUNCH();
     const unsigned gc = (unsigned)std::min<int64_t>(ceil_div(nc, (int64_t)BLK), (int64_t)kNumSMs * 16);
-    fof_cand_info_kernel<<<gc, BLK, 0, s>>>(root, nc, first, st.skey, st.prid, st.gsize, crank, st.cand_anchor,
+    const bool large = ctx.last_max_cell > kAnchorScan;  // (no candidate is left to the second kernel otherwise)
+    uint2 *piece = nullptr;
+    if (large) {
+      // cells of more than kAnchorScan positions, ceil(size / kAnchorScan) pieces each
+      piece = W.carve<uint2>(2 * (size_t)na / kAnchorScan + 1);
+      if (!piece) { set_error("workspace exhausted (candidates)"); return kAlloc; }
+    }
+    fof_cand_anchor_kernel<<<gw, BLK, 0, s>>>(root, nc, st.lab, st.skey, st.cell_start, st.pos, first, crank, piece,
+                                              ctx.d_flags);
+    PYFOF_CHECK_LAUNCH();
+    if (large) {
+      fof_cand_anchor_large_kernel<<<kNumSMs * 4, BLK, 0, s>>>(piece, ctx.d_flags, st.lab, st.skey, st.cell_start,
+                                                               st.gsize, nmin, st.pos, crank, first);
+      PYFOF_CHECK_LAUNCH();
+    }
+    uint32_t *order = nullptr;
+    const size_t before_sort = W.mark();
+    if (ctx.last_max_cell > kCandRun && nc > kCandRun) {
+      PYFOF_CUDA(cudaMemcpyAsync(ctx.h_flags, ctx.d_flags, sizeof(int32_t) * FLAG_COUNT, cudaMemcpyDeviceToHost, s));
+      PYFOF_CUDA(cudaStreamSynchronize(s));
+      if (ctx.h_flags[FLAG_RUN]) {
+        // by first member, then (stable) by cell
+        uint32_t *b[5];
+        for (uint32_t *&p : b)
+          if (!(p = W.carve<uint32_t>(nc))) { set_error("workspace exhausted (candidate order)"); return kAlloc; }
+        uint32_t *k1, *v1, *k2;
+        PYFOF_TRY(radix_sort_pairs(first, nullptr, nc, bits_for((uint64_t)a.total_np - 1), b[0], b[1], b[2], b[3], &k1,
+                                   &v1, W, s));
+        fof_cand_cell_kernel<<<gc, BLK, 0, s>>>(v1, nc, root, st.skey, b[4]);
+        PYFOF_CHECK_LAUNCH();
+        // the keys of the first sort are done with; its values are the input
+        uint32_t *const spare = v1 == b[1] ? b[3] : b[1];
+        uint32_t *const own = v1 == b[1] ? b[1] : b[3];
+        PYFOF_TRY(radix_sort_pairs(b[4], v1, nc, bits_for(st.total_cells - 1), b[0], spare, b[2], own, &k2, &order, W,
+                                   s));
+      }
+    }
+    fof_cand_info_kernel<<<gc, BLK, 0, s>>>(root, nc, first, order, st.skey, st.prid, st.gsize, crank, st.cand_anchor,
                                             st.cand_region, st.cand_np, st.cand_root);
     PYFOF_CHECK_LAUNCH();
+    W.release_to(before_sort);
     fof_member_kernel<<<grid, BLK, 0, s>>>(st.lab, st.gsize, crank, st.pos, na, nmin, write_plain ? 1 : 0, pcand,
                                            a.in_halo, a.halo_id);
     PYFOF_CHECK_LAUNCH();

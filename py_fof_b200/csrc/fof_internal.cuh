@@ -11,7 +11,11 @@ namespace pyfof {
 // Slots of Context::d_flags.
 // FLAG_VD: very dense cells linked by merge sub-cells in the last call
 // FLAG_SPREAD: warps of the key kernel's sample whose particles lie far apart
-enum { FLAG_ERR = 0, FLAG_COUNT_A = 1, FLAG_COUNT_B = 2, FLAG_COUNT_C = 3, FLAG_VD = 4, FLAG_SPREAD = 5, FLAG_COUNT = 8 };
+// FLAG_RUN: very many candidates share a cell; FLAG_PIECES: pieces of their cells
+enum {
+  FLAG_ERR = 0, FLAG_COUNT_A = 1, FLAG_COUNT_B = 2, FLAG_COUNT_C = 3, FLAG_VD = 4, FLAG_SPREAD = 5, FLAG_RUN = 6,
+  FLAG_PIECES = 7, FLAG_COUNT = 8
+};
 
 // One input region (one element of xp_list) with its reference cell grid.
 struct RegionDev {

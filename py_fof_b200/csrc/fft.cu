@@ -18,6 +18,7 @@
 #include <utility>
 
 #include "fft.cuh"
+#include "per_device.cuh"
 
 namespace pyfof {
 
@@ -708,12 +709,13 @@ int32_t allow_smem(K kernel, size_t bytes) {
   return kOk;
 }
 
-// Shared-memory limits of every kernel of grid N, set once per process.
+// Shared-memory limits of every kernel of grid N, set once per device.
 template <typename R, int N>
 int32_t prepare() {
-  static std::once_flag once;
-  static int32_t status = kOk;
-  std::call_once(once, [] {
+  static PerDeviceOnce once;
+  int dev = 0;
+  PYFOF_CUDA(cudaGetDevice(&dev));
+  return once.run(dev, [] {
     const size_t sm = smem_lines_bytes<R, N>();
     int32_t r = kOk;
     if (r == kOk) r = allow_smem(k_x_r2c<R, N>, sm);
@@ -724,9 +726,8 @@ int32_t prepare() {
     if (r == kOk) r = allow_smem(k_lines<R, N, kYInverseAll>, sm);
     if (r == kOk) r = allow_smem(k_lines<R, N, kZInverse>, sm);
     if (r == kOk) r = allow_smem(k_lines<R, N, kZConv>, smem_conv_bytes<R, N>(conv_in_max(N)));
-    status = r;
+    return r;
   });
-  return status;
 }
 
 template <typename R, int N>

@@ -546,7 +546,8 @@ static int32_t run_host(Context &ctx, const double *xp, const double *vp, const 
   int seg_x = -1, seg_m = -1, seg_v = -1;
   {
     const size_t total = sizeof(double) * n * (3 + (vp ? 3 : 0) + (mp ? 1 : 0));
-    if (total >= StagedCopy::kMinBytes && StagedCopy::pageable(xp)) {
+    if (total >= StagedCopy::kMinBytes && StagedCopy::pageable(xp) && (!vp || StagedCopy::readable(vp)) &&
+        (!mp || StagedCopy::readable(mp))) {
       seg_x = copies.add(xd, xp, sizeof(double) * 3 * n, s);
       if (mp) seg_m = copies.add(md, mp, sizeof(double) * n, ctx.aux_stream);
       if (vp) seg_v = copies.add(vd, vp, sizeof(double) * 3 * n, ctx.aux_stream);

@@ -70,6 +70,17 @@ class StagedCopy {
     return at.type == cudaMemoryTypeUnregistered;
   }
 
+  // Whether the worker threads can read `src`: not device memory, which the
+  // runtime's own copy takes like any other.
+  static bool readable(const void *src) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, src) != cudaSuccess) {
+      cudaGetLastError();
+      return true;
+    }
+    return at.type != cudaMemoryTypeDevice;
+  }
+
   ~StagedCopy() { join(); }
 
   // Appends a segment; its copies are issued on stream s.  Returns its index.

@@ -321,7 +321,8 @@ __global__ void __launch_bounds__(BLK) fof_place_kernel(const float4 *__restrict
 }
 
 // Whether the two-step scatter pays: one region, most sampled warps hold
-// particles far apart, and the output (20 B a particle) does not fit half of L2.
+// particles far apart, and the output (16 B a particle) is above 64 MB, half
+// of L2.
 static bool use_partition(int nreg, int64_t n_active, int64_t ntiles, int32_t spread) {
   return nreg == 1 && 16.0 * (double)n_active > 64e6 && (int64_t)spread * 2 >= ntiles * (BLK / 32);
 }

@@ -124,12 +124,12 @@ def _tile_table_note():
 
 
 def _traffic(workload, kernel):
-    """DRAM bytes per algorithmic byte of `kernel`, from a committed ncu
-    summary (profiles/roofline_traffic.json), or None."""
+    """DRAM bytes per algorithmic byte of `kernel` over one call of `workload`,
+    from a committed ncu summary (profiles/roofline_traffic.json), or None."""
     tp = os.path.join(ROOT, "profiles", "roofline_traffic.json")
     if not os.path.exists(tp):
         return None
-    d = json.load(open(tp)).get(kernel)
+    d = json.load(open(tp)).get(workload, {}).get(kernel)
     if not d:
         return None
     return float(d["dram_bytes_per_algorithmic_byte"])

@@ -58,11 +58,12 @@ int32_t pyfof_last_error(char *buf, int64_t len);
  * differently), "unbind_per_halo" (1 = the plain FP64 baseline: one halo per
  * launch sequence), "timing" (1 = record stage times), "unbind_big_np"
  * (particle-mesh halos above this many members run their removal loop
- * spread over the whole GPU; 0 = the default of 32768), "cell_order" (how
- * the particles are put in cell order: 0 = per-cell sorts when cell keys
- * need more than 24 bits and no cell holds more than 8192 particles, else a
- * radix sort; 1 = per-cell sorts whenever no cell holds more than 8192; 2 =
- * always the radix sort; all give the same order). */
+ * spread over the whole GPU; 0 = the default of 32768), "cell_order" (the
+ * order of the particles inside a cell of the linking: 0 = arbitrary, each
+ * particle in its cell's next free slot, nothing is sorted; 1 = the
+ * reference's, ascending index, by a sort of every cell if none holds more
+ * than 8192 particles, else by a radix sort; 2 = the reference's, by the
+ * radix sort; the results are the same). */
 int32_t pyfof_set_option(const char *key, int64_t value);
 
 /* Current value of a pyfof_set_option key.  No reference counterpart. */
@@ -102,7 +103,8 @@ int32_t pyfof_host_free(void *ptr);
  * least np_halo_min members), "dense_cells" (cells given a sub-cell index),
  * "max_cell" (particles in the fullest cell), "vd_cells" (very dense cells,
  * linked by merge sub-cells narrower than link/sqrt(3)), "cell_sorts" (1 when the
- * cell order came from per-cell sorts, 0 from the radix sort),
+ * cells were sorted one by one, 0 when the radix sort or, cell_order 0, no
+ * sort ran),
  * "direct_halos" / "pm_halos" (candidates unbound by direct summation / the
  * particle mesh), "valid_halos" (halos written to the output),
  * "refined_regions" (two-level inner regions), "pm_passes" (passes of the

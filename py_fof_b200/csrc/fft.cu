@@ -7,7 +7,7 @@
 //   stage A  thread (line, s):  Y[s][k1] = sum_q x[s + N2 q] W_N1^(q k1),
 //            times the twiddle W_N^(s k1), written to shared memory;
 //   stage B  thread (line, k1): X[k1 + N1 k2] = sum_s Y[s][k1] W_N2^(s k2).
-// The register DFTs are mixed-radix (4, 2, 3) decompositions unrolled at
+// The register DFTs are mixed-radix (4, 2, 3, 5) decompositions unrolled at
 // compile time with constant twiddles.  A block works on a tile of W lines
 // that are adjacent in memory (consecutive kx), so every global access of a
 // warp covers whole 128-byte segments.  The z pass does forward transform,
@@ -289,8 +289,9 @@ constexpr size_t smem_conv_bytes(int rows) {
 }
 
 // Blocks per SM the registers of a line kernel are limited for.  The FP64 z
-// pass is bound by FP64 issue and the latency between dependent operations,
-// so a few more warps help until the registers spill (256: 2.97 ms a call of
+// pass is bound by the latency between dependent operations (FP64 units 48 to
+// 56 % busy, issue 44 to 46 %, three warps per scheduler), so a few more warps
+// help until the registers spill (256: 2.97 ms a call of
 // the 256^3 box at 3 blocks, 3.28 at 4; 216: 6.7 -> 4.5 ms of the NFW list at
 // 3 instead of 2).  The y passes go without a staging buffer: with one their
 // registers left 2 blocks per SM and they ran a quarter slower.

@@ -177,6 +177,9 @@ inline unsigned table_grid(int64_t n) { return (unsigned)std::min<int64_t>(ceil_
 // its shorter transform lengths.  The kernel is even along every axis, so its
 // forward transform is the inverse one that c2r_full runs.  Once per process
 // and grid size: about a millisecond for 256 points, all lengths together.
+// Where the device has no room for a table (186 MB for the 256-point kernel,
+// 166 MB more while they are made), it and the rest are left out, and their
+// halos run at n points.
 int32_t shorter_tables(GreenTable &t, const double *grid, double2 *spec, ConvBox *dbox, cudaStream_t s) {
   double *h = nullptr, *out = nullptr;
   int32_t r = kOk;
@@ -185,8 +188,11 @@ int32_t shorter_tables(GreenTable &t, const double *grid, double2 *spec, ConvBox
     auto q = std::make_shared<GreenTable>();
     q->n = m;
     q->fp64 = q->scaled = true;
-    PYFOF_CUDA(cudaMalloc(&q->g, sizeof(double) * cnt));
-    PYFOF_CUDA(cudaMalloc(&q->tw, sizeof(double2) * m));
+    if (cudaMalloc(&q->g, sizeof(double) * cnt) != cudaSuccess ||
+        cudaMalloc(&q->tw, sizeof(double2) * m) != cudaSuccess) {
+      cudaGetLastError();
+      return kAlloc;
+    }
     PYFOF_TRY(fill_twiddles<double>((double2 *)q->tw, m, s));
     ConvBox box{};
     for (int d = 0; d < 3; ++d) box.in[d] = box.out[d] = m;
@@ -206,13 +212,12 @@ int32_t shorter_tables(GreenTable &t, const double *grid, double2 *spec, ConvBox
   if (cudaMallocAsync(&h, sizeof(double) * (top / 2 + 1) * top * top, s) != cudaSuccess ||
       cudaMallocAsync(&out, sizeof(double) * top * top * top, s) != cudaSuccess) {
     cudaGetLastError();
-    set_error("device allocation failed (kernel tables)");
     r = kAlloc;
   }
   for (; r == kOk && *l < t.n; ++l) r = one(*l);
   if (h) cudaFreeAsync(h, s);
   if (out) cudaFreeAsync(out, s);
-  return r;
+  return r == kAlloc ? kOk : r;
 }
 
 // Green table of grid n for (soft, range, truncated), cached per device.  Its
@@ -2695,11 +2700,12 @@ int32_t run_pm(Context &ctx, const FofArgs &a, const GridRules &rules, const Mem
   std::vector<Grid> hgrid, rgrid;
   for (int h = 0; h < nh; ++h) {
     const ConvBox b = halo_box(h);
-    hgrid.push_back(Grid{b, h, H[h].n, conv_length(H[h].n, sizeof(R) == 8, b)});
+    hgrid.push_back(Grid{b, h, H[h].n, green_of[H[h].n]->at(conv_length(H[h].n, sizeof(R) == 8, b))->n});
   }
   for (int ia = 0; ia < na; ++ia) {
     const ConvBox b = region_box(ia);
-    rgrid.push_back(Grid{b, ia, act[ia].n_in, conv_length(act[ia].n_in, sizeof(R) == 8, b)});
+    const int n = act[ia].n_in;
+    rgrid.push_back(Grid{b, ia, n, (n == 128 ? g_r2 : g_r4)->at(conv_length(n, sizeof(R) == 8, b))->n});
   }
   order(hgrid);
   order(rgrid);

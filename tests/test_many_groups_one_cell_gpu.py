@@ -67,6 +67,16 @@ def test_runs_above_and_below_the_line_in_one_call():
         assert np.array_equal(part, np.arange(part[0], part[0] + part.size))
 
 
+@pytest.mark.parametrize("order", [0, 1, 2])
+def test_two_regions_and_cell_orders(order):
+    """A list of two knots: the second's ids follow the first's, whatever the
+    order inside the cells."""
+    xs = [_knot(18, 5), _knot(11, 6)]
+    with _native.options(cell_order=order):
+        ids = P._fof_core(xs, np_halo_min=1, **KW)[1]
+    assert np.array_equal(ids, np.arange(1, ids.size + 1))
+
+
 def test_time_is_linear():
     ms = {}
     with _native.options(timing=1):
